@@ -97,7 +97,7 @@ def reference_root():
 def build_oracle(ref=None):
     _run(["make", "-s", "-C", os.path.join(ROOT, "oracle")])
     ref = ref or reference_root()
-    if os.path.isdir(ref):
+    if os.path.isdir(os.path.join(ref, "src")):  # an empty mount point counts as absent
         _run(["make", "-s", "-j8", "-C", os.path.join(ROOT, "oracle", "refbuild"), "REF=" + ref])
 
 
