@@ -5,11 +5,11 @@
 // v + j n, runs the iterated-sparse-sampling CC on the union and stops at the first level with
 // more than `copies` components; the answer is 2^level.
 //
-// Here each level does the keep test of every (copy, edge) pair and hooks kept edges straight
-// into one union-find over n * copies vertices, in slices with the forest flattened between the
-// first ones (the CC of the disjoint union is the
-// union-find of all kept edges; the CC path's sampling round has nothing to skip at these
-// densities), then the roots are counted. The keep test is integer-only and counter-addressed:
+// Here each level hooks the kept edges of every copy into one union-find over n * copies vertices
+// (the CC of the disjoint union is the union-find of all kept edges), then the roots are counted. On
+// larger graphs a sample of the edges comes first: it leaves one giant component per copy, and of the
+// other edges only those with an end outside the giant of some copy are tested and hooked at all
+// (run_level). The keep test is integer-only and counter-addressed:
 // P(Binomial(w, q) > 0) = 1 - (1 - q)^w, so the pair is kept iff the u64 draw x >= F(i, w) with
 // F = (1 - 2^-i)^w in 0.64 fixed point by square-and-multiply over truncating 64x64->128-bit
 // products; x is draw e_local of stream (seed + r, i, j, 1), r the virtual rank whose slice
@@ -35,6 +35,7 @@
 // Graphs with other weights draw a variable number of outputs per edge (a sequential chain per
 // rank), so the replay takes unit weights only.
 #include "cac_internal.h"
+#include "pdl.cuh"
 #include "sitmo.cuh"
 
 #include <algorithm>
@@ -45,9 +46,13 @@ namespace cac {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr uint32_t kSlices = 8;            // hook slices per level on large graphs
-constexpr uint32_t kCompressedSlices = 3;  // slices followed by a full compression
-
+// Graphs with fewer edges hook every edge in one pass: there a level is a few launches either way.
+constexpr uint64_t kSampledEdges = 1u << 15;
+constexpr uint32_t kSampleParts = 128;        // a sampling round takes 128ths of the edges
+constexpr double kRoundDegree[] = {0.8, 0.8, 0.8, 0.8, 1.6};  // kept edges per vertex in each round
+constexpr uint32_t kGiantSample = 1024;       // vertices looked at to find a copy's giant component
+constexpr int kStreamThreads = 1024;          // CTA of the pass over the other edges (the bitmap fills shared memory)
+constexpr uint32_t kSmemWords = 48 * 1024;    // bitmap words in shared memory (1.57 M vertices)
 __device__ __forceinline__ uint64_t keep_threshold(uint32_t level, uint32_t w) {
     const uint64_t base = 0ull - (1ull << (64 - level));
     uint64_t res = base, b = base;
@@ -60,12 +65,21 @@ __device__ __forceinline__ uint64_t keep_threshold(uint32_t level, uint32_t w) {
     return res;
 }
 
-__device__ __forceinline__ uint32_t afind(uint32_t *par, uint32_t v) {
-    uint32_t cur = par[v];
+// The forest of all copies: parent of vertex x in copy j at x * copies + j, so that what one edge needs
+// of all copies lies side by side (4 copies: one 16-byte access per end). Parents are vertices of the
+// same copy, never larger than the child; roots are their own parents.
+struct Forest {
+    uint32_t *par;
+    uint32_t copies;
+    __device__ __forceinline__ uint32_t &at(uint32_t x, uint32_t j) const { return par[x * copies + j]; }
+};
+
+__device__ __forceinline__ uint32_t afind(const Forest &F, uint32_t j, uint32_t v) {  // with path halving
+    uint32_t cur = F.at(v, j);
     if (cur != v) {
         uint32_t prev = v, next;
-        while (cur > (next = par[cur])) {
-            par[prev] = next;
+        while (cur > (next = F.at(cur, j))) {
+            F.at(prev, j) = next;
             prev = cur;
             cur = next;
         }
@@ -73,31 +87,45 @@ __device__ __forceinline__ uint32_t afind(uint32_t *par, uint32_t v) {
     return cur;
 }
 
-__device__ __forceinline__ void aunite(uint32_t *par, uint32_t a, uint32_t b) {
-    uint32_t ra = afind(par, a), rb = afind(par, b);
+__device__ __forceinline__ void aunite(const Forest &F, uint32_t j, uint32_t a, uint32_t b) {
+    uint32_t ra = afind(F, j, a), rb = afind(F, j, b);
     while (ra != rb) {
         if (ra < rb) {
-            const uint32_t old = atomicCAS(&par[rb], rb, ra);
+            const uint32_t old = atomicCAS(&F.at(rb, j), rb, ra);
             if (old == rb) return;
             rb = old;
         } else {
-            const uint32_t old = atomicCAS(&par[ra], ra, rb);
+            const uint32_t old = atomicCAS(&F.at(ra, j), ra, rb);
             if (old == ra) return;
             ra = old;
         }
     }
 }
 
-__global__ void approx_init(uint32_t *par, uint64_t nv) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (uint64_t)gridDim.x * blockDim.x)
-        par[i] = (uint32_t)i;
+__device__ __forceinline__ uint32_t root_of(const Forest &F, uint32_t j, uint32_t cur) {  // without writes
+    uint32_t next;
+    while ((next = F.at(cur, j)) != cur) cur = next;
+    return cur;
+}
+
+// Singletons, one thread per vertex, and the root count at 0.
+__global__ void approx_init(const Forest F, uint32_t n, unsigned int *count) {
+    pdl_wait();
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (tid == 0) *count = 0;
+    for (uint32_t x = tid; x < n; x += stride) {
+        if (F.copies == 4) reinterpret_cast<uint4 *>(F.par)[x] = make_uint4(x, x, x, x);
+        else
+            for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = x;
+    }
 }
 
 // One thread per (copy, edge), one sitmo block per draw: small graphs, where the pass is one
 // latency chain per thread and more threads finish sooner. Copies along blockIdx.y.
-__global__ void approx_keep_hook(uint32_t *par, const uint32_t *__restrict__ U, const uint32_t *__restrict__ V,
-                                 const uint32_t *__restrict__ Wt, uint64_t m, uint32_t n, uint32_t level,
-                                 uint32_t seed, uint32_t ranks, uint64_t portion) {
+__global__ void approx_keep_hook(const Forest F, const uint32_t *__restrict__ U, const uint32_t *__restrict__ V,
+                                 const uint32_t *__restrict__ Wt, uint64_t m, uint32_t level, uint32_t seed,
+                                 uint32_t ranks, uint64_t portion) {
+    pdl_wait();
     const uint32_t j = blockIdx.y;
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t w = Wt[e];
@@ -107,46 +135,39 @@ __global__ void approx_keep_hook(uint32_t *par, const uint32_t *__restrict__ U, 
         const uint64_t local = e - (uint64_t)r * portion;
         const uint64_t x = draw64(seed + r, level, j, 1, 0, local);
         if (x < keep_threshold(level, w)) continue;
-        const uint32_t off = j * n;
-        aunite(par, U[e] + off, V[e] + off);
+        aunite(F, j, U[e], V[e]);
     }
 }
 
-// Large graphs: one thread per (copy, quad): a quad is 4 consecutive edges of one rank's slice, local indices
-// 4 lq .. 4 lq + 3, whose 4 draws are the 4 words of one sitmo block (counter lq). Rank r < P - 1
-// owns Qf = ceil(portion / 4) quads, the last rank the rest of the edges (all of them when
-// portion is 0). Quads [q0, q1) of the flattened list; copies along blockIdx.y.
-__global__ void approx_keep_hook4(uint32_t *par, const uint32_t *__restrict__ U, const uint32_t *__restrict__ V,
-                                  const uint32_t *__restrict__ Wt, uint64_t m, uint32_t n, uint32_t level,
-                                  uint32_t seed, uint32_t ranks, uint64_t portion, uint64_t Qf, uint64_t q0,
-                                  uint64_t q1) {
-    const uint32_t j = blockIdx.y;
-    const uint32_t off = j * n;
-    for (uint64_t gq = q0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gq < q1;
-         gq += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t r;
-        uint64_t lq;
-        if (portion == 0) {
-            r = ranks - 1;
-            lq = gq;
-        } else {
-            const uint64_t rr = gq / Qf;
-            r = rr < ranks - 1 ? (uint32_t)rr : ranks - 1;
-            lq = gq - (uint64_t)r * Qf;
-        }
-        const uint64_t base = (uint64_t)r * portion;                   // first edge of the slice
-        const uint64_t len = r + 1 < ranks ? portion : m - base;       // edges of the slice
-        const u64x4 o = sitmo_block(seed + r, level, j, 1, lq, 0, 0, 0);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint64_t local = 4 * lq + k;
-            if (local >= len) break;
-            const uint64_t e = base + local;
-            const uint32_t w = Wt[e];
-            if (w == 0 || o.x[k] < keep_threshold(level, w)) continue;
-            aunite(par, U[e] + off, V[e] + off);
-        }
-    }
+// Larger graphs take the draws by quads: a quad is 4 consecutive edges of one rank's slice, local
+// indices 4 lq .. 4 lq + 3, whose 4 draws are the 4 words of one sitmo block (counter lq). Rank
+// r < P - 1 owns Qf = ceil(portion / 4) quads, the last rank the rest of the edges (all of them when
+// portion is 0).
+struct Level {
+    const uint32_t *U, *V, *Wt;
+    uint32_t m, n, level, seed, ranks, portion, Qf, Q;
+    uint64_t keep_max;     // seed replay: stream_threshold(level)
+    uint32_t from, to;     // the quads of a sampling round: groups g of 64 with from <= g % kSampleParts < to
+    Forest F;
+    uint32_t *giants;      // copies: the root of each copy's giant component
+    uint32_t *member;      // n: bit j: in the giant of copy j
+    uint32_t *bits;        // n bits: in the giant of every copy
+    uint2 *list;           // (edge, copies it has to be tested in), the first `cap` survivors
+    uint32_t cap;
+    uint32_t *count;       // survivors
+};
+
+struct Quad {
+    uint32_t r, lq, base, len;  // its rank, its index there, the rank's first edge and edge count
+};
+__device__ __forceinline__ Quad quad_of(const Level &L, uint32_t gq) {
+    Quad q;
+    q.r = L.ranks - 1;
+    if (L.portion) q.r = min(gq / L.Qf, L.ranks - 1);
+    q.lq = gq - q.r * L.Qf;
+    q.base = q.r * L.portion;
+    q.len = q.r + 1 < L.ranks ? L.portion : L.m - q.base;
+    return q;
 }
 
 // Binomial(1, p) > 0 on the reference's draws: U = generate_canonical<double, 53> of outputs x0, x1
@@ -172,37 +193,26 @@ __device__ __forceinline__ bool stream_keep(uint64_t S, uint64_t T) {  // S = x0
     return (qr << sh) <= T;
 }
 
-// Seed replay, unit weights: one thread per (copy, quad of 4 slice edges), quads numbered as in
-// approx_keep_hook4. The quad's 4 draws read the 8 consecutive outputs k0 .. k0 + 7 of the rank's
-// engine (output k = half k & 1 of word k >> 1, low half first: lib/prng_engine.hpp:195-212;
+// Seed replay, unit weights: the quad's 4 draws read the 8 consecutive outputs k0 .. k0 + 7 of the
+// rank's engine (output k = half k & 1 of word k >> 1, low half first: lib/prng_engine.hpp:195-212;
 // words 4b .. 4b + 3 form sitmo block b). Draw d's two outputs give S = x0 + x1 2^32, which is
 // word (k0 >> 1) + d itself when k0 is even and the high half of that word joined to the low half
 // of the next when k0 is odd; the words lie in the blocks k0 >> 3 and the one after it.
-__global__ void approx_stream_keep_hook(uint32_t *par, const uint32_t *__restrict__ U, const uint32_t *__restrict__ V,
-                                        uint64_t m, uint32_t n, uint32_t level, uint64_t keep_max, uint32_t copies,
-                                        uint32_t seed, uint32_t ranks, uint64_t portion, uint64_t Qf, uint64_t q0,
-                                        uint64_t q1) {
-    const uint32_t j = blockIdx.y;
-    const uint32_t off = j * n;
-    for (uint64_t gq = q0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gq < q1;
-         gq += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t r;
-        uint64_t lq;
-        if (portion == 0) {
-            r = ranks - 1;
-            lq = gq;
-        } else {
-            const uint64_t rr = gq / Qf;
-            r = rr < ranks - 1 ? (uint32_t)rr : ranks - 1;
-            lq = gq - (uint64_t)r * Qf;
-        }
-        const uint64_t base = (uint64_t)r * portion;
-        const uint64_t len = r + 1 < ranks ? portion : m - base;
-        const uint64_t k0 = (uint64_t)(level - 1) * (2 * (uint64_t)copies * len + 1) + 2 * ((uint64_t)j * len + 4 * lq);
+__device__ __forceinline__ uint64_t stream_output(const Level &L, uint32_t j, uint32_t len, uint32_t local) {
+    return (uint64_t)(L.level - 1) * (2 * (uint64_t)L.F.copies * len + 1) + 2 * ((uint64_t)j * len + local);
+}
+
+// The kept edges of quad q in copy j, bit d for its edge d (edges past the slice's end: 0).
+template <bool kRef>
+__device__ __forceinline__ uint32_t quad_keeps(const Level &L, const Quad &q, uint32_t j) {
+    const uint32_t here = min(4u, q.len - 4 * q.lq);
+    uint32_t mask = 0;
+    if constexpr (kRef) {
+        const uint64_t k0 = stream_output(L, j, q.len, 4 * q.lq);
         const uint64_t b0 = k0 >> 3;
         const unsigned a = (unsigned)(k0 >> 1) & 3u;  // first word inside block b0
         const bool odd = k0 & 1;
-        const uint32_t key = seed + r;
+        const uint32_t key = L.seed + q.r;
         const u64x4 A = sitmo_block(key, 0, 0, 0, b0, 0, 0, 0);
         u64x4 B = A;
         if (a != 0 || odd) B = sitmo_block(key, 0, 0, 0, b0 + 1, 0, 0, 0);
@@ -219,12 +229,189 @@ __global__ void approx_stream_keep_hook(uint32_t *par, const uint32_t *__restric
         }
 #undef CAC_QUAD_DRAWS
 #pragma unroll
-        for (int d = 0; d < 4; d++) {
-            const uint64_t local = 4 * lq + d;
-            if (local >= len) break;
-            if (!stream_keep(S[d], keep_max)) continue;
-            aunite(par, U[base + local] + off, V[base + local] + off);
+        for (int d = 0; d < 4; d++) mask |= (uint32_t)stream_keep(S[d], L.keep_max) << d;
+    } else {
+        const u64x4 o = sitmo_block(L.seed + q.r, L.level, j, 1, q.lq, 0, 0, 0);
+#pragma unroll
+        for (uint32_t d = 0; d < 4; d++) {
+            const uint32_t w = d < here ? L.Wt[q.base + 4 * q.lq + d] : 0;
+            mask |= (uint32_t)(w != 0 && o.x[d] >= keep_threshold(L.level, w)) << d;
         }
+    }
+    return mask & ((1u << here) - 1);
+}
+
+// Whether edge e is kept in copy j, on its own.
+template <bool kRef>
+__device__ __forceinline__ bool edge_kept(const Level &L, uint32_t e, uint32_t j) {
+    const uint32_t r = L.portion ? min(e / L.portion, L.ranks - 1) : L.ranks - 1;
+    const uint32_t base = r * L.portion, local = e - base;
+    if constexpr (kRef) {
+        const uint64_t k0 = stream_output(L, j, r + 1 < L.ranks ? L.portion : L.m - base, local);
+        const uint64_t w0 = draw64(L.seed + r, 0, 0, 0, 0, k0 >> 1);
+        if (!(k0 & 1)) return stream_keep(w0, L.keep_max);
+        return stream_keep((w0 >> 32) | (draw64(L.seed + r, 0, 0, 0, 0, (k0 >> 1) + 1) << 32), L.keep_max);
+    } else {
+        const uint32_t w = L.Wt[e];
+        return w != 0 && draw64(L.seed + r, L.level, j, 1, 0, local) >= keep_threshold(L.level, w);
+    }
+}
+
+// Hooks the kept edges of some quads, a thread per quad and copy, the copies of a quad in neighbouring
+// lanes (what an end needs of 4 copies is one 16-byte access).
+//   kRound  a sampling round: the forest is flat, and every kept edge between two roots makes the smaller
+//           one the parent of the larger, the smallest of all winning (an atomic without a return value:
+//           no walk, no retry; a link that loses is found again by the pass over all edges). Late
+//           rounds have few large trees, whose roots would take thousands of such writes each: a table
+//           of the CTA's writes (lossy; root -> smallest parent given) stops those that change nothing.
+//   kAll    every quad, by union walks
+enum QuadPass { kRound, kAll };
+constexpr uint32_t kGiven = 1024;
+template <bool kRef, QuadPass kPass>
+__global__ void __launch_bounds__(kThreads) approx_quads(const Level L) {
+    pdl_wait();
+    __shared__ unsigned long long given[kPass == kRound ? kGiven : 1];
+    if (kPass == kRound) {
+        for (uint32_t i = threadIdx.x; i < kGiven; i += kThreads) given[i] = ~0ull;
+        __syncthreads();
+    }
+    const uint32_t C = L.F.copies, lane = threadIdx.x & 31, side = min(C, 32u), per = 32 / side;  // quads per warp
+    if (lane >= side * per) return;
+    // the pass's quads, numbered: all, or those of the round
+    const uint32_t w = L.to - L.from, groups = (L.Q + 63) / 64, last = groups % kSampleParts;
+    const uint64_t count = kPass == kAll ? L.Q
+                                         : (uint64_t)64 * (groups / kSampleParts * w + (last > L.from ? min(last, L.to) - L.from : 0));
+    const uint32_t warps = (gridDim.x * kThreads) >> 5;
+    for (uint64_t i = (uint64_t)((blockIdx.x * kThreads + threadIdx.x) >> 5) * per + lane / side; i < count;
+         i += (uint64_t)warps * per) {
+        uint32_t gq = (uint32_t)i;
+        if (kPass == kRound) {
+            const uint32_t g = (uint32_t)(i >> 6);
+            gq = (g / w * kSampleParts + L.from + g % w) * 64 + ((uint32_t)i & 63u);
+            if (gq >= L.Q) continue;
+        }
+        const Quad q = quad_of(L, gq);
+        const uint32_t e0 = q.base + 4 * q.lq;
+        for (uint32_t j = lane % side; j < C; j += side) {
+            const uint32_t mask = quad_keeps<kRef>(L, q, j);
+            uint32_t a[4], b[4];
+#pragma unroll
+            for (uint32_t d = 0; d < 4; d++) {
+                a[d] = b[d] = 0;
+                if ((mask >> d) & 1u) {
+                    a[d] = __ldg(L.U + e0 + d);
+                    b[d] = __ldg(L.V + e0 + d);
+                }
+            }
+#pragma unroll
+            for (uint32_t d = 0; d < 4; d++)
+                if ((mask >> d) & 1u) {
+                    a[d] = L.F.at(a[d], j);
+                    b[d] = L.F.at(b[d], j);
+                }
+#pragma unroll
+            for (uint32_t d = 0; d < 4; d++) {
+                if (a[d] == b[d]) continue;
+                if (kPass == kAll) {
+                    aunite(L.F, j, a[d], b[d]);
+                } else {
+                    const uint32_t hi = max(a[d], b[d]) * C + j, lo = min(a[d], b[d]);
+                    volatile unsigned long long *t = &given[hi * 2654435761u >> 22];
+                    const unsigned long long had = *t;
+                    if ((uint32_t)(had >> 32) == hi && (uint32_t)had <= lo) continue;
+                    atomicMin(&L.F.par[hi], lo);
+                    *t = (unsigned long long)hi << 32 | lo;
+                }
+            }
+        }
+    }
+}
+
+// Tests edge e in the copies of `need` and hooks it there.
+template <bool kRef>
+__device__ __forceinline__ void keep_hook(const Level &L, uint32_t e, uint32_t a, uint32_t b, uint32_t j) {
+    if (edge_kept<kRef>(L, e, j)) aunite(L.F, j, a, b);
+}
+
+// All edges after the sampling rounds, a warp per 256-edge tile as in the filter of the
+// connected-components path: an edge with both ends in the giant of every copy is dropped unseen
+// (whatever its draws say, it joins nothing); of the others, the copies in which an end is outside the
+// giant are noted in the survivor list. Survivors past the end of the list are tested and hooked on the
+// spot. kShared: the bitmap fits shared memory.
+template <bool kRef, bool kShared>
+__global__ void __launch_bounds__(kStreamThreads) approx_stream(const Level L) {
+    pdl_wait();
+    extern __shared__ uint32_t sbits[];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    if (kShared) {
+        for (uint32_t i = threadIdx.x; i < (L.n + 31) / 32; i += blockDim.x) sbits[i] = L.bits[i];
+        __syncthreads();
+    }
+    const uint32_t *bits = kShared ? sbits : L.bits;
+    auto inside = [&](uint32_t x) { return (bits[x >> 5] >> (x & 31)) & 1u; };
+    const uint32_t tiles = (uint32_t)(((uint64_t)L.m + 255) / 256);
+    const uint32_t all = L.F.copies >= 32 ? 0xFFFFFFFFu : (1u << L.F.copies) - 1;
+    for (uint32_t i = blockIdx.x * nwarps + warp; i < tiles; i += gridDim.x * nwarps) {
+        const uint32_t e0 = i * 256;
+        uint32_t a[8], b[8], e[8], keep = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t x = e0 + 128 * h + 4 * lane;
+            uint4 ua = make_uint4(0, 0, 0, 0), va = ua;
+            if (x + 3 < L.m) {
+                ua = __ldcs(reinterpret_cast<const uint4 *>(L.U + x));
+                va = __ldcs(reinterpret_cast<const uint4 *>(L.V + x));
+            } else {
+                if (x < L.m) ua.x = L.U[x], va.x = L.V[x];
+                if (x + 1 < L.m) ua.y = L.U[x + 1], va.y = L.V[x + 1];
+                if (x + 2 < L.m) ua.z = L.U[x + 2], va.z = L.V[x + 2];
+            }
+            a[4 * h] = ua.x, a[4 * h + 1] = ua.y, a[4 * h + 2] = ua.z, a[4 * h + 3] = ua.w;
+            b[4 * h] = va.x, b[4 * h + 1] = va.y, b[4 * h + 2] = va.z, b[4 * h + 3] = va.w;
+#pragma unroll
+            for (int d = 0; d < 4; d++) e[4 * h + d] = x + d;
+        }
+#pragma unroll
+        for (int d = 0; d < 8; d++) {  // (an edge past the end is 0-0: a loop)
+            keep |= (uint32_t)(a[d] != b[d] && !(inside(a[d]) && inside(b[d]))) << d;
+        }
+        if (!__any_sync(0xffffffffu, keep)) continue;
+        uint32_t need[8];
+#pragma unroll
+        for (int d = 0; d < 8; d++) need[d] = (keep >> d) & 1u ? all & ~(L.member[a[d]] & L.member[b[d]]) : 0;
+        const uint32_t mine = __popc(keep);
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        uint32_t at = 0;
+        if (lane == 31) at = atomicAdd(L.count, incl);
+        at = __shfl_sync(0xffffffffu, at, 31) + incl - mine;
+#pragma unroll
+        for (int d = 0; d < 8; d++) {
+            if (!((keep >> d) & 1u)) continue;
+            if (at < L.cap) {
+                L.list[at] = make_uint2(e[d], need[d]);
+            } else {
+                for (uint32_t j = 0; j < L.F.copies; j++)
+                    if ((need[d] >> j) & 1u) keep_hook<kRef>(L, e[d], a[d], b[d], j);
+            }
+            at++;
+        }
+    }
+}
+
+// One thread per (survivor, copy).
+template <bool kRef>
+__global__ void __launch_bounds__(kThreads) approx_survivors(const Level L) {
+    pdl_wait();
+    const uint64_t items = (uint64_t)min(*L.count, L.cap) * L.F.copies;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < items; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t at = (uint32_t)(i / L.F.copies), j = (uint32_t)(i - (uint64_t)at * L.F.copies);
+        const uint2 x = L.list[at];
+        if ((x.y >> j) & 1u) keep_hook<kRef>(L, x.x, L.U[x.x], L.V[x.x], j);
     }
 }
 
@@ -244,22 +431,149 @@ __global__ void approx_slice_sums(const uint32_t *__restrict__ w, uint64_t m, ui
     }
 }
 
-// Full path compression (read-only walks; only roots are written).
-__global__ void approx_compress(uint32_t *par, uint64_t nv) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t cur = par[i], next;
-        if (cur == (uint32_t)i) continue;
-        while ((next = par[cur]) != cur) cur = next;
-        par[i] = cur;
+// Full path compression (read-only walks; only roots are written), a thread per vertex and 4 copies:
+// their parents in one load, the 4 grandparents requested together, then the longer chains.
+__global__ void approx_compress(const Forest F, uint32_t n) {
+    pdl_wait();
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (F.copies == 4) {
+        uint4 *p4 = reinterpret_cast<uint4 *>(F.par);
+        for (uint32_t x = tid; x < n; x += stride) {
+            const uint4 p = p4[x];
+            const uint32_t g0 = F.par[4 * p.x], g1 = F.par[4 * p.y + 1], g2 = F.par[4 * p.z + 2], g3 = F.par[4 * p.w + 3];
+            const uint32_t r0 = g0 == p.x ? g0 : root_of(F, 0, g0), r1 = g1 == p.y ? g1 : root_of(F, 1, g1);
+            const uint32_t r2 = g2 == p.z ? g2 : root_of(F, 2, g2), r3 = g3 == p.w ? g3 : root_of(F, 3, g3);
+            if (r0 != p.x || r1 != p.y || r2 != p.z || r3 != p.w) p4[x] = make_uint4(r0, r1, r2, r3);
+        }
+    } else {
+        for (uint32_t x = tid; x < n; x += stride)
+            for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = root_of(F, j, x);
     }
 }
 
-__global__ void approx_count_roots(const uint32_t *par, uint64_t nv, unsigned int *count) {
+// The giant component of each copy (one CTA per copy): the most frequent root among kGiantSample
+// vertices spread over the copy (the mode of each warp's 32, counted over all; ties to the smaller
+// root). The choice decides which edges are dropped unseen, never the partition.
+__global__ void __launch_bounds__(kGiantSample) approx_giants(const Level L) {
+    pdl_wait();
+    __shared__ uint32_t cand[kGiantSample / 32], cnt[kGiantSample / 32];
+    __shared__ unsigned long long best;
+    const uint32_t i = threadIdx.x, lane = i & 31, w = i >> 5;
+    const uint32_t r = root_of(L.F, blockIdx.x, (uint32_t)(((uint64_t)i * 2654435761u) % L.n));
+    const uint32_t same = __match_any_sync(0xffffffffu, r);
+    const uint32_t c = __popc(same);
+    const uint32_t top = __reduce_max_sync(0xffffffffu, c);
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, c == top ? r : 0xFFFFFFFFu);
+    if (lane == 0) {
+        cand[w] = lo;
+        cnt[w] = 0;
+    }
+    if (i == 0) best = 0;
+    __syncthreads();
+    for (uint32_t k = 0; k < kGiantSample / 32; k++)
+        if (r == cand[k]) atomicAdd(&cnt[k], 1u);
+    __syncthreads();
+    if (i < kGiantSample / 32) atomicMax(&best, ((unsigned long long)cnt[i] << 32) | (0xFFFFFFFFu - cand[i]));
+    __syncthreads();
+    if (i == 0) L.giants[blockIdx.x] = 0xFFFFFFFFu - (uint32_t)best;
+    if (blockIdx.x == 0 && i == 0) *L.count = 0;
+}
+
+// Each vertex's giant memberships, and the bitmap of the vertices that are in the giant of every copy
+// (a warp per 32 vertices). The forest need not be flat: walks without writes.
+__global__ void approx_members(const Level L) {
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31, C = L.F.copies;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, words = (L.n + 31) / 32;
+    const uint32_t all = C >= 32 ? 0xFFFFFFFFu : (1u << C) - 1;
+    for (uint32_t wd = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; wd < words; wd += warps) {
+        const uint32_t x = wd * 32 + lane;
+        uint32_t in = 0;
+        if (x < L.n) {
+            if (C == 4) {
+                const uint4 p = reinterpret_cast<const uint4 *>(L.F.par)[x];
+                const uint32_t g0 = L.F.par[4 * p.x], g1 = L.F.par[4 * p.y + 1];
+                const uint32_t g2 = L.F.par[4 * p.z + 2], g3 = L.F.par[4 * p.w + 3];
+                const uint4 g = *reinterpret_cast<const uint4 *>(L.giants);
+                in = (uint32_t)((g0 == p.x ? g0 : root_of(L.F, 0, g0)) == g.x) |
+                     (uint32_t)((g1 == p.y ? g1 : root_of(L.F, 1, g1)) == g.y) << 1 |
+                     (uint32_t)((g2 == p.z ? g2 : root_of(L.F, 2, g2)) == g.z) << 2 |
+                     (uint32_t)((g3 == p.w ? g3 : root_of(L.F, 3, g3)) == g.w) << 3;
+            } else {
+                for (uint32_t j = 0; j < C; j++) in |= (uint32_t)(root_of(L.F, j, x) == L.giants[j]) << j;
+            }
+            L.member[x] = in;
+        }
+        const uint32_t word = __ballot_sync(0xffffffffu, in == all);
+        if (lane == 0) L.bits[wd] = word;
+    }
+}
+
+__global__ void approx_count_roots(const Forest F, uint32_t n, unsigned int *count) {
+    pdl_wait();
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     uint32_t c = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (uint64_t)gridDim.x * blockDim.x)
-        c += par[i] == (uint32_t)i;
+    for (uint32_t x = tid; x < n; x += stride) {
+        if (F.copies == 4) {
+            const uint4 p = reinterpret_cast<const uint4 *>(F.par)[x];
+            c += (uint32_t)(p.x == x) + (uint32_t)(p.y == x) + (uint32_t)(p.z == x) + (uint32_t)(p.w == x);
+        } else {
+            for (uint32_t j = 0; j < F.copies; j++) c += F.at(x, j) == x;
+        }
+    }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+}
+
+// The hooks of one level (the forest already holds singletons).
+// Union walks from singletons make long parent chains that every walk then pays for (15 M edges, 4
+// copies: 480 us for the first eighth of the edges, 85 us for each of the last). So the forest is built
+// in rounds on small parts of the edges, flattened after each: with kRoundDegree kept edges per vertex
+// in each, 98.7% of a random graph's vertices are in the giant component after the fifth (counted on
+// G(10^6, M); two rounds of twice the edges leave it in small trees). Then some 1.3% of the vertices of
+// a copy are outside, about 2.6% of its edges are tested one by one, and the rest cost two bitmap
+// lookups for all copies together.
+// Bound by: the draws (one or two cipher blocks per quad and copy) and L2 gathers of the rounds at 10^7
+// edges, kernel boundaries at 10^6. Measured per query against eight slices of union walks: G(10^6,
+// 15.2 M edges), unit weights, 4 copies, 1.97 -> 0.75 ms; G(10^5, 1.4 M edges), weights to 42, six
+// levels, 1.79 -> 0.61 ms.
+template <bool kRef>
+int run_level(cac_ctx *ctx, Level L, double kept_degree) {
+    cudaStream_t s = ctx->stream;
+    auto grid = [&](uint64_t work, int per_sm) {
+        return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((work + kThreads - 1) / kThreads, (uint64_t)ctx->num_sms * per_sm));
+    };
+    const unsigned gc = grid(L.n, 8), gq = grid((uint64_t)L.Q * L.F.copies, 8);
+    double sum = 0;
+    for (double d : kRoundDegree) sum += d;
+    if (L.list) {
+        double upto = 0;
+        L.to = 0;
+        for (double d : kRoundDegree) {
+            upto += d;
+            L.from = L.to;
+            L.to = std::min(kSampleParts, (uint32_t)std::ceil(kSampleParts * std::min(1.0, upto / kept_degree)));
+            if (L.to == L.from) continue;
+            CAC_CUDA_TRY(launch_pdl(approx_quads<kRef, kRound>, gq, kThreads, 0, s, L));
+            CAC_CUDA_TRY(launch_pdl(approx_compress, gc, kThreads, 0, s, L.F, L.n));
+        }
+    }
+    if (!L.list || kept_degree < sum) {  // too few edges for a giant component in every copy
+        CAC_CUDA_TRY(launch_pdl(approx_quads<kRef, kAll>, gq, kThreads, 0, s, L));
+    } else {
+        CAC_CUDA_TRY(launch_pdl(approx_giants, L.F.copies, kGiantSample, 0, s, L));
+        CAC_CUDA_TRY(launch_pdl(approx_members, gc, kThreads, 0, s, L));
+        const uint32_t words = (L.n + 31) / 32;
+        const bool shared = words <= kSmemWords;
+        auto kern = shared ? approx_stream<kRef, true> : approx_stream<kRef, false>;
+        CAC_TRY(smem_optin(ctx, kern));
+        const uint64_t tiles = ((uint64_t)L.m + 255) / 256;
+        const unsigned gt = (unsigned)std::min<uint64_t>(tiles / (kStreamThreads / 32) + 1, (uint64_t)ctx->num_sms);
+        CAC_CUDA_TRY(launch_pdl(kern, gt, kStreamThreads, shared ? words * 4 : 0, s, L));
+        CAC_CUDA_TRY(launch_pdl(approx_survivors<kRef>, (unsigned)ctx->num_sms * 8, kThreads, 0, s, L));
+    }
+    CAC_CUDA_TRY(cudaGetLastError());
+    return CAC_OK;
 }
 
 }  // namespace
@@ -288,7 +602,20 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
     // slice but the last empty: no level runs. Unit weights: w_r is the slice length; one rank:
     // the graph's total weight; otherwise the slice sums are taken on the device.
     const bool stats = ranks > 1 && portion > 0 && !g->unit_weights;
-    CAC_TRY(arena_reserve(ctx, align_up(nv * 4 + 4) + 256 + (stats ? align_up((uint64_t)ranks * 8) : 0)));
+    // quads of 4 edges per rank slice
+    const uint64_t Qf = (portion + 3) / 4;
+    const uint64_t Q = portion == 0 ? (g->m + 3) / 4 : (ranks - 1) * Qf + (g->m - (uint64_t)(ranks - 1) * portion + 3) / 4;
+    const bool large = g->m >= kSampledEdges && Q < 0xFFFFFFFFull;
+    const size_t base_bytes = align_up(nv * 4 + 4) + 256 + (stats ? align_up((uint64_t)ranks * 8) : 0);
+    const uint64_t cap = g->m / 4 + 1024;
+    const size_t more = align_up((uint64_t)g->n * 4) + align_up(((uint64_t)g->n + 31) / 32 * 4) +
+                        align_up(cap * 8) + 256;
+    // the survivor list needs 2 bytes an edge more than the forest: without it (it does not fit the
+    // budget, or there are more copies than a mask has bits) every edge is tested and hooked at once
+    const bool sampled = large && copies <= 32 &&
+                         (base_bytes + more <= ctx->arena.cap || !ctx->budget ||
+                          ctx->held - ctx->arena.cap + align_up(base_bytes + more, 1 << 20) <= ctx->budget);
+    CAC_TRY(arena_reserve(ctx, base_bytes + (sampled ? more : 0)));
     arena_reset(ctx);
     uint32_t *par = (uint32_t *)arena_take(ctx, nv * 4 + 4);
     unsigned int *d_count = (unsigned int *)arena_take(ctx, 16);
@@ -314,53 +641,45 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
         iterations = UINT32_MAX;
         for (uint32_t r = 0; r < ranks; r++) iterations = std::min(iterations, level_count(h[r]));
     }
-    // quads of 4 edges per rank slice (see approx_keep_hook4)
-    const uint64_t Qf = (portion + 3) / 4;
-    const uint64_t Q = portion == 0 ? (g->m + 3) / 4 : (ranks - 1) * Qf + (g->m - (uint64_t)(ranks - 1) * portion + 3) / 4;
-    const int gi = (int)std::max<uint64_t>(1, std::min<uint64_t>((nv + kThreads - 1) / kThreads, ctx->num_sms * 8));
+    const int gi = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)g->n + kThreads - 1) / kThreads, ctx->num_sms * 8));
     uint32_t first = 0;
     if (ref_stream) iterations = std::min<uint32_t>(iterations, 52);  // ceil(ln W) <= 45 for W < 2^64
+    Level L{};
+    L.U = g->u;
+    L.V = g->v;
+    L.Wt = g->w;
+    L.m = (uint32_t)g->m;
+    L.n = g->n;
+    L.F = Forest{par, copies};
+    L.seed = seed;
+    L.ranks = ranks;
+    L.portion = (uint32_t)portion;
+    L.Qf = (uint32_t)Qf;
+    L.Q = (uint32_t)Q;
+    if (sampled) {
+        L.member = (uint32_t *)arena_take(ctx, (uint64_t)g->n * 4);
+        L.bits = (uint32_t *)arena_take(ctx, ((uint64_t)g->n + 31) / 32 * 4);
+        L.list = (uint2 *)arena_take(ctx, cap * 8);
+        L.cap = (uint32_t)cap;
+        L.giants = (uint32_t *)arena_take(ctx, 256);
+        L.count = L.giants + 32;
+    }
+    const double mean_weight = g->m ? (double)g->total_weight / (double)g->m : 0;
     for (uint32_t level = 1; level <= iterations && level <= 63; level++) {
-        approx_init<<<gi, kThreads, 0, s>>>(par, nv);
-        // the kept edges are hooked in kSlices slices, the forest flattened after the first few
-        // and the last (the same partition as one pass; one pass from singletons builds long
-        // parent chains on large graphs)
-        if (ref_stream) {
-            const uint64_t keep_max = stream_threshold(level);  // p = 2^-level (ApproximateCut.cpp:37)
-            const uint32_t slices = Q < (1u << 16) ? 1 : kSlices;
-            for (uint32_t sl = 0; sl < slices; sl++) {
-                const uint64_t q0 = Q * sl / slices, q1 = Q * (sl + 1) / slices;
-                if (q1 <= q0) continue;
-                const int ge = (int)std::max<uint64_t>(
-                    1, std::min<uint64_t>((q1 - q0 + kThreads - 1) / kThreads,
-                                          std::max(1, ctx->num_sms * 8 / (int)copies)));
-                approx_stream_keep_hook<<<dim3(ge, copies), kThreads, 0, s>>>(par, g->u, g->v, g->m, g->n, level,
-                                                                              keep_max, copies, seed, ranks,
-                                                                              portion, Qf, q0, q1);
-                if (sl < kCompressedSlices && sl + 1 < slices) approx_compress<<<gi, kThreads, 0, s>>>(par, nv);
-            }
-        } else if (Q < (1u << 16)) {
-            if (g->m) {
-                const int ge = (int)std::max<uint64_t>(
-                    1, std::min<uint64_t>((g->m + kThreads - 1) / kThreads, std::max(1, ctx->num_sms * 8 / (int)copies)));
-                dim3 grid(ge, copies);
-                approx_keep_hook<<<grid, kThreads, 0, s>>>(par, g->u, g->v, g->w, g->m, g->n, level, seed, ranks,
-                                                           portion);
-            }
-        }
-        const uint32_t slices = ref_stream || Q < (1u << 16) ? 0 : kSlices;
-        for (uint32_t sl = 0; sl < slices; sl++) {
-            const uint64_t q0 = Q * sl / slices, q1 = Q * (sl + 1) / slices;
-            if (q1 <= q0) continue;
+        approx_init<<<gi, kThreads, 0, s>>>(L.F, g->n, d_count);
+        L.level = level;
+        L.keep_max = stream_threshold(level);  // p = 2^-level (ApproximateCut.cpp:37)
+        if (large || ref_stream) {
+            const double kept = 1 - std::pow(1 - std::ldexp(1.0, -(int)level), mean_weight);  // share of the edges
+            const double degree = 2.0 * g->m * kept / std::max<uint32_t>(1, g->n);
+            CAC_TRY(ref_stream ? run_level<true>(ctx, L, degree) : run_level<false>(ctx, L, degree));
+        } else if (g->m) {
             const int ge = (int)std::max<uint64_t>(
-                1, std::min<uint64_t>((q1 - q0 + kThreads - 1) / kThreads, std::max(1, ctx->num_sms * 8 / (int)copies)));
-            dim3 grid(ge, copies);
-            approx_keep_hook4<<<grid, kThreads, 0, s>>>(par, g->u, g->v, g->w, g->m, g->n, level, seed, ranks, portion,
-                                                        Qf, q0, q1);
-            if (sl < kCompressedSlices && sl + 1 < slices) approx_compress<<<gi, kThreads, 0, s>>>(par, nv);
+                1, std::min<uint64_t>((g->m + kThreads - 1) / kThreads, std::max(1, ctx->num_sms * 8 / (int)copies)));
+            approx_keep_hook<<<dim3(ge, copies), kThreads, 0, s>>>(L.F, g->u, g->v, g->w, g->m, level, seed, ranks,
+                                                                   portion);
         }
-        CAC_CUDA_TRY(cudaMemsetAsync(d_count, 0, 4, s));
-        approx_count_roots<<<gi, kThreads, 0, s>>>(par, nv, d_count);
+        CAC_CUDA_TRY(launch_pdl(approx_count_roots, (unsigned)gi, kThreads, 0, s, L.F, g->n, d_count));
         CAC_CUDA_TRY(cudaGetLastError());
         CAC_CUDA_TRY(cudaMemcpyAsync(ctx->pinned_u32, d_count, 4, cudaMemcpyDeviceToHost, s));
         CAC_CUDA_TRY(cudaStreamSynchronize(s));

@@ -21,6 +21,7 @@
 // 16-byte vector loads, 4 edges per load pair); parent[n] uint32 (L2-resident for n up to
 // tens of millions: 129 MB of L2); per-tile root counts; labels[n].
 #include "cac_internal.h"
+#include "pdl.cuh"
 #include "sitmo.cuh"
 
 #include <algorithm>
@@ -30,28 +31,6 @@
 
 namespace cac {
 namespace {
-
-// Programmatic dependent launch: a kernel launched with launch_pdl may start while its predecessor
-// on the stream drains; pdl_wait() (griddepcontrol.wait) holds it until the predecessor has
-// completed and its writes are visible, so every kernel calls it before its first dependent
-// access. After an ordinary launch it returns at once. Measured on the CC query (22 kernels in
-// one replayed graph): BA n=1,024,000 194.9 -> 192.8 us, R-MAT scale 22 about 1-3 us.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
 
 constexpr int kThreads = 256;
 constexpr int kTileItems = 4;                        // vertices per thread in the labelling tiles
