@@ -49,6 +49,7 @@ constexpr int kThreads = 256;
 // Graphs with fewer edges hook every edge in one pass: there a level is a few launches either way.
 constexpr uint64_t kSampledEdges = 1u << 15;
 constexpr uint32_t kSampleParts = 128;        // a sampling round takes 128ths of the edges
+constexpr int kHops = 32;                     // longest walk of a compression between rounds
 constexpr double kRoundDegree[] = {0.8, 0.8, 0.8, 0.8, 1.6};  // kept edges per vertex in each round
 constexpr uint32_t kGiantSample = 1024;       // vertices looked at to find a copy's giant component
 constexpr int kStreamThreads = 1024;          // CTA of the pass over the other edges (the bitmap fills shared memory)
@@ -259,7 +260,7 @@ __device__ __forceinline__ bool edge_kept(const Level &L, uint32_t e, uint32_t j
 
 // Hooks the kept edges of some quads, a thread per quad and copy, the copies of a quad in neighbouring
 // lanes (what an end needs of 4 copies is one 16-byte access).
-//   kRound  a sampling round: the forest is flat, and every kept edge between two roots makes the smaller
+//   kRound  a sampling round: the forest is nearly flat, and every kept edge between two parents makes the smaller
 //           one the parent of the larger, the smallest of all winning (an atomic without a return value:
 //           no walk, no retry; a link that loses is found again by the pass over all edges). Late
 //           rounds have few large trees, whose roots would take thousands of such writes each: a table
@@ -268,13 +269,7 @@ __device__ __forceinline__ bool edge_kept(const Level &L, uint32_t e, uint32_t j
 enum QuadPass { kRound, kAll };
 constexpr uint32_t kGiven = 1024;
 template <bool kRef, QuadPass kPass>
-__global__ void __launch_bounds__(kThreads) approx_quads(const Level L) {
-    pdl_wait();
-    __shared__ unsigned long long given[kPass == kRound ? kGiven : 1];
-    if (kPass == kRound) {
-        for (uint32_t i = threadIdx.x; i < kGiven; i += kThreads) given[i] = ~0ull;
-        __syncthreads();
-    }
+__device__ __forceinline__ void hook_quads(const Level &L, unsigned long long *given) {
     const uint32_t C = L.F.copies, lane = threadIdx.x & 31, side = min(C, 32u), per = 32 / side;  // quads per warp
     if (lane >= side * per) return;
     // the pass's quads, numbered: all, or those of the round
@@ -327,17 +322,22 @@ __global__ void __launch_bounds__(kThreads) approx_quads(const Level L) {
     }
 }
 
-// Tests edge e in the copies of `need` and hooks it there.
-template <bool kRef>
-__device__ __forceinline__ void keep_hook(const Level &L, uint32_t e, uint32_t a, uint32_t b, uint32_t j) {
-    if (edge_kept<kRef>(L, e, j)) aunite(L.F, j, a, b);
+template <bool kRef, QuadPass kPass>
+__global__ void __launch_bounds__(kThreads) approx_quads(const Level L) {
+    __shared__ unsigned long long given[kPass == kRound ? kGiven : 1];
+    if (kPass == kRound) {
+        for (uint32_t i = threadIdx.x; i < kGiven; i += kThreads) given[i] = ~0ull;
+        __syncthreads();
+    }
+    pdl_wait();
+    hook_quads<kRef, kPass>(L, given);
 }
 
 // All edges after the sampling rounds, a warp per 256-edge tile as in the filter of the
 // connected-components path: an edge with both ends in the giant of every copy is dropped unseen
 // (whatever its draws say, it joins nothing); of the others, the copies in which an end is outside the
-// giant are noted in the survivor list. Survivors past the end of the list are tested and hooked on the
-// spot. kShared: the bitmap fits shared memory.
+// giant are noted in the survivor list (the first L.cap; past that only counted). kShared: the bitmap fits
+// shared memory.
 template <bool kRef, bool kShared>
 __global__ void __launch_bounds__(kStreamThreads) approx_stream(const Level L) {
     pdl_wait();
@@ -392,26 +392,27 @@ __global__ void __launch_bounds__(kStreamThreads) approx_stream(const Level L) {
 #pragma unroll
         for (int d = 0; d < 8; d++) {
             if (!((keep >> d) & 1u)) continue;
-            if (at < L.cap) {
-                L.list[at] = make_uint2(e[d], need[d]);
-            } else {
-                for (uint32_t j = 0; j < L.F.copies; j++)
-                    if ((need[d] >> j) & 1u) keep_hook<kRef>(L, e[d], a[d], b[d], j);
-            }
+            if (at < L.cap) L.list[at] = make_uint2(e[d], need[d]);
             at++;
         }
     }
 }
 
-// One thread per (survivor, copy).
+// What the stream pass left: one thread per (survivor, copy), or, where the survivors are more than their
+// list holds, every quad by union walks (a quad's 4 draws cost as much as one survivor's).
 template <bool kRef>
-__global__ void __launch_bounds__(kThreads) approx_survivors(const Level L) {
+__global__ void __launch_bounds__(kThreads) approx_rest(const Level L) {
     pdl_wait();
-    const uint64_t items = (uint64_t)min(*L.count, L.cap) * L.F.copies;
+    const uint32_t count = *L.count;
+    if (count > L.cap) {
+        hook_quads<kRef, kAll>(L, nullptr);
+        return;
+    }
+    const uint64_t items = (uint64_t)count * L.F.copies;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < items; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t at = (uint32_t)(i / L.F.copies), j = (uint32_t)(i - (uint64_t)at * L.F.copies);
         const uint2 x = L.list[at];
-        if ((x.y >> j) & 1u) keep_hook<kRef>(L, x.x, L.U[x.x], L.V[x.x], j);
+        if (((x.y >> j) & 1u) && edge_kept<kRef>(L, x.x, j)) aunite(L.F, j, L.U[x.x], L.V[x.x]);
     }
 }
 
@@ -431,8 +432,17 @@ __global__ void approx_slice_sums(const uint32_t *__restrict__ w, uint64_t m, ui
     }
 }
 
-// Full path compression (read-only walks; only roots are written), a thread per vertex and 4 copies:
-// their parents in one load, the 4 grandparents requested together, then the longer chains.
+// An ancestor of v in copy j, the root unless it is more than kHops away.
+__device__ __forceinline__ uint32_t near_of(const Forest &F, uint32_t j, uint32_t cur) {
+    uint32_t next;
+    for (int k = 0; k < kHops && (next = F.at(cur, j)) != cur; k++) cur = next;
+    return cur;
+}
+
+// Compression between the rounds, a thread per vertex and 4 copies: their parents in one load, the 4
+// grandparents requested together, then the longer chains. Walks end after kHops parents: heavy paths
+// numbered along their length make chains of that length, and the rounds do not need a flat forest (what
+// a link at a vertex that is no root any more separates is joined again by the pass over all edges).
 __global__ void approx_compress(const Forest F, uint32_t n) {
     pdl_wait();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -441,13 +451,13 @@ __global__ void approx_compress(const Forest F, uint32_t n) {
         for (uint32_t x = tid; x < n; x += stride) {
             const uint4 p = p4[x];
             const uint32_t g0 = F.par[4 * p.x], g1 = F.par[4 * p.y + 1], g2 = F.par[4 * p.z + 2], g3 = F.par[4 * p.w + 3];
-            const uint32_t r0 = g0 == p.x ? g0 : root_of(F, 0, g0), r1 = g1 == p.y ? g1 : root_of(F, 1, g1);
-            const uint32_t r2 = g2 == p.z ? g2 : root_of(F, 2, g2), r3 = g3 == p.w ? g3 : root_of(F, 3, g3);
+            const uint32_t r0 = g0 == p.x ? g0 : near_of(F, 0, g0), r1 = g1 == p.y ? g1 : near_of(F, 1, g1);
+            const uint32_t r2 = g2 == p.z ? g2 : near_of(F, 2, g2), r3 = g3 == p.w ? g3 : near_of(F, 3, g3);
             if (r0 != p.x || r1 != p.y || r2 != p.z || r3 != p.w) p4[x] = make_uint4(r0, r1, r2, r3);
         }
     } else {
         for (uint32_t x = tid; x < n; x += stride)
-            for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = root_of(F, j, x);
+            for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = near_of(F, j, x);
     }
 }
 
@@ -570,7 +580,7 @@ int run_level(cac_ctx *ctx, Level L, double kept_degree) {
         const uint64_t tiles = ((uint64_t)L.m + 255) / 256;
         const unsigned gt = (unsigned)std::min<uint64_t>(tiles / (kStreamThreads / 32) + 1, (uint64_t)ctx->num_sms);
         CAC_CUDA_TRY(launch_pdl(kern, gt, kStreamThreads, shared ? words * 4 : 0, s, L));
-        CAC_CUDA_TRY(launch_pdl(approx_survivors<kRef>, (unsigned)ctx->num_sms * 8, kThreads, 0, s, L));
+        CAC_CUDA_TRY(launch_pdl(approx_rest<kRef>, (unsigned)ctx->num_sms * 8, kThreads, 0, s, L));
     }
     CAC_CUDA_TRY(cudaGetLastError());
     return CAC_OK;
@@ -607,10 +617,10 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
     const uint64_t Q = portion == 0 ? (g->m + 3) / 4 : (ranks - 1) * Qf + (g->m - (uint64_t)(ranks - 1) * portion + 3) / 4;
     const bool large = g->m >= kSampledEdges && Q < 0xFFFFFFFFull;
     const size_t base_bytes = align_up(nv * 4 + 4) + 256 + (stats ? align_up((uint64_t)ranks * 8) : 0);
-    const uint64_t cap = g->m / 4 + 1024;
+    const uint64_t cap = g->m / 8 + 1024;
     const size_t more = align_up((uint64_t)g->n * 4) + align_up(((uint64_t)g->n + 31) / 32 * 4) +
                         align_up(cap * 8) + 256;
-    // the survivor list needs 2 bytes an edge more than the forest: without it (it does not fit the
+    // the survivor list needs a byte an edge more than the forest: without it (it does not fit the
     // budget, or there are more copies than a mask has bits) every edge is tested and hooked at once
     const bool sampled = large && copies <= 32 &&
                          (base_bytes + more <= ctx->arena.cap || !ctx->budget ||
