@@ -69,10 +69,9 @@ PORT_SLOWDOWN = {
                           "how": _PORT_HOW},
 }
 METRIC = "CC edges/s (parallel_cc, BA n=1,024,000 m=16)"
-# init, sample_draws, 4 x sample_hook (slices of 1, 1, 2 and 4 eighths), 3 x compress4 (after all
-# but the last slice), compress_giant_bitmap, filter, hook_survivors, finalize_count, scan_tiles,
-# rank_roots, label_all
-KERNELS_PER_QUERY = 2 + 4 + 3 + 1 + 2 + 4
+# init, sample_draws, 5 x sample_round, 4 x compress4 (after all but the last), compress_giant_bitmap,
+# filter, hook_survivors, count_roots, rank_roots, label_all
+KERNELS_PER_QUERY = 2 + 5 + 4 + 1 + 2 + 3
 
 
 def _max_over_ranks(x, world):

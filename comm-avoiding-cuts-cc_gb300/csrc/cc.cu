@@ -3,19 +3,20 @@
 //
 // Reference round structure            ->  here
 //   root scatters per-rank draw counts    host restates edgesToSamplePerProcessor (cc_plan)
-//   rank r draws engine()%slice samples   cc_sample_draws / cc_sample_hook: sitmo stream
+//   rank r draws engine()%slice samples   cc_sample_draws / cc_sample_round: sitmo stream
 //     with sitmo(seed + r)                  (seed + r, 0, 0, 0), output k = word k % 8 of block
 //                                           k / 8, the reference's k-th engine output; it picks
 //                                           a 32-edge chunk of the slice (coalesced) instead of
 //                                           one edge
-//   root: shuffle + prefix union-find     lock-free union-find in HBM (atomicCAS hooking of
-//     to one component (Boost sets)         the larger root under the smaller, so roots are
-//                                           component minima; order-free for target 1)
+//   root: shuffle + prefix union-find     rounds of root links in HBM (the smallest root an edge
+//     to one component (Boost sets)         leads to becomes the parent), flattened in between
 //   bcast map, rewrite slice, drop loops  cc_edge_pass: one streaming pass over every edge;
 //     and repeat while edges remain         edges whose endpoints already share a root are the
-//                                           dropped loops, the rest hook (the final round)
+//                                           dropped loops, the rest hook (the final round): lock-
+//                                           free union-find (atomicCAS hooking of the larger root
+//                                           under the smaller, so roots are component minima)
 //   relabel by first appearance           roots = minima, so label = exclusive scan of the
-//                                           root flags (cc_finalize_count/scan/rank/label)
+//                                           root flags (label_components)
 //
 // Memory layout in HBM: edge endpoints as two uint32 arrays u[m], v[m] (structure of arrays,
 // 16-byte vector loads, 4 edges per load pair); parent[n] uint32 (L2-resident for n up to
@@ -28,6 +29,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 namespace cac {
 namespace {
@@ -40,14 +42,21 @@ constexpr int kEdgeThreads = 1024;                   // closing-pass CTA (one pe
 constexpr uint32_t kSmemBitmapWords = 48 * 1024;     // 192 KB of bitmap in shared memory (1.57M vertices)
 constexpr uint32_t kGiantSample = 1024;              // vertices sampled to find the giant component
 constexpr uint32_t kSampleChunk = 32;                // consecutive edges behind one sampling draw
-// Slices of the sampling round, in eighths of its draws: a first slice above an eighth builds long
-// parent chains from the singletons (2/8 first: 451 vs 209 us per BA n=1,024,000 query), later
-// ones mostly hook small trees onto the giant one and can be larger. Every slice but the last is
-// followed by a full compression; the last by the fused compression + giant search + bitmap.
-// Measured per BA n=1,024,000 query against eight even slices (compressions after the first three
-// and the last): 1,1,2,4 202.0 vs 208.8 us; 1,1,1,5 203.3; 1,1,1,1,4 206.6; 1,1,1,1,1,3 204.9.
-// R-MAT scale 22: 1,1,1,5 647.5 vs 666.4 us.
-constexpr uint32_t kSliceEighths[] = {1, 1, 2, 4};
+// Edges per vertex (as degrees: half as many) in each round of forest building. Union walks from
+// singletons make long parent chains that every walk then pays for, so the forest is built in rounds on
+// disjoint parts of the edges, flattened after each; in a round every edge between two roots makes the
+// smaller one the parent of the larger, the smallest of all winning. With these sizes 98.7% of a
+// random graph's vertices are in the giant component after the fifth (counted on G(10^6, M); two rounds
+// of twice the edges leave it in small trees).
+constexpr double kRoundDegree[] = {0.8, 0.8, 0.8, 0.8, 1.6};
+constexpr uint32_t kRoundParts = 128;                // without draws: rounds are 128ths of the 256-edge tiles
+// Without draws, smaller or sparser graphs hook every edge in one pass (below one edge per vertex at each
+// end a random graph has small trees only): G(10^6, M) with average degree 0.1 takes 41 us in one pass
+// and 48 in rounds, with 3 863 and 127, G(17000, M) with degree 2 87 and 66.
+constexpr uint64_t kRoundEdges = 1u << 13;
+constexpr uint32_t kProbes = 128;
+constexpr int kHops = 32;                            // longest walk of a compression between rounds
+constexpr int kRoundThreads = 1024;                  // CTA of a round: the more threads, the more links the table sees
 constexpr uint32_t kMaxRegions = 1024;               // filter CTAs (regions of the survivor buffer)
 // survivor-hook CTAs per SM: about one survivor per thread on BA n=1,024,000 (0.6 M survivors);
 // 8 against 4: 20 vs 22.5 us there, 47 vs 63.5 us on R-MAT scale 22; 16 no better
@@ -162,51 +171,177 @@ __global__ void cc_sample_draws(const RankDesc *__restrict__ ranks, int nranks, 
     }
 }
 
-// One warp per sampled chunk of the draw range [d0, d1): coalesced loads of its edges, each hooked.
-template <bool kCheck>
-__global__ void cc_sample_hook(uint32_t *par, const uint32_t *__restrict__ u, const uint32_t *__restrict__ v,
-                               const uint64_t *__restrict__ chunks, uint64_t d0, uint64_t d1, uint32_t n,
-                               uint32_t *err) {
+// The links of one CTA's part of a round, gathered in shared memory: root -> smallest root it is linked
+// to. Late rounds have few large trees, whose roots would take thousands of atomics from every CTA at
+// once; here each takes one. A root whose entry belongs to another is linked in memory directly; the roots
+// of kProbes vertices, among which the large trees are, get their entries first.
+template <uint32_t kLinks>  // a power of two
+struct Links {
+    uint32_t key[kLinks], val[kLinks];
+    static __device__ __forceinline__ uint32_t entry(uint32_t r) { return (uint32_t)(((uint64_t)(r * 2654435761u) * kLinks) >> 32); }
+    __device__ __forceinline__ void clear() {
+        for (uint32_t i = threadIdx.x; i < kLinks; i += blockDim.x) key[i] = val[i] = 0xFFFFFFFFu;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void claim_large(const uint32_t *par, uint32_t n) {
+        if (threadIdx.x < kProbes) {
+            const uint32_t r = par[(uint32_t)(((uint64_t)(threadIdx.x * 0x9E3779B9u) * n) >> 32)];
+            atomicCAS(&key[entry(r)], 0xFFFFFFFFu, r);
+        }
+        __syncthreads();
+    }
+    // a and b: parents of an edge's ends in a flat forest
+    __device__ __forceinline__ void add(uint32_t *par, uint32_t a, uint32_t b) {
+        if (a == b) return;
+        const uint32_t hi = max(a, b), lo = min(a, b), x = entry(hi);
+        uint32_t k = *(volatile uint32_t *)&key[x];
+        if (k == 0xFFFFFFFFu) k = atomicCAS(&key[x], 0xFFFFFFFFu, hi);
+        if (k != hi && k != 0xFFFFFFFFu) atomicMin(&par[hi], lo);
+        else if (*(volatile uint32_t *)&val[x] > lo) atomicMin(&val[x], lo);
+    }
+    __device__ __forceinline__ void flush(uint32_t *par) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < kLinks; i += blockDim.x)
+            if (val[i] != 0xFFFFFFFFu) atomicMin(&par[key[i]], val[i]);
+    }
+};
+
+// The first round: every vertex is still its own root, and any smaller end will do as its parent (a
+// store; hubs take thousands of links here, and atomics on them took 110 us on R-MAT scale 22).
+__device__ __forceinline__ void first_link(uint32_t *par, uint32_t a, uint32_t b) {
+    if (a != b) par[max(a, b)] = min(a, b);
+}
+
+// One round on the chunks of the draw range [d0, d1): a warp takes two chunks at a time (coalesced loads
+// of their edges, all in flight together).
+template <bool kFirst, bool kCheck>
+__global__ void __launch_bounds__(kRoundThreads, 2) cc_sample_round(uint32_t *par, const uint32_t *__restrict__ u,
+                                                            const uint32_t *__restrict__ v,
+                                                            const uint64_t *__restrict__ chunks, uint64_t d0, uint64_t d1,
+                                                            uint32_t n, uint32_t *err) {
+    __shared__ typename std::conditional<kFirst, char, Links<4 * kRoundThreads>>::type links;
+    if constexpr (!kFirst) links.clear();
     pdl_wait();
+    if constexpr (!kFirst) links.claim_large(par, n);
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t d = d0 + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); d < d1; d += warps) {
-        const uint64_t c = chunks[d];
-        if (lane < (uint32_t)(c >> 32)) {
-            const uint64_t e = (c & 0xFFFFFFFFull) + lane;
-            edge_hook_checked<kCheck>(par, __ldg(u + e), __ldg(v + e), n, err);
+    for (uint64_t d = d0 + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); d < d1; d += 2 * warps) {
+        uint64_t c[2];
+        uint32_t a[2], b[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) c[k] = d + k * warps < d1 ? chunks[d + k * warps] : 0;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            a[k] = b[k] = 0;
+            if (lane < (uint32_t)(c[k] >> 32)) {
+                const uint64_t e = (c[k] & 0xFFFFFFFFull) + lane;
+                a[k] = __ldg(u + e);
+                b[k] = __ldg(v + e);
+                if (kCheck && (a[k] >= n || b[k] >= n)) {
+                    atomicOr(err, kErrBadId);
+                    a[k] = b[k] = 0;
+                }
+            }
+        }
+        if (!kFirst) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                a[k] = par[a[k]];
+                b[k] = par[b[k]];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if constexpr (kFirst) first_link(par, a[k], b[k]);
+            else links.add(par, a[k], b[k]);
         }
     }
+    if constexpr (!kFirst) links.flush(par);
 }
 
-__global__ void cc_compress(uint32_t *par, uint32_t lo, uint32_t hi) {
+// One round on the 256-edge tiles t with from <= t % kRoundParts < to, a warp per tile, its lane l on
+// edges l, 32 + l, ... (all loads of the eight in flight together).
+template <bool kFirst, bool kCheck, int kNT>
+__global__ void __launch_bounds__(kNT, 2048 / kNT) cc_edge_round(uint32_t *par, const uint32_t *__restrict__ u,
+                                                          const uint32_t *__restrict__ v, uint64_t m, uint32_t from,
+                                                          uint32_t to, uint32_t n, uint32_t *err) {
+    __shared__ typename std::conditional<kFirst, char, Links<4 * kNT>>::type links;
+    if constexpr (!kFirst) links.clear();
     pdl_wait();
-    for (uint32_t i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
-        par[i] = find_root_ro(par, i);
+    if constexpr (!kFirst && kNT == kRoundThreads) links.claim_large(par, n);
+    const uint32_t lane = threadIdx.x & 31, w = to - from;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5, tiles = (m + 255) / 256;
+    for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;; i += warps) {
+        const uint64_t t = i / w * kRoundParts + from + i % w;
+        if (t >= tiles) break;
+        uint32_t a[8], b[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint64_t e = t * 256 + 32 * k + lane;
+            a[k] = b[k] = 0;
+            if (e < m) {
+                a[k] = __ldg(u + e);
+                b[k] = __ldg(v + e);
+            }
+            if (kCheck && (a[k] >= n || b[k] >= n)) {
+                atomicOr(err, kErrBadId);
+                a[k] = b[k] = 0;
+            }
+        }
+        if (!kFirst) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                a[k] = par[a[k]];
+                b[k] = par[b[k]];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if constexpr (kFirst) first_link(par, a[k], b[k]);
+            else links.add(par, a[k], b[k]);
+        }
+    }
+    if constexpr (!kFirst) links.flush(par);
 }
 
-// Full compression, 4 consecutive vertices per thread: one 16-byte load of their parents, then
-// the grandparents of all four requested together (most chains end there), then the rare longer
-// chains; one 16-byte store. Only roots are written, as in cc_compress.
-__global__ void cc_compress4(uint32_t *par, uint32_t n4) {
+// An ancestor of v, the root unless it is more than kHops away.
+__device__ __forceinline__ uint32_t find_near(const uint32_t *par, uint32_t v) {
+    uint32_t cur = v, next;
+    for (int k = 0; k < kHops && (next = par[cur]) != cur; k++) cur = next;
+    return cur;
+}
+
+// Compression between the rounds, 4 consecutive vertices per thread: one 16-byte load of their parents,
+// then the grandparents of all four requested together (most chains end there), then the longer chains;
+// one 16-byte store. The last n % 4 vertices are done one by one. Walks end after kHops parents: a path
+// whose vertices are numbered along it makes chains of its own length, and walking these to the end
+// took 9 ms for 300,000 vertices; cut short, every compression divides the depth by kHops. The rounds
+// do not need a flat forest: a link made at a vertex that is no root any more replaces that vertex's
+// parent by another vertex of its component, and what that separates is joined again by the passes over
+// all edges.
+__global__ void cc_compress4(uint32_t *par, uint32_t n) {
     pdl_wait();
     uint4 *p4 = reinterpret_cast<uint4 *>(par);
+    const uint32_t n4 = n / 4;
+    if (blockIdx.x == 0 && threadIdx.x < (n & 3u)) {
+        const uint32_t x = 4 * n4 + threadIdx.x;
+        par[x] = find_near(par, x);
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
         const uint4 p = p4[i];
         const uint32_t v0 = 4 * i;
         uint32_t r0 = p.x, r1 = p.y, r2 = p.z, r3 = p.w;
         const uint32_t g0 = r0 != v0 ? par[r0] : r0, g1 = r1 != v0 + 1 ? par[r1] : r1;
         const uint32_t g2 = r2 != v0 + 2 ? par[r2] : r2, g3 = r3 != v0 + 3 ? par[r3] : r3;
-        r0 = g0 == r0 ? r0 : find_root_ro(par, g0);
-        r1 = g1 == r1 ? r1 : find_root_ro(par, g1);
-        r2 = g2 == r2 ? r2 : find_root_ro(par, g2);
-        r3 = g3 == r3 ? r3 : find_root_ro(par, g3);
+        r0 = g0 == r0 ? r0 : find_near(par, g0);
+        r1 = g1 == r1 ? r1 : find_near(par, g1);
+        r2 = g2 == r2 ? r2 : find_near(par, g2);
+        r3 = g3 == r3 ? r3 : find_near(par, g3);
         if (r0 != p.x || r1 != p.y || r2 != p.z || r3 != p.w) p4[i] = make_uint4(r0, r1, r2, r3);
     }
 }
 
-// Compression of [0, n): the vectorised body over whole 4-vertex groups, the scalar kernel for
-// the tail (the parent array is 256-byte aligned).
+// Compression of [0, n) (the parent array is 256-byte aligned).
 void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s);
 
 // The end of the sampling round in one launch: full compression, the giant component and its
@@ -262,7 +397,7 @@ __global__ void __launch_bounds__(kGiantSample) cc_compress_giant_bitmap(uint32_
 }
 
 // Closing pass without a sampling round: every edge hooks, 4 edges per thread step through
-// 16-byte streaming loads.
+// 16-byte streaming loads, their 8 parents requested together.
 template <bool kVec, bool kCheck>
 __global__ void __launch_bounds__(kThreads) cc_edge_pass(uint32_t *par, const uint32_t *__restrict__ u,
                                                          const uint32_t *__restrict__ v, uint64_t m, uint32_t n,
@@ -276,12 +411,22 @@ __global__ void __launch_bounds__(kThreads) cc_edge_pass(uint32_t *par, const ui
         const uint4 *u4 = reinterpret_cast<const uint4 *>(u);
         const uint4 *v4 = reinterpret_cast<const uint4 *>(v);
         for (uint64_t i = tid; i < m4; i += stride) {
-            const uint4 a = __ldcs(u4 + i);
-            const uint4 b = __ldcs(v4 + i);
-            edge_hook_checked<kCheck>(par, a.x, b.x, n, err);
-            edge_hook_checked<kCheck>(par, a.y, b.y, n, err);
-            edge_hook_checked<kCheck>(par, a.z, b.z, n, err);
-            edge_hook_checked<kCheck>(par, a.w, b.w, n, err);
+            const uint4 qa = __ldcs(u4 + i), qb = __ldcs(v4 + i);
+            uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w}, b[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (kCheck && (a[k] >= n || b[k] >= n)) {
+                    atomicOr(err, kErrBadId);
+                    a[k] = b[k] = 0;
+                }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                a[k] = par[a[k]];
+                b[k] = par[b[k]];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++)  // (equal parents: one component already, the reference drops the edge as a loop)
+                if (a[k] != b[k]) unite(par, a[k], b[k]);
         }
         done = m4 << 2;
     }
@@ -426,20 +571,16 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t x, uint32_t *sh) {
     return t;  // valid in thread 0
 }
 
-// Final compression, root flags and per-tile root counts.
-__global__ void __launch_bounds__(kThreads) cc_finalize_count(uint32_t *par, uint32_t n, uint32_t *tile_counts) {
+// Per-tile root counts.
+__global__ void __launch_bounds__(kThreads) cc_count_roots(const uint32_t *par, uint32_t n, uint32_t *tile_counts) {
     pdl_wait();
     __shared__ uint32_t sh[32];
     const uint64_t base = (uint64_t)blockIdx.x * kTile;
     uint32_t c = 0;
-#pragma unroll 4
+#pragma unroll
     for (int k = 0; k < kTileItems; k++) {
         const uint64_t i = base + (uint64_t)k * kThreads + threadIdx.x;
-        if (i < n) {
-            const uint32_t r = find_root_ro(par, (uint32_t)i);
-            par[i] = r;
-            c += (r == (uint32_t)i);
-        }
+        c += i < n && par[i] == (uint32_t)i;
     }
     const uint32_t t = block_sum(c, sh);
     if (threadIdx.x == 0) tile_counts[blockIdx.x] = t;
@@ -483,11 +624,26 @@ __global__ void __launch_bounds__(1024) cc_scan_tiles(const uint32_t *counts, ui
     if (threadIdx.x == 0) *total = carry;
 }
 
-// Rank of every root: tile offset + exclusive scan of root flags inside the tile.
+// Rank of every root: tile offset + exclusive scan of root flags inside the tile. kOwn: the CTA sums the
+// counts of the tiles before its own (counts), and the last one writes the total; else the offsets
+// come from cc_scan_tiles. Labels of a null array are not written.
+template <bool kOwn>
 __global__ void __launch_bounds__(kThreads) cc_rank_roots(const uint32_t *par, uint32_t n, const uint32_t *offsets,
-                                                          uint32_t *labels) {
+                                                          const uint32_t *counts, uint32_t *total, uint32_t *labels) {
     pdl_wait();
     __shared__ uint32_t sh[32];
+    __shared__ uint32_t s_before;
+    if (kOwn) {
+        uint32_t x = 0;
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kThreads) x += counts[t];
+        x = block_sum(x, sh);
+        if (threadIdx.x == 0) {
+            s_before = x;
+            if (blockIdx.x == gridDim.x - 1) *total = x + counts[blockIdx.x];
+        }
+        __syncthreads();
+    }
+    if (!labels) return;
     const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)threadIdx.x * kTileItems;
     uint32_t flags = 0, c = 0;
 #pragma unroll
@@ -515,19 +671,57 @@ __global__ void __launch_bounds__(kThreads) cc_rank_roots(const uint32_t *par, u
         sh[l] = t;
     }
     __syncthreads();
-    uint32_t r = offsets[blockIdx.x] + (w ? sh[w - 1] : 0) + s - c;
+    uint32_t r = (kOwn ? s_before : offsets[blockIdx.x]) + (w ? sh[w - 1] : 0) + s - c;
 #pragma unroll
     for (int k = 0; k < kTileItems; k++) {
         if ((flags >> k) & 1u) labels[base + k] = r++;
     }
 }
 
-__global__ void cc_label_all(const uint32_t *par, uint32_t n, uint32_t *labels) {
+// Every other vertex takes its root's label (4 vertices per thread, their parents and grandparents
+// requested together; a vertex further down writes its root back, which shortens the walks of others).
+__global__ void __launch_bounds__(kThreads) cc_label_all(uint32_t *par, uint32_t n, uint32_t *labels) {
     pdl_wait();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t r = par[i];
-        if (r != i) labels[i] = labels[r];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
+        uint32_t p[4], r[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) p[k] = i0 + (uint64_t)k * stride < n ? par[i0 + k * stride] : 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) r[k] = par[p[k]];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+            if (r[k] != p[k]) r[k] = find_root_ro(par, r[k]);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t i = i0 + k * stride;
+            if (i0 + (uint64_t)k * stride >= n || r[k] == i) continue;
+            if (r[k] != p[k]) par[i] = r[k];
+            labels[i] = labels[r[k]];
+        }
     }
+}
+
+// Count and labels of a finished forest. Up to kOwnTiles tiles each ranking CTA sums the counts before
+// its own (saves a launch; the sums together read ntiles^2 / 2 counts).
+constexpr uint32_t kOwnTiles = 4096;
+int label_components(int sms, uint32_t *par, uint32_t n, uint32_t ntiles, uint32_t *counts, uint32_t *offsets,
+                     uint32_t *total, uint32_t *labels, cudaStream_t s) {
+    const uint32_t *cpar = par, *ccounts = counts, *coffsets = offsets;
+    CAC_CUDA_TRY(launch_pdl(cc_count_roots, ntiles, kThreads, 0, s, cpar, n, counts));
+    if (ntiles <= kOwnTiles) {
+        CAC_CUDA_TRY(launch_pdl(cc_rank_roots<true>, ntiles, kThreads, 0, s, cpar, n, coffsets, ccounts, total, labels));
+    } else {
+        CAC_CUDA_TRY(launch_pdl(cc_scan_tiles, 1, 1024, 0, s, ccounts, offsets, ntiles, total));
+        if (labels)
+            CAC_CUDA_TRY(launch_pdl(cc_rank_roots<false>, ntiles, kThreads, 0, s, cpar, n, coffsets, ccounts, total, labels));
+    }
+    if (labels) {
+        const uint64_t blocks = ((uint64_t)n + 4 * kThreads - 1) / (4 * kThreads);
+        CAC_CUDA_TRY(launch_pdl(cc_label_all, (unsigned)std::min<uint64_t>(blocks, (uint64_t)sms * 8), kThreads, 0, s, par, n,
+                                labels));
+    }
+    return CAC_OK;
 }
 
 // CTAs of cc_compress_giant_bitmap: two per SM (kGiantSample threads each), fewer for small n.
@@ -543,9 +737,7 @@ int grid_for(cac_ctx *ctx, uint64_t work, int per_sm) {
 }
 
 void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s) {
-    const uint32_t n4 = n / 4;
-    if (n4) launch_pdl(cc_compress4, grid_for(ctx, n4, 8), kThreads, 0, s, par, n4);
-    if (n & 3) launch_pdl(cc_compress, 1, 32, 0, s, par, 4 * n4, n);
+    launch_pdl(cc_compress4, grid_for(ctx, n / 4, 8), kThreads, 0, s, par, n);
 }
 
 }  // namespace
@@ -634,6 +826,49 @@ int record(cac_ctx *ctx, int i, bool capturing) {
     return CAC_OK;
 }
 
+auto pick_edge_round(bool first, bool check, bool wide) {
+    if (first) return check ? (wide ? cc_edge_round<true, true, kRoundThreads> : cc_edge_round<true, true, kThreads>)
+                            : (wide ? cc_edge_round<true, false, kRoundThreads> : cc_edge_round<true, false, kThreads>);
+    return check ? (wide ? cc_edge_round<false, true, kRoundThreads> : cc_edge_round<false, true, kThreads>)
+                 : (wide ? cc_edge_round<false, false, kRoundThreads> : cc_edge_round<false, false, kThreads>);
+}
+
+unsigned round_grid(cac_ctx *ctx, uint64_t warps, int threads = kRoundThreads) {
+    const uint64_t per = threads / 32;
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((warps + per - 1) / per, (uint64_t)ctx->num_sms * 2048 / threads));
+}
+
+// Forest building without draws (every rank returns its whole slice): the rounds of kRoundDegree on
+// parts of the edges; where these take all edges before a giant component forms, one more round over all
+// of them, after which some hundred of 375,000 edges are left to the union walks (counted on G(300000, M),
+// average degree 2.5; 104,000 without it). Bound by the kernel boundaries (a round and its compression
+// take 6 us each). Measured against one pass of union walks: G(300000, M) of average degree 2.5 166 ->
+// 90 us a query, G(10^6, M) of degree 3 863 -> 127, of degree 1.5 153 -> 175; a path of 300,000 vertices
+// numbered along it 217 -> 151.
+int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
+    const double degree = 2.0 * (double)L.m / L.n;
+    if (L.m < kRoundEdges || degree < 1) return CAC_OK;
+    auto round = [&](uint32_t from, uint32_t to) -> int {
+        const uint64_t warps = (L.m / 256 / kRoundParts + 1) * (to - from);
+        const bool wide = warps >= (uint64_t)ctx->num_sms * (kRoundThreads / 32), first = from == 0 && to < kRoundParts;
+        const int threads = wide ? kRoundThreads : kThreads;
+        auto kern = pick_edge_round(first, L.check, wide);
+        CAC_CUDA_TRY(launch_pdl(kern, round_grid(ctx, warps, threads), threads, 0, s, L.par, L.u, L.v, L.m, from, to, L.n, L.err));
+        compress_all(ctx, L.par, L.n, s);
+        return CAC_OK;
+    };
+    double upto = 0;
+    uint32_t to = 0;
+    for (double d : kRoundDegree) {
+        upto += d;
+        const uint32_t from = to;
+        to = std::min(kRoundParts, (uint32_t)std::ceil(kRoundParts * std::min(1.0, upto / degree)));
+        if (to > from) CAC_TRY(round(from, to));
+    }
+    if (to == kRoundParts) CAC_TRY(round(0, kRoundParts));
+    return CAC_OK;
+}
+
 // Enqueues the whole query on the ctx stream (directly, or into a graph being captured).
 int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
     cudaStream_t s = ctx->stream;
@@ -644,25 +879,23 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
     CAC_CUDA_TRY(launch_pdl(cc_init, grid_for(ctx, n, 8), kThreads, 0, s, L.par, n));
     if (L.draws > 0 && m > 0) {
         CAC_CUDA_TRY(cudaMemcpyAsync(L.d_ranks, L.h_ranks, sizeof(RankDesc) * L.ranks, cudaMemcpyHostToDevice, s));
-        // The draws are hooked in the slices of kSliceEighths: forest building from singletons is
-        // the expensive part of CC, and flattening the trees between slices keeps the union walks
-        // of the next slice one or two hops long. (Drawing inside the hooking CTAs instead of in
-        // one kernel up front measured slower: the rank search and the block cipher then sit on
-        // every slice's critical path.)
+        // (Drawing inside the hooking CTAs instead of in one kernel up front measured slower: the rank
+        // search and the block cipher then sit on every round's critical path.)
         CAC_CUDA_TRY(launch_pdl(cc_sample_draws, grid_for(ctx, L.blocks, 8), kThreads, 0, s,
                                 static_cast<const RankDesc *>(L.d_ranks), (int)L.ranks, L.blocks, L.chunks));
-        constexpr uint32_t sub = sizeof(kSliceEighths) / sizeof(kSliceEighths[0]);
-        uint32_t eighths = 0;
-        for (uint32_t k = 0; k < sub; k++) {
-            const uint64_t d0 = L.draws * eighths / 8;
-            eighths += kSliceEighths[k];
-            const uint64_t d1 = L.draws * eighths / 8;
-            if (d1 > d0) {
-                auto hook = L.check ? cc_sample_hook<true> : cc_sample_hook<false>;
-                CAC_CUDA_TRY(launch_pdl(hook, grid_for(ctx, (d1 - d0) * 32, 8), kThreads, 0, s, L.par, L.u, L.v,
-                                        static_cast<const uint64_t *>(L.chunks), d0, d1, n, L.err));
-            }
-            if (k + 1 < sub) compress_all(ctx, L.par, n, s);
+        // the rounds: kRoundDegree, the last one with all draws that are left
+        constexpr uint32_t rounds = sizeof(kRoundDegree) / sizeof(kRoundDegree[0]);
+        uint64_t d1 = 0;
+        double edges = 0;
+        for (uint32_t k = 0; k < rounds && d1 < L.draws; k++) {
+            const uint64_t d0 = d1;
+            edges += kRoundDegree[k] * n / 2;
+            d1 = k + 1 == rounds ? L.draws : std::min<uint64_t>(L.draws, (uint64_t)(edges / kSampleChunk) + 1);
+            auto round = k == 0 ? (L.check ? cc_sample_round<true, true> : cc_sample_round<true, false>)
+                                : (L.check ? cc_sample_round<false, true> : cc_sample_round<false, false>);
+            CAC_CUDA_TRY(launch_pdl(round, round_grid(ctx, (d1 - d0 + 1) / 2), kRoundThreads, 0, s, L.par, L.u, L.v,
+                                    static_cast<const uint64_t *>(L.chunks), d0, d1, n, L.err));
+            if (d1 < L.draws) compress_all(ctx, L.par, n, s);
         }
         CAC_CUDA_TRY(launch_pdl(cc_compress_giant_bitmap, giant_grid(ctx, n), kGiantSample, 0, s, L.par, n, L.giant,
                                 L.bits));
@@ -694,6 +927,7 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
                                                                                        0, s>>>(
                     L.par, L.u + done, L.v + done, m - done, n, L.err);
         } else {
+            CAC_TRY(edge_rounds(ctx, L, s));
             const int grid = grid_for(ctx, (m + 3) / 4, 8);
             auto pass = L.vec ? (L.check ? cc_edge_pass<true, true> : cc_edge_pass<true, false>)
                               : (L.check ? cc_edge_pass<false, true> : cc_edge_pass<false, false>);
@@ -706,15 +940,7 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
     CAC_TRY(record(ctx, 2, capturing));
     // (A single-pass count and rank by decoupled look-back measured slower: BA n=1,024,000 20.4 vs
     // 18.5 us, R-MAT scale 22 48.6 vs 34.0 us for the labelling.)
-    CAC_CUDA_TRY(launch_pdl(cc_finalize_count, L.ntiles, kThreads, 0, s, L.par, n, L.counts));
-    CAC_CUDA_TRY(launch_pdl(cc_scan_tiles, 1, 1024, 0, s, static_cast<const uint32_t *>(L.counts), L.offsets, L.ntiles,
-                            L.total));
-    if (L.labels) {
-        CAC_CUDA_TRY(launch_pdl(cc_rank_roots, L.ntiles, kThreads, 0, s, static_cast<const uint32_t *>(L.par), n,
-                                static_cast<const uint32_t *>(L.offsets), L.labels));
-        CAC_CUDA_TRY(launch_pdl(cc_label_all, grid_for(ctx, n, 8), kThreads, 0, s,
-                                static_cast<const uint32_t *>(L.par), n, L.labels));
-    }
+    CAC_TRY(label_components(ctx->num_sms, L.par, n, L.ntiles, L.counts, L.offsets, L.total, L.labels, s));
     CAC_CUDA_TRY(cudaGetLastError());
     CAC_CUDA_TRY(cudaMemcpyAsync(ctx->pinned_u32, L.total, (kErrWord + 1) * 4, cudaMemcpyDeviceToHost, s));
     CAC_TRY(record(ctx, 3, capturing));
@@ -992,12 +1218,7 @@ int stream_enqueue(cac_ctx *ctx, const StreamLaunch &L, bool capturing) {
     }
     if (!L.filtered) CAC_TRY(record(ctx, 1, capturing));
     CAC_TRY(record(ctx, 2, capturing));
-    cc_finalize_count<<<L.ntiles, kThreads, 0, s>>>(L.par, n, L.counts);
-    cc_scan_tiles<<<1, 1024, 0, s>>>(L.counts, L.offsets, L.ntiles, L.total);
-    if (L.d_labels) {
-        cc_rank_roots<<<L.ntiles, kThreads, 0, s>>>(L.par, n, L.offsets, L.d_labels);
-        cc_label_all<<<grid_for(ctx, n, 8), kThreads, 0, s>>>(L.par, n, L.d_labels);
-    }
+    CAC_TRY(label_components(ctx->num_sms, L.par, n, L.ntiles, L.counts, L.offsets, L.total, L.d_labels, s));
     CAC_CUDA_TRY(cudaGetLastError());
     CAC_CUDA_TRY(cudaMemcpyAsync(ctx->pinned_u32, L.total, (kErrWord + 1) * 4, cudaMemcpyDeviceToHost, s));
     CAC_TRY(record(ctx, 3, capturing));
@@ -1235,12 +1456,7 @@ extern "C" int cac_cc_noalloc(uint32_t n, uint64_t m, const uint32_t *u_dev, con
                                                                                  S->total + kErrWord);
         else cc_edge_pass<false, true><<<grid(m), kThreads, 0, s>>>(S->parent, u_dev, v_dev, m, n, S->total + kErrWord);
     }
-    cc_finalize_count<<<ntiles, kThreads, 0, s>>>(S->parent, n, S->counts);
-    cc_scan_tiles<<<1, 1024, 0, s>>>(S->counts, S->offsets, ntiles, S->total);
-    if (labels_dev) {
-        cc_rank_roots<<<ntiles, kThreads, 0, s>>>(S->parent, n, S->offsets, labels_dev);
-        cc_label_all<<<grid(n), kThreads, 0, s>>>(S->parent, n, labels_dev);
-    }
+    CAC_TRY(label_components(D.sms, S->parent, n, ntiles, S->counts, S->offsets, S->total, labels_dev, s));
     if (num_components_dev) cc_noalloc_count<<<1, 1, 0, s>>>(S->total, num_components_dev);
     CAC_CUDA_TRY(cudaGetLastError());
     return CAC_OK;
