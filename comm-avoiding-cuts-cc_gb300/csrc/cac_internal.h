@@ -159,6 +159,11 @@ CCPlan cc_plan(uint32_t n, uint64_t m, uint32_t ranks);
 // endpoint >= n fails the query with CAC_ERR_INVALID.
 int cc_run(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint32_t *d_v, uint32_t seed,
            uint32_t ranks, uint32_t *d_labels, cac_cc_result *res, bool check_ids = false);
+// The same in one CTA, for graphs that are small by cc_is_small (cc_run takes it by itself); labels to
+// host or device memory.
+bool cc_is_small(uint32_t n, uint64_t m);
+int cc_run_small(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint32_t *d_v, uint32_t *labels,
+                 int labels_where, cac_cc_result *res, bool check_ids);
 size_t cc_scratch_bytes(uint32_t n, uint32_t ranks, uint64_t m);
 // CC of an edge list in host memory: parts copied to d_u/d_v on a second stream while the ctx
 // stream hooks or filters each part that has arrived (cac_cc_edges); labels copied to h_labels.

@@ -560,6 +560,7 @@ int cac_cc(cac_ctx *ctx, const cac_graph *g, uint32_t seed, uint32_t virtual_ran
     }
     CAC_CUDA_TRY(cudaSetDevice(ctx->device));
     if (virtual_ranks == 0) virtual_ranks = 1;
+    if (cc_is_small(g->n, g->m)) return cc_run_small(ctx, g->n, g->m, g->u, g->v, labels, labels_where, res, false);
     uint32_t *d_labels = nullptr;
     if (labels && labels_where == CAC_DEVICE) d_labels = labels;
     if (labels && labels_where == CAC_HOST) {
@@ -609,7 +610,12 @@ int cac_cc_edges(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *u_host, c
             set_error("cac_cc_edges: upload failed");
             st = CAC_ERR_CUDA;
         }
-        if (st == CAC_OK) st = cc_run(ctx, n, m, du, dv, seed, virtual_ranks, labels_host ? dl : nullptr, &r, true);
+        if (st == CAC_OK && cc_is_small(n, m)) {
+            st = cc_run_small(ctx, n, m, du, dv, labels_host, CAC_HOST, &r, true);
+            streamed = true;  // the labels are in place
+        } else if (st == CAC_OK) {
+            st = cc_run(ctx, n, m, du, dv, seed, virtual_ranks, labels_host ? dl : nullptr, &r, true);
+        }
     } else {
         st = cc_run_streamed(ctx, n, m, u_host, v_host, du, dv, labels_host ? dl : nullptr, labels_host, &r);
         streamed = true;

@@ -87,6 +87,11 @@ void finish(cac_server *s, Request *r, int status, const std::string &msg) {
 int run_cc(cac_ctx *ctx, Request *r) {
     const cac_graph *g = r->req.graph;
     cac_cc_result cr{};
+    if (cc_is_small(g->n, g->m)) {
+        CAC_TRY(cc_run_small(ctx, g->n, g->m, g->u, g->v, r->req.labels_host, CAC_HOST, &cr, false));
+        r->resp.num_components = cr.num_components;
+        return CAC_OK;
+    }
     void *d_labels = nullptr;
     if (r->req.labels_host && g->n) CAC_TRY(stream_alloc(ctx, &d_labels, (size_t)g->n * 4));
     int st = cc_run(ctx, g->n, g->m, g->u, g->v, r->req.seed, r->ranks, static_cast<uint32_t *>(d_labels), &cr);

@@ -132,7 +132,9 @@ int cac_cache_convert(const char *input_path, const char *cache_path);
 /* ---- connected components (parallel_cc) ---- */
 typedef struct {
     uint32_t num_components; /* the count parallel_cc prints */
-    uint32_t rounds;         /* sampling rounds + the closing pass over all edges */
+    uint32_t rounds;         /* sampling round (if one ran) + the closing pass over all edges; graphs small
+                                enough for one CTA (up to 16,320 vertices and 65,536 edges) run without
+                                sampling, and all their device time is edge_pass_ms */
     uint64_t sampled_edges;  /* edges drawn in the sampling round */
     float device_ms;         /* device time of the whole call on the ctx stream */
     float edge_pass_ms;      /* device time of the streaming pass over every edge (the loop-dropping
