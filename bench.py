@@ -308,7 +308,7 @@ def run_ks(args, rank, world):
             "dtype": "u64", "data": "synthetic (seeded)", "cut": int(res.cut),
             "config": {"workload": name, "vertices": n, "edges": int(len(u)), "virtual_ranks": ranks,
                        "trials_per_query": res.total_trials, "intermediate_size": res.intermediate,
-                       "quotient_kernel": args.quotient_kernel or "autotuned"},
+                       "quotient_kernel": args.quotient_kernel or "by size"},
             "clocks": clk.summary()}
     peak, peak_kind = _peaks()
     line["work_model"] = _ks_work_model(res.intermediate, res.total_trials / (total_ms / args.steps / 1e3),
@@ -713,7 +713,7 @@ def run_batch(args, rank, world):
             "config": {"workload": "uneven square_root batch", "graphs": r["graphs"], "edges": r["edges"],
                        "trials_per_batch": r["trials_per_batch"], "success_probability": 0.9,
                        "n_range": [64, 8192], "timing": "host wall clock per batch",
-                       "quotient_kernel": args.quotient_kernel or "autotuned"},
+                       "quotient_kernel": args.quotient_kernel or "by size"},
             "queries_per_s": world * r["graphs"] * args.steps / total_s,
             "device_ms_per_batch": r["device_ms_per_batch"], "plain_path_subset": r["plain_path_subset"],
             "results_equal_plain": r["results_equal_plain"], "cuts_exact": r["cuts_exact"],
@@ -879,9 +879,8 @@ def main():
     ap.add_argument("--no-batch", action="store_true", help="skip the batched min-cut measurement")
     ap.add_argument("--no-serve", action="store_true", help="skip the served-stream measurement")
     ap.add_argument("--quotient-kernel", type=int, default=0, choices=[0, 1, 2, 3, 4],
-                    help="ks-er1000 / ks-k4000 / ks-batch / ks-ws32k: 0 autotuned; 1 warp per row, 2 eight warps per row, "
-                         "3 warp per row with bulk-copy staging forced for every Karger-Stein step; 4 the fixed "
-                         "size rule without timing (a profiling aid: under ncu the autotuner's timings are distorted)")
+                    help="ks-er1000 / ks-k4000 / ks-batch / ks-ws32k: 0 and 4 by size; 1 and 3 tiles of output rows, "
+                         "2 eight warps per row forced for every Karger-Stein step")
     args = ap.parse_args()
     if args.steps is None:
         args.steps = {"cc": 20, "cc-rmat22": 20, "ks-batch": 3, "ks-ws32k": 3}.get(args.workload, 10)

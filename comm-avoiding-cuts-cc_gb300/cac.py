@@ -194,8 +194,7 @@ class Context:
         return int(lib().cac_ctx_plan_redos(self.h))
 
     def set_quotient_kernel(self, kind):
-        """0: autotuned; 1 warp per row; 2 eight warps per row; 3 warp per row with bulk-copy staging;
-        4 the fixed size rule (eight warps per row from N = 2000 on), without timing."""
+        """0 and 4: by size; 1 and 3: tiles of output rows; 2: eight warps per output row."""
         _check(lib().cac_ctx_set_quotient_kernel(self.h, kind), "cac_ctx_set_quotient_kernel")
 
     def close(self):

@@ -89,8 +89,7 @@ struct cac_ctx {
     cudaGraphExec_t cc_exec = nullptr;  // its captured launch sequence (second sighting onwards)
     uint32_t *pinned_u32 = nullptr;  // 64 KB pinned staging: [0,256) B scalar results, then descriptors
     void *ks_scratch = nullptr;      // grow-only Karger-Stein scratch buffers (mincut.cu)
-    uint8_t quotient_choice[32] = {};  // autotuned quotient kernel per (N bucket, width); 0: untuned
-    uint8_t quotient_forced = 0;       // a quotient kernel chosen by the caller instead (0: autotuned)
+    uint8_t quotient_forced = 0;       // a quotient kernel chosen by the caller (kQuotient*) instead of by size
     bool plan_ahead = true;            // Karger-Stein levels planned at their target sizes (mincut.cu)
     uint64_t plan_redos = 0;           // runs redone level by level after a child stopped off its target
     cudaStream_t copy_stream = nullptr;  // host-to-device chunks of cac_cc_edges (created on first use)
@@ -265,8 +264,7 @@ inline bool ks_is_dense(const cac_ctx *ctx, uint32_t N, uint64_t m) {
 // are dense join `eng` as matrices, the others are contracted in turn.
 int sparse_phase(cac_ctx *ctx, KsEngine &eng, std::vector<SparseNode> nodes);
 
-// The status and message of a nonzero engine error word (bit 1: a bounded bulk-copy wait ran
-// out; otherwise an inconsistent selection prefix).
+// The status and message of a nonzero engine error word (an inconsistent selection prefix).
 int engine_error(uint32_t err);
 
 struct MincutQuery {
@@ -336,18 +334,11 @@ int merge_edges_multi(cac_ctx *ctx, std::vector<MergeTask> &tasks, uint32_t *oa,
 uint64_t merge_edges_multi_scratch(uint64_t M, uint32_t B);
 int shrink_big(cac_ctx *ctx, const cac_graph *g, uint32_t target, uint32_t B, const uint32_t *k0, const uint32_t *idx,
                uint32_t *d_lab, uint32_t *d_kout, void *scratch);
-// Quotient kernel choices of the autotuner (cac_ctx::quotient_choice), bucketed by
-// floor(log2 N) and entry width.
-constexpr uint8_t kQuotientWarp = 1, kQuotientShared = 2, kQuotientBulk = 3, kQuotientRule = 4;
-// Engine error word bits: 1 an inconsistent selection prefix in a contraction, 2 a bulk-copy wait
-// past its bound, 4 a child planned at its target size that stopped elsewhere (the run is redone
-// without planning ahead)
+// Quotient kernels that a caller can force (cac_ctx_set_quotient_kernel; 0 and 4: by size).
+constexpr uint8_t kQuotientTile = 1, kQuotientShared = 2, kQuotientTileToo = 3;
+// Engine error word bits: 1 an inconsistent selection prefix in a contraction, 4 a child planned at
+// its target size that stopped elsewhere (the run is redone without planning ahead)
 constexpr uint32_t kErrPlan = 4u;
-inline int quotient_bucket(uint32_t N, bool small) {
-    int b = 0;
-    while ((N >> (b + 1)) != 0 && b < 15) b++;
-    return 2 * b + (small ? 1 : 0);
-}
 // Frees the ctx's grow-only Karger-Stein scratch (cac_ctx_destroy).
 void ctx_scratch_free(cac_ctx *ctx);
 // All trials of all queries through one engine, admitted as memory allows.

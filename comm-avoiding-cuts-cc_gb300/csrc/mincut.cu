@@ -17,11 +17,10 @@
 //                                column by block prefix + a 32-entry scan), contraction in draw
 //                                order until max(ceil(n/sqrt 2)+1, 128) vertices, labels by rank
 //                                of the smallest member, member lists by counting sort
-//              quotient_warp_kernel / quotient_shared_row_kernel
-//                                the child's matrix: member rows summed, every column added into
-//                                its label's slot of the output row in shared memory (integer
-//                                atomics); a warp per output row, or a CTA's 8 warps on one row at
-//                                large N (autotuned per size bucket)
+//              quotient_tile_kernel / quotient_shared_row_kernel
+//                                the child's matrix: a few output rows at a time as one tile in shared
+//                                memory, member rows summed on the way in, joined columns added to their
+//                                groups' first ones, those stored; at large N a CTA per output row
 //              sw_leaf_kernel    one 128-thread CTA per leaf (n <= 128), a thread per vertex:
 //                                Stoer-Wagner maximum-adjacency
 //                                phases with Nagamochi-Ono-Ibaraki contractions on the matrix held
@@ -42,7 +41,6 @@
 namespace cac {
 namespace {
 
-constexpr uint32_t kSharedRowMinN = 2000;  // before tuning: quotient steps from this N on use the shared-row kernel
 constexpr uint32_t kSharedRows = 8;         // output rows per CTA of the shared-row quotient
 
 constexpr uint32_t kMaxSmemVertices = kMaxDenseVertices;  // union-find of a contraction held in shared memory
@@ -86,9 +84,11 @@ struct SrcDesc {
 struct TaskDesc {
     uint64_t tag;         // stream key word 2 (1 + heap index)
     uint64_t *cut;        // the trial's cut
-    uint32_t *lab;        // N labels (output)
-    uint32_t *memb_off;   // k + 1 offsets (output)
-    uint32_t *members;    // N vertices grouped by label (output)
+    uint16_t *lab;        // N labels (output; all vertices and counts are at most 16384)
+    uint16_t *memb_off;   // k + 1 offsets (output)
+    uint16_t *members;    // N vertices grouped by label, each group's smallest first (output)
+    uint16_t *cols;       // the quotient's column lists (output, see kColHead)
+    uint32_t *rows;       // k: label | member offset << 16, by falling group size (output)
     uint32_t src;         // index into the SrcDesc array
     uint32_t target;
     uint32_t round;
@@ -112,6 +112,20 @@ struct LeafDesc {
 // Row stride of an N x N node matrix: N rounded up to a multiple of 4 entries, so that every row
 // starts on a 16-byte boundary (16-byte loads). Entries past column N - 1 are never used.
 __host__ __device__ __forceinline__ uint64_t ld_of(uint32_t N) { return ((uint64_t)N + 3) & ~(uint64_t)3; }
+
+// Column lists that a contraction leaves for the quotient, u16 entries:
+//   [0, kEll)  joined[j]: how many small groups have more than j members beside their first
+//   [kColMulti], [kColBig], [kColEll]  small groups with joined members, big groups, list entries
+//   from kColHead: the k groups' first (smallest) vertices in label order; then, list by list
+//   j = 0 .. kEll - 1, the joined[j] small groups' member j + 1 (groups by falling size, so that the
+//   groups still going are a prefix); then the small groups' first vertices in the same order. Each
+//   part is padded to an even count. Big groups have more than kEll members beside their first.
+constexpr uint32_t kEll = 32, kColMulti = 32, kColBig = 33, kColEll = 34, kColHead = 64;
+// u32 words of a contraction's output arrays: rows, then lab, members, memb_off and cols (u16)
+__host__ __device__ __forceinline__ uint32_t even16(uint32_t x) { return (x + 1) / 2; }
+inline uint32_t task_words(uint32_t N) {
+    return N + 2 * even16(N) + even16(N + 1) + even16(kColHead + N + N / 2 + 4);
+}
 
 template <typename Tm>
 __device__ __forceinline__ bool width_is(uint32_t small) {
@@ -248,15 +262,15 @@ __device__ __forceinline__ uint64_t upper_bound_u64(const uint64_t *a, uint64_t 
 
 // Rank-of-minimum relabel of a compressed min-linked union-find (roots are minima): roots get
 // their rank in vertex order, every vertex its root's label. Writes `lab` (global).
-template <int NT>
-__device__ void rank_labels(const uint32_t *par, uint32_t n, uint32_t *lab) {
+template <int NT, typename LabT>
+__device__ void rank_labels(const uint32_t *par, uint32_t n, LabT *lab) {
     uint32_t off = 0;
     for (uint32_t base = 0; base < n; base += NT) {
         const uint32_t v = base + threadIdx.x;
         const uint32_t f = (v < n && par[v] == v) ? 1u : 0u;
         uint32_t tot;
         const uint32_t r = block_excl_scan_u32<NT>(f, tot);
-        if (f) lab[v] = off + r;
+        if (f) lab[v] = (LabT)(off + r);
         off += tot;
     }
     __syncthreads();
@@ -516,30 +530,442 @@ __global__ void __launch_bounds__(NT) contract_kernel(const TaskDesc *__restrict
     __syncthreads();
     rank_labels<NT>(par, N, T.lab);
     const uint32_t k = s_count;
-    // member lists grouped by label (counting sort; order inside a group is irrelevant)
+    // member lists grouped by label, and the quotient's row order and column lists (order inside a group
+    // is irrelevant): cnt[l] first counts the group's members beside its first
+    __shared__ uint32_t s_hist[kEll + 2], s_pos[kEll + 2], s_off[kEll], s_base[2];
+    if (threadIdx.x < kEll + 2) s_hist[threadIdx.x] = 0;
     for (uint32_t l = threadIdx.x; l < k; l += NT) cnt[l] = 0;
     __syncthreads();
-    for (uint32_t v = threadIdx.x; v < N; v += NT) atomicAdd(&cnt[T.lab[v]], 1u);
+    for (uint32_t v = threadIdx.x; v < N; v += NT)
+        if (par[v] != v) atomicAdd(&cnt[T.lab[v]], 1u);
     __syncthreads();
     uint32_t off = 0;
     for (uint32_t base = 0; base < k; base += NT) {
         const uint32_t l = base + threadIdx.x;
         const uint32_t x = l < k ? cnt[l] : 0;
         uint32_t tot;
-        const uint32_t ex = block_excl_scan_u32<NT>(x, tot);
-        if (l < k) {
-            T.memb_off[l] = off + ex;
-            cnt[l] = off + ex;  // becomes the scatter cursor
-        }
+        const uint32_t ex = block_excl_scan_u32<NT>(l < k ? x + 1 : 0, tot);
+        if (l < k) T.memb_off[l] = (uint16_t)(off + ex);
+        if (x) atomicAdd(&s_hist[min(x, kEll + 1)], 1u);
         off += tot;
     }
-    if (threadIdx.x == 0) T.memb_off[k] = N;
+    if (threadIdx.x == 0) T.memb_off[k] = (uint16_t)N;
+    __syncthreads();
+    const uint32_t nbig = s_hist[kEll + 1], lane = threadIdx.x & 31;
+    if (threadIdx.x < kEll) {  // joined[j] = small groups with more than j: a suffix sum over the warp's lanes
+        const uint32_t j = threadIdx.x;
+        uint32_t joined = s_hist[j + 1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_down_sync(0xffffffffu, joined, o);
+            if (j + o < 32) joined += y;
+        }
+        uint32_t incl = joined;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)j >= o) incl += y;
+        }
+        const uint32_t nell = __shfl_sync(0xffffffffu, incl, 31), nmulti = __shfl_sync(0xffffffffu, joined, 0);
+        s_off[j] = incl - joined;
+        s_pos[j] = joined;  // the small groups with exactly j joined members follow those with more
+        T.cols[j] = (uint16_t)joined;
+        if (j == 0) {
+            s_pos[kEll] = 0;
+            s_pos[kEll + 1] = 0;            // big groups: the head of the row order
+            s_pos[0] = nbig + nmulti;       // single vertices: its tail
+            T.cols[kColMulti] = (uint16_t)nmulti;
+            T.cols[kColBig] = (uint16_t)nbig;
+            T.cols[kColEll] = (uint16_t)nell;
+            s_base[0] = kColHead + ((k + 1) & ~1u);
+            s_base[1] = s_base[0] + ((nell + 1) & ~1u);
+        }
+    }
+    __syncthreads();
+    uint16_t *first = T.cols + kColHead, *ell = T.cols + s_base[0], *multi = T.cols + s_base[1];
+    for (uint32_t base = 0; base < k; base += NT) {
+        const uint32_t l = base + threadIdx.x;
+        const uint32_t x = l < k ? cnt[l] : 1u;
+        const uint32_t single = __ballot_sync(0xffffffffu, x == 0);  // most groups: one atomic per warp
+        uint32_t at = 0, pos = 0xFFFFu;
+        if (lane == 0 && single) at = atomicAdd(&s_pos[0], (uint32_t)__popc(single));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(single & ((1u << lane) - 1));
+        if (l < k) {
+            if (x > kEll) at = atomicAdd(&s_pos[kEll + 1], 1u);
+            else if (x) at = nbig + (pos = atomicAdd(&s_pos[x], 1u));
+            T.rows[at] = l | (uint32_t)T.memb_off[l] << 16;
+            cnt[l] = pos << 16;  // becomes (position among the small groups, scatter cursor)
+        }
+    }
     __syncthreads();
     for (uint32_t v = threadIdx.x; v < N; v += NT) {
-        const uint32_t p = atomicAdd(&cnt[T.lab[v]], 1u);
-        T.members[p] = v;
+        const uint32_t l = T.lab[v], at = T.memb_off[l];
+        if (par[v] == v) {
+            T.members[at] = (uint16_t)v;
+            first[l] = (uint16_t)v;
+            const uint32_t pos = cnt[l] >> 16;
+            if (pos != 0xFFFFu) multi[pos] = (uint16_t)v;
+        } else {
+            const uint32_t c = atomicAdd(&cnt[l], 1u), rank = c & 0xFFFFu, pos = c >> 16;
+            T.members[at + 1 + rank] = (uint16_t)v;
+            if (pos != 0xFFFFu) ell[s_off[rank] + pos] = (uint16_t)v;
+        }
     }
     if (threadIdx.x == 0) k_out[blockIdx.x] = k;
+}
+
+// ---------------------------------------------------------------- quotient
+// Q[a][b] = sum over u in group a, v in group b of A[u][v], the diagonal zeroed, with every row's
+// 32-column block prefixes and its sum (the next step's row prep). Two kernels with identical results:
+// tiles of R rows (quotient_tile_kernel) up to kTileMaxN source vertices, one row per CTA
+// (quotient_shared_row_kernel) above.
+//
+// R output rows make a tile: R rows of N entries in shared memory, so that every column index is
+// read once for R rows. The rows of a tile are interleaved in 16-byte chunks (a column's R entries
+// are a constant distance apart, so one address serves R loads), for R = 4 with a spare chunk after
+// each 4 so that neighbouring chunks of a row start in different banks. A CTA of 8 warps works on 8, 4, 2
+// or 1 tiles at a time, 1, 2, 4 or 8 warps on each; tiles are taken from the CTA's share as warps get
+// free. Per tile:
+//   1. the first member row of each output row is copied in asynchronously (16 bytes per copy), the
+//      other members are summed in registers meanwhile, 8 loads in flight, and added (each thread to
+//      the columns that it copied);
+//   2. every joined column is added to its group's first column: a thread per small group walks the
+//      lists of cols (no atomics), a warp per big group sums its members;
+//   3. the groups' first columns are the output row: first[b] grows with b, so the tile is read nearly
+//      in order and each lane stores 4 columns of each row with 16-byte stores; 8 lanes make a
+//      32-column block sum;
+//   4. the block sums become prefixes.
+// Weighted contraction makes groups of hundreds of members at the deeper levels, so the rows are dealt
+// out by falling group size: the R rows of a tile from R different parts of the order, the tiles of a
+// CTA from all over it, the largest first.
+// Bound by latency within each step (loads of step 1, index -> entry chains of 2 and 3): its steps
+// alone take 150 us (1) and 160 us (2 to 4) of the 340 at N = 356, where the bytes read and written
+// take 135 of HBM's time. The forms that this replaces added every source column into its label's slot
+// with a shared atomic. Measured on the levels of a recursion from K4000 (7 trials; us per level of
+// 225 M source entries, contraction drawn by weight), old -> new: N = 182 755 -> 386, 253 540 -> 308,
+// 356 473 -> 341, 709 552 -> 357, 1416 750 -> 477, 2830 553 -> 511; at 4000 one row per CTA takes 340.
+constexpr uint32_t kTileThreads = 256;
+constexpr uint32_t kTileRows = 256;      // most output rows per CTA
+constexpr uint32_t kTileSmem = 74 * 1024;  // three CTAs per SM
+constexpr uint32_t kTileMaxN = 2900;
+
+struct TilePlan {
+    uint32_t rows;   // R
+    uint32_t esize;  // bytes of an entry
+    uint32_t smem;   // bytes of shared memory per CTA
+    uint32_t tiles;  // tiles per group of warps
+};
+
+__host__ __device__ __forceinline__ uint32_t first_pad(uint32_t k) { return (k + 127) & ~127u; }
+// the lists: header, first (padded), joined columns (at most two entries each)
+__host__ __device__ __forceinline__ uint32_t tile_idx_bytes(uint32_t N, uint32_t k) {
+    return (kColHead * 2 + first_pad(k) * 2 + (N - k + 2) * 4 + 15) & ~15u;
+}
+// one tile: its chunks and one of zeros, the block sums of its rows and their diagonal entries
+__host__ __device__ __forceinline__ uint32_t tile_bytes(uint32_t N, uint32_t rows, uint32_t esize) {
+    const uint32_t chunk = 16 * (rows == 4 ? 5 : rows);
+    return (uint32_t)(ld_of(N) * esize / 16 + 1) * chunk + ((rows * ((N + 31) / 32 + 1) * esize + 15) & ~15u);
+}
+// tiles at a time: the most of 8, 4, 2, 1 that fit `smem`
+__host__ __device__ __forceinline__ uint32_t tile_groups(uint32_t N, uint32_t k, const TilePlan &p, uint32_t smem) {
+    const uint32_t idx = tile_idx_bytes(N, k), one = tile_bytes(N, p.rows, p.esize);
+    const uint32_t room = smem > idx ? smem - idx : 0;
+    return room >= 8 * one ? 8u : room >= 4 * one ? 4u : room >= 2 * one ? 2u : 1u;
+}
+
+// tiles per CTA
+__host__ __device__ __forceinline__ uint32_t tile_per_cta(uint32_t groups, const TilePlan &p) {
+    return groups * p.tiles < kTileRows / p.rows ? groups * p.tiles : kTileRows / p.rows;
+}
+
+// One child of a launch.
+struct TileTask {
+    const void *mat;          // N x N
+    const uint16_t *cols, *members, *memb_off;
+    const uint32_t *rows;
+    void *q;                  // k x k
+    uint64_t *rowsum;         // k row sums, then k x ceil(k / 32) block prefixes
+    const uint32_t *kact;     // planned ahead: the contraction's own count, else null
+    uint32_t N, k;
+};
+struct TileArgs {
+    const TileTask *task;
+    const uint64_t *first;    // their first CTAs
+    uint32_t ntasks, uniform; // uniform: CTAs of every task where all have the same number, else 0
+    uint32_t *err;
+    TilePlan plan;
+};
+
+// last i of [0, n) with first[i] <= x (first[0] = 0), by a warp: 32 probes per step
+__device__ __forceinline__ uint32_t warp_last_le(const uint64_t *__restrict__ first, uint32_t n, uint64_t x) {
+    uint32_t lo = 0, len = n;  // the answer is in [lo, lo + len)
+    while (len > 1) {
+        const uint32_t step = (len + 31) / 32, at = lo + step * (threadIdx.x & 31);
+        const uint32_t hits = __popc(__ballot_sync(0xffffffffu, at < lo + len && first[at] <= x));
+        const uint32_t end = lo + len;
+        lo += (hits - 1) * step;
+        len = min(step, end - lo);
+    }
+    return lo;
+}
+
+// asynchronous copy of 16 bytes to shared memory, past L1
+__device__ __forceinline__ void copy16_async(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+__device__ __forceinline__ void vadd(uint4 &a, const uint4 &b) {
+    a.x += b.x;
+    a.y += b.y;
+    a.z += b.z;
+    a.w += b.w;
+}
+__device__ __forceinline__ void vadd(ulonglong2 &a, const ulonglong2 &b) {
+    a.x += b.x;
+    a.y += b.y;
+}
+
+__device__ __forceinline__ void tile_sync(uint32_t group, uint32_t warps) {  // the warps of one tile
+    if (warps == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(warps * 32) : "memory");
+}
+
+template <typename Tm, int R>
+__global__ void __launch_bounds__(kTileThreads, 3) quotient_tile_kernel(const __grid_constant__ TileArgs A) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    using Vec = typename std::conditional<sizeof(Tm) == 4, uint4, ulonglong2>::type;
+    constexpr uint32_t VEC = 16 / sizeof(Tm);        // columns per chunk
+    constexpr uint32_t CS = VEC * (R == 4 ? 5 : R);  // entries from a chunk to the next of its row
+    __shared__ uint32_t s_take[8], s_next;
+    __shared__ uint32_t s_row[kTileRows][2];  // label | members << 16, first member position
+    const uint32_t li = A.uniform ? blockIdx.x / A.uniform : warp_last_le(A.first, A.ntasks, blockIdx.x);
+    const uint32_t cta = A.uniform ? blockIdx.x - li * A.uniform : (uint32_t)(blockIdx.x - A.first[li]);
+    const TileTask T = A.task[li];
+    const uint32_t k = T.k, N = T.N;
+    if (T.kact && *T.kact != k) {  // planned ahead, and this child stopped off its target: redo the run
+        if (threadIdx.x == 0) atomicOr(A.err, kErrPlan);
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t ldN = ld_of(N), ldk = ld_of(k);
+    const uint32_t nch = (uint32_t)(ldN / VEC), nbk = (k + 31) / 32;
+    const uint32_t groups = tile_groups(N, k, A.plan, A.plan.smem), wpt = 8 / groups;  // warps per tile
+    const uint32_t grp = warp / wpt, wl = warp % wpt, tl = wl * 32 + lane, tt = wpt * 32;
+    const Tm *__restrict__ mat = reinterpret_cast<const Tm *>(T.mat);
+    // a vertex as an entry offset in the tile (below 2^16)
+    auto slot = [](uint32_t c) { return c + c / VEC * (CS - VEC); };
+    uint16_t *s_cols = reinterpret_cast<uint16_t *>(dsm), *s_first = s_cols + kColHead;
+    const uint32_t kpad = first_pad(k);
+    const uint32_t nmulti = T.cols[kColMulti], nbig = T.cols[kColBig], nell = T.cols[kColEll];
+    uint16_t *s_ell = s_first + kpad, *s_multi = s_ell + ((nell + 1) & ~1u);
+    // this CTA's tiles: cta, cta + ctas, ...; tile t has the rows at t, t + ntiles, ... of the order
+    const uint32_t ntiles = (k + R - 1) / R, per = tile_per_cta(groups, A.plan), ctas = (ntiles + per - 1) / per;
+    for (uint32_t i = threadIdx.x; i < kColHead; i += kTileThreads) s_cols[i] = T.cols[i];
+    for (uint32_t i = threadIdx.x; i < kpad; i += kTileThreads)  // (padded with the chunk of zeros)
+        s_first[i] = (uint16_t)slot(i < k ? T.cols[kColHead + i] : (uint32_t)ldN);
+    {
+        const uint16_t *ell = T.cols + kColHead + ((k + 1) & ~1u);
+        for (uint32_t i = threadIdx.x; i < ((nell + 1) & ~1u) + nmulti; i += kTileThreads) s_ell[i] = (uint16_t)slot(ell[i]);
+    }
+    for (uint32_t i = threadIdx.x; i < per * R; i += kTileThreads) {
+        const uint32_t t = i / R * ctas + cta, at = t + i % R * ntiles;
+        if (t >= ntiles) break;
+        const uint32_t x = T.rows[at < k ? at : t], l = x & 0xFFFFu;  // (a repeated row stores the same again)
+        s_row[i][0] = l | (uint32_t)(T.memb_off[l + 1] - T.memb_off[l]) << 16;
+        s_row[i][1] = x >> 16;
+    }
+    if (threadIdx.x == 0) s_next = 0;
+    // entry of row r at offset x: tile[x + r * VEC]
+    Tm *tile = reinterpret_cast<Tm *>(dsm + tile_idx_bytes(N, k) + (size_t)grp * tile_bytes(N, R, sizeof(Tm)));
+    Tm *bsum = tile + (nch + 1) * CS, *sdiag = bsum + R * nbk;
+    if (tl < R * VEC) tile[nch * CS + tl] = 0;
+    Tm *Q = reinterpret_cast<Tm *>(T.q);
+    uint64_t *blk = T.rowsum + k;
+    __syncthreads();
+    for (uint32_t it = 0;; it++) {
+        uint32_t mine = it;
+        if (wpt == 1) {
+            if (lane == 0) mine = atomicAdd(&s_next, 1u);
+            mine = __shfl_sync(0xffffffffu, mine, 0);
+        } else if (wpt < 8) {
+            if (tl == 0) s_take[grp] = atomicAdd(&s_next, 1u);
+            tile_sync(grp, wpt);
+            mine = s_take[grp];
+        }
+        if (mine >= per || mine * ctas + cta >= ntiles) break;
+        // 1. member rows
+        uint32_t lab[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            lab[r] = s_row[mine * R + r][0] & 0xFFFFu;
+            const uint32_t f = s_first[lab[r]], v = f / CS * VEC + f % CS;  // the slot's vertex
+            const Tm *row = mat + v * ldN + tl * VEC;
+            Tm *dst = tile + tl * CS + r * VEC;
+            for (uint32_t c = tl; c < nch; c += tt, row += tt * VEC, dst += tt * CS) copy16_async(dst, row);
+        }
+        bool waited = false;
+#pragma unroll 1
+        for (int r = 0; r < R; r++) {
+            const uint32_t size = s_row[mine * R + r][0] >> 16;
+            if (size == 1) continue;
+            const uint32_t q0 = s_row[mine * R + r][1] + 1, q1 = q0 + size - 1;
+            for (uint32_t c = tl; c < nch; c += 2 * tt) {
+                const bool two = c + tt < nch;
+                Vec acc[2] = {Vec{}, Vec{}};
+                for (uint32_t p = q0; p < q1; p += 4) {
+                    Vec q[4][2];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        q[u][0] = q[u][1] = Vec{};
+                        if (p + u < q1) {
+                            const Vec *row = reinterpret_cast<const Vec *>(mat + (uint64_t)T.members[p + u] * ldN) + c;
+                            q[u][0] = __ldg(row);
+                            if (two) q[u][1] = __ldg(row + tt);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        vadd(acc[0], q[u][0]);
+                        vadd(acc[1], q[u][1]);
+                    }
+                }
+                if (!waited) {
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    waited = true;
+                }
+                Vec *d = reinterpret_cast<Vec *>(tile + c * CS + r * VEC);
+                Vec x = *d;
+                vadd(x, acc[0]);
+                *d = x;
+                if (two) {
+                    d = reinterpret_cast<Vec *>(tile + (c + tt) * CS + r * VEC);
+                    x = *d;
+                    vadd(x, acc[1]);
+                    *d = x;
+                }
+            }
+        }
+        if (!waited) asm volatile("cp.async.wait_all;" ::: "memory");
+        tile_sync(grp, wpt);
+        // 2. joined columns -> their groups' first columns
+        for (uint32_t i = tl; i < nmulti; i += tt) {
+            Tm *to = tile + s_multi[i];
+            Tm acc[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) acc[r] = to[r * VEC];
+            const uint16_t *list = s_ell + i;
+            const Tm *from = tile + *list;
+            uint32_t joined = nmulti;
+            for (uint32_t j = 1;; j++) {  // the next list entry is read ahead of this one's column
+                list += joined;
+                joined = j < kEll ? s_cols[j] : 0;
+                const bool more = i < joined;
+                const Tm *next = more ? tile + *list : nullptr;
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] += from[r * VEC];
+                if (!more) break;
+                from = next;
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) to[r * VEC] = acc[r];
+        }
+        for (uint32_t i = wl; i < nbig; i += wpt) {  // (the big groups lead the order)
+            const uint32_t x = T.rows[i], l = x & 0xFFFFu, end = T.memb_off[l + 1];
+            Tm acc[R] = {};
+            for (uint32_t p = (x >> 16) + lane; p < end; p += 32) {
+                const Tm *from = tile + slot(T.members[p]);
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] += from[r * VEC];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+            if (lane == 0)
+#pragma unroll
+                for (int r = 0; r < R; r++) tile[s_first[l] + r * VEC] = acc[r];
+        }
+        tile_sync(grp, wpt);
+        // 3. first columns -> output rows and block sums (the diagonal is taken out in step 4)
+        Tm *out[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) out[r] = Q + lab[r] * ldk + lane * 4;
+        for (uint32_t b0 = wl * 128; b0 < k; b0 += tt * 4) {
+            const uint32_t b = b0 + lane * 4;
+            Tm y[R][4];
+            const uint2 f = *reinterpret_cast<const uint2 *>(s_first + b);
+            const uint32_t x[4] = {f.x & 0xFFFFu, f.x >> 16, f.y & 0xFFFFu, f.y >> 16};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const Tm *from = tile + x[i];
+#pragma unroll
+                for (int r = 0; r < R; r++) y[r][i] = from[r * VEC];
+            }
+            Tm sum[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) sum[r] = (y[r][0] + y[r][1]) + (y[r][2] + y[r][3]);
+            if (b < k) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    Tm *q = out[r] + b0;
+                    if constexpr (sizeof(Tm) == 4) {
+                        *reinterpret_cast<uint4 *>(q) = make_uint4(y[r][0], y[r][1], y[r][2], y[r][3]);
+                    } else {
+                        *reinterpret_cast<ulonglong2 *>(q) = make_ulonglong2(y[r][0], y[r][1]);
+                        *reinterpret_cast<ulonglong2 *>(q + 2) = make_ulonglong2(y[r][2], y[r][3]);
+                    }
+                }
+            }
+            // sums over the block's 8 lanes: the rows are halved among the lanes first, so that 4 rows take
+            // 4 shuffles
+            uint32_t row = 0, step = 1;
+            if constexpr (R == 4) {
+                const bool hi = lane & 1u;
+                const Tm s0 = hi ? sum[0] : sum[2], s1 = hi ? sum[1] : sum[3];
+                sum[0] = (hi ? sum[2] : sum[0]) + __shfl_xor_sync(0xffffffffu, s0, 1);
+                sum[1] = (hi ? sum[3] : sum[1]) + __shfl_xor_sync(0xffffffffu, s1, 1);
+                row = hi ? 2 : 0;
+                step = 2;
+            }
+            const bool hi = lane & step;
+            const Tm s0 = hi ? sum[0] : sum[1];
+            sum[0] = (hi ? sum[1] : sum[0]) + __shfl_xor_sync(0xffffffffu, s0, step);
+            row += hi;
+#pragma unroll
+            for (int o = R; o < 8; o *= 2) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+            if ((lane & 7u) < (uint32_t)R && b / 32 < nbk) bsum[row * nbk + b / 32] = sum[0];
+        }
+        if (tl < R) sdiag[tl] = tile[s_first[s_row[mine * R + tl][0] & 0xFFFFu] + tl * VEC];
+        tile_sync(grp, wpt);
+        // 4. block sums -> prefixes: `side` rows side by side in a warp, `width` lanes each
+        const uint32_t width = nbk <= 8 ? 8u : nbk <= 16 ? 16u : 32u, side = 32 / width;
+        for (uint32_t r0 = wl * side; r0 < (uint32_t)R; r0 += wpt * side) {
+            const uint32_t r = r0 + lane / width, j1 = lane % width;
+            const bool has = r < (uint32_t)R;
+            const uint32_t l = has ? s_row[mine * R + r][0] & 0xFFFFu : 0;
+            Tm carry = 0;
+            for (uint32_t j0 = 0; j0 < nbk; j0 += width) {
+                const uint32_t j = j0 + j1;
+                Tm s = 0;
+                if (has && j < nbk) {
+                    s = bsum[r * nbk + j];
+                    if (j == l / 32) {
+                        s -= sdiag[r];
+                        Q[l * ldk + l] = 0;
+                    }
+                }
+                for (uint32_t o = 1; o < width; o <<= 1) {
+                    const Tm y = __shfl_up_sync(0xffffffffu, s, o, width);
+                    if (j1 >= o) s += y;
+                }
+                s += carry;
+                if (has && j < nbk) blk[(uint64_t)l * nbk + j] = s;
+                carry = __shfl_sync(0xffffffffu, s, width - 1, width);
+            }
+            if (has && j1 == 0) T.rowsum[l] = carry;
+        }
+    }
 }
 
 __device__ __forceinline__ void sadd(uint32_t *p, uint64_t v) { atomicAdd(p, (uint32_t)v); }
@@ -548,10 +974,8 @@ __device__ __forceinline__ void sadd(uint64_t *p, uint64_t v) {
 }
 
 // The quotient for large N: one CTA of 8 warps per group of `rows` consecutive output rows, all
-// warps on the same output row at a time. The warp kernel below gives every warp its own k-entry
-// row in shared memory, which at N in the thousands leaves room for only a few warps per SM; here
-// the CTA shares one row (labels + one row: 8 CTAs, 64 warps per SM at N = 4000), and the warps
-// split the columns: 128-column chunks (one 16-byte load per lane), chunk c to warp c mod 8, four
+// warps on the same output row at a time (labels + one row in shared memory: 5 CTAs, 40 warps per SM
+// at N = 4000, where a tile leaves room for 16). The warps split the columns: 128-column chunks (one 16-byte load per lane), chunk c to warp c mod 8, four
 // chunks per warp in flight. Per output row: zero the row, sum the member rows chunk by chunk and
 // add every column into its label's slot (shared atomics), store the row with the diagonal zeroed
 // and its 32-column block sums, then one warp turns the block sums into the block prefixes and the
@@ -560,6 +984,7 @@ __device__ __forceinline__ void sadd(uint64_t *p, uint64_t v) {
 template <typename Ts, typename Tm>
 __global__ void __launch_bounds__(256, 5) quotient_shared_row_kernel(const TaskDesc *__restrict__ tasks,
                                                                   const SrcDesc *__restrict__ srcs,
+                                                                  const uint32_t *__restrict__ list, uint32_t nlist,
                                                                   const uint32_t *__restrict__ kdim,
                                                                   const uint64_t *__restrict__ group_task_off,
                                                                   uint32_t ntasks, uint32_t rows,
@@ -569,11 +994,12 @@ __global__ void __launch_bounds__(256, 5) quotient_shared_row_kernel(const TaskD
                                                                   uint32_t *err) {
     extern __shared__ __align__(16) unsigned char dsm[];
     const uint64_t gg = blockIdx.x;
-    uint32_t lo = 0, hi = ntasks - 1;
-    while (lo < hi) {  // last task whose first row group <= gg
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (group_task_off[mid] <= gg) lo = mid; else hi = mid - 1;
+    uint32_t at = 0, hi = nlist - 1;
+    while (at < hi) {  // last task of the list whose first row group <= gg
+        const uint32_t mid = (at + hi + 1) >> 1;
+        if (group_task_off[mid] <= gg) at = mid; else hi = mid - 1;
     }
+    const uint32_t lo = list[at];
     const TaskDesc T = tasks[lo];
     const SrcDesc S = srcs[T.src];
     const uint32_t k = kdim[lo];
@@ -582,7 +1008,7 @@ __global__ void __launch_bounds__(256, 5) quotient_shared_row_kernel(const TaskD
         return;
     }
     const uint32_t N = S.N;
-    const uint32_t a0 = (uint32_t)(gg - group_task_off[lo]) * rows, a1 = min(k, a0 + rows);
+    const uint32_t a0 = (uint32_t)(gg - group_task_off[at]) * rows, a1 = min(k, a0 + rows);
     if (!width_is<Tm>(S.small)) return;
     const Tm *mat = reinterpret_cast<const Tm *>(S.mat);
     constexpr int VEC = 16 / sizeof(Tm);  // columns per 16-byte load
@@ -671,322 +1097,6 @@ __global__ void __launch_bounds__(256, 5) quotient_shared_row_kernel(const TaskD
             }
             if (lane == 31) rowsum_out[a] = incl;
         }
-    }
-}
-
-// One CTA per group of `rows` consecutive output rows of one child, one warp per output row at a
-// time. The child's labels are staged in shared memory once per CTA. For output row a the warp
-// sums the member rows of group a (lanes stride the columns, eight independent loads in flight
-// each) and adds every column's sum straight into its label's slot of the warp's output row in
-// shared memory (an integer atomic, exact in any order); then it stores the row with the diagonal
-// zeroed, and writes the row's 32-column block prefixes and its sum (the next step's row prep).
-// Shared memory: the labels, then one k-entry row per warp.
-//   Q[a][b] = sum over u in group a, v in group b of A[u][v]
-template <typename Ts, typename Tm>
-__global__ void __launch_bounds__(256) quotient_warp_kernel(const TaskDesc *__restrict__ tasks,
-                                                            const SrcDesc *__restrict__ srcs,
-                                                            const uint32_t *__restrict__ kdim,
-                                                            const uint64_t *__restrict__ group_task_off,
-                                                            uint32_t ntasks, uint32_t rows,
-                                                            const uint64_t *__restrict__ out_off,
-                                                            unsigned char *out_base, uint32_t lab_words,
-                                                            uint32_t kmax, const uint32_t *__restrict__ kact,
-                                                            uint32_t *err) {
-    // out_off[i]: byte offset of task i's matrix; out_off[ntasks + i]: of its row sums and block
-    // prefixes (the next step's row prep)
-    extern __shared__ __align__(16) unsigned char dsm[];
-    const uint64_t gg = blockIdx.x;
-    uint32_t lo = 0, hi = ntasks - 1;
-    while (lo < hi) {  // last task whose first row group <= gg
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (group_task_off[mid] <= gg) lo = mid; else hi = mid - 1;
-    }
-    const TaskDesc T = tasks[lo];
-    const SrcDesc S = srcs[T.src];
-    const uint32_t k = kdim[lo];
-    if (kact && kact[lo] != k) {  // planned ahead, and this child stopped off its target: redo the run
-        if (threadIdx.x == 0) atomicOr(err, kErrPlan);
-        return;
-    }
-    const uint32_t N = S.N;
-    const uint32_t a0 = (uint32_t)(gg - group_task_off[lo]) * rows, a1 = min(k, a0 + rows);
-    if (!width_is<Tm>(S.small)) return;
-    const Tm *mat = reinterpret_cast<const Tm *>(S.mat);
-    constexpr int VEC = 16 / sizeof(Tm);  // columns per 16-byte load
-    using Vec = typename std::conditional<sizeof(Tm) == 4, uint4, ulonglong2>::type;
-    const uint64_t ldN = ld_of(N);
-    uint32_t *s_lab = reinterpret_cast<uint32_t *>(dsm);  // N
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // Ts: uint32_t when the graph's total weight is below 2^32 (every entry and row sum fits)
-    Ts *qrow = reinterpret_cast<Ts *>(dsm + (size_t)lab_words * 4) + (size_t)warp * kmax;
-    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) s_lab[i] = T.lab[i];
-    __syncthreads();
-    Tm *Qt = reinterpret_cast<Tm *>(out_base + out_off[lo]);
-    uint64_t *rowsum_out = reinterpret_cast<uint64_t *>(out_base + out_off[ntasks + lo]);
-    const uint32_t small = S.small;
-    const uint32_t nbk = (k + 31) / 32;
-    uint64_t *blk = rowsum_out + k;
-    // the warp's row is zeroed once here, then by the output pass of every row as it reads it
-    for (uint32_t b = lane; b < k; b += 32) qrow[b] = 0;
-    __syncwarp();
-    for (uint32_t a = a0 + warp; a < a1; a += nw) {
-        const uint32_t p0 = T.memb_off[a], p1 = T.memb_off[a + 1];
-        // 16-byte loads: lane l reads columns j0 + (32 u + l) VEC .. + VEC - 1 (4 loads per pass);
-        // the padding columns of a row are read but never scattered
-        for (uint32_t j0 = 0; j0 < N; j0 += 4 * 32 * VEC) {
-            Tm x[4][VEC];
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int t = 0; t < VEC; t++) x[u][t] = 0;
-            for (uint32_t p = p0; p < p1; p++) {
-                const Vec *row = reinterpret_cast<const Vec *>(mat + (uint64_t)T.members[p] * ldN);
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const uint32_t c = j0 + (u * 32 + lane) * VEC;
-                    if (c < N) {
-                        const Vec q = __ldg(row + c / VEC);
-                        const Tm *e = reinterpret_cast<const Tm *>(&q);
-#pragma unroll
-                        for (int t = 0; t < VEC; t++) x[u][t] += e[t];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int t = 0; t < VEC; t++) {
-                    const uint32_t j = j0 + (u * 32 + lane) * VEC + t;
-                    if (j < N && x[u][t]) sadd(&qrow[s_lab[j]], (uint64_t)x[u][t]);
-                }
-        }
-        __syncwarp();
-        const uint64_t qb = (uint64_t)a * ld_of(k);
-        uint64_t run = 0;
-        for (uint32_t b0 = 0; b0 < k; b0 += 128) {  // four 32-column blocks per pass (warp-uniform trip count)
-            uint64_t acc[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const uint32_t b = b0 + 32 * u + lane;
-                acc[u] = (b < k && b != a) ? (uint64_t)qrow[b] : 0;
-                if (b < k) {
-                    Qt[qb + b] = (Tm)acc[u];
-                    qrow[b] = 0;  // for the next row (the warp barrier after this row orders it)
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (small) {  // every entry < 2^32: two 32-bit reductions of the 16-bit halves are exact
-                    const uint32_t lo16 = __reduce_add_sync(0xffffffffu, (uint32_t)(acc[u] & 0xFFFFu));
-                    const uint32_t hi16 = __reduce_add_sync(0xffffffffu, (uint32_t)(acc[u] >> 16));
-                    acc[u] = (uint64_t)lo16 + ((uint64_t)hi16 << 16);
-                } else {
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (b0 + 32 * u < k) {
-                    run += acc[u];
-                    if (lane == u) blk[(uint64_t)a * nbk + (b0 >> 5) + u] = run;
-                }
-            }
-        }
-        if (lane == 0) rowsum_out[a] = run;
-        __syncwarp();
-    }
-}
-
-// ---------------------------------------------------------------- bulk-copy quotient
-// The warp-per-row quotient with its member rows staged in shared memory by the bulk-copy (TMA)
-// engine instead of loaded into registers: every warp walks its stream of (output row a, member u)
-// pairs; while it adds row u of the source into its label slots from shared memory, the copy
-// engine already fetches the next member row into the warp's other buffer (one 1-D
-// cp.async.bulk per row, completion counted on an mbarrier per buffer). So a warp always has a
-// whole row in flight, and its registers hold no row data. Rows start on 16-byte boundaries (ld_of
-// pads every row to 4 entries) and their length is a multiple of 16 bytes, as the bulk copy needs.
-// Every wait on an mbarrier is bounded: when the bound is reached the kernel sets bit 1 of the
-// engine's error word, waits (bounded again) for the copies it still has in flight and returns.
-constexpr uint32_t kBulkSpin = 1u << 20;  // bound on one mbarrier wait (polls with a short sleep)
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-
-// lane 0: one bulk copy of `bytes` from global `src` into shared `dst`, completing on `bar`
-__device__ __forceinline__ void bulk_row(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-
-// wait until the barrier's phase `parity` has completed; false when the bound ran out
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kBulkSpin; i++) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(smem_addr(bar)), "r"(parity)
-            : "memory");
-        if (done) return true;
-        __nanosleep(32);
-    }
-    return false;
-}
-
-template <typename Ts, typename Tm>
-__global__ void __launch_bounds__(256) quotient_bulk_kernel(const TaskDesc *__restrict__ tasks,
-                                                            const SrcDesc *__restrict__ srcs,
-                                                            const uint32_t *__restrict__ kdim,
-                                                            const uint64_t *__restrict__ group_task_off,
-                                                            uint32_t ntasks, uint32_t rows,
-                                                            const uint64_t *__restrict__ out_off,
-                                                            unsigned char *out_base, uint32_t lab_words,
-                                                            uint32_t kmax, uint32_t row_words, uint32_t *err,
-                                                            const uint32_t *__restrict__ kact) {
-    extern __shared__ __align__(16) unsigned char dsm[];  // bulk copies need 16-byte alignment
-    const uint64_t gg = blockIdx.x;
-    uint32_t lo = 0, hi = ntasks - 1;
-    while (lo < hi) {  // last task whose first row group <= gg
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (group_task_off[mid] <= gg) lo = mid; else hi = mid - 1;
-    }
-    const TaskDesc T = tasks[lo];
-    const SrcDesc S = srcs[T.src];
-    const uint32_t k = kdim[lo];
-    if (kact && kact[lo] != k) {  // planned ahead, and this child stopped off its target: redo the run
-        if (threadIdx.x == 0) atomicOr(err, kErrPlan);
-        return;
-    }
-    const uint32_t N = S.N;
-    const uint32_t a0 = (uint32_t)(gg - group_task_off[lo]) * rows, a1 = min(k, a0 + rows);
-    if (!width_is<Tm>(S.small)) return;
-    const Tm *mat = reinterpret_cast<const Tm *>(S.mat);
-    constexpr int VEC = 16 / sizeof(Tm);
-    using Vec = typename std::conditional<sizeof(Tm) == 4, uint4, ulonglong2>::type;
-    const uint64_t ldN = ld_of(N);
-    const uint32_t row_bytes = (uint32_t)(ldN * sizeof(Tm));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // shared memory: 16 mbarriers | labels | per warp: two row buffers, then its k-entry row
-    uint64_t *bars = reinterpret_cast<uint64_t *>(dsm);
-    uint32_t *s_lab = reinterpret_cast<uint32_t *>(dsm + 128);
-    const size_t per_warp = (((size_t)row_words * sizeof(Tm)) * 2 + (size_t)kmax * sizeof(Ts) + 15) & ~(size_t)15;
-    unsigned char *wbase = dsm + 128 + (((size_t)lab_words * 4 + 15) & ~(size_t)15) + (size_t)warp * per_warp;
-    Tm *const buf0 = reinterpret_cast<Tm *>(wbase);
-    Tm *const buf1 = reinterpret_cast<Tm *>(wbase + (size_t)row_words * sizeof(Tm));
-    Ts *qrow = reinterpret_cast<Ts *>(wbase + (size_t)row_words * sizeof(Tm) * 2);
-    uint64_t *bar = bars + 2 * warp;
-    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) s_lab[i] = T.lab[i];
-    if (lane == 0) {
-        mbar_init(bar, 1);
-        mbar_init(bar + 1, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    Tm *Qt = reinterpret_cast<Tm *>(out_base + out_off[lo]);
-    uint64_t *rowsum_out = reinterpret_cast<uint64_t *>(out_base + out_off[ntasks + lo]);
-    const uint32_t small = S.small;
-    const uint32_t nbk = (k + 31) / 32;
-    uint64_t *blk = rowsum_out + k;
-    // the warp's stream: rows a = a0 + warp, a0 + warp + nw, ...; members p of each row
-    uint32_t a = a0 + warp;
-    if (a >= a1) return;  // no row for this warp (its barriers were never armed)
-    uint32_t p = T.memb_off[a], pend = T.memb_off[a + 1];
-    // per buffer: the phase to wait for next, and whether a copy into it is in flight (bits 0, 1)
-    uint32_t parity = 0, inflight = 1;
-    bool failed = false;
-    if (lane == 0) bulk_row(buf0, mat + (uint64_t)T.members[p] * ldN, row_bytes, bar);
-    for (uint32_t b = lane; b < k; b += 32) qrow[b] = 0;
-    __syncwarp();
-    for (uint32_t item = 0;; item++) {
-        const int cur = item & 1, nxt = cur ^ 1;
-        // the next item of the stream, fetched while this one is added
-        const bool row_done = p + 1 >= pend;
-        uint32_t na = a, np = p + 1, npend = pend;
-        if (row_done) {
-            na = a + nw;
-            if (na < a1) {
-                np = T.memb_off[na];
-                npend = T.memb_off[na + 1];
-            }
-        }
-        const bool has_next = na < a1;
-        if (has_next) {
-            if (lane == 0) bulk_row(nxt ? buf1 : buf0, mat + (uint64_t)T.members[np] * ldN, row_bytes, bar + nxt);
-            inflight |= 1u << nxt;
-        }
-        if (!mbar_wait(bar + cur, (parity >> cur) & 1u)) {
-            failed = true;
-            break;
-        }
-        parity ^= 1u << cur;
-        inflight &= ~(1u << cur);
-        // add the member row into the label slots of the warp's output row
-        const Vec *row = reinterpret_cast<const Vec *>(cur ? buf1 : buf0);
-        for (uint32_t c = lane * VEC; c < N; c += 32 * VEC) {
-            const Vec q = row[c / VEC];
-            const Tm *e = reinterpret_cast<const Tm *>(&q);
-#pragma unroll
-            for (int t = 0; t < VEC; t++)
-                if (c + t < N && e[t]) sadd(&qrow[s_lab[c + t]], (uint64_t)e[t]);
-        }
-        __syncwarp();  // every lane is done with buf[cur] (it is refilled two items on)
-        if (row_done) {
-            // row a is complete: store it with the diagonal zeroed, its block prefixes and its sum
-            const uint64_t qb = (uint64_t)a * ld_of(k);
-            uint64_t run = 0;
-            for (uint32_t b0 = 0; b0 < k; b0 += 128) {
-                uint64_t acc[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const uint32_t b = b0 + 32 * u + lane;
-                    acc[u] = (b < k && b != a) ? (uint64_t)qrow[b] : 0;
-                    if (b < k) Qt[qb + b] = (Tm)acc[u];
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (small) {
-                        const uint32_t lo16 = __reduce_add_sync(0xffffffffu, (uint32_t)(acc[u] & 0xFFFFu));
-                        const uint32_t hi16 = __reduce_add_sync(0xffffffffu, (uint32_t)(acc[u] >> 16));
-                        acc[u] = (uint64_t)lo16 + ((uint64_t)hi16 << 16);
-                    } else {
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (b0 + 32 * u < k) {
-                        run += acc[u];
-                        if (lane == u) blk[(uint64_t)a * nbk + (b0 >> 5) + u] = run;
-                    }
-                }
-            }
-            if (lane == 0) rowsum_out[a] = run;
-            __syncwarp();
-            for (uint32_t b = lane; b < k; b += 32) qrow[b] = 0;
-            __syncwarp();
-        }
-        if (!has_next) break;
-        a = na;
-        p = np;
-        pend = npend;
-    }
-    if (failed) {
-        if (lane == 0) atomicOr(err, 2u);
-        // let the copies still in flight land before the shared memory is released
-        for (int b = 0; b < 2; b++)
-            if ((inflight >> b) & 1u) mbar_wait(bar + b, (parity >> b) & 1u);
     }
 }
 
@@ -1392,10 +1502,7 @@ int KsEngine::read_err(uint32_t *err) {
 }
 
 int engine_error(uint32_t err) {
-    if (err & 2u) {
-        set_error("Karger-Stein quotient: a bulk-copy wait exceeded its bound");
-        return CAC_ERR_TIMEOUT;
-    }
+    (void)err;  // one cause is left (kErrPlan redoes the run instead)
     set_error("inconsistent selection prefix in the contraction kernel");
     return CAC_ERR_CUDA;
 }
@@ -1561,7 +1668,7 @@ int KsEngine::step() {
     uint64_t tscratch = 0;
     uint32_t maxN = 0;
     for (const KTask &t : tasks) {
-        tscratch += 3 * (uint64_t)t.src.N + 1;
+        tscratch += task_words(t.src.N);
         maxN = std::max(maxN, t.src.N);
     }
     CAC_TRY(d_tscratch.ensure(tscratch * 4));
@@ -1578,10 +1685,13 @@ int KsEngine::step() {
         d.k0 = t.src.k0;
         d.idx = t.src.idx;
         d.pad = t.src.small;  // entries (and row sums) below 2^32
-        d.lab = d_tscratch.as<uint32_t>() + ts;
-        d.members = d.lab + t.src.N;
-        d.memb_off = d.members + t.src.N;
-        ts += 3 * (uint64_t)t.src.N + 1;
+        const uint32_t N = t.src.N;
+        d.rows = d_tscratch.as<uint32_t>() + ts;
+        d.lab = reinterpret_cast<uint16_t *>(d.rows + N);
+        d.members = d.lab + 2 * even16(N);
+        d.memb_off = d.members + 2 * even16(N);
+        d.cols = d.memb_off + 2 * even16(N + 1);
+        ts += task_words(N);
     }
     CAC_TRY(d_kout.ensure(tasks.size() * 4));
     // one descriptor copy for the sources, the row-prep list and the tasks
@@ -1636,154 +1746,121 @@ int KsEngine::step() {
     std::vector<uint64_t> out_off(2 * tasks.size(), 0);
     std::vector<uint32_t> kq(tasks.size(), 0);
     uint64_t out_bytes = 0;
-    bool all_small = true;
-    uint32_t kmax = 0;
     for (size_t i = 0; i < tasks.size(); i++) {
         const uint32_t k = kk[i] == kDropped ? 0 : kk[i];
         kq[i] = k;
         out_off[i] = out_bytes;
         out_bytes += ((uint64_t)k * ld_of(k) * (tasks[i].src.small ? 4 : 8) + 15) / 16 * 16;
-        all_small = all_small && tasks[i].src.small;
-        kmax = std::max(kmax, k);
     }
     for (size_t i = 0; i < tasks.size(); i++) {
         out_off[tasks.size() + i] = out_bytes;
         out_bytes += ((kq[i] + (uint64_t)kq[i] * ((kq[i] + 31) / 32)) * 8 + 15) / 16 * 16;
     }
-    // Three quotient kernels, identical outputs: warp-per-row (8 or 4 warps, one k-entry row per
-    // warp in shared memory; where three of its CTAs fit an SM: labels + rows within 80 KB), its
-    // bulk-copy variant, and shared-row (8 warps on one output row). Which is fastest depends on
-    // N, k and the task count, so the step autotunes: the first sizeable step of each
-    // (power-of-two bucket of N, entry width) on this ctx times them on its own data and keeps the
-    // fastest; smaller steps before that use the rule measured on GB300 (shared-row from N = 2000
-    // on).
-    const size_t stage_words = ((size_t)maxN + 3) & ~(size_t)3;  // N u32 labels, 16-byte rounded
-    const size_t rs_bytes = all_small ? 4 : 8;
-    const uint32_t qwarps = stage_words * 4 + 8 * rs_bytes * (size_t)kmax <= 80 * 1024   ? 8u
-                            : stage_words * 4 + 4 * rs_bytes * (size_t)kmax <= 80 * 1024 ? 4u
-                                                                                         : 0u;
-    auto group_offsets = [&](uint32_t rows, std::vector<uint64_t> &gto) {
-        gto.assign(tasks.size(), 0);
-        uint64_t g = 0;
-        for (size_t i = 0; i < tasks.size(); i++) {
-            gto[i] = g;
-            g += (kq[i] + rows - 1) / rows;
-        }
-        return g;
-    };
-    std::vector<uint64_t> gto_warp, gto_shared;
-    const uint64_t groups_warp = qwarps ? group_offsets(qwarps * 4, gto_warp) : 0;
-    const uint64_t groups_shared = group_offsets(kSharedRows, gto_shared);
-    // the bulk-copy variant of the warp quotient: labels, then per warp two staged member rows
-    // and its output row; 8 warps where two CTAs fit an SM, else 4 where one does
-    const size_t row_words = (size_t)ld_of(maxN);
-    const size_t bulk_per_warp = ((row_words * (all_small ? 4 : 8)) * 2 + (size_t)kmax * rs_bytes + 15) & ~(size_t)15;
-    const size_t bulk_base = 128 + ((stage_words * 4 + 15) & ~(size_t)15);
-    const uint32_t bwarps = bulk_base + 8 * bulk_per_warp <= 113 * 1024   ? 8u
-                            : bulk_base + 4 * bulk_per_warp <= 226 * 1024 ? 4u
-                                                                          : 0u;
-    std::vector<uint64_t> gto_bulk;
-    const uint64_t groups_bulk = bwarps ? group_offsets(bwarps * 4, gto_bulk) : 0;
+    // Two quotient kernels, identical outputs: tiles up to kTileMaxN source vertices (a launch per entry
+    // width), one row per CTA above; the caller may force one, where it fits.
     MatBuf *out = nullptr;
-    if (groups_shared) {
+    if (out_bytes) {
         CAC_TRY(alloc(out_bytes, &out));
-        // one descriptor copy for the output offsets, the children's sizes and the row groups
-        CAC_TRY(post_st.begin(Staging::bytes_of(out_off) + Staging::bytes_of(kq) + Staging::bytes_of(gto_shared) +
-                              Staging::bytes_of(gto_warp) + Staging::bytes_of(gto_bulk)));
+        unsigned char *obase = static_cast<unsigned char *>(out->p);
+        struct TileList {
+            TilePlan plan;
+            std::vector<TileTask> task;
+            std::vector<uint64_t> first;
+            uint64_t ctas = 0;
+            uint32_t uniform = 0;
+        } tl[2];
+        tl[0].plan = TilePlan{4, 4, 0, 1};  // u32 entries
+        tl[1].plan = TilePlan{2, 8, 0, 1};  // u64
+        std::vector<uint32_t> shared;
+        std::vector<uint64_t> gto;
+        uint64_t groups_shared = 0;
+        uint32_t shared_n = 0, shared_k = 0;
+        bool shared_small = true;
+        const uint8_t forced = ctx_->quotient_forced;
+        for (size_t i = 0; i < tasks.size(); i++) {
+            const uint32_t N = tasks[i].src.N, k = kq[i];
+            if (!k) continue;
+            TileList &l = tl[tasks[i].src.small ? 0 : 1];
+            const uint32_t need = tile_idx_bytes(N, k) +
+                                  tile_groups(N, k, l.plan, kTileSmem) * tile_bytes(N, l.plan.rows, l.plan.esize);
+            const bool tiles = forced == kQuotientShared                                     ? false
+                               : forced == kQuotientTile || forced == kQuotientTileToo ? need <= 226 * 1024
+                                                                                       : N <= kTileMaxN;
+            if (tiles) {
+                l.plan.smem = std::max(l.plan.smem, need);
+                l.task.push_back(TileTask{tasks[i].src.mat, td[i].cols, td[i].members, td[i].memb_off, td[i].rows,
+                                          obase + out_off[i], reinterpret_cast<uint64_t *>(obase + out_off[tasks.size() + i]),
+                                          kact ? kact + i : nullptr, N, k});
+            } else {
+                shared.push_back((uint32_t)i);
+                gto.push_back(groups_shared);
+                groups_shared += (k + kSharedRows - 1) / kSharedRows;
+                shared_n = std::max(shared_n, N);
+                shared_k = std::max(shared_k, k);
+                shared_small = shared_small && tasks[i].src.small;
+            }
+        }
+        for (TileList &l : tl) {
+            // tiles per group of warps: a CTA's lists are staged once for all of them, but a last wave of
+            // long CTAs costs more than the staging (448 children of N = 709: 16 tiles 357 us, 8 414; 240
+            // of N = 501: 131 and 110)
+            for (l.plan.tiles = 16;; l.plan.tiles /= 2) {
+                l.first.clear();
+                l.ctas = 0;
+                uint64_t same = 0;
+                bool uniform = true;
+                for (const TileTask &t : l.task) {
+                    const uint32_t g = tile_groups(t.N, t.k, l.plan, l.plan.smem);
+                    const uint32_t per = tile_per_cta(g, l.plan), nt = (t.k + l.plan.rows - 1) / l.plan.rows;
+                    const uint64_t ctas = (nt + per - 1) / per;
+                    if (l.first.empty()) same = ctas;
+                    uniform = uniform && ctas == same;
+                    l.first.push_back(l.ctas);
+                    l.ctas += ctas;
+                }
+                l.uniform = uniform ? (uint32_t)same : 0;
+                if (l.plan.tiles == 1 || 2 * l.ctas >= (uint64_t)ctx_->num_sms * (l.plan.tiles == 16 ? 9 : 2)) break;
+            }
+        }
+        // one descriptor copy for the output offsets, the children's sizes and the launch lists
+        size_t bytes = Staging::bytes_of(out_off) + Staging::bytes_of(kq) + Staging::bytes_of(shared) + Staging::bytes_of(gto);
+        for (const TileList &l : tl) bytes += Staging::bytes_of(l.task) + Staging::bytes_of(l.first);
+        CAC_TRY(post_st.begin(bytes));
         const uint64_t *dv_qoff = post_st.put(out_off);
         const uint32_t *dv_k = post_st.put(kq);
-        const uint64_t *dv_gto_shared = post_st.put(gto_shared);
-        const uint64_t *dv_gto_warp = post_st.put(gto_warp);
-        const uint64_t *dv_gto_bulk = post_st.put(gto_bulk);
+        const uint32_t *dv_shared = post_st.put(shared);
+        const uint64_t *dv_gto = post_st.put(gto);
+        TileArgs args[2];
+        for (int i = 0; i < 2; i++)
+            args[i] = TileArgs{post_st.put(tl[i].task), post_st.put(tl[i].first), (uint32_t)tl[i].task.size(), tl[i].uniform,
+                               d_err, tl[i].plan};
         CAC_TRY(post_st.flush());
-        unsigned char *obase = static_cast<unsigned char *>(out->p);
-        const uint32_t ntk = (uint32_t)tasks.size();
-        auto launch_shared = [&]() -> int {
-            const size_t ssm = stage_words * 4 + (((size_t)kmax * rs_bytes + 15) & ~(size_t)15) +
-                               ((size_t)kmax / 32 + 1) * 8;
+        if (tl[0].ctas) {
+            CAC_TRY(smem_optin(ctx_, quotient_tile_kernel<uint32_t, 4>));
+            quotient_tile_kernel<uint32_t, 4><<<(unsigned)tl[0].ctas, kTileThreads, tl[0].plan.smem, s>>>(args[0]);
+        }
+        if (tl[1].ctas) {
+            CAC_TRY(smem_optin(ctx_, quotient_tile_kernel<uint64_t, 2>));
+            quotient_tile_kernel<uint64_t, 2><<<(unsigned)tl[1].ctas, kTileThreads, tl[1].plan.smem, s>>>(args[1]);
+        }
+        if (groups_shared) {
+            // shared rows are u32 only when every task's sums fit (all sources small)
+            const size_t words = ((size_t)shared_n + 3) & ~(size_t)3, es = shared_small ? 4 : 8;
+            const size_t ssm = words * 4 + (((size_t)shared_k * es + 15) & ~(size_t)15) + ((size_t)shared_k / 32 + 1) * 8;
             std::vector<decltype(&quotient_shared_row_kernel<uint32_t, uint32_t>)> kerns;
-            if (all_small) kerns.push_back(quotient_shared_row_kernel<uint32_t, uint32_t>);
+            if (shared_small) kerns.push_back(quotient_shared_row_kernel<uint32_t, uint32_t>);
             else {
                 if (t32) kerns.push_back(quotient_shared_row_kernel<uint64_t, uint32_t>);
                 if (t64) kerns.push_back(quotient_shared_row_kernel<uint64_t, uint64_t>);
             }
             for (auto kern : kerns) {
                 CAC_TRY(smem_optin(ctx_, kern));
-                kern<<<(unsigned)groups_shared, 256, ssm, s>>>(dv_task, dv_src, dv_k, dv_gto_shared, ntk, kSharedRows,
-                                                               dv_qoff, obase, (uint32_t)stage_words, kmax, kact,
-                                                               d_err);
+                kern<<<(unsigned)groups_shared, 256, ssm, s>>>(dv_task, dv_src, dv_shared, (uint32_t)shared.size(), dv_k, dv_gto,
+                                                               (uint32_t)tasks.size(), kSharedRows, dv_qoff, obase,
+                                                               (uint32_t)words, shared_k, kact, d_err);
             }
-            CAC_CUDA_TRY(cudaGetLastError());
-            return CAC_OK;
-        };
-        auto launch_warp = [&]() -> int {
-            // shared rows are u32 only when every task's sums fit (all sources small)
-            const size_t wsm = stage_words * 4 + (size_t)qwarps * kmax * rs_bytes;
-            std::vector<decltype(&quotient_warp_kernel<uint32_t, uint32_t>)> kerns;
-            if (all_small) kerns.push_back(quotient_warp_kernel<uint32_t, uint32_t>);
-            else {
-                if (t32) kerns.push_back(quotient_warp_kernel<uint64_t, uint32_t>);
-                if (t64) kerns.push_back(quotient_warp_kernel<uint64_t, uint64_t>);
-            }
-            for (auto kern : kerns) {
-                CAC_TRY(smem_optin(ctx_, kern));
-                kern<<<(unsigned)groups_warp, qwarps * 32, wsm, s>>>(dv_task, dv_src, dv_k, dv_gto_warp, ntk,
-                                                                     qwarps * 4, dv_qoff, obase,
-                                                                     (uint32_t)stage_words, kmax, kact, d_err);
-            }
-            CAC_CUDA_TRY(cudaGetLastError());
-            return CAC_OK;
-        };
-        auto launch_bulk = [&]() -> int {
-            const size_t bsm = bulk_base + bwarps * bulk_per_warp;
-            std::vector<decltype(&quotient_bulk_kernel<uint32_t, uint32_t>)> kerns;
-            if (all_small) kerns.push_back(quotient_bulk_kernel<uint32_t, uint32_t>);
-            else {
-                if (t32) kerns.push_back(quotient_bulk_kernel<uint64_t, uint32_t>);
-                if (t64) kerns.push_back(quotient_bulk_kernel<uint64_t, uint64_t>);
-            }
-            for (auto kern : kerns) {
-                CAC_TRY(smem_optin(ctx_, kern));
-                kern<<<(unsigned)groups_bulk, bwarps * 32, bsm, s>>>(dv_task, dv_src, dv_k, dv_gto_bulk, ntk,
-                                                                     bwarps * 4, dv_qoff, obase,
-                                                                     (uint32_t)stage_words, kmax,
-                                                                     (uint32_t)row_words, d_err, kact);
-            }
-            CAC_CUDA_TRY(cudaGetLastError());
-            return CAC_OK;
-        };
-        uint8_t &tuned = ctx_->quotient_forced ? ctx_->quotient_forced
-                                               : ctx_->quotient_choice[quotient_bucket(maxN, all_small)];
-        const bool sizeable = groups_shared >= (uint64_t)4 * ctx_->num_sms;  // enough work to time
-        if (!qwarps && !bwarps) {
-            CAC_TRY(launch_shared());
-        } else if (tuned == kQuotientShared) {
-            CAC_TRY(launch_shared());
-        } else if (tuned == kQuotientWarp && qwarps) {
-            CAC_TRY(launch_warp());
-        } else if (tuned == kQuotientBulk && bwarps) {
-            CAC_TRY(launch_bulk());
-        } else if (!sizeable || tuned) {  // too small to time, already timed, or kQuotientRule forced
-            CAC_TRY(maxN >= kSharedRowMinN || !qwarps ? launch_shared() : launch_warp());
-        } else {
-            // all write the same matrices, row sums and prefixes: time each on this step's data
-            cudaEvent_t *ev = ctx_->ev;
-            float t_warp = 1e30f, t_shared = 0, t_bulk = 1e30f;
-            CAC_CUDA_TRY(cudaEventRecord(ev[4], s));
-            if (qwarps) CAC_TRY(launch_warp());
-            CAC_CUDA_TRY(cudaEventRecord(ev[5], s));
-            if (bwarps) CAC_TRY(launch_bulk());
-            CAC_CUDA_TRY(cudaEventRecord(ev[6], s));
-            CAC_TRY(launch_shared());
-            CAC_CUDA_TRY(cudaEventRecord(ev[7], s));
-            CAC_CUDA_TRY(cudaEventSynchronize(ev[7]));
-            if (qwarps) CAC_CUDA_TRY(cudaEventElapsedTime(&t_warp, ev[4], ev[5]));
-            if (bwarps) CAC_CUDA_TRY(cudaEventElapsedTime(&t_bulk, ev[5], ev[6]));
-            CAC_CUDA_TRY(cudaEventElapsedTime(&t_shared, ev[6], ev[7]));
-            tuned = t_shared <= t_warp && t_shared <= t_bulk ? kQuotientShared
-                    : t_bulk < t_warp                        ? kQuotientBulk
-                                                             : kQuotientWarp;
         }
+        CAC_CUDA_TRY(cudaGetLastError());
     }
     // the sources are read by everything enqueued above: their buffers may now be released
     for (MatBuf *b : consumed) release(b);

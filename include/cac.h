@@ -82,13 +82,10 @@ int cac_ctx_create(const cac_config *config, cac_ctx **out);
  * trials' draws, never the validity of a cut; a lower limit moves more of the recursion to the
  * sparse form. */
 int cac_ctx_set_dense_limit(cac_ctx *ctx, uint32_t max_dense_vertices);
-/* The quotient kernel of the dense Karger-Stein steps: 0 (default) lets the ctx time the candidates
- * on the first sizeable step of each size bucket and keep the fastest; 1 warp per output row,
- * 2 eight warps per output row, 3 warp per output row with member rows staged by bulk copies, 4 the
- * fixed size rule without timing (eight warps per row from 2000 source vertices on, else one; for
- * profilers, whose serialised replays distort the timings). All give identical matrices; a kernel
- * that does not fit a step's shared memory is replaced by one that does. (No reference
- * counterpart: a tuning control.) */
+/* The quotient kernel of the dense Karger-Stein steps: 0 (default) and 4 choose by size (tiles of
+ * output rows up to 2900 source vertices, eight warps per output row above); 1 and 3 force the tiles,
+ * 2 eight warps per row. All give identical matrices; a kernel that does not fit a step's shared
+ * memory is replaced by one that does. (No reference counterpart: a tuning control.) */
 int cac_ctx_set_quotient_kernel(cac_ctx *ctx, int kind);
 /* Karger-Stein levels planned ahead (default 1): every child is taken to stop at its target size,
  * so the levels of a run follow one another without reading the children's sizes back; a child
