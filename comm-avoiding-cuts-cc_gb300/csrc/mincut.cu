@@ -21,10 +21,10 @@
 //                                the child's matrix: a few output rows at a time as one tile in shared
 //                                memory, member rows summed on the way in, joined columns added to their
 //                                groups' first ones, those stored; at large N a CTA per output row
-//              sw_leaf_kernel    one 128-thread CTA per leaf (n <= 128), a thread per vertex:
+//              sw_leaf_kernel    one warp per leaf (n <= 128), four vertices per lane:
 //                                Stoer-Wagner maximum-adjacency
 //                                phases with Nagamochi-Ono-Ibaraki contractions on the matrix held
-//                                in shared memory (circulant half storage); atomicMin into the
+//                                in shared memory (its lower triangle); atomicMin into the
 //                                trial's cut
 // The random stream of every draw is addressed by (seed + r, i, tag, 0) and (round, draw index),
 // tag 1 for Stage 1 and 1 + h for the Karger-Stein child with heap index h, so a CPU replay of
@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(256, 5) quotient_shared_row_kernel(const TaskD
     }
 }
 
-// Exact minimum cut of one leaf (n <= 128) by one CTA of 128 threads: maximum-adjacency orderings
+// Exact minimum cut of one leaf (n <= 128) by one warp, four vertices per lane: maximum-adjacency orderings
 // as in the reference's Stoer-Wagner base case (co_mincut_base_case.hpp:52-144), with the
 // Nagamochi-Ono-Ibaraki contraction rule (Nagamochi & Ibaraki 1992; Nagamochi, Ono & Ibaraki
 // 1994): when vertex w's key reaches q >= lambda while vertex v is scanned, then lambda(v, w) >= q,
@@ -1109,15 +1109,24 @@ __global__ void __launch_bounds__(256, 5) quotient_shared_row_kernel(const TaskD
 // certified edges plus the last two vertices (the cut of the phase updates lambda), so far fewer
 // orderings are needed than the n - 1 of plain Stoer-Wagner; the returned value is the exact
 // minimum cut of the leaf.
-//   Thread v owns vertex v. A step of an ordering is one warp argmax of (key, smallest vertex), a
-//   cross-warp maximum through a double-buffered shared word per warp (one barrier per step), and
-//   one key update per thread from the scanned vertex's row. Every certified edge and the pair
-//   (second to last, last) joins a vertex to one scanned before it, so when all but the first
-//   vertex of the ordering are so joined the leaf contracts to one vertex and the ordering's result
-//   is final: a barrier count decides this without building the contraction (the usual case:
-//   Karger-Stein leaves of 128 vertices mostly finish in one ordering). Otherwise the pairs are
-//   joined by a union-find over vertex slots and the matrix entries are merged pair by pair.
-//   Keys stay below 2^56 (total graph weight checked on the host); u32 matrices keep 32-bit keys.
+//   A vertex is one word, key << 8 | 255 - vertex, 0 once it is scanned, so the next vertex (largest
+// key, smallest id) is one maximum over the warp; 32-bit words while the leaf weighs less than 2^24,
+// else 64. Every certified edge and the pair (second to last, last) joins a vertex to one scanned
+// before it, so when all but the first vertex of the ordering are so joined the leaf contracts to one
+// vertex and the ordering's result is final (the usual case: Karger-Stein leaves of 128 vertices
+// mostly finish in one ordering). Otherwise the joined vertices are merged into the roots of their
+// trees, row by row.
+//   The matrix is kept as its lower triangle, (i, j < i) at i (i - 1) / 2 + j: the entries (x, v) of 32
+// consecutive v lie in 32 different banks on either side of x (triangular numbers take every residue
+// of a power of two once), and 128 vertices take half the shared memory of the full matrix: six leaves
+// per SM. It is copied in asynchronously, all rows in flight.
+//   Bound by the latency of a step (maximum, four shared loads, add: about 130 cycles), not by issue or
+// memory, so the step holds no branch and no barrier. A 128-thread CTA per leaf with a thread per
+// vertex (a barrier and a cross-warp maximum per step, half matrix in 32 KB) took 714 us for the 14,336
+// leaves of K4000's 56 trials, 73 us for the 480 of ER(1000, 0.05)'s 60 and 9.7 ms in 64 graphs' batch;
+// this takes 300 us, 36 us and 3.6 ms. With the update under a branch per vertex a step took 570 cycles
+// (789 us); with the unions walked by one lane a merge took 300 cycles more.
+//   Keys stay below 2^56 (total graph weight checked on the host).
 __device__ __forceinline__ uint64_t warp_min_u64(uint64_t x) {
     const uint32_t hi = (uint32_t)(x >> 32);
     const uint32_t top = __reduce_min_sync(0xffffffffu, hi);
@@ -1125,217 +1134,180 @@ __device__ __forceinline__ uint64_t warp_min_u64(uint64_t x) {
     return ((uint64_t)top << 32) | lo;
 }
 
-// Circulant half storage of a symmetric N x N matrix with a zero diagonal: row i holds the entries
-// (i, (i + d) mod N) for d = 1 .. H, H = floor(N / 2), so every pair is stored once (twice when N
-// is even and d = N / 2; both copies are kept equal). A warp reading the entries (x, v) for its
-// lanes' v touches consecutive words for the v after x and words H - 1 apart for the v before x,
-// so neither half has bank conflicts; a 128-vertex leaf takes half the shared memory of the full
-// matrix and twice as many leaves are resident per SM.
-__device__ __forceinline__ uint32_t cpos(uint32_t i, uint32_t j, uint32_t N, uint32_t H) {
-    const uint32_t d = j >= i ? j - i : j + N - i;
-    return d <= H ? i * H + d - 1 : j * H + (N - d) - 1;
-}
-
-template <typename Tm>
-__device__ __forceinline__ void cset(Tm *M, uint32_t i, uint32_t j, uint32_t N, uint32_t H, Tm val) {
-    const uint32_t d = j >= i ? j - i : j + N - i;
-    if (d <= H) {
-        M[i * H + d - 1] = val;
-        if (d == H && !(N & 1u)) M[j * H + H - 1] = val;  // the twin of an even-N antipodal pair
-    } else {
-        M[j * H + (N - d) - 1] = val;
-    }
-}
-
-__device__ __forceinline__ uint64_t warp_max_u64(uint64_t x) {
+__device__ __forceinline__ uint64_t warp_max(uint64_t x) {
     const uint32_t hi = (uint32_t)(x >> 32);
     const uint32_t top = __reduce_max_sync(0xffffffffu, hi);
     const uint32_t lo = __reduce_max_sync(0xffffffffu, hi == top ? (uint32_t)x : 0u);
     return ((uint64_t)top << 32) | lo;
 }
+__device__ __forceinline__ uint32_t warp_max(uint32_t x) { return __reduce_max_sync(0xffffffffu, x); }
 
-constexpr uint32_t kLeafThreads = 128;
+constexpr uint32_t kLeafThreads = 32;
+__device__ __forceinline__ uint32_t tri(uint32_t i) { return i * (i - 1) / 2; }
+__device__ __forceinline__ uint32_t tpos(uint32_t i, uint32_t j) { return i > j ? tri(i) + j : tri(j) + i; }
+
+template <typename Tm>
+__device__ __forceinline__ void copy_entry_async(Tm *dst, const Tm *src) {
+    if constexpr (sizeof(Tm) == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+}
+
+// The orderings; returns the leaf's minimum cut. Kt: the vertex words. root: 128 bytes of shared memory.
+template <typename Tm, typename Kt>
+__device__ __forceinline__ uint64_t leaf_cut(Tm *M, uint32_t N, uint64_t lambda, uint8_t *root) {
+    const uint32_t lane = threadIdx.x;
+    // at[q]: the vertex whose entries the lane reads in place q, 0 where it has none (the loads are not
+    // predicated: what an inactive or scanned vertex reads is dropped)
+    uint32_t v[4], at[4], tat[4];
+    bool active[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        v[q] = lane + 32 * q;
+        active[q] = v[q] < N;
+        at[q] = active[q] ? v[q] : 0;
+        tat[q] = tri(at[q]);
+    }
+    auto entry = [&](int q, uint32_t x, uint32_t tx) { return at[q] > x ? tat[q] + x : tx + at[q]; };
+    uint32_t cnt = N;
+    while (cnt > 1) {
+        const Kt lam = (Kt)lambda << 8;
+        Kt P[4];
+        uint32_t mark[4];  // vertex to contract into, 255: none
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            P[q] = active[q] ? (Kt)(255u - v[q]) : (Kt)0;
+            mark[q] = 255u;
+        }
+        uint32_t prev = 0;
+        for (uint32_t step = 1; step < cnt; step++) {
+            const Kt m01 = P[0] > P[1] ? P[0] : P[1], m23 = P[2] > P[3] ? P[2] : P[3];
+            const Kt best = warp_max(m01 > m23 ? m01 : m23);
+            const uint32_t sv = 255u - ((uint32_t)best & 255u), ts = tri(sv);
+            prev = sv;
+            Tm c[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) c[q] = M[entry(q, sv, ts)];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const bool open = P[q] != 0 && P[q] != best;
+                const Kt next = P[q] + ((Kt)c[q] << 8);
+                P[q] = open ? next : (Kt)0;
+                mark[q] = open && c[q] != 0 && next >= lam ? sv : mark[q];  // lambda(sv, v) >= key: contractible
+            }
+        }
+        const Kt m01 = P[0] > P[1] ? P[0] : P[1], m23 = P[2] > P[3] ? P[2] : P[3];
+        const Kt best = warp_max(m01 > m23 ? m01 : m23);
+        const uint32_t last = 255u - ((uint32_t)best & 255u);
+        lambda = (uint64_t)(best >> 8) < lambda ? (uint64_t)(best >> 8) : lambda;
+        // one vertex left when every vertex but the first of the ordering is joined to an earlier one
+        uint32_t linked = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) linked += __popc(__ballot_sync(0xffffffffu, active[q] && (mark[q] != 255u || v[q] == last)));
+        if (linked + 1 >= cnt) break;
+        // the roots of the marks' trees by pointer doubling (a tree is at most 127 edges deep), then
+        // (prev, last) joins two of them
+#pragma unroll
+        for (int q = 0; q < 4; q++) root[v[q]] = (uint8_t)(mark[q] != 255u ? mark[q] : v[q]);
+        __syncwarp();
+        uint32_t rt[4];
+#pragma unroll 1
+        for (uint32_t deep = 1; deep < 128; deep *= 2) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) rt[q] = root[root[v[q]]];
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 4; q++) root[v[q]] = (uint8_t)rt[q];
+            __syncwarp();
+        }
+        const uint32_t into = root[prev], from = root[last];
+        // each vertex that is no root is merged into its own
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) {
+            const uint32_t mine = v[0] + 32 * k;
+            const uint32_t r = root[mine];
+            const uint32_t to = r == from ? into : r;
+            bool on = false;
+#pragma unroll
+            for (int q = 0; q < 4; q++) on = q == k ? active[q] : on;
+            uint32_t gone = __ballot_sync(0xffffffffu, on && to != mine);
+            cnt -= __popc(gone);
+            while (gone) {
+                const uint32_t l = __ffs(gone) - 1;
+                gone &= gone - 1;
+                const uint32_t y = l + 32 * k, x = __shfl_sync(0xffffffffu, to, l);
+                const uint32_t tx = tri(x), ty = tri(y);
+                Tm a[4], b[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    a[q] = M[entry(q, x, tx)];
+                    b[q] = M[entry(q, y, ty)];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (active[q] && v[q] != x && v[q] != y) M[entry(q, x, tx)] = a[q] + b[q];
+                    active[q] = active[q] && v[q] != y;
+                }
+                __syncwarp();
+            }
+        }
+    }
+    return lambda;
+}
 
 template <typename Tm>
 __global__ void __launch_bounds__(kLeafThreads) sw_leaf_kernel(const LeafDesc *__restrict__ leaves) {
     extern __shared__ __align__(16) unsigned char dsm[];
-    Tm *M = reinterpret_cast<Tm *>(dsm);
-    __shared__ uint8_t uf[128];
-    __shared__ uint32_t pairs[128];
-    __shared__ uint32_t npairs;
-    __shared__ __align__(16) uint64_t wbest[2][4];
-    __shared__ __align__(16) uint32_t wbest32[2][4];
-    __shared__ uint64_t wsum[4];
+    Tm *M = reinterpret_cast<Tm *>(dsm);  // N (N - 1) / 2 entries and one that is read but not used
+    __shared__ uint8_t root[128];
     const LeafDesc L = leaves[blockIdx.x];
-    const uint32_t N = L.N, H = N / 2;
-    const uint32_t v = threadIdx.x, lane = v & 31u, warp = v >> 5;
-    // circulant half: thread v loads offset d = v % 64 + 1 of every second row (rows v / 64,
-    // v / 64 + 2, ...), eight rows per pass in flight
+    const uint32_t N = L.N, lane = threadIdx.x;
     {
-        const Tm *src = reinterpret_cast<const Tm *>(L.mat);
+        const Tm *src = reinterpret_cast<const Tm *>(L.mat) + lane;
         const uint64_t ldN = ld_of(N);
-        const uint32_t d = (v & 63u) + 1, r0 = v >> 6;
-        const bool has = d <= H;
-        for (uint32_t i0 = r0; i0 < N; i0 += 16) {
-            Tm a[8];
+        Tm *dst = M + lane;
+#pragma unroll 4
+        for (uint32_t i = 1; i < N; i++) {
+            src += ldN;
 #pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const uint32_t i = i0 + 2 * r;
-                uint32_t j = i + d;
-                j = j >= N ? j - N : j;
-                a[r] = (i < N && has) ? __ldg(src + (uint64_t)i * ldN + j) : (Tm)0;
-            }
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const uint32_t i = i0 + 2 * r;
-                if (i < N && has) M[i * H + d - 1] = a[r];
-            }
+            for (uint32_t j = 0; j < 128; j += 32)
+                if (lane + j < i) copy_entry_async(dst + j, src + j);
+            dst += i;
         }
     }
-    uf[v] = (uint8_t)v;
-    bool active = v < N;
-    __syncthreads();
     // lambda starts at the minimum weighted degree (a cut of the leaf): the row sums that came with
-    // the matrix, else summed here (row v's own half, then the entries (v - e, v) stored in the rows
-    // before it)
-    uint64_t deg = kU64Max;
-    if (active) {
-        if (L.rowsum) {
-            deg = __ldg(L.rowsum + v);
-        } else {
-            deg = 0;
-            for (uint32_t e = 1; e <= H; e++) deg += (uint64_t)M[v * H + e - 1];
-            for (uint32_t e = 1; e + H < N; e++) deg += (uint64_t)M[(v >= e ? v - e : v + N - e) * H + e - 1];
+    // the matrix, else summed here
+    uint64_t deg[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) deg[q] = L.rowsum && lane + 32 * q < N ? __ldg(L.rowsum + lane + 32 * q) : 0;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    uint64_t low = kU64Max, sum = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t v = lane + 32 * q;
+        if (v < N) {
+            if (!L.rowsum)
+                for (uint32_t j = 0; j < N; j++) deg[q] += j == v ? 0 : (uint64_t)M[tpos(v, j)];
+            low = deg[q] < low ? deg[q] : low;
+            sum += deg[q];
         }
     }
-    {
-        const uint64_t wm = warp_min_u64(deg);
-        // the degree sum (u32 matrices: every degree below 2^32, summed as two 16-bit halves)
-        const uint32_t d = active && deg < (1ull << 32) ? (uint32_t)deg : 0u;
-        const uint64_t ws = (uint64_t)__reduce_add_sync(0xffffffffu, d & 0xFFFFu) +
-                            ((uint64_t)__reduce_add_sync(0xffffffffu, d >> 16) << 16);
-        if (lane == 0) {
-            wbest[1][warp] = wm;  // the first step writes wbest[0]
-            wsum[warp] = ws;
-        }
+    const uint64_t lambda = warp_min_u64(low);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    // a key never exceeds the leaf's total weight (half its degree sum, which merges only lower)
+    uint64_t cut;
+    if constexpr (sizeof(Tm) == 4) {
+        cut = sum < (1ull << 25) ? leaf_cut<Tm, uint32_t>(M, N, lambda, root)
+                                 : leaf_cut<Tm, uint64_t>(M, N, lambda, root);
+    } else {
+        cut = leaf_cut<Tm, uint64_t>(M, N, lambda, root);
     }
-    __syncthreads();
-    uint64_t lambda = wbest[1][0], deg_sum = wsum[0];
-    for (int w = 1; w < 4; w++) {
-        lambda = wbest[1][w] < lambda ? wbest[1][w] : lambda;
-        deg_sum += wsum[w];
-    }
-    // a key never exceeds the leaf's total weight (half its degree sum, which merges only lower):
-    // below 2^24, (key << 8 | 255 - v) is one 32-bit word and the argmax one reduction
-    const bool packed32 = sizeof(Tm) == 4 && deg_sum < (1ull << 25);
-    using Kt = typename std::conditional<sizeof(Tm) == 4, uint32_t, uint64_t>::type;
-    uint32_t cnt = N, par = 0;
-    while (cnt > 1) {
-        Kt key = 0;
-        const Kt lam = lambda > (uint64_t)(Kt)~(Kt)0 ? (Kt)~(Kt)0 : (Kt)lambda;
-        bool in_a = false;
-        uint32_t mark = 0xFFu;  // vertex to contract into, 0xFF: none
-        uint32_t prev = 0, last = 0;
-        uint64_t cut_phase = 0;
-        for (uint32_t step = 0; step < cnt; step++) {
-            const bool elig = active && !in_a;
-            uint32_t sv;
-            uint64_t top_key;
-            if (packed32) {
-                const uint32_t wb = __reduce_max_sync(0xffffffffu, elig ? (((uint32_t)key << 8) | (255u - v)) : 0u);
-                if (lane == 0) wbest32[par][warp] = wb;
-                __syncthreads();
-                const uint4 b = *reinterpret_cast<const uint4 *>(&wbest32[par][0]);
-                par ^= 1u;
-                const uint32_t best = max(max(b.x, b.y), max(b.z, b.w));
-                sv = 255u - (best & 255u);
-                top_key = best >> 8;
-            } else {
-            uint64_t wb;  // this warp's best as (key << 8 | 255 - vertex), 0 for none
-            if constexpr (sizeof(Tm) == 4) {
-                const uint32_t top = __reduce_max_sync(0xffffffffu, elig ? key : 0u);
-                const uint32_t vmin = __reduce_min_sync(0xffffffffu, (elig && key == top) ? v : 255u);
-                wb = vmin == 255u ? 0 : (((uint64_t)top << 8) | (uint64_t)(255u - vmin));
-            } else {
-                wb = warp_max_u64(elig ? ((key << 8) | (uint64_t)(255u - v)) : 0);
-            }
-            if (lane == 0) wbest[par][warp] = wb;
-            __syncthreads();
-            const ulonglong2 b01 = *reinterpret_cast<const ulonglong2 *>(&wbest[par][0]);
-            const ulonglong2 b23 = *reinterpret_cast<const ulonglong2 *>(&wbest[par][2]);
-            par ^= 1u;
-            const uint64_t m01 = b01.x > b01.y ? b01.x : b01.y, m23 = b23.x > b23.y ? b23.x : b23.y;
-            const uint64_t best = m01 > m23 ? m01 : m23;
-            sv = 255u - (uint32_t)(best & 255u);
-            top_key = best >> 8;
-            }
-            if (sv >= N) {  // no candidate: cannot happen (cnt - step vertices are unscanned)
-                cut_phase = kU64Max;
-                break;
-            }
-            if (step + 1 == cnt) {
-                last = sv;
-                cut_phase = top_key;
-                break;
-            }
-            in_a = in_a || v == sv;
-            prev = sv;
-            if (active && !in_a) {
-                const Kt c = (Kt)M[cpos(sv, v, N, H)];
-                key += c;
-                if (c && key >= lam) mark = sv;  // lambda(sv, v) >= key: contractible
-            }
-        }
-        if (cut_phase == kU64Max) break;
-        lambda = cut_phase < lambda ? cut_phase : lambda;
-        // one vertex left when every vertex but the first of the ordering is joined to an earlier one
-        const uint32_t linked = (uint32_t)__syncthreads_count(active && (mark != 0xFFu || v == last));
-        if (linked + 1 >= cnt) break;
-        // contraction list: (prev, last), then every certified edge (mark[v], v)
-        if (v == 0) {
-            pairs[0] = (prev << 8) | last;
-            npairs = 1;
-        }
-        __syncthreads();
-        if (active && mark != 0xFFu) pairs[atomicAdd(&npairs, 1u)] = (mark << 8) | v;
-        __syncthreads();
-        // thread 0 joins the pairs' slots (union-find with path halving) and rewrites the list as
-        // the (root, root) merges actually made
-        if (v == 0) {
-            const uint32_t np = npairs;
-            uint32_t made = 0;
-            for (uint32_t q = 0; q < np && cnt - made > 1; q++) {
-                uint32_t x = pairs[q] >> 8, y = pairs[q] & 255u;
-                while (uf[x] != x) {
-                    uf[x] = uf[uf[x]];
-                    x = uf[x];
-                }
-                while (uf[y] != y) {
-                    uf[y] = uf[uf[y]];
-                    y = uf[y];
-                }
-                if (x == y) continue;  // already merged
-                uf[y] = (uint8_t)x;
-                pairs[made++] = (x << 8) | y;
-            }
-            npairs = made;
-        }
-        __syncthreads();
-        const uint32_t nm = npairs;
-        if (cnt - nm <= 1) break;
-        for (uint32_t q = 0; q < nm; q++) {
-            const uint32_t x = pairs[q] >> 8, y = pairs[q] & 255u;
-            // merge y into x: entry (x, v) += entry (y, v) for every other active v
-            if (active && v != x && v != y) {
-                const Tm val = M[cpos(x, v, N, H)] + M[cpos(y, v, N, H)];
-                cset(M, x, v, N, H, val);
-            }
-            if (v == y) active = false;
-            __syncthreads();
-        }
-        cnt -= nm;
-    }
-    if (v == 0) atomicMin((unsigned long long *)L.cut, (unsigned long long)lambda);
+    if (lane == 0) atomicMin((unsigned long long *)L.cut, (unsigned long long)cut);
 }
 
 __global__ void fill_u64(uint64_t *p, uint64_t n, uint64_t value) {
@@ -1459,7 +1431,7 @@ int upload(cac_ctx *ctx, DevBuf &buf, const std::vector<T> &v) {
     return CAC_OK;
 }
 
-size_t leaf_smem(uint32_t N, bool small) { return (size_t)N * (N / 2) * (small ? 4 : 8); }
+size_t leaf_smem(uint32_t N, bool small) { return ((size_t)N * (N - 1) / 2 + 1) * (small ? 4 : 8); }
 size_t contract_smem(uint32_t N) { return kBatch * sizeof(uint2) + kCoarseRows * sizeof(uint64_t) + (size_t)2 * N * 4; }
 
 }  // namespace
@@ -1561,7 +1533,7 @@ int KsEngine::step() {
     uint32_t *d_err = static_cast<DevBuf *>(d_err_)->as<uint32_t>();
     std::vector<MatBuf *> consumed;
 
-    // leaves (n <= 128) -> exact cut; grouped by size and entry width, one launch each
+    // leaves (n <= 128) -> exact cut, one launch per entry width
     std::vector<LeafDesc> leaves;
     std::vector<KNode> inner;
     for (const KNode &nd : nodes_) {
@@ -1576,27 +1548,19 @@ int KsEngine::step() {
         }
     }
     nodes_.clear();
-    std::sort(leaves.begin(), leaves.end(),
-              [](const LeafDesc &a, const LeafDesc &b) { return a.N != b.N ? a.N > b.N : a.small > b.small; });
-    // the leaves, grouped by size and entry width, one launch each (after the descriptor copy)
-    auto launch_leaves = [&](const LeafDesc *d_leaves) -> int {
-        size_t first = 0;
-        while (first < leaves.size()) {
-            size_t last = first;
-            while (last < leaves.size() && leaves[last].N == leaves[first].N && leaves[last].small == leaves[first].small)
-                last++;
-            const uint32_t N = leaves[first].N;
-            const LeafDesc *dl = d_leaves + first;
-            if (leaves[first].small) {
-                const size_t sm = leaf_smem(N, true);
-                CAC_TRY(smem_optin(ctx_, sw_leaf_kernel<uint32_t>));
-                sw_leaf_kernel<uint32_t><<<(unsigned)(last - first), kLeafThreads, sm, s>>>(dl);
-            } else {
-                const size_t sm = leaf_smem(N, false);
-                CAC_TRY(smem_optin(ctx_, sw_leaf_kernel<uint64_t>));
-                sw_leaf_kernel<uint64_t><<<(unsigned)(last - first), kLeafThreads, sm, s>>>(dl);
-            }
-            first = last;
+    const size_t leaves32 = (size_t)(std::partition(leaves.begin(), leaves.end(), [](const LeafDesc &l) { return l.small != 0; }) -
+                                     leaves.begin());
+    auto launch_leaves = [&](const LeafDesc *d_leaves) -> int {  // (after the descriptor copy)
+        uint32_t n32 = 2, n64 = 2;
+        for (const LeafDesc &l : leaves) (l.small ? n32 : n64) = std::max(l.small ? n32 : n64, l.N);
+        if (leaves32) {
+            CAC_TRY(smem_optin(ctx_, sw_leaf_kernel<uint32_t>));
+            sw_leaf_kernel<uint32_t><<<(unsigned)leaves32, kLeafThreads, leaf_smem(n32, true), s>>>(d_leaves);
+        }
+        if (leaves32 < leaves.size()) {
+            CAC_TRY(smem_optin(ctx_, sw_leaf_kernel<uint64_t>));
+            sw_leaf_kernel<uint64_t><<<(unsigned)(leaves.size() - leaves32), kLeafThreads, leaf_smem(n64, false), s>>>(d_leaves +
+                                                                                                                      leaves32);
         }
         CAC_CUDA_TRY(cudaGetLastError());
         return CAC_OK;
