@@ -11,10 +11,10 @@
 //   Stage 2  dense_build_kernel: the t x t adjacency matrix of the contracted graph in HBM
 //            (u64 entries, global atomics per edge).
 //   Stage 3  Karger-Stein, level-synchronous over all trials of a wave:
-//              prep_rows_kernel / prefix_rows_kernel  row sums + 32-column block prefixes of every
-//                                                     matrix that is contracted this level
-//              contract_kernel   one CTA per child: draws (row by binary search over row prefixes,
-//                                column by block prefix + a 32-entry scan), contraction in draw
+//              prep_rows_kernel  row sums + 32-column block prefixes of the matrices that came
+//                                without them
+//              contract_kernel   one CTA per child: draws (row by a scan of the row sums, block
+//                                by its prefixes, column by a scan of the block), contraction in draw
 //                                order until max(ceil(n/sqrt 2)+1, 128) vertices, labels by rank
 //                                of the smallest member, member lists by counting sort
 //              quotient_tile_kernel / quotient_shared_row_kernel
@@ -46,6 +46,7 @@ constexpr uint32_t kSharedRows = 8;         // output rows per CTA of the shared
 constexpr uint32_t kMaxSmemVertices = kMaxDenseVertices;  // union-find of a contraction held in shared memory
 constexpr int kBatch = 1024;                  // draws gathered before the ordered contraction
 constexpr int kNT = 512;                      // threads of the per-trial / per-task CTAs
+constexpr uint32_t kRootFlag = 0x80000000u;   // a contraction's vertex word: label, first of its group
 constexpr uint32_t kDropped = 0xFFFFFFFFu;    // task whose source matrix has no edges left
 constexpr uint64_t kU64Max = 0xFFFFFFFFFFFFFFFFull;
 
@@ -74,7 +75,7 @@ struct DenseDesc {
 
 struct SrcDesc {
     const void *mat;      // N x N row-major, u32 entries when `small`, else u64
-    uint64_t *rowpre;     // N: inclusive prefix of row sums
+    uint64_t *rowsum;     // N row sums
     uint64_t *blk;        // N x nb: per row, inclusive prefix of 32-column block sums
     uint64_t *cut;        // the trial's cut (root matrices deliver the minimum weighted degree bound)
     uint32_t N, nb;
@@ -170,14 +171,6 @@ __device__ __forceinline__ uint32_t block_excl_scan_u32(uint32_t x, uint32_t &to
     return (uint32_t)r;
 }
 
-__device__ __forceinline__ uint32_t sfind(uint32_t *par, uint32_t x) {
-    while (par[x] != x) {
-        par[x] = par[par[x]];
-        x = par[x];
-    }
-    return x;
-}
-
 __device__ __forceinline__ uint32_t sfind_ro(const uint32_t *par, uint32_t x) {
     uint32_t nx;
     while ((nx = par[x]) != x) x = nx;
@@ -191,9 +184,9 @@ __device__ __forceinline__ uint32_t sfind_ro(const uint32_t *par, uint32_t x) {
 // at most once, so the count cannot fall below target, and since draws after the one that reaches
 // target link nothing, the partition equals the sequential one. A successful CAS always joins
 // two different components, so the number of links is the exact count drop. Repeated until the
-// target or the end of the batch; the last few links (need <= 16) are made by thread 0 in draw
-// order. Endpoints of linked draws are pointed at their roots after each step.
-constexpr uint32_t kSeqTail = 16;
+// target or the end of the batch; the last few links (need <= kWarpTail) are made by one warp the
+// same way, without block barriers. Endpoints of linked draws are pointed at their roots after each step.
+constexpr uint32_t kWarpTail = 32;
 
 template <int NT>
 __device__ void contract_batch(uint32_t *par, const uint2 *sb, uint32_t nb, uint32_t target, uint32_t *s_count,
@@ -205,17 +198,38 @@ __device__ void contract_batch(uint32_t *par, const uint2 *sb, uint32_t nb, uint
         const uint32_t c = *s_count;
         if (c <= target || j0 >= nb) break;
         const uint32_t need = c - target;
-        if (need <= kSeqTail) {
-            if (threadIdx.x == 0) {
+        if (need <= kWarpTail) {
+            if (threadIdx.x < 32) {
+                // 32 draws at a time: those that are loops already stay so; the first `left` others are
+                // linked (at most once each, so the count cannot fall below target), the rest looked at again
+                const uint32_t lane = threadIdx.x;
                 uint32_t cc = c;
-                for (uint32_t j = j0; j < nb && cc > target; j++) {
-                    const uint32_t x = sfind(par, sb[j].x), y = sfind(par, sb[j].y);
-                    if (x != y) {
-                        if (x < y) par[y] = x; else par[x] = y;
-                        cc--;
+                for (uint32_t j = j0; j < nb && cc > target;) {
+                    uint32_t x = 0, y = 0;
+                    if (j + lane < nb) {
+                        x = sb[j + lane].x;
+                        y = sb[j + lane].y;
+                        while (vp[x] != x) x = vp[x];
+                        while (vp[y] != y) y = vp[y];
                     }
+                    const uint32_t open = __ballot_sync(0xffffffffu, x != y), left = cc - target;
+                    const bool mine = x != y && (uint32_t)__popc(open & ((1u << lane) - 1)) < left;
+                    const uint32_t taken = __ballot_sync(0xffffffffu, mine);
+                    bool linked = false;
+                    while (mine && x != y) {
+                        const uint32_t hi = x > y ? x : y, lo = x > y ? y : x;
+                        linked = atomicCAS(&par[hi], hi, lo) == hi;
+                        if (linked) break;
+                        x = hi;  // hi was linked meanwhile: find both roots again
+                        y = lo;
+                        while (vp[x] != x) x = vp[x];
+                        while (vp[y] != y) y = vp[y];
+                    }
+                    cc -= __popc(__ballot_sync(0xffffffffu, linked));
+                    j += taken != open ? 32 - __clz(taken) : 32;
+                    __syncwarp();
                 }
-                *s_count = cc;
+                if (lane == 0) *s_count = cc;
             }
             __syncthreads();
             break;
@@ -431,127 +445,224 @@ __global__ void prep_rows_kernel(const SrcDesc *__restrict__ srcs, const uint64_
         }
     }
     if (lane == 0) {
-        S.rowpre[i] = run;
+        S.rowsum[i] = run;
         if (S.is_root) atomicMin((unsigned long long *)S.cut, (unsigned long long)run);
     }
 }
 
-// One CTA per source: row sums -> inclusive prefix (in place).
-template <int NT>
-__global__ void __launch_bounds__(NT) prefix_rows_kernel(const SrcDesc *__restrict__ srcs) {
-    const SrcDesc S = srcs[blockIdx.x];
-    uint64_t carry = 0;
-    for (uint32_t base = 0; base < S.N; base += NT) {
-        const uint32_t i = base + threadIdx.x;
-        const uint64_t x = i < S.N ? S.rowpre[i] : 0;
-        uint64_t tot;
-        const uint64_t ex = block_excl_scan_u64<NT>(x, tot);
-        if (i < S.N) S.rowpre[i] = carry + ex + x;
-        carry += tot;
+// One CTA per child: contracts the child's copy of the source to its target and writes the labels, member
+// lists and the quotient's lists. The row sums that came with the source are scanned here (one segment of
+// `cr` rows per entry of a coarse index in shared memory; cr = 1 up to kCoarseRows vertices), so a step needs
+// no kernel for their prefix. Draws are made as the contraction asks for them -- at least as many as links
+// are still wanted -- not a whole round of N at once: the stream is indexed by the draw, so those not made
+// change nothing. A draw: its stream block (four draws each) and position, its row by the index, its
+// 32-column block by eight-way search of the row's block prefixes, its column from one 128-byte load of
+// the block (u32).
+//   Bound by the latency of the serial phases (block prefix and column loads, about 20 block barriers,
+// the union-find), so what counts is how many CTAs an SM holds: kContractSmall threads up to
+// kContractSmallN source vertices, kContractMid up to kContractMidN, else kNT.
+//   With 512 threads at every size, a prefix kernel per step, whole rounds of draws (a stream block each),
+// binary searches in global memory and labels read back from there, K4000's 11 levels took 1.11 ms and
+// 0.09 ms of prefixes (14,336 sources of N = 182: 347 us), the three of ER(1000, 0.05) 67 us and 15 us, a
+// 64-graph batch 12.7 ms and 0.57 ms; this takes 0.52 ms (129 us), 42 us and 5.3 ms.
+constexpr uint32_t kContractSmall = 128, kContractSmallN = 256;
+constexpr uint32_t kContractMid = 256, kContractMidN = 724;
+
+__host__ __device__ __forceinline__ uint32_t contract_batch_cap(uint32_t N) { return N < kBatch ? (N + 3) & ~3u : kBatch; }
+
+// first index i in [0, len) with a[i] > y (a non-decreasing, a[len-1] > y), in global memory: seven probes in
+// flight per step; `before` receives a[i-1] (0 for i = 0)
+__device__ __forceinline__ uint32_t upper_bound8(const uint64_t *a, uint32_t len, uint64_t y, uint64_t &before) {
+    uint32_t lo = 0;
+    before = 0;
+    for (;;) {
+        const uint32_t s = (len + 7) / 8, last = lo + len - 1;
+        uint64_t x[7];
+#pragma unroll
+        for (uint32_t i = 0; i < 7; i++) x[i] = __ldg(a + min(lo + (i + 1) * s - 1, last));
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 7; i++)
+            if (x[i] <= y) {
+                c++;
+                before = x[i];
+            }
+        lo += c * s;
+        if (s == 1) return min(lo, last);
+        len = min(s, last + 1 - lo);
     }
 }
 
+// the column of one 32-column block (row starts are 16-byte aligned, so the block is too): first of the
+// block's `lim` entries whose running sum exceeds rem; lim if none does
+__device__ __forceinline__ uint32_t block_column(const uint32_t *p, uint32_t lim, uint64_t rem) {
+    uint4 x[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) x[q] = 4u * q < lim ? __ldg(reinterpret_cast<const uint4 *>(p) + q) : make_uint4(0, 0, 0, 0);
+    uint32_t acc = 0, c = 0;
+    const uint32_t r = (uint32_t)rem;  // row sums are below 2^32
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const uint32_t e[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            acc += 4u * q + i < lim ? e[i] : 0u;  // (entries past the last column are not defined)
+            c += acc <= r ? 1u : 0u;
+        }
+    }
+    return min(c, lim);
+}
+__device__ __forceinline__ uint32_t block_column(const uint64_t *p, uint32_t lim, uint64_t rem) {
+    uint64_t acc = 0;
+    uint32_t c = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        ulonglong2 x[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            x[q] = 16u * h + 2u * q < lim ? __ldg(reinterpret_cast<const ulonglong2 *>(p) + 8 * h + q) : make_ulonglong2(0, 0);
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            acc += 16u * h + 2u * q < lim ? x[q].x : 0ull;
+            c += acc <= rem ? 1u : 0u;
+            acc += 16u * h + 2u * q + 1 < lim ? x[q].y : 0ull;
+            c += acc <= rem ? 1u : 0u;
+        }
+    }
+    return min(c, lim);
+}
+
 template <int NT, typename Tm>
-__global__ void __launch_bounds__(NT) contract_kernel(const TaskDesc *__restrict__ tasks,
-                                                      const SrcDesc *__restrict__ srcs, uint32_t *__restrict__ k_out,
+__global__ void __launch_bounds__(NT, 1024 / NT) contract_kernel(const TaskDesc *__restrict__ tasks, const SrcDesc *__restrict__ srcs,
+                                                      const uint32_t *__restrict__ list, uint32_t *__restrict__ k_out,
                                                       uint32_t *err) {
     extern __shared__ __align__(16) unsigned char dsm[];
-    uint2 *sb = reinterpret_cast<uint2 *>(dsm);
-    uint64_t *crow = reinterpret_cast<uint64_t *>(dsm + kBatch * sizeof(uint2));  // coarse row index
     __shared__ uint32_t s_count, s_nlog;
-    const TaskDesc T = tasks[blockIdx.x];
+    const uint32_t task = list[blockIdx.x];
+    const TaskDesc T = tasks[task];
     const SrcDesc S = srcs[T.src];
-    const uint32_t N = S.N;
-    uint32_t *par = reinterpret_cast<uint32_t *>(dsm + kBatch * sizeof(uint2) + kCoarseRows * sizeof(uint64_t));
-    uint32_t *cnt = par + N;  // counting-sort counters, N entries
     if (!width_is<Tm>(S.small)) return;
+    const uint32_t N = S.N, cap = contract_batch_cap(N), lane = threadIdx.x & 31;
+    // row prefix at the end of every `cr`-row segment (every row when N <= kCoarseRows)
+    const uint32_t cr = (N + kCoarseRows - 1) / kCoarseRows;
+    const uint32_t ncr = (N + cr - 1) / cr;
+    uint64_t *crow = reinterpret_cast<uint64_t *>(dsm);         // ncr entries: coarse row index
+    uint2 *sb = reinterpret_cast<uint2 *>(crow + ncr);          // cap draws
+    uint32_t *par = reinterpret_cast<uint32_t *>(sb + cap);     // N: union-find, then label | root flag
+    uint32_t *cnt = par + N;                                    // N: labels of roots, then member offsets
+    uint32_t *num = cnt + N;                                    // N: members beside the first, then scatter cursors
     const Tm *mat = reinterpret_cast<const Tm *>(S.mat);
-    const uint64_t W = S.rowpre[N - 1];
+    for (uint32_t v = threadIdx.x; v < N; v += NT) {
+        par[v] = v;
+        num[v] = 0;
+    }
+    if (threadIdx.x == 0) s_count = N;
+    uint64_t W;
+    {  // a thread's segments are consecutive, so one block scan orders them all
+        const uint32_t per = (ncr + NT - 1) / NT, i0 = min(threadIdx.x * per, ncr), i1 = min(i0 + per, ncr);
+        uint64_t sum = 0;
+        for (uint32_t r = i0 * cr; r < min(i1 * cr, N); r++) sum += __ldg(S.rowsum + r);
+        uint64_t run = block_excl_scan_u64<NT>(sum, W);
+        for (uint32_t i = i0; i < i1; i++) {
+            for (uint32_t r = i * cr; r < min((i + 1) * cr, N); r++) run += __ldg(S.rowsum + r);
+            crow[i] = run;
+        }
+    }
     if (W == 0) {  // no edges between the vertices: the cut is 0, nothing to contract
         if (threadIdx.x == 0) {
-            k_out[blockIdx.x] = kDropped;
+            k_out[task] = kDropped;
             atomicMin((unsigned long long *)T.cut, 0ull);
         }
         return;
     }
-    // row prefix at the end of every `cr`-row segment (every row when N <= kCoarseRows)
-    const uint32_t cr = (N + kCoarseRows - 1) / kCoarseRows;
-    const uint32_t ncr = (N + cr - 1) / cr;
-    for (uint32_t v = threadIdx.x; v < N; v += NT) par[v] = v;
-    for (uint32_t i = threadIdx.x; i < ncr; i += NT) crow[i] = S.rowpre[min(N, (i + 1) * cr) - 1];
-    if (threadIdx.x == 0) s_count = N;
     __syncthreads();
-    for (uint32_t base = 0; base < N; base += kBatch) {
-        const uint32_t nb = min((uint32_t)kBatch, N - base);
+    for (uint32_t base = 0; base < N;) {
+        // a little more than the links still wanted, whole passes of the CTA
+        const uint32_t need = s_count - T.target;
+        const uint32_t nb = min(min(cap, N - base), (need + need / 8 + 32 + NT - 1) / NT * NT);
+        for (uint32_t q = threadIdx.x; 4 * q < nb; q += NT) {
+            const u64x4 o = sitmo_block(T.k0, T.idx, T.tag, 0, (base >> 2) + q, T.round, 0, 0);
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                const uint64_t y = mulhi64(o.x[i], W);
+                sb[4 * q + i] = make_uint2((uint32_t)y, (uint32_t)(y >> 32));
+            }
+        }
+        __syncthreads();
         for (uint32_t j = threadIdx.x; j < nb; j += NT) {
-            const uint64_t y = mulhi64(draw64(T.k0, T.idx, T.tag, 0, T.round, base + j), W);
+            const uint2 yy = sb[j];
+            const uint64_t y = (uint64_t)yy.y << 32 | yy.x;
             // row: first whose inclusive prefix exceeds y (segment in shared memory, then inside it)
             const uint32_t sg = (uint32_t)upper_bound_u64(crow, ncr, y);
-            uint32_t a;
-            uint64_t before;
-            if (cr == 1) {
-                a = sg;
-                before = a ? crow[a - 1] : 0;
-            } else {
-                const uint32_t r0 = sg * cr;
-                a = r0 + (uint32_t)upper_bound_u64(S.rowpre + r0, min(cr, N - r0), y);
-                before = a ? S.rowpre[a - 1] : 0;
-            }
-            const uint64_t rem = y - before;
-            const uint64_t *B = S.blk + (uint64_t)a * S.nb;
-            const uint32_t b = (uint32_t)upper_bound_u64(B, S.nb, rem);
-            const uint64_t rem2 = rem - (b ? B[b - 1] : 0);
-            const uint64_t rb = (uint64_t)a * ld_of(N) + (uint64_t)b * 32;
-            const uint32_t lim = min(32u, N - b * 32);
-            // column: first whose running sum exceeds rem2, eight entries loaded together per step
-            uint64_t acc = 0;
-            uint32_t c = lim;
-            for (uint32_t c0 = 0; c0 < lim && c == lim; c0 += 8) {
-                uint64_t x[8];
-#pragma unroll
-                for (int k = 0; k < 8; k++) x[k] = c0 + k < lim ? (uint64_t)__ldg(mat + rb + c0 + k) : 0;
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    acc += x[k];
-                    if (c == lim && c0 + k < lim && acc > rem2) c = c0 + k;
+            uint32_t a = sg * cr;
+            uint64_t before = sg ? crow[sg - 1] : 0;
+            if (cr > 1) {
+                const uint32_t r1 = min(a + cr, N) - 1;
+                for (; a < r1; a++) {
+                    const uint64_t x = __ldg(S.rowsum + a);
+                    if (before + x > y) break;
+                    before += x;
                 }
             }
+            const uint64_t rem = y - before;
+            uint64_t left;
+            const uint32_t b = upper_bound8(S.blk + (uint64_t)a * S.nb, S.nb, rem, left);
+            const uint32_t lim = min(32u, N - b * 32);
+            uint32_t c = block_column(mat + (uint64_t)a * ld_of(N) + (uint64_t)b * 32, lim, rem - left);
             if (c >= lim) {  // cannot happen with consistent prefixes; record and clamp
                 atomicOr(err, 1u);
                 c = lim - 1;
             }
             sb[j] = make_uint2(a, b * 32 + c);
         }
-        __syncthreads();
         contract_batch<NT>(par, sb, nb, T.target, &s_count, &s_nlog);
         if (s_count <= T.target) break;
+        base += nb;
     }
-    for (uint32_t v = threadIdx.x; v < N; v += NT) par[v] = sfind_ro(par, v);
-    __syncthreads();
-    rank_labels<NT>(par, N, T.lab);
     const uint32_t k = s_count;
+    // labels: a root's rank among the roots, every vertex its root's. groups of 32 vertices are ranked by ballots
+    // and one block scan over the groups' counts (at most NT of them)
+    __shared__ uint32_t s_group[NT];
+    const uint32_t groups = (N + 31) / 32;
+    for (uint32_t g = threadIdx.x / 32; g < groups; g += NT / 32) {
+        const uint32_t v = g * 32 + lane;
+        uint32_t r = v;
+        if (v < N) par[v] = r = sfind_ro(par, v);
+        const uint32_t roots = __ballot_sync(0xffffffffu, v < N && r == v);
+        if (lane == 0) s_group[g] = __popc(roots);
+    }
+    __syncthreads();
+    uint32_t total;
+    uint32_t ex = block_excl_scan_u32<NT>(threadIdx.x < groups ? s_group[threadIdx.x] : 0, total);
+    if (threadIdx.x < groups) s_group[threadIdx.x] = ex;
+    __syncthreads();
+    for (uint32_t g = threadIdx.x / 32; g < groups; g += NT / 32) {
+        const uint32_t v = g * 32 + lane;
+        const bool root = v < N && par[v] == v;
+        const uint32_t roots = __ballot_sync(0xffffffffu, root);
+        if (root) cnt[v] = s_group[g] + __popc(roots & ((1u << lane) - 1));
+    }
     // member lists grouped by label, and the quotient's row order and column lists (order inside a group
-    // is irrelevant): cnt[l] first counts the group's members beside its first
+    // is irrelevant): num[l] first counts the group's members beside its first
     __shared__ uint32_t s_hist[kEll + 2], s_pos[kEll + 2], s_off[kEll], s_base[2];
     if (threadIdx.x < kEll + 2) s_hist[threadIdx.x] = 0;
-    for (uint32_t l = threadIdx.x; l < k; l += NT) cnt[l] = 0;
     __syncthreads();
-    for (uint32_t v = threadIdx.x; v < N; v += NT)
-        if (par[v] != v) atomicAdd(&cnt[T.lab[v]], 1u);
-    __syncthreads();
-    uint32_t off = 0;
-    for (uint32_t base = 0; base < k; base += NT) {
-        const uint32_t l = base + threadIdx.x;
-        const uint32_t x = l < k ? cnt[l] : 0;
-        uint32_t tot;
-        const uint32_t ex = block_excl_scan_u32<NT>(l < k ? x + 1 : 0, tot);
-        if (l < k) T.memb_off[l] = (uint16_t)(off + ex);
-        if (x) atomicAdd(&s_hist[min(x, kEll + 1)], 1u);
-        off += tot;
+    for (uint32_t v = threadIdx.x; v < N; v += NT) {
+        const uint32_t r = par[v], l = cnt[r];
+        T.lab[v] = (uint16_t)l;
+        if (r != v) atomicAdd(&num[l], 1u);
+        par[v] = r == v ? l | kRootFlag : l;
     }
-    if (threadIdx.x == 0) T.memb_off[k] = (uint16_t)N;
     __syncthreads();
-    const uint32_t nbig = s_hist[kEll + 1], lane = threadIdx.x & 31;
+    const uint32_t lgroups = (k + 31) / 32;
+    for (uint32_t g = threadIdx.x / 32; g < lgroups; g += NT / 32) {
+        const uint32_t l = g * 32 + lane, x = l < k ? num[l] : 0;
+        if (x) atomicAdd(&s_hist[min(x, kEll + 1)], 1u);
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, l < k ? x + 1 : 0);
+        if (lane == 0) s_group[g] = sum;
+    }
+    __syncthreads();
+    const uint32_t nbig = s_hist[kEll + 1];
     if (threadIdx.x < kEll) {  // joined[j] = small groups with more than j: a suffix sum over the warp's lanes
         const uint32_t j = threadIdx.x;
         uint32_t joined = s_hist[j + 1];
@@ -581,11 +692,20 @@ __global__ void __launch_bounds__(NT) contract_kernel(const TaskDesc *__restrict
             s_base[1] = s_base[0] + ((nell + 1) & ~1u);
         }
     }
+    ex = block_excl_scan_u32<NT>(threadIdx.x < lgroups ? s_group[threadIdx.x] : 0, total);
+    if (threadIdx.x < lgroups) s_group[threadIdx.x] = ex;
+    if (threadIdx.x == 0) T.memb_off[k] = (uint16_t)N;
     __syncthreads();
     uint16_t *first = T.cols + kColHead, *ell = T.cols + s_base[0], *multi = T.cols + s_base[1];
-    for (uint32_t base = 0; base < k; base += NT) {
-        const uint32_t l = base + threadIdx.x;
-        const uint32_t x = l < k ? cnt[l] : 1u;
+    for (uint32_t g = threadIdx.x / 32; g < lgroups; g += NT / 32) {
+        const uint32_t l = g * 32 + lane, x = l < k ? num[l] : 1u;
+        uint32_t incl = l < k ? x + 1 : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const uint32_t off = s_group[g] + incl - (x + 1);
         const uint32_t single = __ballot_sync(0xffffffffu, x == 0);  // most groups: one atomic per warp
         uint32_t at = 0, pos = 0xFFFFu;
         if (lane == 0 && single) at = atomicAdd(&s_pos[0], (uint32_t)__popc(single));
@@ -593,25 +713,27 @@ __global__ void __launch_bounds__(NT) contract_kernel(const TaskDesc *__restrict
         if (l < k) {
             if (x > kEll) at = atomicAdd(&s_pos[kEll + 1], 1u);
             else if (x) at = nbig + (pos = atomicAdd(&s_pos[x], 1u));
-            T.rows[at] = l | (uint32_t)T.memb_off[l] << 16;
-            cnt[l] = pos << 16;  // becomes (position among the small groups, scatter cursor)
+            T.rows[at] = l | off << 16;
+            T.memb_off[l] = (uint16_t)off;
+            cnt[l] = off;
+            num[l] = pos << 16;  // becomes (position among the small groups, scatter cursor)
         }
     }
     __syncthreads();
     for (uint32_t v = threadIdx.x; v < N; v += NT) {
-        const uint32_t l = T.lab[v], at = T.memb_off[l];
-        if (par[v] == v) {
+        const uint32_t l = par[v] & ~kRootFlag, at = cnt[l];
+        if (par[v] & kRootFlag) {
             T.members[at] = (uint16_t)v;
             first[l] = (uint16_t)v;
-            const uint32_t pos = cnt[l] >> 16;
+            const uint32_t pos = num[l] >> 16;
             if (pos != 0xFFFFu) multi[pos] = (uint16_t)v;
         } else {
-            const uint32_t c = atomicAdd(&cnt[l], 1u), rank = c & 0xFFFFu, pos = c >> 16;
+            const uint32_t c = atomicAdd(&num[l], 1u), rank = c & 0xFFFFu, pos = c >> 16;
             T.members[at + 1 + rank] = (uint16_t)v;
             if (pos != 0xFFFFu) ell[s_off[rank] + pos] = (uint16_t)v;
         }
     }
-    if (threadIdx.x == 0) k_out[blockIdx.x] = k;
+    if (threadIdx.x == 0) k_out[task] = k;
 }
 
 // ---------------------------------------------------------------- quotient
@@ -1432,7 +1554,9 @@ int upload(cac_ctx *ctx, DevBuf &buf, const std::vector<T> &v) {
 }
 
 size_t leaf_smem(uint32_t N, bool small) { return ((size_t)N * (N - 1) / 2 + 1) * (small ? 4 : 8); }
-size_t contract_smem(uint32_t N) { return kBatch * sizeof(uint2) + kCoarseRows * sizeof(uint64_t) + (size_t)2 * N * 4; }
+size_t contract_smem(uint32_t N) {
+    return (size_t)std::min(N, kCoarseRows) * sizeof(uint64_t) + contract_batch_cap(N) * sizeof(uint2) + (size_t)3 * N * 4;
+}
 
 }  // namespace
 
@@ -1617,24 +1741,20 @@ int KsEngine::step() {
         S.is_root = nd.is_root;
         S.small = nd.small;
         if (nd.pre) {
-            S.rowpre = nd.pre;
+            S.rowsum = nd.pre;
         } else {
-            S.rowpre = d_prep.as<uint64_t>() + pe;
+            S.rowsum = d_prep.as<uint64_t>() + pe;
             pe += nd.N + (uint64_t)nd.N * S.nb;
             row_off.push_back(rows);
             rows += nd.N;
         }
-        S.blk = S.rowpre + nd.N;
+        S.blk = S.rowsum + nd.N;
         if (!nd.pre) psrcs.push_back(S);
     }
 
     // contraction of every child
     uint64_t tscratch = 0;
-    uint32_t maxN = 0;
-    for (const KTask &t : tasks) {
-        tscratch += task_words(t.src.N);
-        maxN = std::max(maxN, t.src.N);
-    }
+    for (const KTask &t : tasks) tscratch += task_words(t.src.N);
     CAC_TRY(d_tscratch.ensure(tscratch * 4));
     std::vector<TaskDesc> td(tasks.size());
     uint64_t ts = 0;
@@ -1658,13 +1778,28 @@ int KsEngine::step() {
         ts += task_words(N);
     }
     CAC_TRY(d_kout.ensure(tasks.size() * 4));
-    // one descriptor copy for the sources, the row-prep list and the tasks
+    // the contraction's launches: tasks by the size class of their source and its entry width
+    std::vector<uint32_t> list;
+    uint32_t list_num[6] = {}, list_max[6] = {};
+    auto class_of = [](const KNode &src) {
+        return (src.N <= kContractSmallN ? 4 : src.N <= kContractMidN ? 2 : 0) + (src.small ? 0 : 1);
+    };
+    for (int c = 0; c < 6; c++) {
+        for (size_t i = 0; i < tasks.size(); i++) {
+            if (class_of(tasks[i].src) != c) continue;
+            list.push_back((uint32_t)i);
+            list_num[c]++;
+            list_max[c] = std::max(list_max[c], tasks[i].src.N);
+        }
+    }
+    // one descriptor copy for the sources, the row-prep list, the tasks and their launch lists
     CAC_TRY(pre_st.begin(Staging::bytes_of(srcs) + Staging::bytes_of(row_off) + Staging::bytes_of(psrcs) +
-                         Staging::bytes_of(td)));
+                         Staging::bytes_of(td) + Staging::bytes_of(list)));
     const SrcDesc *dv_src = pre_st.put(srcs);
     const uint64_t *dv_rowoff = pre_st.put(row_off);
     const SrcDesc *dv_psrc = pre_st.put(psrcs);
     const TaskDesc *dv_task = pre_st.put(td);
+    const uint32_t *dv_list = pre_st.put(list);
     CAC_TRY(pre_st.flush());
     if (rows) {
         bool p32 = false, p64 = false;
@@ -1675,20 +1810,28 @@ int KsEngine::step() {
         if (p64)
             prep_rows_kernel<uint64_t><<<pg, 256, 0, s>>>(dv_psrc, dv_rowoff, (uint32_t)row_off.size(), rows);
     }
-    prefix_rows_kernel<kNT><<<(unsigned)srcs.size(), kNT, 0, s>>>(dv_src);
     bool t32 = false, t64 = false;  // entry widths present among the tasks' sources
     for (const KTask &t : tasks) (t.src.small ? t32 : t64) = true;
     {
-        const size_t sm = contract_smem(maxN);
-        if (t32) {
-            CAC_TRY(smem_optin(ctx_, contract_kernel<kNT, uint32_t>));
-            contract_kernel<kNT, uint32_t><<<(unsigned)tasks.size(), kNT, sm, s>>>(
-                dv_task, dv_src, d_kout.as<uint32_t>(), d_err);
-        }
-        if (t64) {
-            CAC_TRY(smem_optin(ctx_, contract_kernel<kNT, uint64_t>));
-            contract_kernel<kNT, uint64_t><<<(unsigned)tasks.size(), kNT, sm, s>>>(
-                dv_task, dv_src, d_kout.as<uint32_t>(), d_err);
+        // the largest sources first; a launch takes what its size class has of one entry width
+        const uint32_t *d_list = dv_list;
+        auto launch = [&](auto nt, auto tm, uint32_t big, uint32_t num) -> int {
+            if (!num) return CAC_OK;
+            auto kern = contract_kernel<decltype(nt)::value, decltype(tm)>;
+            CAC_TRY(smem_optin(ctx_, kern));
+            kern<<<num, decltype(nt)::value, contract_smem(big), s>>>(dv_task, dv_src, d_list, d_kout.as<uint32_t>(), d_err);
+            d_list += num;
+            return CAC_OK;
+        };
+        for (int c = 0; c < 6; c++) {
+            const uint32_t big = list_max[c], num = list_num[c];
+            using std::integral_constant;
+            if (c == 0) CAC_TRY(launch(integral_constant<int, kNT>(), uint32_t(), big, num));
+            if (c == 1) CAC_TRY(launch(integral_constant<int, kNT>(), uint64_t(), big, num));
+            if (c == 2) CAC_TRY(launch(integral_constant<int, kContractMid>(), uint32_t(), big, num));
+            if (c == 3) CAC_TRY(launch(integral_constant<int, kContractMid>(), uint64_t(), big, num));
+            if (c == 4) CAC_TRY(launch(integral_constant<int, kContractSmall>(), uint32_t(), big, num));
+            if (c == 5) CAC_TRY(launch(integral_constant<int, kContractSmall>(), uint64_t(), big, num));
         }
         CAC_CUDA_TRY(cudaGetLastError());
     }
