@@ -199,6 +199,7 @@ __device__ void contract_batch(uint32_t *par, const uint2 *sb, uint32_t nb, uint
         if (c <= target || j0 >= nb) break;
         const uint32_t need = c - target;
         if (need <= kWarpTail) {
+            __syncthreads();  // every warp has read *s_count before the tail writes it
             if (threadIdx.x < 32) {
                 // 32 draws at a time: those that are loops already stay so; the first `left` others are
                 // linked (at most once each, so the count cannot fall below target), the rest looked at again
