@@ -471,16 +471,18 @@ constexpr uint32_t kContractMid = 256, kContractMidN = 724;
 
 __host__ __device__ __forceinline__ uint32_t contract_batch_cap(uint32_t N) { return N < kBatch ? (N + 3) & ~3u : kBatch; }
 
-// first index i in [0, len) with a[i] > y (a non-decreasing, a[len-1] > y), in global memory: seven probes in
-// flight per step; `before` receives a[i-1] (0 for i = 0)
-__device__ __forceinline__ uint32_t upper_bound8(const uint64_t *a, uint32_t len, uint64_t y, uint64_t &before) {
-    uint32_t lo = 0;
+// first index i in [0, end) with a[i] > y (a non-decreasing, a[end-1] > y), in global memory: seven probes in
+// flight per step; `before` receives a[i-1] (0 for i = 0). In [0, end) whatever a holds: below a child that a
+// run planned ahead and that stopped off its target, matrices and prefixes were never written (the run is
+// redone, but these contractions still draw from them).
+__device__ __forceinline__ uint32_t upper_bound8(const uint64_t *a, uint32_t end, uint64_t y, uint64_t &before) {
+    uint32_t lo = 0, len = end;
     before = 0;
     for (;;) {
-        const uint32_t s = (len + 7) / 8, last = lo + len - 1;
+        const uint32_t s = (len + 7) / 8;
         uint64_t x[7];
 #pragma unroll
-        for (uint32_t i = 0; i < 7; i++) x[i] = __ldg(a + min(lo + (i + 1) * s - 1, last));
+        for (uint32_t i = 0; i < 7; i++) x[i] = __ldg(a + min(lo + (i + 1) * s - 1, end - 1));
         uint32_t c = 0;
 #pragma unroll
         for (uint32_t i = 0; i < 7; i++)
@@ -488,9 +490,9 @@ __device__ __forceinline__ uint32_t upper_bound8(const uint64_t *a, uint32_t len
                 c++;
                 before = x[i];
             }
-        lo += c * s;
-        if (s == 1) return min(lo, last);
-        len = min(s, last + 1 - lo);
+        lo = min(lo + c * s, end - 1);
+        if (s == 1) return lo;
+        len = min(s, end - lo);
     }
 }
 

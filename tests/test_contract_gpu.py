@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+import graphgen
 import pyoracle as O
 
 pytestmark = pytest.mark.gpu
@@ -27,3 +28,23 @@ def _weights(n, kind, seed):
 def test_trial_matches_replay(ctx, n, kind):
     mat = _weights(n, kind, n)
     assert ctx.ks_dense(mat, 3, 1, 5) == O.ks_dense(mat, 3, 1, 5)
+
+
+@pytest.mark.parametrize("n", [300, 700, 1500])
+def test_children_below_a_missed_target_stay_in_range(libcac, n):
+    # a run planned ahead whose first children stop off their target draws, below them, from matrices and
+    # prefixes that hold what earlier runs left in the memory
+    for seed in range(3):
+        c = libcac.Context(0)
+        try:
+            c.generate("erdos_renyi_m", seed=seed, n=2 * n, avg_degree=200, wmax=9).trials(seed, 1, 4)
+            c.generate("watts_strogatz", seed=seed, n=3 * n, k=20, p=0.3, wmax=1 << 20).trials(seed, 1, 4)
+            n, u, v, w = graphgen.complete(n, seed, wmax=1)
+            w = np.asarray(w, np.uint32).copy()
+            w[0] = 1 << 31  # nearly every draw
+            got = c.graph(n, u, v, w).trials(seed=3, virtual_ranks=1, trials_per_rank=2)
+            assert c.plan_redos() == 1
+            for i in range(2):
+                assert int(got[0, i]) == O.mincut_trial(n, u, v, w, 3, 0, i)
+        finally:
+            c.close()
