@@ -42,3 +42,26 @@ def test_leaf_path_and_star(ctx):
     star[0, 1:] = star[1:, 0] = 9
     for mat in (path, path[::-1, ::-1].copy(), star):
         assert ctx.exact_cut_small(mat) == O.stoer_wagner_dense(mat)
+
+
+# leaves solved straight from their source: 1 to 51 joined vertices, above 179 none; both entry widths,
+# groups of one to dozens of members, planned ahead (a graph's trials) and level by level (a matrix)
+@pytest.mark.parametrize("wmax", [9, 1 << 20, 1 << 31])
+@pytest.mark.parametrize("hub", [False, True])
+@pytest.mark.parametrize("n", [129, 130, 159, 160, 161, 178, 179, 180, 181])
+def test_trial_with_leaf_children(ctx, n, hub, wmax):
+    rng = np.random.default_rng(n + hub)
+    u, v = np.triu_indices(n, 1)
+    w = rng.integers(1, wmax, len(u), endpoint=True).astype(np.uint64)
+    if hub:  # most draws join a few vertices
+        heavy = (v < 12) | (rng.random(len(u)) < 0.01)
+        w = np.where(heavy, w, w // 9 + 1)
+    keep = rng.random(len(u)) < 0.7
+    u, v, w = u[keep].astype(np.uint32), v[keep].astype(np.uint32), w[keep].astype(np.uint32)
+    got = ctx.graph(n, u, v, w).trials(seed=5, virtual_ranks=1, trials_per_rank=2)
+    for i in range(2):
+        assert int(got[0, i]) == O.mincut_trial(n, u, v, w, 5, 0, i)
+    mat = np.zeros((n, n), np.uint64)
+    mat[u, v] = w
+    mat[v, u] = w
+    assert ctx.ks_dense(mat, 5, 0, 1) == O.ks_dense(mat, 5, 0, 1)
