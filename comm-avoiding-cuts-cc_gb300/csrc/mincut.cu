@@ -1278,7 +1278,7 @@ __device__ __forceinline__ uint64_t warp_max(uint64_t x) {
 }
 __device__ __forceinline__ uint32_t warp_max(uint32_t x) { return __reduce_max_sync(0xffffffffu, x); }
 
-constexpr uint32_t kLeafThreads = 32;
+constexpr uint32_t kLeafThreads = 128;  // they load; warp 0 solves
 __device__ __forceinline__ uint32_t tri(uint32_t i) { return i * (i - 1) / 2; }
 __device__ __forceinline__ uint32_t tpos(uint32_t i, uint32_t j) { return i > j ? tri(i) + j : tri(j) + i; }
 
@@ -1394,6 +1394,26 @@ __device__ __forceinline__ uint64_t leaf_cut(Tm *M, uint32_t N, uint64_t lambda,
     return lambda;
 }
 
+// The lower triangle, asynchronously: warp w copies rows 1 + w, 1 + w + 4, ... (a lone warp took 15 thousand
+// cycles to issue the copies, about as long as an ordering takes). row(i): where row i is; col(q): the column there
+// of the lane's vertex lane + 32 q.
+template <typename Tm, typename Row, typename Col>
+__device__ __forceinline__ void leaf_copy(Tm *M, uint32_t N, Row row, Col col) {
+    constexpr uint32_t kWarps = kLeafThreads / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    uint32_t c[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) c[q] = col(q);
+#pragma unroll 4
+    for (uint32_t i = 1 + warp; i < N; i += kWarps) {
+        const Tm *src = row(i);
+        Tm *dst = M + tri(i) + lane;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++)
+            if (lane + 32 * q < i) copy_entry_async(dst + 32 * q, src + c[q]);
+    }
+}
+
 // From the matrix and the degrees of the lane's vertices: lambda starts at the minimum weighted degree (a
 // cut of the leaf).
 template <typename Tm>
@@ -1426,26 +1446,16 @@ __global__ void __launch_bounds__(kLeafThreads) sw_leaf_kernel(const LeafDesc *_
     Tm *M = reinterpret_cast<Tm *>(dsm);  // N (N - 1) / 2 entries and one that is read but not used
     __shared__ uint8_t root[128];
     const LeafDesc L = leaves[blockIdx.x];
-    const uint32_t N = L.N, lane = threadIdx.x;
-    {
-        const Tm *src = reinterpret_cast<const Tm *>(L.mat) + lane;
-        const uint64_t ldN = ld_of(N);
-        Tm *dst = M + lane;
-#pragma unroll 4
-        for (uint32_t i = 1; i < N; i++) {
-            src += ldN;
-#pragma unroll
-            for (uint32_t j = 0; j < 128; j += 32)
-                if (lane + j < i) copy_entry_async(dst + j, src + j);
-            dst += i;
-        }
-    }
+    const uint32_t N = L.N, lane = threadIdx.x & 31;
+    leaf_copy(M, N, [&](uint32_t i) { return reinterpret_cast<const Tm *>(L.mat) + i * ld_of(N); },
+              [&](int q) { return lane + 32 * q; });
     // degrees: the row sums that came with the matrix, else summed here
     uint64_t deg[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) deg[q] = L.rowsum && lane + 32 * q < N ? __ldg(L.rowsum + lane + 32 * q) : 0;
     asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         const uint32_t v = lane + 32 * q;
@@ -1476,38 +1486,34 @@ __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *
     __shared__ unsigned long long s_deg[kLeafN];
     __shared__ uint16_t s_first[kLeafN], s_joined[kLeafN];  // s_joined: vertex | label << 8
     __shared__ uint8_t root[kLeafN];
-    const uint32_t task = list[blockIdx.x], lane = threadIdx.x;
+    const uint32_t task = list[blockIdx.x], lane = threadIdx.x & 31;
     const TaskDesc T = tasks[task];
     const SrcDesc S = srcs[T.src];
     const uint32_t N = S.N, k = T.target;
     if (k_act[task] != k) {  // planned ahead, and this child stopped off its target: redo the run
-        if (lane == 0) atomicOr(err, kErrPlan);
+        if (threadIdx.x == 0) atomicOr(err, kErrPlan);
         return;
     }
     const Tm *mat = reinterpret_cast<const Tm *>(S.mat);
     const uint64_t ldN = ld_of(N);
+    if (threadIdx.x < kLeafN) s_first[threadIdx.x] = threadIdx.x < k ? T.cols[kColHead + threadIdx.x] : (uint16_t)0;
+    __syncthreads();
     uint32_t f[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) f[q] = s_first[lane + 32 * q];
+    leaf_copy(M, k, [&](uint32_t i) { return mat + s_first[i] * ldN; }, [&](int q) { return f[q]; });
+    if (threadIdx.x >= 32) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        return;
+    }
     uint64_t deg[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        const uint32_t l = lane + 32 * q;
-        f[q] = l < k ? T.cols[kColHead + l] : 0;
-        deg[q] = l < k ? __ldg(S.rowsum + f[q]) : 0;
-        s_first[l] = (uint16_t)f[q];
-        s_deg[l] = 0;
+        deg[q] = lane + 32 * q < k ? __ldg(S.rowsum + f[q]) : 0;
+        s_deg[lane + 32 * q] = 0;
     }
     __syncwarp();
-    {
-        Tm *dst = M + lane;
-#pragma unroll 4
-        for (uint32_t i = 1; i < k; i++) {
-            const Tm *src = mat + s_first[i] * ldN;
-#pragma unroll
-            for (uint32_t q = 0; q < 4; q++)
-                if (lane + 32 * q < i) copy_entry_async(dst + 32 * q, src + f[q]);
-            dst += i;
-        }
-    }
     // the joined vertices, ascending
     uint32_t joined = 0;
     for (uint32_t v0 = 0; v0 < N; v0 += 32) {
@@ -1538,7 +1544,7 @@ __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *
         }
         if (!waited) {
             asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncwarp();
+            __syncthreads();
             waited = true;
         }
 #pragma unroll
@@ -1564,7 +1570,7 @@ __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *
     }
     if (!waited) {
         asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
+        __syncthreads();
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) deg[q] += s_deg[lane + 32 * q];
