@@ -1278,7 +1278,7 @@ __device__ __forceinline__ uint64_t warp_max(uint64_t x) {
 }
 __device__ __forceinline__ uint32_t warp_max(uint32_t x) { return __reduce_max_sync(0xffffffffu, x); }
 
-constexpr uint32_t kLeafThreads = 128;  // they load; warp 0 solves
+constexpr uint32_t kLeafThreads = 128, kLeafWarps = kLeafThreads / 32;  // they load; warp 0 solves
 __device__ __forceinline__ uint32_t tri(uint32_t i) { return i * (i - 1) / 2; }
 __device__ __forceinline__ uint32_t tpos(uint32_t i, uint32_t j) { return i > j ? tri(i) + j : tri(j) + i; }
 
@@ -1399,13 +1399,12 @@ __device__ __forceinline__ uint64_t leaf_cut(Tm *M, uint32_t N, uint64_t lambda,
 // of the lane's vertex lane + 32 q.
 template <typename Tm, typename Row, typename Col>
 __device__ __forceinline__ void leaf_copy(Tm *M, uint32_t N, Row row, Col col) {
-    constexpr uint32_t kWarps = kLeafThreads / 32;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x / 32;
     uint32_t c[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) c[q] = col(q);
 #pragma unroll 4
-    for (uint32_t i = 1 + warp; i < N; i += kWarps) {
+    for (uint32_t i = 1 + warp; i < N; i += kLeafWarps) {
         const Tm *src = row(i);
         Tm *dst = M + tri(i) + lane;
 #pragma unroll
@@ -1468,14 +1467,13 @@ __global__ void __launch_bounds__(kLeafThreads) sw_leaf_kernel(const LeafDesc *_
 // The leaf of a contraction to kLeafN vertices, straight from its source (N <= 179): its matrix, the child's
 // quotient, is never written. The entries between first vertices of two groups are copied as in
 // sw_leaf_kernel, at the columns of the first vertices (ascending, so the copies stay nearly coalesced);
-// then the row of each joined vertex is added to its group's, four rows in flight: to the other groups'
-// entries from the first vertices' columns, a lane per group without conflicts, and from the columns of
-// the joined vertices before it with shared atomics (several may have one group). The degrees are the
-// source's row sums, less twice what lies inside the groups.
+// then the row of each joined vertex is added to its group's, four rows in flight per warp, from the first
+// vertices' columns and from those of the joined vertices before it, with shared atomics. The degrees are
+// the source's row sums, less twice what lies inside the groups.
 //   Before, the last level's quotients were written and read back: K4000 14,336 quotients of N = 181 and
-// their leaves 485 + 300 us, now 424 us; the plain Karger-Stein query on Watts-Strogatz n = 32,000 (524,288
-// children of N = 130 at a time) 18.7 + 8.3 ms, now 13.1 ms, and 37 GB less memory; ER(1000, 0.05) 44 +
-// 36 us, now 64 us.
+// their leaves 485 + 300 us, now 364 us; the plain Karger-Stein query on Watts-Strogatz n = 32,000 (524,288
+// children of N = 130 at a time) 18.7 + 8.3 ms, now 10.4 ms, and 37 GB less memory; ER(1000, 0.05) 44 +
+// 36 us, now 48 us. (One warp for the copies and the joined rows: 424 us, 13.1 ms, 64 us.)
 template <typename Tm>
 __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *__restrict__ tasks,
                                                                 const SrcDesc *__restrict__ srcs,
@@ -1486,7 +1484,7 @@ __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *
     __shared__ unsigned long long s_deg[kLeafN];
     __shared__ uint16_t s_first[kLeafN], s_joined[kLeafN];  // s_joined: vertex | label << 8
     __shared__ uint8_t root[kLeafN];
-    const uint32_t task = list[blockIdx.x], lane = threadIdx.x & 31;
+    const uint32_t task = list[blockIdx.x], lane = threadIdx.x & 31, warp = threadIdx.x / 32;
     const TaskDesc T = tasks[task];
     const SrcDesc S = srcs[T.src];
     const uint32_t N = S.N, k = T.target;
@@ -1502,40 +1500,30 @@ __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *
 #pragma unroll
     for (int q = 0; q < 4; q++) f[q] = s_first[lane + 32 * q];
     leaf_copy(M, k, [&](uint32_t i) { return mat + s_first[i] * ldN; }, [&](int q) { return f[q]; });
-    if (threadIdx.x >= 32) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        return;
-    }
-    uint64_t deg[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        deg[q] = lane + 32 * q < k ? __ldg(S.rowsum + f[q]) : 0;
-        s_deg[lane + 32 * q] = 0;
-    }
-    __syncwarp();
-    // the joined vertices, ascending
+    if (threadIdx.x < kLeafN) s_deg[threadIdx.x] = threadIdx.x < k ? __ldg(S.rowsum + s_first[threadIdx.x]) : 0;
+    __syncthreads();
+    // the joined vertices, ascending (every warp counts them, warp 0 lists them)
     uint32_t joined = 0;
     for (uint32_t v0 = 0; v0 < N; v0 += 32) {
         const uint32_t v = v0 + lane, l = v < N ? T.lab[v] : 0;
         const bool j = v < N && s_first[l] != v;
         const uint32_t js = __ballot_sync(0xffffffffu, j);
-        if (j) {
+        if (j && warp == 0) {
             s_joined[joined + __popc(js & ((1u << lane) - 1))] = (uint16_t)(v | l << 8);
             atomicAdd(&s_deg[l], (unsigned long long)__ldg(S.rowsum + v));
         }
         joined += __popc(js);
     }
-    __syncwarp();
+    __syncthreads();
     uint32_t other[2];  // the lane's joined vertices: lane and lane + 32
 #pragma unroll
     for (int q = 0; q < 2; q++) other[q] = lane + 32 * q < joined ? s_joined[lane + 32 * q] : 0;
     bool waited = false;
-    for (uint32_t p0 = 0; p0 < joined; p0 += 4) {
+    for (uint32_t p0 = 0; p0 < joined || !waited; p0 += 4 * kLeafWarps) {
         Tm a[4][4], b[4][2];
 #pragma unroll
         for (uint32_t u = 0; u < 4; u++) {
-            const uint32_t p = p0 + u;
+            const uint32_t p = p0 + u * kLeafWarps + warp;
             const Tm *row = mat + (p < joined ? s_joined[p] & 255u : 0) * ldN;
 #pragma unroll
             for (int q = 0; q < 4; q++) a[u][q] = p < joined && lane + 32 * q < k ? __ldg(row + f[q]) : Tm(0);
@@ -1549,31 +1537,24 @@ __global__ void __launch_bounds__(kLeafThreads) sw_child_kernel(const TaskDesc *
         }
 #pragma unroll
         for (uint32_t u = 0; u < 4; u++) {
-            if (p0 + u >= joined) break;
-            const uint32_t to = s_joined[p0 + u] >> 8, tt = tri(to);
+            const uint32_t p = p0 + u * kLeafWarps + warp;
+            if (p >= joined) break;
+            const uint32_t to = s_joined[p] >> 8, tt = tri(to);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const uint32_t l = lane + 32 * q;
-                if (l == to) deg[q] -= 2 * (uint64_t)a[u][q];
-                else if (l < k) M[l > to ? tri(l) + to : tt + l] += a[u][q];
+            for (int q = 0; q < 6; q++) {
+                const uint32_t l = q < 4 ? lane + 32 * q : other[q - 4] >> 8;
+                const Tm x = q < 4 ? a[u][q] : b[u][q - 4];
+                if (x == 0) continue;
+                if (l == to) atomicAdd(&s_deg[to], 0ull - 2 * (unsigned long long)x);
+                else sadd(&M[l > to ? tri(l) + to : tt + l], x);
             }
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const uint32_t l = other[q] >> 8;
-                if (b[u][q] == 0) continue;
-                if (l == to) atomicAdd(&s_deg[to], 0ull - 2 * (unsigned long long)b[u][q]);
-                else sadd(&M[tpos(l, to)], b[u][q]);
-            }
-            __syncwarp();
         }
     }
-    if (!waited) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-    }
+    __syncthreads();
+    if (warp > 0) return;
+    uint64_t deg[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) deg[q] += s_deg[lane + 32 * q];
+    for (int q = 0; q < 4; q++) deg[q] = s_deg[lane + 32 * q];
     leaf_solve(M, k, deg, root, T.cut);
 }
 
