@@ -411,39 +411,90 @@ __global__ void dense_build_kernel(const DenseDesc *__restrict__ descs) {
 
 // ---------------------------------------------------------------- stage 3: Karger-Stein
 
+// last i of [0, n) with first[i] <= x (first[0] = 0), by a warp: 32 probes per step
+__device__ __forceinline__ uint32_t warp_last_le(const uint64_t *__restrict__ first, uint32_t n, uint64_t x) {
+    uint32_t lo = 0, len = n;  // the answer is in [lo, lo + len)
+    while (len > 1) {
+        const uint32_t step = (len + 31) / 32, at = lo + step * (threadIdx.x & 31);
+        const uint32_t hits = __popc(__ballot_sync(0xffffffffu, at < lo + len && first[at] <= x));
+        const uint32_t end = lo + len;
+        lo += (hits - 1) * step;
+        len = min(step, end - lo);
+    }
+    return lo;
+}
+
 // One warp per matrix row: 32-column block prefixes and the row sum.
+//   u32 entries: 16-byte loads, four in flight (512 columns, 16 blocks); the eight lanes of a block add up
+// by a transposing reduction (4 shuffles for the 4 loads), one shuffle puts the 16 sums in order and a
+// 16-lane scan makes them prefixes. Row sums are below 2^32. Bound by memory and, for short rows, by the
+// latency of the search for the row's source (32-way) and of its loads.
+//   K4000's root (4000 rows) and 16.4 GB of children of N = 2005 of the Watts-Strogatz query: 54 us and
+// 3.0 ms; with a load per 32 columns, 64-bit shuffles (10 per block) and a binary search 181 us and 6.6 ms.
 template <typename Tm>
 __global__ void prep_rows_kernel(const SrcDesc *__restrict__ srcs, const uint64_t *__restrict__ row_off,
                                  uint32_t nsrc, uint64_t total_rows) {
     const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31;
     if (gw >= total_rows) return;
-    uint32_t lo = 0, hi = nsrc - 1;
-    while (lo < hi) {  // last source whose first row <= gw
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (row_off[mid] <= gw) lo = mid; else hi = mid - 1;
-    }
-    const SrcDesc S = srcs[lo];
-    const uint64_t i = gw - row_off[lo];
+    const uint32_t si = warp_last_le(row_off, nsrc, gw);  // last source whose first row <= gw
+    const SrcDesc S = srcs[si];
+    const uint64_t i = gw - row_off[si];
     if (!width_is<Tm>(S.small)) return;
     const Tm *mat = reinterpret_cast<const Tm *>(S.mat) + i * ld_of(S.N);
+    uint64_t *blk = S.blk + i * S.nb;
     uint64_t run = 0;
-    for (uint32_t b0 = 0; b0 < S.nb; b0 += 8) {  // eight 32-column blocks per pass, loads in flight together
-        uint64_t x[8];
+    if constexpr (sizeof(Tm) == 4) {
+        for (uint32_t c0 = 0; c0 < S.N; c0 += 512) {
+            uint32_t x[4];
+            uint4 v[4];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const uint32_t j = (b0 + u) * 32 + lane;
-            x[u] = (b0 + u < S.nb && j < S.N) ? (uint64_t)__ldg(mat + j) : 0;
+            for (uint32_t u = 0; u < 4; u++) {
+                const uint32_t c = c0 + u * 128 + lane * 4;
+                v[u] = c < S.N ? __ldg(reinterpret_cast<const uint4 *>(mat + c)) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {  // (entries past the last column are not defined)
+                const uint32_t c = c0 + u * 128 + lane * 4;
+                x[u] = v[u].x + (c + 1 < S.N ? v[u].y : 0) + (c + 2 < S.N ? v[u].z : 0) + (c + 3 < S.N ? v[u].w : 0);
+            }
+            // of each pair of loads a lane keeps one and hands the other over: load u = bits 2, 1 of the lane
+            const bool hi = lane & 4, mid = lane & 2;
+            uint32_t s0 = hi ? x[2] : x[0], s1 = hi ? x[3] : x[1];
+            s0 += __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 4);
+            s1 += __shfl_xor_sync(0xffffffffu, hi ? x[1] : x[3], 4);
+            uint32_t t = mid ? s1 : s0;
+            t += __shfl_xor_sync(0xffffffffu, mid ? s0 : s1, 2);
+            t += __shfl_xor_sync(0xffffffffu, t, 1);
+            // block b of the 16: load b / 4, lanes 8 (b % 4) ..
+            const uint32_t b = lane & 15;
+            uint32_t p = __shfl_sync(0xffffffffu, t, (b & 3) * 8 + (b >> 2) * 2);
+#pragma unroll
+            for (uint32_t o = 1; o < 16; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, p, o);
+                if (b >= o) p += y;
+            }
+            if (lane < 16 && c0 / 32 + b < S.nb) blk[c0 / 32 + b] = run + p;
+            run += __shfl_sync(0xffffffffu, p, 15);
         }
+    } else {
+        for (uint32_t b0 = 0; b0 < S.nb; b0 += 8) {  // eight 32-column blocks per pass, loads in flight together
+            uint64_t x[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+            for (int u = 0; u < 8; u++) {
+                const uint32_t j = (b0 + u) * 32 + lane;
+                x[u] = (b0 + u < S.nb && j < S.N) ? (uint64_t)__ldg(mat + j) : 0;
+            }
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] += __shfl_xor_sync(0xffffffffu, x[u], o);
-        }
+            for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            run += x[u];
-            if (lane == u && b0 + u < S.nb) S.blk[i * S.nb + b0 + u] = run;
+                for (int u = 0; u < 8; u++) x[u] += __shfl_xor_sync(0xffffffffu, x[u], o);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                run += x[u];
+                if (lane == u && b0 + u < S.nb) blk[b0 + u] = run;
+            }
         }
     }
     if (lane == 0) {
@@ -831,19 +882,6 @@ struct TileArgs {
     uint32_t *err;
     TilePlan plan;
 };
-
-// last i of [0, n) with first[i] <= x (first[0] = 0), by a warp: 32 probes per step
-__device__ __forceinline__ uint32_t warp_last_le(const uint64_t *__restrict__ first, uint32_t n, uint64_t x) {
-    uint32_t lo = 0, len = n;  // the answer is in [lo, lo + len)
-    while (len > 1) {
-        const uint32_t step = (len + 31) / 32, at = lo + step * (threadIdx.x & 31);
-        const uint32_t hits = __popc(__ballot_sync(0xffffffffu, at < lo + len && first[at] <= x));
-        const uint32_t end = lo + len;
-        lo += (hits - 1) * step;
-        len = min(step, end - lo);
-    }
-    return lo;
-}
 
 // asynchronous copy of 16 bytes to shared memory, past L1
 __device__ __forceinline__ void copy16_async(void *dst, const void *src) {
