@@ -276,6 +276,36 @@ __device__ __forceinline__ uint64_t upper_bound_u64(const uint64_t *a, uint64_t 
     return lo;
 }
 
+// first index i in [0, end) with a[i] > y (a non-decreasing, a[end-1] > y), in global memory: seven probes in
+// flight per step; `before` receives a[i-1] (0 for i = 0). In [0, end) whatever a holds: below a child that a
+// run planned ahead and that stopped off its target, matrices and prefixes were never written (the run is
+// redone, but these contractions still draw from them).
+// kConst: nothing writes a during the kernel.
+template <bool kConst>
+__device__ __forceinline__ uint32_t upper_bound8(const uint64_t *a, uint32_t end, uint64_t y, uint64_t &before) {
+    uint32_t lo = 0, len = end;
+    before = 0;
+    for (;;) {
+        const uint32_t s = (len + 7) / 8;
+        uint64_t x[7];
+#pragma unroll
+        for (uint32_t i = 0; i < 7; i++) {
+            const uint64_t *p = a + min(lo + (i + 1) * s - 1, end - 1);
+            x[i] = kConst ? __ldg(p) : *p;
+        }
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 7; i++)
+            if (x[i] <= y) {
+                c++;
+                before = x[i];
+            }
+        lo = min(lo + c * s, end - 1);
+        if (s == 1) return lo;
+        len = min(s, end - lo);
+    }
+}
+
 // Rank-of-minimum relabel of a compressed min-linked union-find (roots are minima): roots get
 // their rank in vertex order, every vertex its root's label. Writes `lab` (global).
 template <int NT, typename LabT>
@@ -300,11 +330,15 @@ __device__ void rank_labels(const uint32_t *par, uint32_t n, LabT *lab) {
 // ---------------------------------------------------------------- stage 1
 
 // Stage 1 of one trial per CTA. Per round: the weights of the edges that are not loops and their
-// inclusive prefix in edge order (warp w owns a contiguous range, its lanes read consecutive
-// edges; warp sums, one block-level offset step, then a warp scan per 32 edges writes the
-// prefix), a coarse index of the prefix at the end of every `cs`-edge segment in shared memory,
-// then (vertex count) draws in batches: each draw finds its segment in the shared index and its
-// edge by a short binary search inside the segment, and the batch is contracted in draw order.
+// inclusive prefix in edge order, in one pass (warp w owns a contiguous range of whole coarse segments and
+// scans it from 0; four consecutive edges per lane, so one warp scan per 128), and a coarse index in shared memory of the prefix at the end
+// of every `cs`-edge segment, to which the warps' offsets are added; then draws in batches, little
+// more than the links still wanted (a stream block each four): a draw finds its segment in the shared
+// index and its edge by eight-way search inside the segment, less its warp's offset, and the batch is
+// contracted in draw order.
+//   Bound by latency: the passes over the edges and, per batch, the chain of a draw and of its union.
+//   60 trials of ER(1000, 0.05) 34 us, the trials of a 64-graph batch 9.3 ms; with two passes over the
+// edges (sums, then prefixes), 32 edges at a time, a block per draw and binary searches 39 us and 10.1 ms.
 constexpr uint32_t kCoarse = 2048;      // Stage 1 coarse prefix index entries (shared memory)
 constexpr uint32_t kCoarseRows = 1024;  // contraction: coarse row-prefix index entries (shared memory)
 
@@ -316,7 +350,7 @@ __global__ void __launch_bounds__(NT) iss_shrink_kernel(const ShrinkDesc *__rest
     uint64_t *coarse = reinterpret_cast<uint64_t *>(dsm + kBatch * sizeof(uint2));
     uint32_t *par = reinterpret_cast<uint32_t *>(dsm + kBatch * sizeof(uint2) + kCoarse * sizeof(uint64_t));
     __shared__ uint32_t s_count, s_nlog;
-    __shared__ uint64_t s_w[NW];
+    __shared__ uint64_t s_w[NW], s_off[NW];
     const ShrinkDesc D = descs[blockIdx.x];
     const uint32_t n = D.n, target = D.target;
     const uint64_t m = D.m;
@@ -328,52 +362,92 @@ __global__ void __launch_bounds__(NT) iss_shrink_kernel(const ShrinkDesc *__rest
     for (uint32_t v = threadIdx.x; v < n; v += NT) par[v] = v;
     if (threadIdx.x == 0) s_count = n;
     __syncthreads();
-    const uint64_t wseg = (m + NW - 1) / NW;
-    const uint64_t wlo = min(m, (uint64_t)warp * wseg), whi = min(m, wlo + wseg);
-    // coarse segments of a multiple of 32 edges, at most kCoarse of them
+    // coarse segments of a multiple of 32 edges, at most kCoarse of them; a warp owns whole ones
     const uint64_t cs = max((uint64_t)32, ((m + kCoarse - 1) / kCoarse + 31) / 32 * 32);
-    const uint32_t ncs = (uint32_t)((m + cs - 1) / cs);
+    const uint32_t ncs = (uint32_t)((m + cs - 1) / cs), own = (ncs + NW - 1) / NW;
+    const uint64_t wlo = min(m, (uint64_t)warp * own * cs), whi = min(m, wlo + own * cs);
+    const uint32_t csg = (uint32_t)(cs / 32);
+    const bool wide = (((uintptr_t)U | (uintptr_t)V | (uintptr_t)Wt) & 15) == 0;
     for (uint64_t rnd = 0; s_count > target; rnd++) {
-        uint64_t wsum = 0;
-        for (uint64_t e = wlo + lane; e < whi; e += 32)
-            if (par[U[e]] != par[V[e]]) wsum += Wt[e];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-        if (lane == 0) s_w[warp] = wsum;
-        __syncthreads();
-        uint64_t carry = 0, W = 0;
-        for (int i = 0; i < NW; i++) {
-            if (i < warp) carry += s_w[i];
-            W += s_w[i];
-        }
-        for (uint64_t e0 = wlo; e0 < whi; e0 += 32) {
-            const uint64_t e = e0 + lane;
-            uint64_t x = (e < whi && par[U[e]] != par[V[e]]) ? Wt[e] : 0;
+        uint64_t carry = 0;
+        for (uint64_t e0 = wlo; e0 < whi; e0 += 128) {
+            const uint64_t e = e0 + 4 * lane;
+            uint4 u = make_uint4(0, 0, 0, 0), v = u, w = u;
+            if (wide && e + 4 <= whi) {
+                u = __ldg(reinterpret_cast<const uint4 *>(U + e));
+                v = __ldg(reinterpret_cast<const uint4 *>(V + e));
+                w = __ldg(reinterpret_cast<const uint4 *>(Wt + e));
+            } else {
+                if (e < whi) u.x = __ldg(U + e), v.x = __ldg(V + e), w.x = __ldg(Wt + e);
+                if (e + 1 < whi) u.y = __ldg(U + e + 1), v.y = __ldg(V + e + 1), w.y = __ldg(Wt + e + 1);
+                if (e + 2 < whi) u.z = __ldg(U + e + 2), v.z = __ldg(V + e + 2), w.z = __ldg(Wt + e + 2);
+                if (e + 3 < whi) u.w = __ldg(U + e + 3), v.w = __ldg(V + e + 3), w.w = __ldg(Wt + e + 3);
+            }
+            uint64_t x[4];
+            x[0] = par[u.x] != par[v.x] ? w.x : 0;
+            x[1] = x[0] + (par[u.y] != par[v.y] ? w.y : 0);
+            x[2] = x[1] + (par[u.z] != par[v.z] ? w.z : 0);
+            x[3] = x[2] + (par[u.w] != par[v.w] ? w.w : 0);
+            uint64_t incl = x[3];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
+                const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
             }
-            if (e < whi) pre[e] = carry + x;
-            carry += __shfl_sync(0xffffffffu, x, 31);
+            const uint64_t off = carry + incl - x[3];
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] += off;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+            if (e + 4 <= whi) {
+                reinterpret_cast<ulonglong2 *>(pre + e)[0] = make_ulonglong2(x[0], x[1]);
+                reinterpret_cast<ulonglong2 *>(pre + e)[1] = make_ulonglong2(x[2], x[3]);
+            } else {
+                for (int i = 0; i < 4 && e + i < whi; i++) pre[e + i] = i == 0 ? x[0] : i == 1 ? x[1] : x[2];
+            }
+            // the end of a segment (lanes 7, 15, 23 and 31 end 32 edges) or of the list (x[3]: past it, weights are 0)
+            if ((lane & 7) == 7 && e < whi) {
+                const uint32_t groups = (uint32_t)(e / 32) + 1;
+                if (groups % csg == 0) coarse[groups / csg - 1] = x[3];
+            }
+            if (e < m && e + 4 >= m) coarse[ncs - 1] = x[3];
+        }
+        if (lane == 0) s_w[warp] = carry;
+        __syncthreads();
+        uint64_t W = 0;
+        for (int i = 0; i < NW; i++) W += s_w[i];
+        if (W == 0) break;  // the remaining graph has no edges between its vertices
+        if (threadIdx.x < NW) {
+            uint64_t before = 0;
+            for (int i = 0; i < (int)threadIdx.x; i++) before += s_w[i];
+            s_off[threadIdx.x] = before;
         }
         __syncthreads();
-        if (W == 0) break;  // the remaining graph has no edges between its vertices
-        for (uint32_t i = threadIdx.x; i < ncs; i += NT) coarse[i] = pre[min(m, (i + 1) * cs) - 1];
-        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < ncs; i += NT) coarse[i] += s_off[i / own];
         const uint32_t c_start = s_count;
-        for (uint32_t base = 0; base < c_start; base += kBatch) {
-            const uint32_t nb = min((uint32_t)kBatch, c_start - base);
-            for (uint32_t j = threadIdx.x; j < nb; j += NT) {
-                const uint64_t y = mulhi64(draw64(D.k0, D.idx, 1, 0, rnd, base + j), W);
-                const uint64_t sg = upper_bound_u64(coarse, ncs, y);
-                const uint64_t s0 = sg * cs;
-                const uint64_t e = s0 + upper_bound_u64(pre + s0, min(cs, m - s0), y);
-                sb[j] = make_uint2(U[e], V[e]);
+        __syncthreads();
+        for (uint32_t base = 0; base < c_start;) {
+            const uint32_t need = s_count - target;
+            const uint32_t nb = min(min((uint32_t)kBatch, c_start - base), (need + need / 8 + 32 + NT - 1) / NT * NT);
+            for (uint32_t q = threadIdx.x; 4 * q < nb; q += NT) {
+                const u64x4 o = sitmo_block(D.k0, D.idx, 1, 0, (base >> 2) + q, rnd, 0, 0);
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++) {
+                    const uint64_t y = mulhi64(o.x[i], W);
+                    sb[4 * q + i] = make_uint2((uint32_t)y, (uint32_t)(y >> 32));
+                }
             }
             __syncthreads();
+            for (uint32_t j = threadIdx.x; j < nb; j += NT) {
+                const uint64_t y = (uint64_t)sb[j].y << 32 | sb[j].x;
+                const uint32_t sg = (uint32_t)upper_bound_u64(coarse, ncs, y);
+                const uint64_t s0 = sg * cs;
+                uint64_t before;
+                const uint64_t e = s0 + upper_bound8<false>(pre + s0, (uint32_t)min(cs, m - s0), y - s_off[sg / own], before);
+                sb[j] = make_uint2(__ldg(U + e), __ldg(V + e));
+            }
             contract_batch<NT>(par, sb, nb, target, &s_count, &s_nlog);
             if (s_count <= target) break;
+            base += nb;
         }
         for (uint32_t v = threadIdx.x; v < n; v += NT) par[v] = sfind_ro(par, v);
         __syncthreads();
@@ -523,31 +597,6 @@ constexpr uint32_t kContractMid = 256, kContractMidN = 724;
 
 __host__ __device__ __forceinline__ uint32_t contract_batch_cap(uint32_t N) { return N < kBatch ? (N + 3) & ~3u : kBatch; }
 
-// first index i in [0, end) with a[i] > y (a non-decreasing, a[end-1] > y), in global memory: seven probes in
-// flight per step; `before` receives a[i-1] (0 for i = 0). In [0, end) whatever a holds: below a child that a
-// run planned ahead and that stopped off its target, matrices and prefixes were never written (the run is
-// redone, but these contractions still draw from them).
-__device__ __forceinline__ uint32_t upper_bound8(const uint64_t *a, uint32_t end, uint64_t y, uint64_t &before) {
-    uint32_t lo = 0, len = end;
-    before = 0;
-    for (;;) {
-        const uint32_t s = (len + 7) / 8;
-        uint64_t x[7];
-#pragma unroll
-        for (uint32_t i = 0; i < 7; i++) x[i] = __ldg(a + min(lo + (i + 1) * s - 1, end - 1));
-        uint32_t c = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < 7; i++)
-            if (x[i] <= y) {
-                c++;
-                before = x[i];
-            }
-        lo = min(lo + c * s, end - 1);
-        if (s == 1) return lo;
-        len = min(s, end - lo);
-    }
-}
-
 // the column of one 32-column block (row starts are 16-byte aligned, so the block is too): first of the
 // block's `lim` entries whose running sum exceeds rem; lim if none does
 __device__ __forceinline__ uint32_t block_column(const uint32_t *p, uint32_t lim, uint64_t rem) {
@@ -661,7 +710,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) contract_kernel(const TaskDesc 
             }
             const uint64_t rem = y - before;
             uint64_t left;
-            const uint32_t b = upper_bound8(S.blk + (uint64_t)a * S.nb, S.nb, rem, left);
+            const uint32_t b = upper_bound8<true>(S.blk + (uint64_t)a * S.nb, S.nb, rem, left);
             const uint32_t lim = min(32u, N - b * 32);
             uint32_t c = block_column(mat + (uint64_t)a * ld_of(N) + (uint64_t)b * 32, lim, rem - left);
             if (c >= lim) {  // cannot happen with consistent prefixes; record and clamp
@@ -2314,6 +2363,7 @@ int admit(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
 // launch and two host synchronisations per query.
 int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan *> &qs) {
     cudaStream_t s = ctx->stream;
+    auto pre_words_of = [](uint64_t m) { return std::max<uint64_t>((m + 3) & ~3ull, 4); };  // (16-byte stores)
     struct Item {
         const QueryPlan *q;
         uint64_t i;
@@ -2333,7 +2383,7 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
         uint64_t mmax = 1;
         while (c1 < items.size() && c1 - c0 < 65535) {
             const cac_graph *g = items[c1].q->g;
-            const uint64_t pw = std::max<uint64_t>(g->m, 1), lw = g->n;
+            const uint64_t pw = pre_words_of(g->m), lw = g->n;
             if (c1 > c0 && (pre_words + pw) * 8 + (lab_words + lw) * 4 > (4ull << 30)) break;
             pre_words += pw;
             lab_words += lw;
@@ -2362,7 +2412,7 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
             D.target = q.t;
             D.k0 = q.seed + (uint32_t)(i / q.per_rank);
             D.idx = (uint32_t)(i % q.per_rank);
-            po += std::max<uint64_t>(q.g->m, 1);
+            po += pre_words_of(q.g->m);
             lo += q.g->n;
         }
         const size_t sm = kBatch * sizeof(uint2) + kCoarse * sizeof(uint64_t) + (size_t)nmax * 4;
