@@ -337,7 +337,7 @@ __device__ void rank_labels(const uint32_t *par, uint32_t n, LabT *lab) {
 // index and its edge by eight-way search inside the segment, less its warp's offset, and the batch is
 // contracted in draw order.
 //   Bound by latency: the passes over the edges and, per batch, the chain of a draw and of its union.
-//   60 trials of ER(1000, 0.05) 34 us, the trials of a 64-graph batch 9.3 ms; with two passes over the
+//   60 trials of ER(1000, 0.05) 32 us, the trials of a 64-graph batch 8.6 ms; with two passes over the
 // edges (sums, then prefixes), 32 edges at a time, a block per draw and binary searches 39 us and 10.1 ms.
 constexpr uint32_t kCoarse = 2048;      // Stage 1 coarse prefix index entries (shared memory)
 constexpr uint32_t kCoarseRows = 1024;  // contraction: coarse row-prefix index entries (shared memory)
