@@ -335,7 +335,7 @@ uint64_t merge_edges_multi_scratch(uint64_t M, uint32_t B);
 int shrink_big(cac_ctx *ctx, const cac_graph *g, uint32_t target, uint32_t B, const uint32_t *k0, const uint32_t *idx,
                uint32_t *d_lab, uint32_t *d_kout, void *scratch);
 // Quotient kernels that a caller can force (cac_ctx_set_quotient_kernel; 0 and 4: by size).
-constexpr uint8_t kQuotientTile = 1, kQuotientShared = 2, kQuotientTileToo = 3;
+constexpr uint8_t kQuotientAuto = 0, kQuotientTile = 1, kQuotientShared = 2, kQuotientTileToo = 3;
 // Engine error word bits: 1 an inconsistent selection prefix in a contraction, 4 a child planned at
 // its target size that stopped elsewhere (the run is redone without planning ahead)
 constexpr uint32_t kErrPlan = 4u;

@@ -17,7 +17,7 @@
 //                                by its prefixes, column by a scan of the block), contraction in draw
 //                                order until max(ceil(n/sqrt 2)+1, 128) vertices, labels by rank
 //                                of the smallest member, member lists by counting sort
-//              quotient_tile_kernel / quotient_shared_row_kernel
+//              quotient_tri_kernel / quotient_tile_kernel / quotient_shared_row_kernel
 //                                the child's matrix: a few output rows at a time as one tile in shared
 //                                memory, member rows summed on the way in, joined columns added to their
 //                                groups' first ones, those stored; at large N a CTA per output row
@@ -95,7 +95,8 @@ struct TaskDesc {
     uint32_t target;
     uint32_t round;
     uint32_t k0, idx;     // stream key words 0, 1
-    uint32_t leaf;        // planned to be a leaf: only the labels and first vertices are wanted
+    uint32_t brief;       // a child planned to be solved or built from its triangle: only the labels and first
+                          // vertices are wanted
 };
 
 struct LeafDesc {
@@ -746,7 +747,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) contract_kernel(const TaskDesc 
         const uint32_t roots = __ballot_sync(0xffffffffu, root);
         if (root) cnt[v] = s_group[g] + __popc(roots & ((1u << lane) - 1));
     }
-    if (T.leaf) {
+    if (T.brief) {
         __syncthreads();
         for (uint32_t v = threadIdx.x; v < N; v += NT) {
             const uint32_t r = par[v], l = cnt[r];
@@ -850,11 +851,27 @@ __global__ void __launch_bounds__(NT, 1024 / NT) contract_kernel(const TaskDesc 
     if (threadIdx.x == 0) k_out[task] = k;
 }
 
+// ---------------------------------------------------------------- lower triangles in shared memory
+// Entry (i, j < i) at i (i - 1) / 2 + j: the entries (x, v) of 32 consecutive v lie in 32 different banks on
+// either side of x (triangular numbers take every residue of a power of two once).
+__device__ __forceinline__ uint32_t tri(uint32_t i) { return i * (i - 1) / 2; }
+__device__ __forceinline__ uint32_t tpos(uint32_t i, uint32_t j) { return i > j ? tri(i) + j : tri(j) + i; }
+
+template <typename Tm>
+__device__ __forceinline__ void copy_entry_async(Tm *dst, const Tm *src) {
+    if constexpr (sizeof(Tm) == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+}
+
 // ---------------------------------------------------------------- quotient
 // Q[a][b] = sum over u in group a, v in group b of A[u][v], the diagonal zeroed, with every row's
-// 32-column block prefixes and its sum (the next step's row prep). Two kernels with identical results:
-// tiles of R rows (quotient_tile_kernel) up to kTileMaxN source vertices, one row per CTA
-// (quotient_shared_row_kernel) above.
+// 32-column block prefixes and its sum (the next step's row prep). Three kernels with identical results:
+// the lower triangle of a small child (quotient_tri_kernel, see tri_fits), tiles of R rows (quotient_tile_kernel)
+// up to kTileMaxN source vertices, one row per CTA (quotient_shared_row_kernel) above.
 //
 // R output rows make a tile: R rows of N entries in shared memory, so that every column index is
 // read once for R rows. The rows of a tile are interleaved in 16-byte chunks (a column's R entries
@@ -1196,6 +1213,137 @@ __device__ __forceinline__ void sadd(uint64_t *p, uint64_t v) {
     atomicAdd(reinterpret_cast<unsigned long long *>(p), (unsigned long long)v);
 }
 
+// Small children: one CTA per child, the child's lower triangle in shared memory. A warp per row copies the
+// entries between first vertices from the source, at the columns of the first vertices (ascending, so the
+// copies stay nearly coalesced); then a warp per joined vertex adds its row to its group's, from the first
+// vertices' columns and from those of the joined vertices before it, with shared atomics; then a warp per
+// row stores it, with its 32-column block prefixes and its sum. Half of the source is read, and a child takes
+// half the instructions of its tiles, whose setup per CTA and per tile it also spares.
+//   Taken while the triangle leaves room for three CTAs per SM (u32 entries: k <= 192; u64: 136): the
+// children of K4000's levels of N = 255 and 182 took 320 and 350 us as tiles and take 244 and 287 us, those
+// of the Watts-Strogatz query 11.7 and 14.0 ms a group, now 7.8 and 9.1. Larger ones would leave one CTA per SM
+// or few warps, where the tiles keep three. Up to kTriSmallBytes six CTAs of 128 threads fit.
+constexpr int kTriThreads = 256, kTriSmall = 128;
+constexpr uint32_t kTriSmallBytes = 36 * 1024;
+constexpr uint32_t kTriMaxK = 192, kTriMaxJoined = 96;
+__host__ __device__ __forceinline__ uint32_t tri_bytes(uint32_t k, uint32_t esize) { return (k * (k - 1) / 2 + 1) * esize; }
+__host__ __device__ __forceinline__ bool tri_fits(uint32_t N, uint32_t k, uint32_t small) {
+    return k >= 2 && N - k <= kTriMaxJoined && tri_bytes(k, small ? 4 : 8) <= tri_bytes(kTriMaxK, 4);
+}
+
+__device__ __forceinline__ uint32_t warp_sum(uint32_t x) { return __reduce_add_sync(0xffffffffu, x); }
+__device__ __forceinline__ uint64_t warp_sum(uint64_t x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+template <int NT, typename Tm>
+__global__ void __launch_bounds__(NT, 768 / NT) quotient_tri_kernel(
+    const TaskDesc *__restrict__ tasks, const SrcDesc *__restrict__ srcs, const uint32_t *__restrict__ list,
+    const uint32_t *__restrict__ ks, const uint64_t *__restrict__ out_off, uint32_t ntasks, unsigned char *out_base,
+    const uint32_t *__restrict__ k_act, uint32_t *err) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    constexpr uint32_t kWarps = NT / 32, Q = kTriMaxK / 32, B = kTriMaxJoined / 32;
+    Tm *M = reinterpret_cast<Tm *>(dsm);
+    __shared__ uint16_t s_first[kTriMaxK];
+    __shared__ uint32_t s_joined[kTriMaxJoined], s_count;  // vertex | label << 16
+    const uint32_t task = list[blockIdx.x], k = ks[task], lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    if (k_act && k_act[task] != k) {  // planned ahead, and this child stopped off its target: redo the run
+        if (threadIdx.x == 0) atomicOr(err, kErrPlan);
+        return;
+    }
+    const TaskDesc T = tasks[task];
+    const SrcDesc S = srcs[T.src];
+    const uint32_t N = S.N;
+    const Tm *__restrict__ mat = reinterpret_cast<const Tm *>(S.mat);
+    const uint64_t ldN = ld_of(N);
+    for (uint32_t l = threadIdx.x; l < kTriMaxK; l += NT) s_first[l] = l < k ? T.cols[kColHead + l] : (uint16_t)0;
+    if (threadIdx.x == 0) s_count = 0;
+    __syncthreads();
+    for (uint32_t v0 = warp * 32; v0 < N; v0 += NT) {
+        const uint32_t v = v0 + lane, l = v < N ? T.lab[v] : 0;
+        const bool j = v < N && s_first[l] != v;
+        const uint32_t js = __ballot_sync(0xffffffffu, j);
+        uint32_t at = 0;
+        if (lane == 0 && js) at = atomicAdd(&s_count, (uint32_t)__popc(js));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(js & ((1u << lane) - 1));
+        if (j) s_joined[at] = v | l << 16;
+    }
+    uint32_t f[Q];
+#pragma unroll
+    for (uint32_t q = 0; q < Q; q++) f[q] = s_first[lane + 32 * q];
+#pragma unroll 2
+    for (uint32_t i = 1 + warp; i < k; i += kWarps) {
+        const Tm *src = mat + s_first[i] * ldN;
+        Tm *dst = M + tri(i) + lane;
+#pragma unroll
+        for (uint32_t q = 0; q < Q; q++)
+            if (lane + 32 * q < i) copy_entry_async(dst + 32 * q, src + f[q]);
+    }
+    __syncthreads();
+    const uint32_t joined = s_count;
+    uint32_t other[B];  // the lane's joined vertices
+#pragma unroll
+    for (uint32_t q = 0; q < B; q++) other[q] = lane + 32 * q < joined ? s_joined[lane + 32 * q] : 0;
+    bool waited = false;
+    for (uint32_t p0 = 0; p0 < joined || !waited; p0 += 2 * kWarps) {
+        Tm a[2][Q + B];
+#pragma unroll
+        for (uint32_t u = 0; u < 2; u++) {
+            const uint32_t p = p0 + u * kWarps + warp;
+            const Tm *row = mat + (p < joined ? s_joined[p] & 0xFFFFu : 0) * ldN;
+#pragma unroll
+            for (uint32_t q = 0; q < Q; q++) a[u][q] = p < joined && lane + 32 * q < k ? __ldg(row + f[q]) : Tm(0);
+#pragma unroll
+            for (uint32_t q = 0; q < B; q++)
+                a[u][Q + q] = p < joined && lane + 32 * q < p ? __ldg(row + (other[q] & 0xFFFFu)) : Tm(0);
+        }
+        if (!waited) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            waited = true;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 2; u++) {
+            const uint32_t p = p0 + u * kWarps + warp;
+            if (p >= joined) break;
+            const uint32_t to = s_joined[p] >> 16, tt = tri(to);
+#pragma unroll
+            for (uint32_t q = 0; q < Q + B; q++) {
+                const uint32_t l = q < Q ? lane + 32 * q : other[q - Q] >> 16;
+                if (a[u][q] != 0 && l != to) sadd(&M[l > to ? tri(l) + to : tt + l], a[u][q]);
+            }
+        }
+    }
+    __syncthreads();
+    const uint64_t ldk = ld_of(k);
+    const uint32_t nbk = (k + 31) / 32;
+    Tm *out = reinterpret_cast<Tm *>(out_base + out_off[task]);
+    uint64_t *sums = reinterpret_cast<uint64_t *>(out_base + out_off[ntasks + task]), *blk = sums + k;
+    for (uint32_t l = warp; l < k; l += kWarps) {
+        const uint32_t tl = tri(l);
+        Tm x[Q], run = 0, mine = 0;  // (a row sum fits an entry)
+#pragma unroll
+        for (uint32_t q = 0; q < Q; q++) {
+            const uint32_t c = lane + 32 * q;
+            x[q] = c < k && c != l ? M[c > l ? tri(c) + l : tl + c] : Tm(0);
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < Q; q++) {
+            if (lane + 32 * q < k) out[l * ldk + lane + 32 * q] = x[q];
+            x[q] = warp_sum(x[q]);
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < Q; q++) {
+            run += x[q];
+            if (lane == q) mine = run;
+        }
+        if (lane < nbk) blk[(uint64_t)l * nbk + lane] = mine;
+        if (lane == 0) sums[l] = run;
+    }
+}
+
 // The quotient for large N: one CTA of 8 warps per group of `rows` consecutive output rows, all
 // warps on the same output row at a time (labels + one row in shared memory: 5 CTAs, 40 warps per SM
 // at N = 4000, where a tile leaves room for 16). The warps split the columns: 128-column chunks (one 16-byte load per lane), chunk c to warp c mod 8, four
@@ -1366,19 +1514,6 @@ __device__ __forceinline__ uint64_t warp_max(uint64_t x) {
 __device__ __forceinline__ uint32_t warp_max(uint32_t x) { return __reduce_max_sync(0xffffffffu, x); }
 
 constexpr uint32_t kLeafThreads = 128, kLeafWarps = kLeafThreads / 32;  // they load; warp 0 solves
-__device__ __forceinline__ uint32_t tri(uint32_t i) { return i * (i - 1) / 2; }
-__device__ __forceinline__ uint32_t tpos(uint32_t i, uint32_t j) { return i > j ? tri(i) + j : tri(j) + i; }
-
-template <typename Tm>
-__device__ __forceinline__ void copy_entry_async(Tm *dst, const Tm *src) {
-    if constexpr (sizeof(Tm) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                     : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                     : "memory");
-}
-
 // The orderings; returns the leaf's minimum cut. Kt: the vertex words. root: 128 bytes of shared memory.
 template <typename Tm, typename Kt>
 __device__ __forceinline__ uint64_t leaf_cut(Tm *M, uint32_t N, uint64_t lambda, uint8_t *root) {
@@ -1999,7 +2134,8 @@ int KsEngine::step() {
         d.round = t.round;
         d.k0 = t.src.k0;
         d.idx = t.src.idx;
-        d.leaf = plan_ahead_ && t.target <= kLeafN;
+        d.brief = plan_ahead_ &&
+                  (t.target <= kLeafN || (ctx_->quotient_forced == kQuotientAuto && tri_fits(t.src.N, t.target, t.src.small)));
         const uint32_t N = t.src.N;
         d.rows = d_tscratch.as<uint32_t>() + ts;
         d.lab = reinterpret_cast<uint16_t *>(d.rows + N);
@@ -2097,8 +2233,8 @@ int KsEngine::step() {
         out_off[tasks.size() + i] = out_bytes;
         out_bytes += ((kq[i] + (uint64_t)kq[i] * ((kq[i] + 31) / 32)) * 8 + 15) / 16 * 16;
     }
-    // Two quotient kernels, identical outputs: tiles up to kTileMaxN source vertices (a launch per entry
-    // width), one row per CTA above; the caller may force one, where it fits.
+    // Three quotient kernels, identical outputs: triangles for small children, tiles up to kTileMaxN source
+    // vertices, one row per CTA above; the caller may force tiles (where they fit) or rows.
     MatBuf *out = nullptr;
     if (out_bytes || !leaf_list[0].empty() || !leaf_list[1].empty()) {
         if (out_bytes) CAC_TRY(alloc(out_bytes, &out));
@@ -2112,8 +2248,9 @@ int KsEngine::step() {
         } tl[2];
         tl[0].plan = TilePlan{4, 4, 0, 1};  // u32 entries
         tl[1].plan = TilePlan{2, 8, 0, 1};  // u64
-        std::vector<uint32_t> shared;
+        std::vector<uint32_t> shared, tris[3];  // (tris: u32 entries, small and larger; u64)
         std::vector<uint64_t> gto;
+        uint32_t tri_k[3] = {2, 2, 2};
         uint64_t groups_shared = 0;
         uint32_t shared_n = 0, shared_k = 0;
         bool shared_small = true;
@@ -2121,6 +2258,12 @@ int KsEngine::step() {
         for (size_t i = 0; i < tasks.size(); i++) {
             const uint32_t N = tasks[i].src.N, k = kq[i];
             if (!k) continue;
+            if (forced == kQuotientAuto && tri_fits(N, k, tasks[i].src.small)) {
+                const int w = !tasks[i].src.small ? 2 : tri_bytes(k, 4) <= kTriSmallBytes ? 0 : 1;
+                tris[w].push_back((uint32_t)i);
+                tri_k[w] = std::max(tri_k[w], k);
+                continue;
+            }
             TileList &l = tl[tasks[i].src.small ? 0 : 1];
             const uint32_t need = tile_idx_bytes(N, k) +
                                   tile_groups(N, k, l.plan, kTileSmem) * tile_bytes(N, l.plan.rows, l.plan.esize);
@@ -2165,7 +2308,8 @@ int KsEngine::step() {
         }
         // one descriptor copy for the output offsets, the children's sizes and the launch lists
         size_t bytes = Staging::bytes_of(out_off) + Staging::bytes_of(kq) + Staging::bytes_of(shared) +
-                       Staging::bytes_of(gto) + Staging::bytes_of(leaf_list[0]) + Staging::bytes_of(leaf_list[1]);
+                       Staging::bytes_of(gto) + Staging::bytes_of(leaf_list[0]) + Staging::bytes_of(leaf_list[1]) +
+                       Staging::bytes_of(tris[0]) + Staging::bytes_of(tris[1]) + Staging::bytes_of(tris[2]);
         for (const TileList &l : tl) bytes += Staging::bytes_of(l.task) + Staging::bytes_of(l.first);
         CAC_TRY(post_st.begin(bytes));
         const uint64_t *dv_qoff = post_st.put(out_off);
@@ -2177,6 +2321,7 @@ int KsEngine::step() {
             args[i] = TileArgs{post_st.put(tl[i].task), post_st.put(tl[i].first), (uint32_t)tl[i].task.size(), tl[i].uniform,
                                d_err, tl[i].plan};
         const uint32_t *dv_leaf32 = post_st.put(leaf_list[0]), *dv_leaf64 = post_st.put(leaf_list[1]);
+        const uint32_t *dv_tri[3] = {post_st.put(tris[0]), post_st.put(tris[1]), post_st.put(tris[2])};
         CAC_TRY(post_st.flush());
         if (plan_ahead_) CAC_TRY(launch_contractions());
         if (!leaf_list[0].empty()) {
@@ -2189,6 +2334,16 @@ int KsEngine::step() {
             sw_child_kernel<uint64_t><<<(unsigned)leaf_list[1].size(), kLeafThreads, leaf_smem(kLeafN, false), s>>>(
                 dv_task, dv_src, dv_leaf64, d_kout.as<uint32_t>(), d_err);
         }
+        auto launch_tri = [&](auto kern, int threads, int w) -> int {
+            if (tris[w].empty()) return CAC_OK;
+            CAC_TRY(smem_optin(ctx_, kern));
+            kern<<<(unsigned)tris[w].size(), threads, tri_bytes(tri_k[w], w == 2 ? 8 : 4), s>>>(
+                dv_task, dv_src, dv_tri[w], dv_k, dv_qoff, (uint32_t)tasks.size(), obase, kact, d_err);
+            return CAC_OK;
+        };
+        CAC_TRY(launch_tri(quotient_tri_kernel<kTriThreads, uint32_t>, kTriThreads, 1));
+        CAC_TRY(launch_tri(quotient_tri_kernel<kTriSmall, uint32_t>, kTriSmall, 0));
+        CAC_TRY(launch_tri(quotient_tri_kernel<kTriThreads, uint64_t>, kTriThreads, 2));
         if (tl[0].ctas) {
             CAC_TRY(smem_optin(ctx_, quotient_tile_kernel<uint32_t, 4>));
             quotient_tile_kernel<uint32_t, 4><<<(unsigned)tl[0].ctas, kTileThreads, tl[0].plan.smem, s>>>(args[0]);
