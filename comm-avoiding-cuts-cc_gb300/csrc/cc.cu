@@ -345,6 +345,13 @@ __global__ void cc_compress4(uint32_t *par, uint32_t n) {
 // Compression of [0, n) (the parent array is 256-byte aligned).
 void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s);
 
+// The bitmap's allocation: a word per 32 vertices, then, for graphs whose bitmap does not fit in shared memory,
+// a byte per 32 vertices (a bit per four of them), read as words.
+__host__ __device__ __forceinline__ uint32_t quad_words_at(uint32_t nwords) { return (nwords + 3) & ~3u; }
+size_t bitmap_bytes(size_t nwords) {
+    return nwords * 4 + 4 + (nwords > kSmemBitmapWords ? 16 + (nwords + 3) / 4 * 4 : 0);
+}
+
 // The end of the sampling round in one launch: full compression, the giant component and its
 // membership bitmap. Every CTA (kGiantSample threads) first finds the giant itself, from the
 // roots of the same kGiantSample vertices (fixed spread of positions): every warp finds the mode
@@ -394,6 +401,14 @@ __global__ void __launch_bounds__(kGiantSample) cc_compress_giant_bitmap(uint32_
         }
         const uint32_t word = __ballot_sync(0xffffffffu, in);
         if (lane == 0) bits[wd] = word;
+        if (nw > kSmemBitmapWords && lane == 0) {  // a bit per four vertices: all of them are in the giant
+            uint32_t b = word & (word >> 1);
+            b &= b >> 2;
+            b &= 0x11111111u;
+            b = (b | b >> 3) & 0x03030303u;
+            b = (b | b >> 6) & 0x000F000Fu;
+            reinterpret_cast<uint8_t *>(bits + quad_words_at((uint32_t)nw))[wd] = (uint8_t)(b | b >> 12);
+        }
     }
 }
 
@@ -441,8 +456,16 @@ __global__ void __launch_bounds__(kThreads) cc_edge_pass(uint32_t *par, const ui
 // `surv` (region = the CTA's contiguous range of 256-edge tiles, so no global counter is
 // contended). A warp owns a tile: lane l reads edges 4l..4l+3 and 128+4l..128+4l+3 of it with
 // two fully coalesced 512-byte loads per endpoint array, keeps 8 edges in flight, and appends its
-// survivors after one warp scan and one shared-memory atomic. The membership bitmap's first
-// `swords` words are staged in shared memory, the rest read through the read-only path.
+// survivors after one warp scan and one shared-memory atomic.
+//   The membership bitmap is staged in shared memory. Above kSmemBitmapWords it does not fit: a lane
+// whose word is elsewhere makes a 32-byte access of the L2 each time, and these bound the pass (R-MAT scale 22,
+// 30% of the endpoints: 262 us). Staged instead is the bitmap of whole quads of vertices in the
+// giant (up to 6.3 M vertices; the ids beyond it, and those of other quads, are looked up in the full one): 98% of
+// R-MAT's endpoints are in such quads although 40% of its vertices are isolated, since a vertex and its
+// neighbours in the numbering have like degrees. Where few are (a giant of half the vertices, spread
+// evenly), the first part of the full bitmap is the better one: a CTA counts what its first two tiles per
+// warp find in the quads and takes the other if that is less than the share of ids it would hold.
+// R-MAT scale 22, 67 M edges: 204 us (the full bitmap's first part alone 262 us).
 template <bool kAllSmem, bool kCheck>
 __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__restrict__ u,
                                                           const uint32_t *__restrict__ v, uint64_t tiles,
@@ -451,19 +474,31 @@ __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__rest
                                                           uint32_t n, uint32_t *err) {
     pdl_wait();
     extern __shared__ uint32_t sbits[];
-    __shared__ uint32_t s_n;
+    __shared__ uint32_t s_n, s_found;
     const uint32_t swords = min(nwords, (uint32_t)kSmemBitmapWords);
-    for (uint32_t i = threadIdx.x; i < swords; i += blockDim.x) sbits[i] = gbits[i];
-    if (threadIdx.x == 0) s_n = 0;
+    // words staged: of the quads' bitmap first, where the full one does not fit
+    uint32_t qwords = kAllSmem ? 0u : min((nwords + 3) / 4, (uint32_t)kSmemBitmapWords);
+    if (kAllSmem)
+        for (uint32_t i = threadIdx.x; i < swords; i += blockDim.x) sbits[i] = gbits[i];
+    else
+        for (uint32_t i = threadIdx.x; i < qwords; i += blockDim.x) sbits[i] = gbits[quad_words_at(nwords) + i];
+    if (threadIdx.x == 0) s_n = s_found = 0;
     __syncthreads();
     const uint64_t per = (tiles + gridDim.x - 1) / gridDim.x;
     const uint64_t t0 = min(tiles, (uint64_t)blockIdx.x * per), t1 = min(tiles, t0 + per);
     uint2 *out = surv + t0 * 256;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    auto in_giant = [&](uint32_t x) -> bool {
+    // the word that holds x's bit, or all ones if its quad is in the giant (loads are predicated, not
+    // branched to: those of the 16 endpoints of a lane's tile are in flight together)
+    auto look = [&](uint32_t x) -> uint32_t {
         const uint32_t w = x >> 5;
-        const uint32_t word = (kAllSmem || w < swords) ? sbits[w] : __ldg(gbits + w);
-        return (word >> (x & 31)) & 1u;
+        if (kAllSmem) return sbits[w];
+        const uint32_t at = qwords ? x >> 7 : w, staged = qwords ? qwords : swords;
+        uint32_t word = sbits[at < staged ? at : 0];
+        const bool known = at < staged && (!qwords || (word >> (x >> 2 & 31)) & 1u);
+        if (qwords) word = 0xFFFFFFFFu;
+        if (!known) word = __ldg(gbits + w);
+        return word;
     };
     const uint4 *u4 = reinterpret_cast<const uint4 *>(u);
     const uint4 *v4 = reinterpret_cast<const uint4 *>(v);
@@ -471,12 +506,17 @@ __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__rest
         const uint32_t a[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
         const uint32_t b[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
         uint32_t keep = 0, bad = 0;
+        uint32_t wa[8], wb[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const bool ok = !kCheck || (a[k] < n && b[k] < n);  // an invalid edge is neither tested nor kept
             bad |= !ok;
-            keep |= (uint32_t)(ok && !(in_giant(ok ? a[k] : 0u) && in_giant(ok ? b[k] : 0u))) << k;
+            wa[k] = look(ok ? a[k] : 0u);
+            wb[k] = look(ok ? b[k] : 0u);
+            if (kCheck && !ok) wa[k] = wb[k] = 0xFFFFFFFFu;
         }
+#pragma unroll
+        for (int k = 0; k < 8; k++) keep |= (~((wa[k] >> (a[k] & 31)) & (wb[k] >> (b[k] & 31))) & 1u) << k;
         if (kCheck && bad) atomicOr(err, kErrBadId);
         const uint32_t cnt = __popc(keep);
         uint32_t incl = cnt;
@@ -495,7 +535,7 @@ __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__rest
             if ((keep >> k) & 1u) out[base++] = make_uint2(a[k], b[k]);
     };
     // two tiles per warp step: all eight 512-byte loads are issued before either tile is used
-    for (uint64_t t = t0 + 2 * (uint64_t)warp; t < t1; t += 2 * (uint64_t)nwarps) {
+    auto step = [&](uint64_t t) {
         const bool two = t + 1 < t1;
         const uint4 z = make_uint4(0, 0, 0, 0);
         const uint4 ua = __ldcs(u4 + t * 64 + lane), ub = __ldcs(u4 + t * 64 + 32 + lane);
@@ -504,7 +544,28 @@ __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__rest
         const uint4 vc = two ? __ldcs(v4 + (t + 1) * 64 + lane) : z, vd = two ? __ldcs(v4 + (t + 1) * 64 + 32 + lane) : z;
         process(ua, ub, va, vb);
         if (two) process(uc, ud, vc, vd);
+    };
+    uint64_t t = t0 + 2 * (uint64_t)warp;
+    if constexpr (!kAllSmem) {
+        // what the quads would find in the CTA's first tiles (one endpoint in eight)
+        uint32_t found = 0;
+        if (t < t1) {
+            const uint32_t x[2] = {__ldg(u + t * 256 + 4 * lane), __ldg(v + t * 256 + 4 * lane)};
+#pragma unroll
+            for (int k = 0; k < 2; k++) found += x[k] >> 7 < qwords && (sbits[x[k] >> 7] >> (x[k] >> 2 & 31)) & 1u;
+        }
+        found = __reduce_add_sync(0xffffffffu, found);
+        if (lane == 0 && found) atomicAdd(&s_found, found);
+        const uint64_t warps_in = t1 > t0 ? min((uint64_t)nwarps, (t1 - t0 + 1) / 2) : 0;
+        __syncthreads();
+        if ((uint64_t)s_found * nwords < 64 * warps_in * swords) {
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < swords; i += blockDim.x) sbits[i] = gbits[i];
+            qwords = 0;
+            __syncthreads();
+        }
     }
+    for (; t < t1; t += 2 * (uint64_t)nwarps) step(t);
     __syncthreads();
     if (threadIdx.x == 0) counts[blockIdx.x] = s_n;
 }
@@ -873,7 +934,7 @@ size_t cc_scratch_bytes(uint32_t n, uint32_t ranks, uint64_t m) {
     const size_t ntiles = ((size_t)n + kTile - 1) / kTile;
     const size_t nwords = ((size_t)n + 31) / 32;
     return align_up((size_t)n * 4) + 2 * align_up(ntiles * 4 + 4) + align_up(256) +
-           align_up(sizeof(RankDesc) * (size_t)ranks) + align_up(nwords * 4 + 4) + align_up(kMaxRegions * 4) +
+           align_up(sizeof(RankDesc) * (size_t)ranks) + align_up(bitmap_bytes(nwords)) + align_up(kMaxRegions * 4) +
            align_up((m + 4 * (uint64_t)kMaxRegions) * 8);
 }
 
@@ -1116,7 +1177,7 @@ int cc_run(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint
     L.giant = L.total + 8;
     L.err = L.total + kErrWord;
     L.d_ranks = (RankDesc *)arena_take(ctx, sizeof(RankDesc) * ranks);
-    L.bits = (uint32_t *)arena_take(ctx, (size_t)L.nwords * 4 + 4);
+    L.bits = (uint32_t *)arena_take(ctx, bitmap_bytes(L.nwords));
     L.region_counts = (uint32_t *)arena_take(ctx, kMaxRegions * 4);
     L.surv = (uint2 *)arena_take(ctx, (m + 4 * (uint64_t)kMaxRegions) * 8);
     L.chunks = (uint64_t *)arena_take(ctx, chunk_slots * 8);
@@ -1377,7 +1438,7 @@ int cc_run_streamed(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *h_u, c
     L.filtered = L.vec && seg > 0;
     const uint64_t max_gap = L.filtered ? m - (kStreamPieces - 1) * seg - piece : 0;
     CAC_TRY(arena_reserve(ctx, align_up((size_t)n * 4) + 2 * align_up((size_t)L.ntiles * 4 + 4) + align_up(256) +
-                                   (L.filtered ? align_up((size_t)L.nwords * 4 + 4) + align_up(kMaxRegions * 4) +
+                                   (L.filtered ? align_up(bitmap_bytes(L.nwords)) + align_up(kMaxRegions * 4) +
                                                      align_up((max_gap + 4 * (uint64_t)kMaxRegions) * 8)
                                                : 0)));
     arena_reset(ctx);
@@ -1387,7 +1448,7 @@ int cc_run_streamed(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *h_u, c
     L.total = (uint32_t *)arena_take(ctx, 256);
     L.giant = L.total + 8;
     if (L.filtered) {
-        L.bits = (uint32_t *)arena_take(ctx, (size_t)L.nwords * 4 + 4);
+        L.bits = (uint32_t *)arena_take(ctx, bitmap_bytes(L.nwords));
         L.region_counts = (uint32_t *)arena_take(ctx, kMaxRegions * 4);
         L.surv = (uint2 *)arena_take(ctx, (max_gap + 4 * (uint64_t)kMaxRegions) * 8);
         CAC_TRY(smem_optin(ctx, cc_filter<true, true>));
