@@ -46,7 +46,8 @@ namespace cac {
 namespace {
 
 constexpr int kThreads = 256;
-// Graphs with fewer edges hook every edge in one pass: there a level is a few launches either way.
+// Graphs with fewer edges (and more than kSmallN vertices) hook every edge in one pass: there a level is a few
+// launches either way.
 constexpr uint64_t kSampledEdges = 1u << 15;
 constexpr uint32_t kSampleParts = 128;        // a sampling round takes 128ths of the edges
 constexpr int kHops = 32;                     // longest walk of a compression between rounds
@@ -121,26 +122,7 @@ __global__ void approx_init(const Forest F, uint32_t n, unsigned int *count) {
     }
 }
 
-// One thread per (copy, edge), one sitmo block per draw: small graphs, where the pass is one
-// latency chain per thread and more threads finish sooner. Copies along blockIdx.y.
-__global__ void approx_keep_hook(const Forest F, const uint32_t *__restrict__ U, const uint32_t *__restrict__ V,
-                                 const uint32_t *__restrict__ Wt, uint64_t m, uint32_t level, uint32_t seed,
-                                 uint32_t ranks, uint64_t portion) {
-    pdl_wait();
-    const uint32_t j = blockIdx.y;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t w = Wt[e];
-        if (w == 0) continue;
-        const uint64_t q = portion ? e / portion : (uint64_t)ranks;
-        const uint32_t r = q < ranks ? (uint32_t)q : ranks - 1;
-        const uint64_t local = e - (uint64_t)r * portion;
-        const uint64_t x = draw64(seed + r, level, j, 1, 0, local);
-        if (x < keep_threshold(level, w)) continue;
-        aunite(F, j, U[e], V[e]);
-    }
-}
-
-// Larger graphs take the draws by quads: a quad is 4 consecutive edges of one rank's slice, local
+// The draws are taken by quads: a quad is 4 consecutive edges of one rank's slice, local
 // indices 4 lq .. 4 lq + 3, whose 4 draws are the 4 words of one sitmo block (counter lq). Rank
 // r < P - 1 owns Qf = ceil(portion / 4) quads, the last rank the rest of the edges (all of them when
 // portion is 0).
@@ -181,7 +163,7 @@ __device__ __forceinline__ Quad quad_of(const Level &L, uint32_t gq) {
 // the midpoint between b and the double below it (a tie rounds to b, whose significand is even
 // for i <= 52), i.e. iff R <= T(i) with T(1) = 2^63 + 2^9 and T(i) = 2^(64-i) + 2^10 for
 // 2 <= i <= 52 (levels stop at ceil(ln W) <= 45). R = 2^64 is U = 1, clamped below 1: never kept.
-uint64_t stream_threshold(uint32_t level) {
+__host__ __device__ __forceinline__ uint64_t stream_threshold(uint32_t level) {
     return level == 1 ? (1ull << 63) + (1ull << 9) : (1ull << (64 - level)) + (1ull << 10);
 }
 
@@ -204,8 +186,15 @@ __device__ __forceinline__ uint64_t stream_output(const Level &L, uint32_t j, ui
 }
 
 // The kept edges of quad q in copy j, bit d for its edge d (edges past the slice's end: 0).
+// Thresholds: `table` holds those of weights below kTable (a square-and-multiply of up to 16 wide
+// products each, as many instructions as the cipher for a quad of small weights).
+constexpr uint32_t kTable = 256;
+__device__ __forceinline__ void fill_thresholds(uint64_t *table, uint32_t level) {  // (a barrier follows)
+    for (uint32_t w = threadIdx.x; w < kTable; w += blockDim.x) table[w] = w ? keep_threshold(level, w) : 0;
+}
+
 template <bool kRef>
-__device__ __forceinline__ uint32_t quad_keeps(const Level &L, const Quad &q, uint32_t j) {
+__device__ __forceinline__ uint32_t quad_keeps(const Level &L, const Quad &q, uint32_t j, const uint64_t *table) {
     const uint32_t here = min(4u, q.len - 4 * q.lq);
     uint32_t mask = 0;
     if constexpr (kRef) {
@@ -236,7 +225,8 @@ __device__ __forceinline__ uint32_t quad_keeps(const Level &L, const Quad &q, ui
 #pragma unroll
         for (uint32_t d = 0; d < 4; d++) {
             const uint32_t w = d < here ? L.Wt[q.base + 4 * q.lq + d] : 0;
-            mask |= (uint32_t)(w != 0 && o.x[d] >= keep_threshold(L.level, w)) << d;
+            const uint64_t least = w < kTable ? table[w] : keep_threshold(L.level, w);
+            mask |= (uint32_t)(w != 0 && o.x[d] >= least) << d;
         }
     }
     return mask & ((1u << here) - 1);
@@ -269,7 +259,7 @@ __device__ __forceinline__ bool edge_kept(const Level &L, uint32_t e, uint32_t j
 enum QuadPass { kRound, kAll };
 constexpr uint32_t kGiven = 1024;
 template <bool kRef, QuadPass kPass>
-__device__ __forceinline__ void hook_quads(const Level &L, unsigned long long *given) {
+__device__ __forceinline__ void hook_quads(const Level &L, unsigned long long *given, const uint64_t *table) {
     const uint32_t C = L.F.copies, lane = threadIdx.x & 31, side = min(C, 32u), per = 32 / side;  // quads per warp
     if (lane >= side * per) return;
     // the pass's quads, numbered: all, or those of the round
@@ -288,7 +278,7 @@ __device__ __forceinline__ void hook_quads(const Level &L, unsigned long long *g
         const Quad q = quad_of(L, gq);
         const uint32_t e0 = q.base + 4 * q.lq;
         for (uint32_t j = lane % side; j < C; j += side) {
-            const uint32_t mask = quad_keeps<kRef>(L, q, j);
+            const uint32_t mask = quad_keeps<kRef>(L, q, j, table);
             uint32_t a[4], b[4];
 #pragma unroll
             for (uint32_t d = 0; d < 4; d++) {
@@ -325,12 +315,13 @@ __device__ __forceinline__ void hook_quads(const Level &L, unsigned long long *g
 template <bool kRef, QuadPass kPass>
 __global__ void __launch_bounds__(kThreads) approx_quads(const Level L) {
     __shared__ unsigned long long given[kPass == kRound ? kGiven : 1];
-    if (kPass == kRound) {
+    __shared__ uint64_t table[kRef ? 1 : kTable];
+    if (kPass == kRound)
         for (uint32_t i = threadIdx.x; i < kGiven; i += kThreads) given[i] = ~0ull;
-        __syncthreads();
-    }
+    if (!kRef) fill_thresholds(table, L.level);
+    __syncthreads();
     pdl_wait();
-    hook_quads<kRef, kPass>(L, given);
+    hook_quads<kRef, kPass>(L, given, table);
 }
 
 // All edges after the sampling rounds, a warp per 256-edge tile as in the filter of the
@@ -405,7 +396,10 @@ __global__ void __launch_bounds__(kThreads) approx_rest(const Level L) {
     pdl_wait();
     const uint32_t count = *L.count;
     if (count > L.cap) {
-        hook_quads<kRef, kAll>(L, nullptr);
+        __shared__ uint64_t table[kRef ? 1 : kTable];
+        if (!kRef) fill_thresholds(table, L.level);
+        __syncthreads();
+        hook_quads<kRef, kAll>(L, nullptr, table);
         return;
     }
     const uint64_t items = (uint64_t)count * L.F.copies;
@@ -534,6 +528,84 @@ __global__ void approx_count_roots(const Forest F, uint32_t n, unsigned int *cou
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
+
+// Small graphs: one CTA per (copy, level), the copy's forest in shared memory, several levels in one
+// launch. A thread takes a quad at a time; links are unions with path halving (shared CAS of the larger
+// root onto the smaller). A copy that has become one tree is decided, whatever its other edges: on the dense
+// graphs of small n that takes a few n ln n of them. The root count goes to the host's page.
+//   Bound by the cipher of the levels that are decided last (all quads) and by the launch and its wait, of
+// which there was one of each, and three kernels or more, per level. Level by level over the whole
+// device (and, to 2^15 edges, a thread per edge and a block per draw) / here: R-MAT scale 9, m = 2,048 40 / 29 us;
+// G(16,000, m = 128,000), 8 levels 623 / 163 us; G(1000, m = 125,000), 10 levels 2.0 ms / 121 us; R-MAT scale 14,
+// m = 114,688, disconnected and so decided by its first level 161 / 141 us.
+//   The rule (approx_is_small): the forest fits in 64 KB of shared memory, and one CTA's pass over the edges is
+// no longer than two levels of rounds over the whole device (70 us each): with 2^20 edges it would be 0.9 ms.
+constexpr uint32_t kSmallThreads = 1024, kSmallN = 16384, kSmallM = 1u << 17;
+
+__device__ __forceinline__ uint32_t small_find(volatile uint32_t *par, uint32_t v) {
+    uint32_t p = par[v];
+    while (p != v) {
+        const uint32_t g = par[p];
+        if (g == p) return p;
+        par[v] = g;  // (a vertex that is no root never becomes one: any ancestor may be written)
+        v = g;
+        p = par[v];
+    }
+    return v;
+}
+
+template <bool kRef>
+__global__ void __launch_bounds__(kSmallThreads) approx_small(const Level base, uint32_t *__restrict__ roots) {
+    extern __shared__ uint32_t par[];
+    __shared__ uint32_t s_links;
+    __shared__ uint64_t table[kRef ? 1 : kTable];
+    Level L = base;
+    L.level += blockIdx.y;
+    L.keep_max = stream_threshold(L.level);
+    const uint32_t j = blockIdx.x, lane = threadIdx.x & 31;
+    for (uint32_t v = threadIdx.x; v < L.n; v += kSmallThreads) par[v] = v;
+    if (threadIdx.x == 0) s_links = 0;
+    if (!kRef) fill_thresholds(table, L.level);
+    __syncthreads();
+    for (uint32_t q0 = threadIdx.x - lane; q0 < L.Q; q0 += kSmallThreads) {  // (a warp's lanes stay together)
+        if (*(volatile uint32_t *)&s_links + 1 >= L.n) break;
+        uint32_t links = 0;
+        if (q0 + lane < L.Q) {
+            const Quad q = quad_of(L, q0 + lane);
+            const uint32_t mask = quad_keeps<kRef>(L, q, j, table), e0 = q.base + 4 * q.lq;
+            uint32_t a[4], b[4];
+#pragma unroll
+            for (uint32_t d = 0; d < 4; d++) {
+                a[d] = b[d] = 0;
+                if ((mask >> d) & 1u) {
+                    a[d] = __ldg(L.U + e0 + d);
+                    b[d] = __ldg(L.V + e0 + d);
+                }
+            }
+#pragma unroll 1
+            for (uint32_t d = 0; d < 4; d++) {
+                uint32_t x = d == 0 ? a[0] : d == 1 ? a[1] : d == 2 ? a[2] : a[3];
+                uint32_t y = d == 0 ? b[0] : d == 1 ? b[1] : d == 2 ? b[2] : b[3];
+                while (x != y) {
+                    x = small_find(par, x);
+                    y = small_find(par, y);
+                    if (x == y) break;
+                    const uint32_t hi = max(x, y), lo = min(x, y);
+                    if (atomicCAS(&par[hi], hi, lo) == hi) {
+                        links++;
+                        break;
+                    }
+                }
+            }
+        }
+        links = __reduce_add_sync(0xffffffffu, links);
+        if (lane == 0 && links) atomicAdd(&s_links, links);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) roots[blockIdx.y * gridDim.x + j] = L.n - s_links;
+}
+
+bool approx_is_small(uint32_t n, uint64_t m) { return n <= kSmallN && m <= kSmallM; }
 
 // The hooks of one level (the forest already holds singletons).
 // Union walks from singletons make long parent chains that every walk then pays for (15 M edges, 4
@@ -674,20 +746,35 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
         L.giants = (uint32_t *)arena_take(ctx, 256);
         L.count = L.giants + 32;
     }
+    iterations = std::min<uint32_t>(iterations, 63);
+    const bool small = approx_is_small(g->n, g->m) && copies <= 8192;  // (the host's page holds a launch's counts)
+    if (small) {
+        auto kern = ref_stream ? approx_small<true> : approx_small<false>;
+        CAC_TRY(smem_optin(ctx, kern));
+        // as many levels as fill the device with one CTA per SM
+        const uint32_t wide = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)ctx->num_sms, 8192) / copies);
+        for (uint32_t level = 1; level <= iterations && !first; level += wide) {
+            const uint32_t here = std::min(wide, iterations + 1 - level);
+            L.level = level;
+            kern<<<dim3(copies, here), kSmallThreads, (size_t)g->n * 4, s>>>(L, ctx->pinned_u32);
+            CAC_CUDA_TRY(cudaGetLastError());
+            CAC_CUDA_TRY(cudaStreamSynchronize(s));
+            for (uint32_t i = 0; i < here && !first; i++) {
+                uint64_t total = 0;
+                for (uint32_t j = 0; j < copies; j++) total += ctx->pinned_u32[i * copies + j];
+                if (total > copies) first = level + i;
+            }
+        }
+    }
     const double mean_weight = g->m ? (double)g->total_weight / (double)g->m : 0;
-    for (uint32_t level = 1; level <= iterations && level <= 63; level++) {
+    for (uint32_t level = 1; level <= iterations && !small; level++) {
         approx_init<<<gi, kThreads, 0, s>>>(L.F, g->n, d_count);
         L.level = level;
         L.keep_max = stream_threshold(level);  // p = 2^-level (ApproximateCut.cpp:37)
-        if (large || ref_stream) {
+        if (g->m) {
             const double kept = 1 - std::pow(1 - std::ldexp(1.0, -(int)level), mean_weight);  // share of the edges
             const double degree = 2.0 * g->m * kept / std::max<uint32_t>(1, g->n);
             CAC_TRY(ref_stream ? run_level<true>(ctx, L, degree) : run_level<false>(ctx, L, degree));
-        } else if (g->m) {
-            const int ge = (int)std::max<uint64_t>(
-                1, std::min<uint64_t>((g->m + kThreads - 1) / kThreads, std::max(1, ctx->num_sms * 8 / (int)copies)));
-            approx_keep_hook<<<dim3(ge, copies), kThreads, 0, s>>>(L.F, g->u, g->v, g->w, g->m, level, seed, ranks,
-                                                                   portion);
         }
         CAC_CUDA_TRY(launch_pdl(approx_count_roots, (unsigned)gi, kThreads, 0, s, L.F, g->n, d_count));
         CAC_CUDA_TRY(cudaGetLastError());
