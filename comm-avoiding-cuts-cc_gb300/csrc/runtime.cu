@@ -247,6 +247,50 @@ __global__ void degree_add(const uint32_t *u, const uint32_t *v, const uint32_t 
     }
 }
 
+// The same for dense graphs whose total weight is below 2^32: each CTA adds up its edges in 32-bit
+// counters in shared memory, then adds those to the result. A warp whose edges have one first end (lists
+// sorted by vertex) adds it once.
+//   Bound by the shared atomics; the kernel above by those of the L2 on few addresses: K4000, 8 M edges on
+// 4,000 vertices, 466 us, here 51 us. Taken for n up to kDegreeVertices (three quarters of the shared
+// memory) from 64 edges per vertex on, with so many CTAs that what they add at the end is a quarter of
+// what they were given.
+constexpr uint32_t kDegreeVertices = 40 * 1024, kDegreeThreads = 1024;
+__global__ void __launch_bounds__(kDegreeThreads) degree_add_shared(const uint32_t *__restrict__ u, const uint32_t *__restrict__ v,
+                                                                    const uint32_t *__restrict__ w, uint64_t m, uint32_t n,
+                                                                    unsigned long long *deg) {
+    extern __shared__ uint32_t part[];
+    for (uint32_t i = threadIdx.x; i < n; i += kDegreeThreads) part[i] = 0;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t stride = (uint64_t)gridDim.x * kDegreeThreads;
+    for (uint64_t e0 = (uint64_t)blockIdx.x * kDegreeThreads + threadIdx.x - lane; e0 < m; e0 += 2 * stride) {
+        uint32_t a[2], b[2], x[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint64_t e = e0 + k * stride + lane;
+            a[k] = b[k] = x[k] = 0;
+            if (e < m) {
+                a[k] = __ldcs(u + e);
+                b[k] = __ldcs(v + e);
+                x[k] = a[k] != b[k] ? __ldcs(w + e) : 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (__all_sync(0xffffffffu, a[k] == __shfl_sync(0xffffffffu, a[k], 0))) {
+                const uint32_t sum = __reduce_add_sync(0xffffffffu, x[k]);
+                if (lane == 0 && sum) atomicAdd(&part[a[k]], sum);
+            } else if (x[k]) {
+                atomicAdd(&part[a[k]], x[k]);
+            }
+            if (x[k]) atomicAdd(&part[b[k]], x[k]);
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += kDegreeThreads)
+        if (part[i]) atomicAdd(deg + i, (unsigned long long)part[i]);
+}
+
 // Minimum over n degrees: a warp minimum, then one atomicMin per warp.
 __global__ void degree_min(const unsigned long long *deg, uint32_t n, unsigned long long *out) {
     unsigned long long x = ~0ull;
@@ -289,8 +333,14 @@ int graph_min_degree(cac_ctx *ctx, cac_graph *g, uint64_t *out) {
         cudaError_t e = cudaMemsetAsync(deg, 0, (size_t)g->n * 8, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(res, 0xFF, 8, s);
         if (e == cudaSuccess && g->m) {
-            degree_add<<<grid1(ctx, g->m), 256, 0, s>>>(g->u, g->v, g->w, g->m, deg);
-            e = cudaGetLastError();
+            if (g->n <= kDegreeVertices && g->m / 64 >= g->n && g->total_weight < (1ull << 32)) {
+                const unsigned ctas = (unsigned)std::min<uint64_t>((uint64_t)ctx->num_sms, g->m / (4ull * g->n));
+                if (smem_optin(ctx, degree_add_shared) != CAC_OK) e = cudaErrorInvalidValue;
+                else degree_add_shared<<<ctas, kDegreeThreads, (size_t)g->n * 4, s>>>(g->u, g->v, g->w, g->m, g->n, deg);
+            } else {
+                degree_add<<<grid1(ctx, g->m), 256, 0, s>>>(g->u, g->v, g->w, g->m, deg);
+            }
+            if (e == cudaSuccess) e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
             degree_min<<<grid1(ctx, g->n), 256, 0, s>>>(deg, g->n, res);
