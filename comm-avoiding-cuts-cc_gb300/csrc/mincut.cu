@@ -55,7 +55,7 @@ constexpr uint64_t kU64Max = 0xFFFFFFFFFFFFFFFFull;
 struct ShrinkDesc {
     const uint32_t *U, *V, *W;
     uint64_t m;
-    uint64_t *pre;     // m: inclusive prefix of the non-loop weights
+    uint64_t *pre;     // ceil(m / 4): inclusive prefix of the non-loop weights at the end of each four edges
     uint32_t *lab;     // n: output labels (rank of the smallest member)
     uint32_t *k_out;   // output: number of vertices left
     uint32_t n, target;
@@ -332,14 +332,16 @@ __device__ void rank_labels(const uint32_t *par, uint32_t n, LabT *lab) {
 
 // Stage 1 of one trial per CTA. Per round: the weights of the edges that are not loops and their
 // inclusive prefix in edge order, in one pass (warp w owns a contiguous range of whole coarse segments and
-// scans it from 0; four consecutive edges per lane, so one warp scan per 128), and a coarse index in shared memory of the prefix at the end
-// of every `cs`-edge segment, to which the warps' offsets are added; then draws in batches, little
+// scans it from 0; four consecutive edges per lane, so one warp scan per 128), kept at the end of each four edges,
+// and a coarse index in shared memory of the prefix at the end of every `cs`-edge segment, to which the warps' offsets are added; then draws in batches, little
 // more than the links still wanted (a stream block each four): a draw finds its segment in the shared
-// index and its edge by eight-way search inside the segment, less its warp's offset, and the batch is
-// contracted in draw order.
+// index, its four edges by eight-way search inside the segment, less its warp's offset, and its edge from
+// their weights again, by the components of the round's start (16 bits a vertex, kept beside the
+// union-find); the batch is contracted in draw order.
 //   Bound by latency: the passes over the edges and, per batch, the chain of a draw and of its union.
-//   60 trials of ER(1000, 0.05) 32 us, the trials of a 64-graph batch 8.6 ms; with two passes over the
-// edges (sums, then prefixes), 32 edges at a time, a block per draw and binary searches 39 us and 10.1 ms.
+//   60 trials of ER(1000, 0.05) 26 us, the trials of a 64-graph batch 6.7 ms. With a prefix per edge (8 bytes
+// written per edge and round) 32 us and 8.6 ms; with two passes over the edges (sums, then prefixes), 32 edges
+// at a time, a block per draw and binary searches 39 us and 10.1 ms.
 constexpr uint32_t kCoarse = 2048;      // Stage 1 coarse prefix index entries (shared memory)
 constexpr uint32_t kCoarseRows = 1024;  // contraction: coarse row-prefix index entries (shared memory)
 
@@ -360,7 +362,11 @@ __global__ void __launch_bounds__(NT) iss_shrink_kernel(const ShrinkDesc *__rest
     const uint32_t *__restrict__ Wt = D.W;
     uint64_t *pre = D.pre;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t v = threadIdx.x; v < n; v += NT) par[v] = v;
+    uint16_t *start = reinterpret_cast<uint16_t *>(par + n);  // the components when the round began
+    for (uint32_t v = threadIdx.x; v < n; v += NT) {
+        par[v] = v;
+        start[v] = (uint16_t)v;
+    }
     if (threadIdx.x == 0) s_count = n;
     __syncthreads();
     // coarse segments of a multiple of 32 edges, at most kCoarse of them; a warp owns whole ones
@@ -369,48 +375,43 @@ __global__ void __launch_bounds__(NT) iss_shrink_kernel(const ShrinkDesc *__rest
     const uint64_t wlo = min(m, (uint64_t)warp * own * cs), whi = min(m, wlo + own * cs);
     const uint32_t csg = (uint32_t)(cs / 32);
     const bool wide = (((uintptr_t)U | (uintptr_t)V | (uintptr_t)Wt) & 15) == 0;
+    // edges e .. e + 3 of those below `end`, else 0-0
+    auto quad_at = [&](uint64_t e, uint64_t end, uint4 &u, uint4 &v, uint4 &w) {
+        u = v = w = make_uint4(0, 0, 0, 0);
+        if (wide && e + 4 <= end) {
+            u = __ldg(reinterpret_cast<const uint4 *>(U + e));
+            v = __ldg(reinterpret_cast<const uint4 *>(V + e));
+            w = __ldg(reinterpret_cast<const uint4 *>(Wt + e));
+        } else {
+            if (e < end) u.x = __ldg(U + e), v.x = __ldg(V + e), w.x = __ldg(Wt + e);
+            if (e + 1 < end) u.y = __ldg(U + e + 1), v.y = __ldg(V + e + 1), w.y = __ldg(Wt + e + 1);
+            if (e + 2 < end) u.z = __ldg(U + e + 2), v.z = __ldg(V + e + 2), w.z = __ldg(Wt + e + 2);
+            if (e + 3 < end) u.w = __ldg(U + e + 3), v.w = __ldg(V + e + 3), w.w = __ldg(Wt + e + 3);
+        }
+    };
     for (uint64_t rnd = 0; s_count > target; rnd++) {
         uint64_t carry = 0;
         for (uint64_t e0 = wlo; e0 < whi; e0 += 128) {
             const uint64_t e = e0 + 4 * lane;
-            uint4 u = make_uint4(0, 0, 0, 0), v = u, w = u;
-            if (wide && e + 4 <= whi) {
-                u = __ldg(reinterpret_cast<const uint4 *>(U + e));
-                v = __ldg(reinterpret_cast<const uint4 *>(V + e));
-                w = __ldg(reinterpret_cast<const uint4 *>(Wt + e));
-            } else {
-                if (e < whi) u.x = __ldg(U + e), v.x = __ldg(V + e), w.x = __ldg(Wt + e);
-                if (e + 1 < whi) u.y = __ldg(U + e + 1), v.y = __ldg(V + e + 1), w.y = __ldg(Wt + e + 1);
-                if (e + 2 < whi) u.z = __ldg(U + e + 2), v.z = __ldg(V + e + 2), w.z = __ldg(Wt + e + 2);
-                if (e + 3 < whi) u.w = __ldg(U + e + 3), v.w = __ldg(V + e + 3), w.w = __ldg(Wt + e + 3);
-            }
-            uint64_t x[4];
-            x[0] = par[u.x] != par[v.x] ? w.x : 0;
-            x[1] = x[0] + (par[u.y] != par[v.y] ? w.y : 0);
-            x[2] = x[1] + (par[u.z] != par[v.z] ? w.z : 0);
-            x[3] = x[2] + (par[u.w] != par[v.w] ? w.w : 0);
-            uint64_t incl = x[3];
+            uint4 u, v, w;
+            quad_at(e, whi, u, v, w);
+            const uint64_t sum = (uint64_t)(par[u.x] != par[v.x] ? w.x : 0) + (par[u.y] != par[v.y] ? w.y : 0) +
+                                 (par[u.z] != par[v.z] ? w.z : 0) + (par[u.w] != par[v.w] ? w.w : 0);
+            uint64_t incl = sum;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += y;
             }
-            const uint64_t off = carry + incl - x[3];
-#pragma unroll
-            for (int i = 0; i < 4; i++) x[i] += off;
+            const uint64_t end = carry + incl;
             carry += __shfl_sync(0xffffffffu, incl, 31);
-            if (e + 4 <= whi) {
-                reinterpret_cast<ulonglong2 *>(pre + e)[0] = make_ulonglong2(x[0], x[1]);
-                reinterpret_cast<ulonglong2 *>(pre + e)[1] = make_ulonglong2(x[2], x[3]);
-            } else {
-                for (int i = 0; i < 4 && e + i < whi; i++) pre[e + i] = i == 0 ? x[0] : i == 1 ? x[1] : x[2];
-            }
-            // the end of a segment (lanes 7, 15, 23 and 31 end 32 edges) or of the list (x[3]: past it, weights are 0)
+            if (e < whi) pre[e / 4] = end;
+            // the end of a segment (lanes 7, 15, 23 and 31 end 32 edges) or of the list
             if ((lane & 7) == 7 && e < whi) {
                 const uint32_t groups = (uint32_t)(e / 32) + 1;
-                if (groups % csg == 0) coarse[groups / csg - 1] = x[3];
+                if (groups % csg == 0) coarse[groups / csg - 1] = end;
             }
-            if (e < m && e + 4 >= m) coarse[ncs - 1] = x[3];
+            if (e < m && e + 4 >= m) coarse[ncs - 1] = end;
         }
         if (lane == 0) s_w[warp] = carry;
         __syncthreads();
@@ -441,16 +442,30 @@ __global__ void __launch_bounds__(NT) iss_shrink_kernel(const ShrinkDesc *__rest
             for (uint32_t j = threadIdx.x; j < nb; j += NT) {
                 const uint64_t y = (uint64_t)sb[j].y << 32 | sb[j].x;
                 const uint32_t sg = (uint32_t)upper_bound_u64(coarse, ncs, y);
-                const uint64_t s0 = sg * cs;
+                const uint64_t s0 = sg * cs, off = s_off[sg / own];
                 uint64_t before;
-                const uint64_t e = s0 + upper_bound8<false>(pre + s0, (uint32_t)min(cs, m - s0), y - s_off[sg / own], before);
-                sb[j] = make_uint2(__ldg(U + e), __ldg(V + e));
+                const uint32_t quad = upper_bound8<false>(pre + s0 / 4, (uint32_t)((min(cs, m - s0) + 3) / 4), y - off, before);
+                if (quad == 0) before = sg % own ? coarse[sg - 1] - off : 0;
+                // the quad's edges again, with the components of the round's start
+                const uint64_t e = s0 + 4 * quad;
+                uint4 u, v, w;
+                quad_at(e, m, u, v, w);
+                const uint64_t rem = y - off - before;
+                const uint64_t p1 = start[u.x] != start[v.x] ? w.x : 0, p2 = p1 + (start[u.y] != start[v.y] ? w.y : 0),
+                               p3 = p2 + (start[u.z] != start[v.z] ? w.z : 0);
+                const uint32_t a = rem < p1 ? u.x : rem < p2 ? u.y : rem < p3 ? u.z : u.w;
+                const uint32_t b = rem < p1 ? v.x : rem < p2 ? v.y : rem < p3 ? v.z : v.w;
+                sb[j] = make_uint2(a, b);
             }
             contract_batch<NT>(par, sb, nb, target, &s_count, &s_nlog);
             if (s_count <= target) break;
             base += nb;
         }
-        for (uint32_t v = threadIdx.x; v < n; v += NT) par[v] = sfind_ro(par, v);
+        for (uint32_t v = threadIdx.x; v < n; v += NT) {
+            const uint32_t r = sfind_ro(par, v);
+            par[v] = r;
+            start[v] = (uint16_t)r;
+        }
         __syncthreads();
     }
     rank_labels<NT>(par, n, D.lab);
@@ -2518,7 +2533,7 @@ int admit(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
 // launch and two host synchronisations per query.
 int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan *> &qs) {
     cudaStream_t s = ctx->stream;
-    auto pre_words_of = [](uint64_t m) { return std::max<uint64_t>((m + 3) & ~3ull, 4); };  // (16-byte stores)
+    auto pre_words_of = [](uint64_t m) { return std::max<uint64_t>((m + 3) / 4, 1); };
     struct Item {
         const QueryPlan *q;
         uint64_t i;
@@ -2570,7 +2585,7 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
             po += pre_words_of(q.g->m);
             lo += q.g->n;
         }
-        const size_t sm = kBatch * sizeof(uint2) + kCoarse * sizeof(uint64_t) + (size_t)nmax * 4;
+        const size_t sm = kBatch * sizeof(uint2) + kCoarse * sizeof(uint64_t) + (size_t)nmax * 6;
         CAC_TRY(upload(ctx, d_sd, sd));
         // fewer trials than SMs: one trial per SM either way, so each trial gets 1024 threads
         if (B < (uint32_t)ctx->num_sms) {
