@@ -345,11 +345,13 @@ __global__ void cc_compress4(uint32_t *par, uint32_t n) {
 // Compression of [0, n) (the parent array is 256-byte aligned).
 void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s);
 
-// The bitmap's allocation: a word per 32 vertices, then, for graphs whose bitmap does not fit in shared memory,
-// a byte per 32 vertices (a bit per four of them), read as words.
-__host__ __device__ __forceinline__ uint32_t quad_words_at(uint32_t nwords) { return (nwords + 3) & ~3u; }
-size_t bitmap_bytes(size_t nwords) {
-    return nwords * 4 + 4 + (nwords > kSmemBitmapWords ? 16 + (nwords + 3) / 4 * 4 : 0);
+// A byte per 32 vertices, a bit per four of them (read as words): for graphs whose bitmap does not fit in
+// shared memory, where the budget has room for it.
+size_t quad_bytes(uint32_t nwords) { return nwords > kSmemBitmapWords ? (size_t)(nwords + 3) / 4 * 4 : 0; }
+bool quads_fit(const cac_ctx *ctx, size_t base, uint32_t nwords) {
+    const size_t more = align_up(quad_bytes(nwords));
+    return more && (base + more <= ctx->arena.cap || !ctx->budget ||
+                    ctx->held - ctx->arena.cap + align_up(base + more, 1 << 20) <= ctx->budget);
 }
 
 // The end of the sampling round in one launch: full compression, the giant component and its
@@ -363,7 +365,7 @@ size_t bitmap_bytes(size_t nwords) {
 // writes the root back when it differs (only roots are written, as in cc_compress4), and the
 // warp's ballot of (root == giant) is the word. CTA 0 records the giant for the next kernels.
 __global__ void __launch_bounds__(kGiantSample) cc_compress_giant_bitmap(uint32_t *par, uint32_t n, uint32_t *giant,
-                                                                         uint32_t *bits) {
+                                                                         uint32_t *bits, uint8_t *quads) {
     pdl_wait();
     __shared__ uint32_t cand[kGiantSample / 32], cnt[kGiantSample / 32];
     __shared__ unsigned long long best;
@@ -401,13 +403,13 @@ __global__ void __launch_bounds__(kGiantSample) cc_compress_giant_bitmap(uint32_
         }
         const uint32_t word = __ballot_sync(0xffffffffu, in);
         if (lane == 0) bits[wd] = word;
-        if (nw > kSmemBitmapWords && lane == 0) {  // a bit per four vertices: all of them are in the giant
+        if (quads && lane == 0) {  // a bit per four vertices: all of them are in the giant
             uint32_t b = word & (word >> 1);
             b &= b >> 2;
             b &= 0x11111111u;
             b = (b | b >> 3) & 0x03030303u;
             b = (b | b >> 6) & 0x000F000Fu;
-            reinterpret_cast<uint8_t *>(bits + quad_words_at((uint32_t)nw))[wd] = (uint8_t)(b | b >> 12);
+            quads[wd] = (uint8_t)(b | b >> 12);
         }
     }
 }
@@ -470,18 +472,18 @@ template <bool kAllSmem, bool kCheck>
 __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__restrict__ u,
                                                           const uint32_t *__restrict__ v, uint64_t tiles,
                                                           const uint32_t *__restrict__ gbits, uint32_t nwords,
-                                                          uint2 *__restrict__ surv, uint32_t *__restrict__ counts,
+                                                          const uint32_t *__restrict__ quads, uint2 *__restrict__ surv, uint32_t *__restrict__ counts,
                                                           uint32_t n, uint32_t *err) {
     pdl_wait();
     extern __shared__ uint32_t sbits[];
     __shared__ uint32_t s_n, s_found;
     const uint32_t swords = min(nwords, (uint32_t)kSmemBitmapWords);
     // words staged: of the quads' bitmap first, where the full one does not fit
-    uint32_t qwords = kAllSmem ? 0u : min((nwords + 3) / 4, (uint32_t)kSmemBitmapWords);
-    if (kAllSmem)
+    uint32_t qwords = kAllSmem || !quads ? 0u : min((nwords + 3) / 4, (uint32_t)kSmemBitmapWords);
+    if (!qwords)
         for (uint32_t i = threadIdx.x; i < swords; i += blockDim.x) sbits[i] = gbits[i];
     else
-        for (uint32_t i = threadIdx.x; i < qwords; i += blockDim.x) sbits[i] = gbits[quad_words_at(nwords) + i];
+        for (uint32_t i = threadIdx.x; i < qwords; i += blockDim.x) sbits[i] = quads[i];
     if (threadIdx.x == 0) s_n = s_found = 0;
     __syncthreads();
     const uint64_t per = (tiles + gridDim.x - 1) / gridDim.x;
@@ -558,7 +560,7 @@ __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__rest
         if (lane == 0 && found) atomicAdd(&s_found, found);
         const uint64_t warps_in = t1 > t0 ? min((uint64_t)nwarps, (t1 - t0 + 1) / 2) : 0;
         __syncthreads();
-        if ((uint64_t)s_found * nwords < 64 * warps_in * swords) {
+        if (qwords && (uint64_t)s_found * nwords < 64 * warps_in * swords) {
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < swords; i += blockDim.x) sbits[i] = gbits[i];
             qwords = 0;
@@ -934,7 +936,7 @@ size_t cc_scratch_bytes(uint32_t n, uint32_t ranks, uint64_t m) {
     const size_t ntiles = ((size_t)n + kTile - 1) / kTile;
     const size_t nwords = ((size_t)n + 31) / 32;
     return align_up((size_t)n * 4) + 2 * align_up(ntiles * 4 + 4) + align_up(256) +
-           align_up(sizeof(RankDesc) * (size_t)ranks) + align_up(bitmap_bytes(nwords)) + align_up(kMaxRegions * 4) +
+           align_up(sizeof(RankDesc) * (size_t)ranks) + align_up(nwords * 4 + 4) + align_up(kMaxRegions * 4) +
            align_up((m + 4 * (uint64_t)kMaxRegions) * 8);
 }
 
@@ -953,6 +955,7 @@ struct CCLaunch {
     RankDesc *d_ranks = nullptr;
     const RankDesc *h_ranks = nullptr;
     uint32_t ntiles = 0, nwords = 0;
+    uint8_t *quads = nullptr;                    // see quad_bytes
     uint64_t blocks = 0, draws = 0, drawn = 0;  // sitmo blocks, chunk draws, sampled edges
     uint64_t *chunks = nullptr;                  // per draw: first edge | count << 32
     uint32_t *err = nullptr;                     // total + kErrWord
@@ -1038,7 +1041,7 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
             if (d1 < L.draws) compress_all(ctx, L.par, n, s);
         }
         CAC_CUDA_TRY(launch_pdl(cc_compress_giant_bitmap, giant_grid(ctx, n), kGiantSample, 0, s, L.par, n, L.giant,
-                                L.bits));
+                                L.bits, L.quads));
     }
     CAC_TRY(record(ctx, 1, capturing));
     if (m > 0) {
@@ -1053,7 +1056,8 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
                 auto filt = L.nwords <= kSmemBitmapWords ? (L.check ? cc_filter<true, true> : cc_filter<true, false>)
                                                          : (L.check ? cc_filter<false, true> : cc_filter<false, false>);
                 CAC_CUDA_TRY(launch_pdl(filt, regions, kEdgeThreads, sm, s, L.u, L.v, tiles,
-                                        static_cast<const uint32_t *>(L.bits), L.nwords, L.surv, L.region_counts, n,
+                                        static_cast<const uint32_t *>(L.bits), L.nwords,
+                                        reinterpret_cast<const uint32_t *>(L.quads), L.surv, L.region_counts, n,
                                         L.err));
             }
             CAC_TRY(record(ctx, 4, capturing));
@@ -1168,7 +1172,9 @@ int cc_run(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint
     L.vec = ((reinterpret_cast<uintptr_t>(d_u) | reinterpret_cast<uintptr_t>(d_v)) & 15) == 0;
     L.check = check_ids;
 
-    CAC_TRY(arena_reserve(ctx, cc_scratch_bytes(n, ranks, m) + align_up(chunk_slots * 8)));
+    const size_t base = cc_scratch_bytes(n, ranks, m) + align_up(chunk_slots * 8);
+    const bool quads = quads_fit(ctx, base, L.nwords);
+    CAC_TRY(arena_reserve(ctx, base + (quads ? align_up(quad_bytes(L.nwords)) : 0)));
     arena_reset(ctx);
     L.par = (uint32_t *)arena_take(ctx, (size_t)n * 4);
     L.counts = (uint32_t *)arena_take(ctx, (size_t)L.ntiles * 4 + 4);
@@ -1177,10 +1183,11 @@ int cc_run(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint
     L.giant = L.total + 8;
     L.err = L.total + kErrWord;
     L.d_ranks = (RankDesc *)arena_take(ctx, sizeof(RankDesc) * ranks);
-    L.bits = (uint32_t *)arena_take(ctx, bitmap_bytes(L.nwords));
+    L.bits = (uint32_t *)arena_take(ctx, (size_t)L.nwords * 4 + 4);
     L.region_counts = (uint32_t *)arena_take(ctx, kMaxRegions * 4);
     L.surv = (uint2 *)arena_take(ctx, (m + 4 * (uint64_t)kMaxRegions) * 8);
     L.chunks = (uint64_t *)arena_take(ctx, chunk_slots * 8);
+    if (quads) L.quads = (uint8_t *)arena_take(ctx, quad_bytes(L.nwords));
 
     // rank descriptors go through the ctx's pinned staging page when they fit (async copy)
     std::vector<RankDesc> hv;
@@ -1301,6 +1308,7 @@ struct StreamLaunch {
     uint32_t *bits = nullptr, *region_counts = nullptr;
     uint2 *surv = nullptr;
     uint32_t ntiles = 0, nwords = 0;
+    uint8_t *quads = nullptr;                    // see quad_bytes
     bool vec = false, filtered = false;
     std::vector<std::pair<uint64_t, uint64_t>> parts;  // (first edge, count): pieces, then gaps
 };
@@ -1364,7 +1372,7 @@ int stream_enqueue(cac_ctx *ctx, const StreamLaunch &L, bool capturing) {
             cc_edge_pass<false, true><<<grid_for(ctx, len, 8), kThreads, 0, s>>>(L.par, L.d_u + e0, L.d_v + e0, len, n,
                                                                            L.total + kErrWord);
             if (L.filtered && c + 1 == kStreamPieces) {
-                cc_compress_giant_bitmap<<<giant_grid(ctx, n), kGiantSample, 0, s>>>(L.par, n, L.giant, L.bits);
+                cc_compress_giant_bitmap<<<giant_grid(ctx, n), kGiantSample, 0, s>>>(L.par, n, L.giant, L.bits, L.quads);
                 CAC_TRY(record(ctx, 1, capturing));
             } else if (c + 1 < L.parts.size()) {
                 compress_all(ctx, L.par, n, s);
@@ -1377,7 +1385,8 @@ int stream_enqueue(cac_ctx *ctx, const StreamLaunch &L, bool capturing) {
             if (tiles) {
                 const size_t sm = (size_t)std::min(L.nwords, kSmemBitmapWords) * 4;
                 auto filt = L.nwords <= kSmemBitmapWords ? cc_filter<true, true> : cc_filter<false, true>;
-                filt<<<regions, kEdgeThreads, sm, s>>>(L.d_u + e0, L.d_v + e0, tiles, L.bits, L.nwords, L.surv,
+                filt<<<regions, kEdgeThreads, sm, s>>>(L.d_u + e0, L.d_v + e0, tiles, L.bits, L.nwords,
+                                                       reinterpret_cast<const uint32_t *>(L.quads), L.surv,
                                                        L.region_counts, n, L.total + kErrWord);
                 cc_hook_survivors<<<(unsigned)ctx->num_sms * kSurvivorBlocksPerSm, kThreads, 0, s>>>(L.par, L.surv, L.region_counts,
                                                                                    regions, tper * 256);
@@ -1437,10 +1446,12 @@ int cc_run_streamed(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *h_u, c
                                : 0;
     L.filtered = L.vec && seg > 0;
     const uint64_t max_gap = L.filtered ? m - (kStreamPieces - 1) * seg - piece : 0;
-    CAC_TRY(arena_reserve(ctx, align_up((size_t)n * 4) + 2 * align_up((size_t)L.ntiles * 4 + 4) + align_up(256) +
-                                   (L.filtered ? align_up(bitmap_bytes(L.nwords)) + align_up(kMaxRegions * 4) +
-                                                     align_up((max_gap + 4 * (uint64_t)kMaxRegions) * 8)
-                                               : 0)));
+    const size_t base = align_up((size_t)n * 4) + 2 * align_up((size_t)L.ntiles * 4 + 4) + align_up(256) +
+                        (L.filtered ? align_up((size_t)L.nwords * 4 + 4) + align_up(kMaxRegions * 4) +
+                                          align_up((max_gap + 4 * (uint64_t)kMaxRegions) * 8)
+                                    : 0);
+    const bool quads = L.filtered && quads_fit(ctx, base, L.nwords);
+    CAC_TRY(arena_reserve(ctx, base + (quads ? align_up(quad_bytes(L.nwords)) : 0)));
     arena_reset(ctx);
     L.par = (uint32_t *)arena_take(ctx, (size_t)n * 4);
     L.counts = (uint32_t *)arena_take(ctx, (size_t)L.ntiles * 4 + 4);
@@ -1448,9 +1459,10 @@ int cc_run_streamed(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *h_u, c
     L.total = (uint32_t *)arena_take(ctx, 256);
     L.giant = L.total + 8;
     if (L.filtered) {
-        L.bits = (uint32_t *)arena_take(ctx, bitmap_bytes(L.nwords));
+        L.bits = (uint32_t *)arena_take(ctx, (size_t)L.nwords * 4 + 4);
         L.region_counts = (uint32_t *)arena_take(ctx, kMaxRegions * 4);
         L.surv = (uint2 *)arena_take(ctx, (max_gap + 4 * (uint64_t)kMaxRegions) * 8);
+        if (quads) L.quads = (uint8_t *)arena_take(ctx, quad_bytes(L.nwords));
         CAC_TRY(smem_optin(ctx, cc_filter<true, true>));
         CAC_TRY(smem_optin(ctx, cc_filter<false, true>));
         CAC_TRY(smem_optin(ctx, cc_filter<true, false>));

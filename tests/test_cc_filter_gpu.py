@@ -38,3 +38,27 @@ def test_labels_above_the_line(ctx, n, kind):
 def test_rmat_22(ctx):
     n, u, v, _ = graphgen.rmat(22, 4, 3)
     _check(ctx, n, u, v)
+
+
+def test_budget_without_room_for_the_quads(libcac):
+    import cac
+    n, m = LINE + 40001, 3 << 20
+    rng = np.random.default_rng(3)
+    u, v = (rng.integers(0, n, m).astype(np.uint32) for _ in range(2))
+    want_count, want = O.cc_labels(n, u, v)
+    with cac.Context(0) as c:
+        c.graph(n, u, v).connected_components(seed=1)
+        full = c.device_bytes
+    answered = 0
+    for budget in range(full - (2 << 20), full + (64 << 20), 1 << 18):  # from the first that suffices
+        with cac.Context(0, hbm_budget_bytes=budget) as c:
+            try:
+                count, lab, _ = c.graph(n, u, v).connected_components(seed=1)
+            except cac.CacError:
+                assert not answered
+                continue
+            answered += 1
+            assert count == want_count and np.array_equal(lab, want)
+        if answered == 8:
+            break
+    assert answered
