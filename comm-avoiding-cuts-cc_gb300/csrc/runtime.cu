@@ -440,7 +440,7 @@ int cac_ctx_set_quotient_kernel(cac_ctx *ctx, int kind) {
         set_error("cac_ctx_set_quotient_kernel: kind must be 0 (by size), 1, 2, 3 or 4");
         return CAC_ERR_INVALID;
     }
-    ctx->quotient_forced = (uint8_t)kind;
+    ctx->quotient_forced = kind == 4 ? kQuotientAuto : (uint8_t)kind;
     return CAC_OK;
 }
 
