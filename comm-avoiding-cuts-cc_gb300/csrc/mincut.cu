@@ -2034,7 +2034,16 @@ int KsEngine::step() {
     DevBuf &d_kout = *static_cast<DevBuf *>(d_kout_), &d_prep = *static_cast<DevBuf *>(d_prep_);
     DevBuf &d_tscratch = *static_cast<DevBuf *>(d_tscratch_);
     uint32_t *d_err = static_cast<DevBuf *>(d_err_)->as<uint32_t>();
-    std::vector<MatBuf *> consumed;
+    // the buffers of the nodes and tasks taken from the lists, released when the step ends: what it enqueued
+    // reads them (freeing is ordered by the stream), and a step that fails keeps none
+    struct Consumed {
+        KsEngine &eng;
+        std::vector<MatBuf *> bufs;
+        ~Consumed() {
+            for (MatBuf *b : bufs) eng.release(b);
+        }
+        void push_back(MatBuf *b) { bufs.push_back(b); }
+    } consumed{*this, {}};
 
     // leaves (n <= 128) -> exact cut, one launch per entry width
     std::vector<LeafDesc> leaves;
@@ -2096,10 +2105,7 @@ int KsEngine::step() {
         consumed.push_back(t.src.buf);
     }
     carried_.clear();
-    if (tasks.empty()) {
-        for (MatBuf *b : consumed) release(b);
-        return CAC_OK;
-    }
+    if (tasks.empty()) return CAC_OK;
     // sources whose row sums and block prefixes came with their matrix (warp quotient) skip the
     // row prep; the others (roots, large-N quotients) are prepped here from their own list
     std::vector<SrcDesc> srcs(src_nodes.size()), psrcs;
@@ -2251,6 +2257,16 @@ int KsEngine::step() {
     // Three quotient kernels, identical outputs: triangles for small children, tiles up to kTileMaxN source
     // vertices, one row per CTA above; the caller may force tiles (where they fit) or rows.
     MatBuf *out = nullptr;
+    struct Output {  // released again if the step ends before a child holds it
+        KsEngine &eng;
+        MatBuf *&buf;
+        ~Output() {
+            if (buf && buf->refs == 0) {
+                buf->refs = 1;
+                eng.release(buf);
+            }
+        }
+    } output{*this, out};
     if (out_bytes || !leaf_list[0].empty() || !leaf_list[1].empty()) {
         if (out_bytes) CAC_TRY(alloc(out_bytes, &out));
         unsigned char *obase = out ? static_cast<unsigned char *>(out->p) : nullptr;
@@ -2386,8 +2402,6 @@ int KsEngine::step() {
         }
         CAC_CUDA_TRY(cudaGetLastError());
     }
-    // the sources are read by everything enqueued above: their buffers may now be released
-    for (MatBuf *b : consumed) release(b);
     for (size_t i = 0; i < tasks.size(); i++) {
         const KTask &t = tasks[i];
         outstanding[t.src.query]--;
@@ -2410,10 +2424,6 @@ int KsEngine::step() {
             c.round += 1;
             carried_.push_back(c);
         }
-    }
-    if (out && out->refs == 0) {  // every child was dropped
-        out->refs = 1;
-        release(out);
     }
     return CAC_OK;
 }
