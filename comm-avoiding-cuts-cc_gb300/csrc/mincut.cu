@@ -332,9 +332,10 @@ __device__ void rank_labels(const uint32_t *par, uint32_t n, LabT *lab) {
 
 // Stage 1 of one trial per CTA. Per round: the weights of the edges that are not loops and their
 // inclusive prefix in edge order, in one pass (warp w owns a contiguous range of whole coarse segments and
-// scans it from 0; four consecutive edges per lane, so one warp scan per 128), kept at the end of each four edges,
-// and a coarse index in shared memory of the prefix at the end of every `cs`-edge segment, to which the warps' offsets are added; then draws in batches, little
-// more than the links still wanted (a stream block each four): a draw finds its segment in the shared
+// scans it from 0; four consecutive edges per lane, so one warp scan per 128), kept at the end of each
+// four edges, and a coarse index in shared memory of the prefix at the end of every `cs`-edge segment,
+// to which the warps' offsets are added; then draws in batches, little more than the links still
+// wanted (a stream block each four): a draw finds its segment in the shared
 // index, its four edges by eight-way search inside the segment, less its warp's offset, and its edge from
 // their weights again, by the components of the round's start (16 bits a vertex, kept beside the
 // union-find); the batch is contracted in draw order.
