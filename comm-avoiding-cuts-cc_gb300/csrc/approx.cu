@@ -35,6 +35,7 @@
 // Graphs with other weights draw a variable number of outputs per edge (a sequential chain per
 // rank), so the replay takes unit weights only.
 #include "cac_internal.h"
+#include "grid_loop.cuh"
 #include "pdl.cuh"
 #include "sitmo.cuh"
 
@@ -113,13 +114,12 @@ __device__ __forceinline__ uint32_t root_of(const Forest &F, uint32_t j, uint32_
 // Singletons, one thread per vertex, and the root count at 0.
 __global__ void approx_init(const Forest F, uint32_t n, unsigned int *count) {
     pdl_wait();
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    if (tid == 0) *count = 0;
-    for (uint32_t x = tid; x < n; x += stride) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
+    grid_stride(n, [&](uint32_t x) {
         if (F.copies == 4) reinterpret_cast<uint4 *>(F.par)[x] = make_uint4(x, x, x, x);
         else
             for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = x;
-    }
+    });
 }
 
 // The draws are taken by quads: a quad is 4 consecutive edges of one rank's slice, local
@@ -439,19 +439,19 @@ __device__ __forceinline__ uint32_t near_of(const Forest &F, uint32_t j, uint32_
 // a link at a vertex that is no root any more separates is joined again by the pass over all edges).
 __global__ void approx_compress(const Forest F, uint32_t n) {
     pdl_wait();
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (F.copies == 4) {
         uint4 *p4 = reinterpret_cast<uint4 *>(F.par);
-        for (uint32_t x = tid; x < n; x += stride) {
+        grid_stride(n, [&](uint32_t x) {
             const uint4 p = p4[x];
             const uint32_t g0 = F.par[4 * p.x], g1 = F.par[4 * p.y + 1], g2 = F.par[4 * p.z + 2], g3 = F.par[4 * p.w + 3];
             const uint32_t r0 = g0 == p.x ? g0 : near_of(F, 0, g0), r1 = g1 == p.y ? g1 : near_of(F, 1, g1);
             const uint32_t r2 = g2 == p.z ? g2 : near_of(F, 2, g2), r3 = g3 == p.w ? g3 : near_of(F, 3, g3);
             if (r0 != p.x || r1 != p.y || r2 != p.z || r3 != p.w) p4[x] = make_uint4(r0, r1, r2, r3);
-        }
+        });
     } else {
-        for (uint32_t x = tid; x < n; x += stride)
+        grid_stride(n, [&](uint32_t x) {
             for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = near_of(F, j, x);
+        });
     }
 }
 
@@ -515,16 +515,15 @@ __global__ void approx_members(const Level L) {
 
 __global__ void approx_count_roots(const Forest F, uint32_t n, unsigned int *count) {
     pdl_wait();
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     uint32_t c = 0;
-    for (uint32_t x = tid; x < n; x += stride) {
+    grid_stride(n, [&](uint32_t x) {
         if (F.copies == 4) {
             const uint4 p = reinterpret_cast<const uint4 *>(F.par)[x];
             c += (uint32_t)(p.x == x) + (uint32_t)(p.y == x) + (uint32_t)(p.z == x) + (uint32_t)(p.w == x);
         } else {
             for (uint32_t j = 0; j < F.copies; j++) c += F.at(x, j) == x;
         }
-    }
+    });
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }

@@ -22,6 +22,7 @@
 // 16-byte vector loads, 4 edges per load pair); parent[n] uint32 (L2-resident for n up to
 // tens of millions: 129 MB of L2); per-tile root counts; labels[n].
 #include "cac_internal.h"
+#include "grid_loop.cuh"
 #include "pdl.cuh"
 #include "sitmo.cuh"
 
@@ -136,7 +137,7 @@ __device__ __forceinline__ void edge_hook_checked(uint32_t *par, uint32_t a, uin
 
 __global__ void cc_init(uint32_t *par, uint32_t n) {
     pdl_wait();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) par[i] = i;
+    grid_stride(n, [&](uint32_t i) { par[i] = i; });
 }
 
 // The draws of the sampling round, one thread per sitmo block (8 draws of one rank). The reference
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(kThreads) cc_hook_survivors(uint32_t *par, con
     if (threadIdx.x == kThreads - 1 && nregions == kMaxRegions) pre[kMaxRegions] = acc;
     __syncthreads();
     const uint32_t total = pre[nregions];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    grid_stride(total, [&](uint32_t i) {
         uint32_t lo = 0, hi = nregions - 1;  // last region whose first survivor <= i
         while (lo < hi) {
             const uint32_t mid = (lo + hi + 1) >> 1;
@@ -618,7 +619,7 @@ __global__ void __launch_bounds__(kThreads) cc_hook_survivors(uint32_t *par, con
         }
         const uint2 e = surv[(uint64_t)lo * region_stride + (i - pre[lo])];
         edge_hook(par, e.x, e.y);
-    }
+    });
 }
 
 __device__ __forceinline__ uint32_t block_sum(uint32_t x, uint32_t *sh) {
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(kThreads) cc_rank_roots(const uint32_t *par, u
 __global__ void __launch_bounds__(kThreads) cc_label_all(uint32_t *par, uint32_t n, uint32_t *labels) {
     pdl_wait();
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
+    grid_stride(n, [&](uint32_t i0) {
         uint32_t p[4], r[4];
 #pragma unroll
         for (uint32_t k = 0; k < 4; k++) p[k] = i0 + (uint64_t)k * stride < n ? par[i0 + k * stride] : 0;
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(kThreads) cc_label_all(uint32_t *par, uint32_t
             if (r[k] != p[k]) par[i] = r[k];
             labels[i] = labels[r[k]];
         }
-    }
+    }, 4);
 }
 
 // Count and labels of a finished forest. Up to kOwnTiles tiles each ranking CTA sums the counts before
