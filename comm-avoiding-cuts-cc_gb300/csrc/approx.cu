@@ -566,8 +566,11 @@ __global__ void __launch_bounds__(kSmallThreads) approx_small(const Level base, 
     if (threadIdx.x == 0) s_links = 0;
     if (!kRef) fill_thresholds(table, L.level);
     __syncthreads();
-    for (uint32_t q0 = threadIdx.x - lane; q0 < L.Q; q0 += kSmallThreads) {  // (a warp's lanes stay together)
-        if (*(volatile uint32_t *)&s_links + 1 >= L.n) break;
+    for (uint32_t q0 = threadIdx.x - lane; q0 < L.Q; q0 += kSmallThreads) {
+        // other warps add to the count meanwhile: one lane's look at it decides for the warp, whose lanes
+        // meet again in the sum below
+        const uint32_t seen = lane == 0 ? *(volatile uint32_t *)&s_links : 0;
+        if (__shfl_sync(0xffffffffu, seen, 0) + 1 >= L.n) break;
         uint32_t links = 0;
         if (q0 + lane < L.Q) {
             const Quad q = quad_of(L, q0 + lane);
