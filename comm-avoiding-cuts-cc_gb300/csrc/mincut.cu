@@ -37,6 +37,7 @@
 #include <cstring>
 #include <numeric>
 #include <type_traits>
+#include <utility>
 
 namespace cac {
 namespace {
@@ -2026,6 +2027,39 @@ void KsEngine::add(const KNode &nd) {
     outstanding[nd.query]++;
 }
 
+namespace {
+
+// A buffer that a scope has allocated and holds one reference on until it ends, however it ends.
+struct Held {
+    KsEngine &eng;
+    MatBuf *buf = nullptr;
+    explicit Held(KsEngine &e) : eng(e) {}
+    Held(const Held &) = delete;
+    Held &operator=(const Held &) = delete;
+    ~Held() { eng.release(buf); }
+    int alloc(size_t bytes) {
+        CAC_TRY(eng.alloc(bytes, &buf));
+        buf->refs++;
+        return CAC_OK;
+    }
+    unsigned char *at(uint64_t off) const { return buf ? static_cast<unsigned char *>(buf->p) + off : nullptr; }
+};
+
+// Sparse roots on their way to sparse_phase, which takes over their references.
+struct SparseRoots {
+    KsEngine &eng;
+    std::vector<SparseNode> nodes;
+    explicit SparseRoots(KsEngine &e) : eng(e) {}
+    SparseRoots(const SparseRoots &) = delete;
+    SparseRoots &operator=(const SparseRoots &) = delete;
+    ~SparseRoots() {
+        for (const SparseNode &nd : nodes) eng.release(nd.buf);
+    }
+    std::vector<SparseNode> take() { return std::exchange(nodes, {}); }
+};
+
+}  // namespace
+
 int KsEngine::step() {
     cudaStream_t s = ctx_->stream;
     if (release_err_) {
@@ -2035,32 +2069,34 @@ int KsEngine::step() {
     DevBuf &d_kout = *static_cast<DevBuf *>(d_kout_), &d_prep = *static_cast<DevBuf *>(d_prep_);
     DevBuf &d_tscratch = *static_cast<DevBuf *>(d_tscratch_);
     uint32_t *d_err = static_cast<DevBuf *>(d_err_)->as<uint32_t>();
-    // the buffers of the nodes and tasks taken from the lists, released when the step ends: what it enqueued
-    // reads them (freeing is ordered by the stream), and a step that fails keeps none
+    // the buffers of all nodes and tasks, which leave the lists here: released when the step ends, as what it
+    // enqueued reads them (freeing is ordered by the stream), and at whatever point it fails
     struct Consumed {
         KsEngine &eng;
         std::vector<MatBuf *> bufs;
         ~Consumed() {
             for (MatBuf *b : bufs) eng.release(b);
         }
-        void push_back(MatBuf *b) { bufs.push_back(b); }
     } consumed{*this, {}};
+    const std::vector<KNode> nodes = std::exchange(nodes_, {});
+    const std::vector<KTask> carried = std::exchange(carried_, {});
+    consumed.bufs.reserve(nodes.size() + carried.size());
+    for (const KNode &nd : nodes) consumed.bufs.push_back(nd.buf);
+    for (const KTask &t : carried) consumed.bufs.push_back(t.src.buf);
 
     // leaves (n <= 128) -> exact cut, one launch per entry width
     std::vector<LeafDesc> leaves;
     std::vector<KNode> inner;
-    for (const KNode &nd : nodes_) {
+    for (const KNode &nd : nodes) {
         if (nd.N <= 128) {
             if (nd.N >= 2) {
                 leaves.push_back(LeafDesc{nd.mat, nd.cut, nd.pre, nd.N, nd.small});
             }
-            consumed.push_back(nd.buf);
             outstanding[nd.query]--;
         } else {
             inner.push_back(nd);
         }
     }
-    nodes_.clear();
     const size_t leaves32 = (size_t)(std::partition(leaves.begin(), leaves.end(), [](const LeafDesc &l) { return l.small != 0; }) -
                                      leaves.begin());
     auto launch_leaves = [&](const LeafDesc *d_leaves) -> int {  // (after the descriptor copy)
@@ -2090,22 +2126,19 @@ int KsEngine::step() {
     // sources: inner nodes (two children each) and the matrices of tasks continuing another round
     std::vector<KTask> tasks;
     std::vector<KNode> src_nodes;
-    tasks.reserve(2 * inner.size() + carried_.size());
-    src_nodes.reserve(inner.size() + carried_.size());
+    tasks.reserve(2 * inner.size() + carried.size());
+    src_nodes.reserve(inner.size() + carried.size());
     for (const KNode &nd : inner) {
         src_nodes.push_back(nd);
         const uint32_t target = (uint32_t)ks_target((int)nd.N);
         for (uint64_t c = 0; c < 2; c++) tasks.push_back(KTask{nd, 2 * nd.h + c, 0, target, (uint32_t)(src_nodes.size() - 1)});
         outstanding[nd.query]++;  // two tasks replace the node
-        consumed.push_back(nd.buf);
     }
-    for (KTask t : carried_) {
+    for (KTask t : carried) {
         src_nodes.push_back(t.src);
         t.src_index = (uint32_t)(src_nodes.size() - 1);
         tasks.push_back(t);
-        consumed.push_back(t.src.buf);
     }
-    carried_.clear();
     if (tasks.empty()) return CAC_OK;
     // sources whose row sums and block prefixes came with their matrix (warp quotient) skip the
     // row prep; the others (roots, large-N quotients) are prepped here from their own list
@@ -2257,20 +2290,10 @@ int KsEngine::step() {
     }
     // Three quotient kernels, identical outputs: triangles for small children, tiles up to kTileMaxN source
     // vertices, one row per CTA above; the caller may force tiles (where they fit) or rows.
-    MatBuf *out = nullptr;
-    struct Output {  // released again if the step ends before a child holds it
-        KsEngine &eng;
-        MatBuf *&buf;
-        ~Output() {
-            if (buf && buf->refs == 0) {
-                buf->refs = 1;
-                eng.release(buf);
-            }
-        }
-    } output{*this, out};
+    Held out(*this);
     if (out_bytes || !leaf_list[0].empty() || !leaf_list[1].empty()) {
-        if (out_bytes) CAC_TRY(alloc(out_bytes, &out));
-        unsigned char *obase = out ? static_cast<unsigned char *>(out->p) : nullptr;
+        if (out_bytes) CAC_TRY(out.alloc(out_bytes));
+        unsigned char *obase = out.at(0);
         struct TileList {
             TilePlan plan;
             std::vector<TileTask> task;
@@ -2412,10 +2435,10 @@ int KsEngine::step() {
         nd.h = t.h;
         nd.N = k;
         nd.is_root = 0;
-        nd.mat = static_cast<unsigned char *>(out->p) + out_off[i];
-        nd.pre = reinterpret_cast<uint64_t *>(static_cast<unsigned char *>(out->p) + out_off[tasks.size() + i]);
-        nd.buf = out;
-        out->refs++;
+        nd.mat = out.at(out_off[i]);
+        nd.pre = reinterpret_cast<uint64_t *>(out.at(out_off[tasks.size() + i]));
+        nd.buf = out.buf;
+        out.buf->refs++;
         outstanding[nd.query]++;
         if (k <= t.target) {
             nodes_.push_back(nd);
@@ -2510,25 +2533,23 @@ int admit(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
     }
     if (q.t >= n) {
         // no pre-contraction: every trial starts from the same dense matrix, built once
-        MatBuf *root = nullptr;
+        Held root(eng);
         const size_t bytes = (size_t)n * ld_of(n) * (small ? 4 : 8);
-        CAC_TRY(eng.alloc(bytes, &root));
-        CAC_CUDA_TRY(cudaMemsetAsync(root->p, 0, bytes, s));
+        CAC_TRY(root.alloc(bytes));
+        CAC_CUDA_TRY(cudaMemsetAsync(root.at(0), 0, bytes, s));
         if (m) {
             DevBuf &d = scratch(ctx, kSlotDd);
-            std::vector<DenseDesc> dd{DenseDesc{g->u, g->v, g->w, nullptr, root->p, m, n, small}};
+            std::vector<DenseDesc> dd{DenseDesc{g->u, g->v, g->w, nullptr, root.at(0), m, n, small}};
             CAC_TRY(upload(ctx, d, dd));
             dim3 grid((unsigned)std::max<uint64_t>(1, std::min<uint64_t>((m + 255) / 256, (uint64_t)ctx->num_sms * 8)), 1);
             dense_build_kernel<<<grid, 256, 0, s>>>(d.as<DenseDesc>());
             CAC_CUDA_TRY(cudaGetLastError());
             CAC_CUDA_TRY(cudaStreamSynchronize(s));  // the descriptor buffer goes out of scope
         }
-        root->refs++;  // held until every root node has been added
         for (uint64_t i = 0; i < q.trials; i++) {
             const uint32_t r = (uint32_t)(i / q.per_rank), idx = (uint32_t)(i % q.per_rank);
-            eng.add(KNode{q.cuts + i, q.seed + r, idx, 1, n, 1, small, q.query, root->p, root});
+            eng.add(KNode{q.cuts + i, q.seed + r, idx, 1, n, 1, small, q.query, root.at(0), root.buf});
         }
-        eng.release(root);
         return CAC_OK;
     }
     // Stage 1: the global-memory rounds of shrink_big.cu above 16384 vertices, else the
@@ -2619,13 +2640,13 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
             CAC_CUDA_TRY(cudaStreamSynchronize(s));
         }
         // trials contracted to more than the dense limit: sparse roots (sorted, merged edge lists)
-        std::vector<SparseNode> sparse;
+        SparseRoots sparse(eng);
         for (uint32_t b = 0; b < B; b++) {
             const QueryPlan &q = *items[c0 + b].q;
             if (q.t <= ctx->dense_limit) continue;
             SparseNode nd;
             CAC_TRY(sparse_root(ctx, eng, q, q.cuts + items[c0 + b].i, sd[b].k0, sd[b].idx, sd[b].lab, kdim[b], &nd));
-            sparse.push_back(nd);
+            sparse.nodes.push_back(nd);
             kdim[b] = 0;  // no dense matrix
         }
         uint64_t bytes = 0;
@@ -2633,16 +2654,16 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
             const uint64_t esize = items[c0 + b].q->g->total_weight < (1ull << 32) ? 4 : 8;
             bytes += ((uint64_t)kdim[b] * ld_of(kdim[b]) * esize + 15) / 16 * 16;
         }
-        MatBuf *roots = nullptr;
-        CAC_TRY(eng.alloc(std::max<uint64_t>(bytes, 16), &roots));
-        CAC_CUDA_TRY(cudaMemsetAsync(roots->p, 0, bytes, s));
+        Held roots(eng);
+        CAC_TRY(roots.alloc(std::max<uint64_t>(bytes, 16)));
+        CAC_CUDA_TRY(cudaMemsetAsync(roots.at(0), 0, bytes, s));
         std::vector<DenseDesc> dd(B);
         uint64_t off = 0;
         for (uint32_t b = 0; b < B; b++) {
             const cac_graph *g = items[c0 + b].q->g;
             const uint32_t small = g->total_weight < (1ull << 32) ? 1u : 0u;
             // no scatter for a trial without a matrix (its labels would index past the buffer)
-            dd[b] = DenseDesc{g->u, g->v, g->w, sd[b].lab, static_cast<unsigned char *>(roots->p) + off,
+            dd[b] = DenseDesc{g->u, g->v, g->w, sd[b].lab, roots.at(off),
                               kdim[b] >= 2 ? g->m : 0, kdim[b], small};
             if (planned) {
                 dd[b].k_act = sd[b].k_out;
@@ -2656,7 +2677,6 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
                   B);
         dense_build_kernel<<<grid, 256, 0, s>>>(d_dd.as<DenseDesc>());
         CAC_CUDA_TRY(cudaGetLastError());
-        roots->refs++;
         for (uint32_t b = 0; b < B; b++) {
             const QueryPlan &q = *items[c0 + b].q;
             const uint64_t i = items[c0 + b].i;
@@ -2666,13 +2686,12 @@ int admit_stage1(cac_ctx *ctx, KsEngine &eng, const std::vector<const QueryPlan 
                 fill_u64<<<1, 32, 0, s>>>(q.cuts + i, 1, 0);
                 continue;
             }
-            eng.add(KNode{q.cuts + i, sd[b].k0, sd[b].idx, 1, kdim[b], 1, dd[b].small, q.query, dd[b].mat, roots});
+            eng.add(KNode{q.cuts + i, sd[b].k0, sd[b].idx, 1, kdim[b], 1, dd[b].small, q.query, dd[b].mat, roots.buf});
         }
-        eng.release(roots);
         // the scratch is refilled from the host for the next chunk (later kernels on the stream
         // are ordered after these, so the last chunk needs no wait)
         if (c1 < items.size()) CAC_CUDA_TRY(cudaStreamSynchronize(s));
-        if (!sparse.empty()) CAC_TRY(sparse_phase(ctx, eng, std::move(sparse)));
+        if (!sparse.nodes.empty()) CAC_TRY(sparse_phase(ctx, eng, sparse.take()));
         c0 = c1;
     }
     return CAC_OK;
@@ -2708,13 +2727,13 @@ int admit_big(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
         // trials contracted above the dense limit become sparse roots; otherwise more than 16384
         // vertices are left only when Stage 1 stopped with no edge between them (a disconnected
         // graph): every vertex is isolated and the trial's cut is exactly 0
-        std::vector<SparseNode> sparse;
+        SparseRoots sparse(eng);
         for (uint32_t b = 0; b < B; b++) {
             if (q.t > ctx->dense_limit) {
                 SparseNode nd;
                 CAC_TRY(sparse_root(ctx, eng, q, q.cuts + c0 + b, k0[b], idx[b], d_lab.as<uint32_t>() + (size_t)b * n,
                                     kdim[b], &nd));
-                sparse.push_back(nd);
+                sparse.nodes.push_back(nd);
                 kdim[b] = 0;
             } else if (kdim[b] > kMaxSmemVertices) {
                 kdim[b] = 0;
@@ -2723,15 +2742,15 @@ int admit_big(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
         const uint64_t esize = small ? 4 : 8;
         uint64_t bytes = 0;
         for (uint32_t b = 0; b < B; b++) bytes += ((uint64_t)kdim[b] * ld_of(kdim[b]) * esize + 15) / 16 * 16;
-        MatBuf *roots = nullptr;
-        CAC_TRY(eng.alloc(std::max<uint64_t>(bytes, 16), &roots));
-        CAC_CUDA_TRY(cudaMemsetAsync(roots->p, 0, bytes, s));
+        Held roots(eng);
+        CAC_TRY(roots.alloc(std::max<uint64_t>(bytes, 16)));
+        CAC_CUDA_TRY(cudaMemsetAsync(roots.at(0), 0, bytes, s));
         std::vector<DenseDesc> dd(B);
         uint64_t off = 0;
         for (uint32_t b = 0; b < B; b++) {
             // no scatter for a trial without a matrix (its labels would index past the buffer)
             dd[b] = DenseDesc{g->u, g->v, g->w, d_lab.as<uint32_t>() + (size_t)b * n,
-                              static_cast<unsigned char *>(roots->p) + off, kdim[b] >= 2 ? m : 0, kdim[b], small};
+                              roots.at(off), kdim[b] >= 2 ? m : 0, kdim[b], small};
             off += ((uint64_t)kdim[b] * ld_of(kdim[b]) * esize + 15) / 16 * 16;
         }
         CAC_TRY(upload(ctx, d_dd, dd));
@@ -2740,7 +2759,6 @@ int admit_big(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
             dense_build_kernel<<<grid, 256, 0, s>>>(d_dd.as<DenseDesc>());
             CAC_CUDA_TRY(cudaGetLastError());
         }
-        roots->refs++;
         for (uint32_t b = 0; b < B; b++) {
             const uint64_t i = c0 + b;
             if (q.t > ctx->dense_limit) continue;  // a sparse root
@@ -2748,11 +2766,10 @@ int admit_big(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
                 fill_u64<<<1, 32, 0, s>>>(q.cuts + i, 1, 0);
                 continue;
             }
-            eng.add(KNode{q.cuts + i, k0[b], idx[b], 1, kdim[b], 1, small, q.query, dd[b].mat, roots});
+            eng.add(KNode{q.cuts + i, k0[b], idx[b], 1, kdim[b], 1, small, q.query, dd[b].mat, roots.buf});
         }
-        eng.release(roots);
         if (c0 + chunk < q.trials) CAC_CUDA_TRY(cudaStreamSynchronize(s));  // the scratch is reused by the next chunk
-        if (!sparse.empty()) CAC_TRY(sparse_phase(ctx, eng, std::move(sparse)));
+        if (!sparse.nodes.empty()) CAC_TRY(sparse_phase(ctx, eng, sparse.take()));
     }
     return CAC_OK;
 }
@@ -2799,17 +2816,17 @@ int admit_groups(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
         };
         if (q.t > ctx->dense_limit) {
             // sparse roots: the merged contracted graph, shared by the group's two recursions
-            std::vector<SparseNode> sparse;
+            SparseRoots sparse(eng);
             for (uint32_t b = 0; b < B; b++) {
                 SparseNode nd;
                 CAC_TRY(sparse_root(ctx, eng, q, q.cuts + c0 + b, q.seed + (uint32_t)(c0 + b), 0, lab_of(b), kdim[b],
                                     &nd));
-                sparse.push_back(nd);
+                sparse.nodes.push_back(nd);
                 nd.idx = 1;
                 if (nd.buf) nd.buf->refs++;
-                sparse.push_back(nd);
+                sparse.nodes.push_back(nd);
             }
-            CAC_TRY(sparse_phase(ctx, eng, std::move(sparse)));
+            CAC_TRY(sparse_phase(ctx, eng, sparse.take()));
             continue;
         }
         // dense roots (more than 16384 vertices left only when Stage 1 found no edge between
@@ -2819,13 +2836,13 @@ int admit_groups(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
         const uint64_t esize = small ? 4 : 8;
         uint64_t bytes = 0;
         for (uint32_t b = 0; b < B; b++) bytes += ((uint64_t)kdim[b] * ld_of(kdim[b]) * esize + 15) / 16 * 16;
-        MatBuf *roots = nullptr;
-        CAC_TRY(eng.alloc(std::max<uint64_t>(bytes, 16), &roots));
-        CAC_CUDA_TRY(cudaMemsetAsync(roots->p, 0, bytes, s));
+        Held roots(eng);
+        CAC_TRY(roots.alloc(std::max<uint64_t>(bytes, 16)));
+        CAC_CUDA_TRY(cudaMemsetAsync(roots.at(0), 0, bytes, s));
         std::vector<DenseDesc> dd(B);
         uint64_t off = 0;
         for (uint32_t b = 0; b < B; b++) {
-            dd[b] = DenseDesc{g->u, g->v, g->w, lab_of(b), static_cast<unsigned char *>(roots->p) + off,
+            dd[b] = DenseDesc{g->u, g->v, g->w, lab_of(b), roots.at(off),
                               kdim[b] >= 2 ? m : 0, kdim[b], small};
             off += ((uint64_t)kdim[b] * ld_of(kdim[b]) * esize + 15) / 16 * 16;
         }
@@ -2837,7 +2854,6 @@ int admit_groups(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
             dense_build_kernel<<<grid, 256, 0, s>>>(d_dd.as<DenseDesc>());
             CAC_CUDA_TRY(cudaGetLastError());
         }
-        roots->refs++;
         for (uint32_t b = 0; b < B; b++) {
             const uint64_t i = c0 + b;
             if (kdim[b] < 2) {
@@ -2845,9 +2861,8 @@ int admit_groups(cac_ctx *ctx, KsEngine &eng, const QueryPlan &q) {
                 continue;
             }
             for (uint32_t j = 0; j < 2; j++)
-                eng.add(KNode{q.cuts + i, q.seed + (uint32_t)i, j, 1, kdim[b], 1, small, q.query, dd[b].mat, roots});
+                eng.add(KNode{q.cuts + i, q.seed + (uint32_t)i, j, 1, kdim[b], 1, small, q.query, dd[b].mat, roots.buf});
         }
-        eng.release(roots);
         if (c0 + chunk < q.trials) CAC_CUDA_TRY(cudaStreamSynchronize(s));  // the scratch is reused
     }
     return CAC_OK;
