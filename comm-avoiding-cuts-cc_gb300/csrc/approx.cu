@@ -111,15 +111,14 @@ __device__ __forceinline__ uint32_t root_of(const Forest &F, uint32_t j, uint32_
     return cur;
 }
 
-// Singletons, one thread per vertex, and the root count at 0.
+// Singletons, one thread per vertex of 4 copies, else per vertex and copy, and the root count at 0.
 __global__ void approx_init(const Forest F, uint32_t n, unsigned int *count) {
     pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
-    grid_stride(n, [&](uint32_t x) {
-        if (F.copies == 4) reinterpret_cast<uint4 *>(F.par)[x] = make_uint4(x, x, x, x);
-        else
-            for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = x;
-    });
+    if (F.copies == 4)
+        grid_stride(n, [&](uint32_t x) { reinterpret_cast<uint4 *>(F.par)[x] = make_uint4(x, x, x, x); });
+    else
+        grid_stride(n * F.copies, [&](uint32_t i) { F.par[i] = i / F.copies; });
 }
 
 // The draws are taken by quads: a quad is 4 consecutive edges of one rank's slice, local
@@ -434,7 +433,9 @@ __device__ __forceinline__ uint32_t near_of(const Forest &F, uint32_t j, uint32_
 }
 
 // Compression between the rounds, a thread per vertex and 4 copies: their parents in one load, the 4
-// grandparents requested together, then the longer chains. Walks end after kHops parents: heavy paths
+// grandparents requested together, then the longer chains. With other numbers of copies a thread per vertex
+// and copy, neighbouring lanes on neighbouring words (37 copies of 300,000 vertices: 38 us; 184 us by
+// vertices). Walks end after kHops parents: heavy paths
 // numbered along their length make chains of that length, and the rounds do not need a flat forest (what
 // a link at a vertex that is no root any more separates is joined again by the pass over all edges).
 __global__ void approx_compress(const Forest F, uint32_t n) {
@@ -449,8 +450,9 @@ __global__ void approx_compress(const Forest F, uint32_t n) {
             if (r0 != p.x || r1 != p.y || r2 != p.z || r3 != p.w) p4[x] = make_uint4(r0, r1, r2, r3);
         });
     } else {
-        grid_stride(n, [&](uint32_t x) {
-            for (uint32_t j = 0; j < F.copies; j++) F.at(x, j) = near_of(F, j, x);
+        grid_stride(n * F.copies, [&](uint32_t i) {
+            const uint32_t x = i / F.copies, r = near_of(F, i - x * F.copies, x);
+            if (r != x) F.par[i] = r;
         });
     }
 }
@@ -621,16 +623,19 @@ bool approx_is_small(uint32_t n, uint64_t m) { return n <= kSmallN && m <= kSmal
 // edges, kernel boundaries at 10^6. Measured per query against eight slices of union walks: G(10^6,
 // 15.2 M edges), unit weights, 4 copies, 1.97 -> 0.75 ms; G(10^5, 1.4 M edges), weights to 42, six
 // levels, 1.79 -> 0.61 ms.
+// The rounds need the forest alone, so they come first also where there is no survivor list and every quad
+// is tested after them: G(10^6, 15.2 M edges) in a budget without room for it 1.28 ms by slices, 1.74 by one pass from
+// singletons, 0.65 so; 37 copies of G(300,000, 3.9 M edges), two levels, 5.6, 15.4 and 4.8 ms.
 template <bool kRef>
-int run_level(cac_ctx *ctx, Level L, double kept_degree) {
+int run_level(cac_ctx *ctx, Level L, double kept_degree, bool rounds) {
     cudaStream_t s = ctx->stream;
     auto grid = [&](uint64_t work, int per_sm) {
         return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((work + kThreads - 1) / kThreads, (uint64_t)ctx->num_sms * per_sm));
     };
-    const unsigned gc = grid(L.n, 8), gq = grid((uint64_t)L.Q * L.F.copies, 8);
+    const unsigned gc = grid(L.F.copies == 4 ? L.n : (uint64_t)L.n * L.F.copies, 8), gq = grid((uint64_t)L.Q * L.F.copies, 8);
     double sum = 0;
     for (double d : kRoundDegree) sum += d;
-    if (L.list) {
+    if (rounds) {
         double upto = 0;
         L.to = 0;
         for (double d : kRoundDegree) {
@@ -695,7 +700,7 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
     const size_t more = align_up((uint64_t)g->n * 4) + align_up(((uint64_t)g->n + 31) / 32 * 4) +
                         align_up(cap * 8) + 256;
     // the survivor list needs a byte an edge more than the forest: without it (it does not fit the
-    // budget, or there are more copies than a mask has bits) every edge is tested and hooked at once
+    // budget, or there are more copies than a mask has bits) every edge is tested after the rounds
     const bool sampled = large && copies <= 32 &&
                          (base_bytes + more <= ctx->arena.cap || !ctx->budget ||
                           ctx->held - ctx->arena.cap + align_up(base_bytes + more, 1 << 20) <= ctx->budget);
@@ -725,7 +730,7 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
         iterations = UINT32_MAX;
         for (uint32_t r = 0; r < ranks; r++) iterations = std::min(iterations, level_count(h[r]));
     }
-    const int gi = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)g->n + kThreads - 1) / kThreads, ctx->num_sms * 8));
+    const int gi = (int)std::max<uint64_t>(1, std::min<uint64_t>(((copies == 4 ? g->n : nv) + kThreads - 1) / kThreads, ctx->num_sms * 8));
     uint32_t first = 0;
     if (ref_stream) iterations = std::min<uint32_t>(iterations, 52);  // ceil(ln W) <= 45 for W < 2^64
     Level L{};
@@ -776,7 +781,7 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
         if (g->m) {
             const double kept = 1 - std::pow(1 - std::ldexp(1.0, -(int)level), mean_weight);  // share of the edges
             const double degree = 2.0 * g->m * kept / std::max<uint32_t>(1, g->n);
-            CAC_TRY(ref_stream ? run_level<true>(ctx, L, degree) : run_level<false>(ctx, L, degree));
+            CAC_TRY(ref_stream ? run_level<true>(ctx, L, degree, large) : run_level<false>(ctx, L, degree, large));
         }
         CAC_CUDA_TRY(launch_pdl(approx_count_roots, (unsigned)gi, kThreads, 0, s, L.F, g->n, d_count));
         CAC_CUDA_TRY(cudaGetLastError());
