@@ -609,6 +609,21 @@ __global__ void __launch_bounds__(kSmallThreads) approx_small(const Level base, 
     if (threadIdx.x == 0) roots[blockIdx.y * gridDim.x + j] = L.n - s_links;
 }
 
+// Device memory of one call, given back (in the stream's order) when the call ends.
+struct Temporary {
+    cac_ctx *ctx;
+    void *p = nullptr;
+    size_t bytes = 0;
+    explicit Temporary(cac_ctx *c) : ctx(c) {}
+    Temporary(const Temporary &) = delete;
+    Temporary &operator=(const Temporary &) = delete;
+    ~Temporary() { stream_free(ctx, p, bytes); }
+    int get(size_t n) {
+        bytes = n;
+        return stream_alloc(ctx, &p, n);
+    }
+};
+
 bool approx_is_small(uint32_t n, uint64_t m) { return n <= kSmallN && m <= kSmallM; }
 
 // The hooks of one level (the forest already holds singletons).
@@ -700,12 +715,13 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
     const size_t more = align_up((uint64_t)g->n * 4) + align_up(((uint64_t)g->n + 31) / 32 * 4) +
                         align_up(cap * 8) + 256;
     // the survivor list needs a byte an edge more than the forest: without it (it does not fit the
-    // budget, or there are more copies than a mask has bits) every edge is tested after the rounds
-    const bool sampled = large && copies <= 32 &&
-                         (base_bytes + more <= ctx->arena.cap || !ctx->budget ||
-                          ctx->held - ctx->arena.cap + align_up(base_bytes + more, 1 << 20) <= ctx->budget);
-    CAC_TRY(arena_reserve(ctx, base_bytes + (sampled ? more : 0)));
+    // budget, or there are more copies than a mask has bits) every edge is tested after the rounds. Under a budget it is
+    // the query's own (5 us a call) and not the arena's, which keeps what it has: room that other calls need
+    bool sampled = large && copies <= 32;
+    Temporary extra(ctx);
+    CAC_TRY(arena_reserve(ctx, base_bytes + (sampled && !ctx->budget ? more : 0)));
     arena_reset(ctx);
+    if (sampled && ctx->budget) sampled = ctx->held + more <= ctx->budget && extra.get(more) == CAC_OK;
     uint32_t *par = (uint32_t *)arena_take(ctx, nv * 4 + 4);
     unsigned int *d_count = (unsigned int *)arena_take(ctx, 16);
     CAC_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
@@ -746,11 +762,17 @@ int approx_run(cac_ctx *ctx, const cac_graph *g, double p, uint32_t seed, uint32
     L.Qf = (uint32_t)Qf;
     L.Q = (uint32_t)Q;
     if (sampled) {
-        L.member = (uint32_t *)arena_take(ctx, (uint64_t)g->n * 4);
-        L.bits = (uint32_t *)arena_take(ctx, ((uint64_t)g->n + 31) / 32 * 4);
-        L.list = (uint2 *)arena_take(ctx, cap * 8);
+        char *at = static_cast<char *>(extra.p ? extra.p : arena_take(ctx, more));
+        auto take = [&](size_t bytes) {
+            char *p = at;
+            at += align_up(bytes);
+            return p;
+        };
+        L.member = (uint32_t *)take((uint64_t)g->n * 4);
+        L.bits = (uint32_t *)take(((uint64_t)g->n + 31) / 32 * 4);
+        L.list = (uint2 *)take(cap * 8);
         L.cap = (uint32_t)cap;
-        L.giants = (uint32_t *)arena_take(ctx, 256);
+        L.giants = (uint32_t *)take(256);
         L.count = L.giants + 32;
     }
     iterations = std::min<uint32_t>(iterations, 63);
