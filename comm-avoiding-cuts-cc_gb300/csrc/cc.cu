@@ -347,12 +347,12 @@ __global__ void cc_compress4(uint32_t *par, uint32_t n) {
 void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s);
 
 // A byte per 32 vertices, a bit per four of them (read as words): for graphs whose bitmap does not fit in
-// shared memory, where the budget has room for it.
+// shared memory. They take no scratch of their own (the arena keeps what it once had, and under a budget other
+// calls need the room), but lie in memory that is idle between the sample and the labels: `spare`, of `bytes`.
 size_t quad_bytes(uint32_t nwords) { return nwords > kSmemBitmapWords ? (size_t)(nwords + 3) / 4 * 4 : 0; }
-bool quads_fit(const cac_ctx *ctx, size_t base, uint32_t nwords) {
-    const size_t more = align_up(quad_bytes(nwords));
-    return more && (base + more <= ctx->arena.cap || !ctx->budget ||
-                    ctx->held - ctx->arena.cap + align_up(base + more, 1 << 20) <= ctx->budget);
+uint8_t *quads_in(void *spare, size_t bytes, uint32_t nwords) {
+    const size_t need = quad_bytes(nwords);
+    return need && need <= bytes ? static_cast<uint8_t *>(spare) : nullptr;
 }
 
 // The end of the sampling round in one launch: full compression, the giant component and its
@@ -1173,9 +1173,7 @@ int cc_run(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint
     L.vec = ((reinterpret_cast<uintptr_t>(d_u) | reinterpret_cast<uintptr_t>(d_v)) & 15) == 0;
     L.check = check_ids;
 
-    const size_t base = cc_scratch_bytes(n, ranks, m) + align_up(chunk_slots * 8);
-    const bool quads = quads_fit(ctx, base, L.nwords);
-    CAC_TRY(arena_reserve(ctx, base + (quads ? align_up(quad_bytes(L.nwords)) : 0)));
+    CAC_TRY(arena_reserve(ctx, cc_scratch_bytes(n, ranks, m) + align_up(chunk_slots * 8)));
     arena_reset(ctx);
     L.par = (uint32_t *)arena_take(ctx, (size_t)n * 4);
     L.counts = (uint32_t *)arena_take(ctx, (size_t)L.ntiles * 4 + 4);
@@ -1188,7 +1186,7 @@ int cc_run(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *d_u, const uint
     L.region_counts = (uint32_t *)arena_take(ctx, kMaxRegions * 4);
     L.surv = (uint2 *)arena_take(ctx, (m + 4 * (uint64_t)kMaxRegions) * 8);
     L.chunks = (uint64_t *)arena_take(ctx, chunk_slots * 8);
-    if (quads) L.quads = (uint8_t *)arena_take(ctx, quad_bytes(L.nwords));
+    L.quads = quads_in(L.chunks, chunk_slots * 8, L.nwords);  // (the last round has read the draws by then)
 
     // rank descriptors go through the ctx's pinned staging page when they fit (async copy)
     std::vector<RankDesc> hv;
@@ -1447,12 +1445,10 @@ int cc_run_streamed(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *h_u, c
                                : 0;
     L.filtered = L.vec && seg > 0;
     const uint64_t max_gap = L.filtered ? m - (kStreamPieces - 1) * seg - piece : 0;
-    const size_t base = align_up((size_t)n * 4) + 2 * align_up((size_t)L.ntiles * 4 + 4) + align_up(256) +
-                        (L.filtered ? align_up((size_t)L.nwords * 4 + 4) + align_up(kMaxRegions * 4) +
-                                          align_up((max_gap + 4 * (uint64_t)kMaxRegions) * 8)
-                                    : 0);
-    const bool quads = L.filtered && quads_fit(ctx, base, L.nwords);
-    CAC_TRY(arena_reserve(ctx, base + (quads ? align_up(quad_bytes(L.nwords)) : 0)));
+    CAC_TRY(arena_reserve(ctx, align_up((size_t)n * 4) + 2 * align_up((size_t)L.ntiles * 4 + 4) + align_up(256) +
+                                   (L.filtered ? align_up((size_t)L.nwords * 4 + 4) + align_up(kMaxRegions * 4) +
+                                                     align_up((max_gap + 4 * (uint64_t)kMaxRegions) * 8)
+                                               : 0)));
     arena_reset(ctx);
     L.par = (uint32_t *)arena_take(ctx, (size_t)n * 4);
     L.counts = (uint32_t *)arena_take(ctx, (size_t)L.ntiles * 4 + 4);
@@ -1463,7 +1459,7 @@ int cc_run_streamed(cac_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *h_u, c
         L.bits = (uint32_t *)arena_take(ctx, (size_t)L.nwords * 4 + 4);
         L.region_counts = (uint32_t *)arena_take(ctx, kMaxRegions * 4);
         L.surv = (uint2 *)arena_take(ctx, (max_gap + 4 * (uint64_t)kMaxRegions) * 8);
-        if (quads) L.quads = (uint8_t *)arena_take(ctx, quad_bytes(L.nwords));
+        if (d_labels) L.quads = quads_in(d_labels, (size_t)n * 4, L.nwords);  // (labels are written last)
         CAC_TRY(smem_optin(ctx, cc_filter<true, true>));
         CAC_TRY(smem_optin(ctx, cc_filter<false, true>));
         CAC_TRY(smem_optin(ctx, cc_filter<true, false>));
