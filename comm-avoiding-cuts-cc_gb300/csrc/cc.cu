@@ -791,12 +791,14 @@ int label_components(int sms, uint32_t *par, uint32_t n, uint32_t ntiles, uint32
 
 // A whole query in one CTA, the forest in shared memory (small graphs: the launches of the form above
 // cost more than their work). Three passes over the edges -- the smallest neighbour as parent, the same
-// between roots, union walks for what is left -- with a full compression after each, then every thread
+// between roots, union walks for what is left -- with a compression after each, which walks to the root after the
+// last only (see cc_compress4; the last pass joins all edges whatever the first two left), then every thread
 // ranks the roots of its own run of vertices. The count, the error word and, for host labels, the labels
 // go straight into pinned host memory, so that the one wait after the launch is the whole read-back.
 // Bound by the latency of its passes (shared-memory unions, edges from L2). Measured per query, labels
 // into a host array, against the 16 launches: R-MAT scale 10 with 8192 edges 94 -> 26 us, G(16000, M) with
-// 64,000 edges 133 -> 78.
+// 64,000 edges 133 -> 78. Device time at 16,320 vertices: a path numbered along its length 171 -> 55 (61 with walks to the
+// root after every pass), relabelled 106 -> 39, a ring lattice of degree 8 224 -> 62, a star 33 -> 28.
 constexpr int kSmallThreads = 1024;
 template <bool kCheck>
 __global__ void __launch_bounds__(kSmallThreads) cc_small(const uint32_t *__restrict__ u, const uint32_t *__restrict__ v,
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(kSmallThreads) cc_small(const uint32_t *__rest
             }
         }
         __syncthreads();
-        for (uint32_t i = t; i < n; i += kSmallThreads) par[i] = find_root_ro(par, i);
+        for (uint32_t i = t; i < n; i += kSmallThreads) par[i] = pass < 2 ? find_near(par, i) : find_root_ro(par, i);
         __syncthreads();
     }
     // ranks: thread t owns the vertices [t per, (t + 1) per)
