@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(NT) iss_shrink_kernel(const ShrinkDesc *__rest
                 const uint32_t groups = (uint32_t)(e / 32) + 1;
                 if (groups % csg == 0) coarse[groups / csg - 1] = end;
             }
-            if (e < m && e + 4 >= m) coarse[ncs - 1] = end;
+            if (e < whi && e + 4 >= m) coarse[ncs - 1] = end;  // (by the warp that owns the last edge)
         }
         if (lane == 0) s_w[warp] = carry;
         __syncthreads();
