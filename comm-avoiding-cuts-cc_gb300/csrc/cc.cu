@@ -56,6 +56,11 @@ constexpr uint32_t kRoundParts = 128;                // without draws: rounds ar
 // end a random graph has small trees only): G(10^6, M) with average degree 0.1 takes 41 us in one pass
 // and 48 in rounds, with 3 863 and 127, G(17000, M) with degree 2 87 and 66.
 constexpr uint64_t kRoundEdges = 1u << 13;
+// Up to this average degree the rounds are those of sparse_rounds, of kFullRounds - 1 below kFewRoundEdges edges.
+// Device us by them and by edge_rounds: G(10^6, M) of degree 2.25 145 and 626, 2.5 147 and 118, 3 167 and 121;
+// a 1000 x 1000 grid (4) 132 and 110.
+constexpr double kSparseDegree = 2.4;
+constexpr uint64_t kFewRoundEdges = 1u << 18;
 constexpr uint32_t kProbes = 128;
 constexpr int kHops = 32;                            // longest walk of a compression between rounds
 constexpr int kRoundThreads = 1024;                  // CTA of a round: the more threads, the more links the table sees
@@ -66,6 +71,9 @@ constexpr unsigned kSurvivorBlocksPerSm = 8;
 constexpr uint32_t kStreamPieces = 8;                // sample pieces (and gaps) of a host edge list
 constexpr uint32_t kErrWord = 9;                     // a query's error word (after its count and giant root)
 constexpr uint32_t kErrBadId = 1;                    // an edge endpoint was >= n (the edge was skipped)
+constexpr uint32_t kFullRounds = 4;                  // most rounds of sparse_rounds after its first
+constexpr uint32_t kOpenWord = 10;                   // the open edges that each of them found
+constexpr uint32_t kQueryWords = kOpenWord + kFullRounds;  // words in use of the total's 64
 
 struct RankDesc {
     uint64_t slice_off;
@@ -261,6 +269,14 @@ __global__ void __launch_bounds__(kRoundThreads, 2) cc_sample_round(uint32_t *pa
     if constexpr (!kFirst) links.flush(par);
 }
 
+// Rounds on the edges that an earlier round left open (their ends under different parents): what comes after one
+// that found few of them is left out.
+struct OpenCount {
+    const uint32_t *before = nullptr;  // the open edges that the round before found, or null: not to be left out
+    uint32_t few = 0;
+    __device__ __forceinline__ bool skip() const { return before && *before <= few; }
+};
+
 // One round on the 256-edge tiles t with from <= t % kRoundParts < to, a warp per tile, its lane l on
 // edges l, 32 + l, ... (all loads of the eight in flight together).
 template <bool kFirst, bool kCheck, int kNT>
@@ -306,6 +322,70 @@ __global__ void __launch_bounds__(kNT, 2048 / kNT) cc_edge_round(uint32_t *par, 
     if constexpr (!kFirst) links.flush(par);
 }
 
+// One round on all edges, a CTA per contiguous range of tiles, which writes the open ones (as the pairs of
+// their ends' parents) to its region of `list`, as cc_filter does with its survivors.
+template <bool kCheck, int kNT>
+__global__ void __launch_bounds__(kNT, 2048 / kNT) cc_open_edges(uint32_t *par, const uint32_t *__restrict__ u,
+                                                          const uint32_t *__restrict__ v, uint64_t m, uint32_t n,
+                                                          uint2 *__restrict__ list, uint32_t *__restrict__ counts,
+                                                          uint32_t *open, uint32_t *err) {
+    __shared__ Links<4 * kNT> links;
+    __shared__ uint32_t s_n;
+    links.clear();
+    if (threadIdx.x == 0) s_n = 0;
+    pdl_wait();
+    if (kNT == kRoundThreads) links.claim_large(par, n);
+    else __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t tiles = (m + 255) / 256, per = (tiles + gridDim.x - 1) / gridDim.x;
+    const uint64_t t0 = min(tiles, (uint64_t)blockIdx.x * per), t1 = min(tiles, t0 + per);
+    uint2 *out = list + t0 * 256;
+    for (uint64_t t = t0 + (threadIdx.x >> 5); t < t1; t += kNT / 32) {
+        uint32_t a[8], b[8], mine = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint64_t e = t * 256 + 32 * k + lane;
+            a[k] = b[k] = 0;
+            if (e < m) {
+                a[k] = __ldg(u + e);
+                b[k] = __ldg(v + e);
+            }
+            if (kCheck && (a[k] >= n || b[k] >= n)) {
+                atomicOr(err, kErrBadId);
+                a[k] = b[k] = 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            a[k] = par[a[k]];
+            b[k] = par[b[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            mine += a[k] != b[k];
+            links.add(par, a[k], b[k]);
+        }
+        if (!__any_sync(0xffffffffu, mine)) continue;
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        uint32_t at = 0;
+        if (lane == 31) at = atomicAdd(&s_n, incl);
+        at = __shfl_sync(0xffffffffu, at, 31) + incl - mine;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (a[k] != b[k]) out[at++] = make_uint2(a[k], b[k]);
+    }
+    links.flush(par);
+    if (threadIdx.x == 0) {
+        counts[blockIdx.x] = s_n;
+        if (s_n) atomicAdd(open, s_n);
+    }
+}
+
 // An ancestor of v, the root unless it is more than kHops away.
 __device__ __forceinline__ uint32_t find_near(const uint32_t *par, uint32_t v) {
     uint32_t cur = v, next;
@@ -321,8 +401,9 @@ __device__ __forceinline__ uint32_t find_near(const uint32_t *par, uint32_t v) {
 // do not need a flat forest: a link made at a vertex that is no root any more replaces that vertex's
 // parent by another vertex of its component, and what that separates is joined again by the passes over
 // all edges.
-__global__ void cc_compress4(uint32_t *par, uint32_t n) {
+__global__ void cc_compress4(uint32_t *par, uint32_t n, const OpenCount left) {
     pdl_wait();
+    if (left.skip()) return;
     uint4 *p4 = reinterpret_cast<uint4 *>(par);
     const uint32_t n4 = n / 4;
     if (blockIdx.x == 0 && threadIdx.x < (n & 3u)) {
@@ -344,7 +425,7 @@ __global__ void cc_compress4(uint32_t *par, uint32_t n) {
 }
 
 // Compression of [0, n) (the parent array is 256-byte aligned).
-void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s);
+void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s, OpenCount left = {});
 
 // A byte per 32 vertices, a bit per four of them (read as words): for graphs whose bitmap does not fit in
 // shared memory. They take no scratch of their own (the arena keeps what it once had, and under a budget other
@@ -573,16 +654,10 @@ __global__ void __launch_bounds__(kEdgeThreads) cc_filter(const uint32_t *__rest
     if (threadIdx.x == 0) counts[blockIdx.x] = s_n;
 }
 
-// Union of the surviving edges (the reference's next round on the remaining slice). Regions of
-// the filter CTAs are addressed through the prefix of their counts.
-__global__ void __launch_bounds__(kThreads) cc_hook_survivors(uint32_t *par, const uint2 *__restrict__ surv,
-                                                              const uint32_t *__restrict__ counts, uint32_t nregions,
-                                                              uint64_t region_stride) {
-    pdl_wait();
-    __shared__ uint32_t pre[kMaxRegions + 1];
+// Exclusive prefix of the region counts: four per thread, then a block scan of the sums.
+__device__ __forceinline__ void region_prefix(const uint32_t *__restrict__ counts, uint32_t nregions, uint32_t *pre) {
     __shared__ uint32_t wsum[kThreads / 32];
     static_assert(kMaxRegions == 4 * kThreads, "four region counts per thread");
-    // exclusive prefix of the region counts: four per thread, then a block scan of the sums
     uint32_t c[4], local = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -610,14 +685,52 @@ __global__ void __launch_bounds__(kThreads) cc_hook_survivors(uint32_t *par, con
     }
     if (threadIdx.x == kThreads - 1 && nregions == kMaxRegions) pre[kMaxRegions] = acc;
     __syncthreads();
-    const uint32_t total = pre[nregions];
-    grid_stride(total, [&](uint32_t i) {
-        uint32_t lo = 0, hi = nregions - 1;  // last region whose first survivor <= i
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (pre[mid] <= i) lo = mid; else hi = mid - 1;
-        }
-        const uint2 e = surv[(uint64_t)lo * region_stride + (i - pre[lo])];
+}
+
+__device__ __forceinline__ uint2 region_edge(const uint2 *__restrict__ list, const uint32_t *pre, uint32_t nregions,
+                                             uint64_t region_stride, uint32_t i) {
+    uint32_t lo = 0, hi = nregions - 1;  // last region whose first edge <= i
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (pre[mid] <= i) lo = mid; else hi = mid - 1;
+    }
+    return list[(uint64_t)lo * region_stride + (i - pre[lo])];
+}
+
+// One more round on the edges that cc_open_edges left.
+__global__ void __launch_bounds__(kThreads, 8) cc_list_round(uint32_t *par, const uint2 *__restrict__ list,
+                                                          const uint32_t *__restrict__ counts, uint32_t nregions,
+                                                          uint64_t region_stride, const OpenCount left, uint32_t *open) {
+    __shared__ Links<4 * kThreads> links;
+    __shared__ uint32_t pre[kMaxRegions + 1];
+    __shared__ uint32_t s_open;
+    links.clear();
+    if (threadIdx.x == 0) s_open = 0;
+    pdl_wait();
+    if (left.skip()) return;
+    region_prefix(counts, nregions, pre);
+    uint32_t mine = 0;
+    grid_stride(pre[nregions], [&](uint32_t i) {
+        const uint2 e = region_edge(list, pre, nregions, region_stride, i);
+        const uint32_t a = par[e.x], b = par[e.y];
+        mine += a != b;
+        links.add(par, a, b);
+    });
+    if (mine) atomicAdd(&s_open, mine);
+    links.flush(par);
+    if (threadIdx.x == 0 && s_open) atomicAdd(open, s_open);
+}
+
+// Union of the surviving edges (the reference's next round on the remaining slice). Regions of
+// the filter CTAs are addressed through the prefix of their counts.
+__global__ void __launch_bounds__(kThreads) cc_hook_survivors(uint32_t *par, const uint2 *__restrict__ surv,
+                                                              const uint32_t *__restrict__ counts, uint32_t nregions,
+                                                              uint64_t region_stride) {
+    pdl_wait();
+    __shared__ uint32_t pre[kMaxRegions + 1];
+    region_prefix(counts, nregions, pre);
+    grid_stride(pre[nregions], [&](uint32_t i) {
+        const uint2 e = region_edge(surv, pre, nregions, region_stride, i);
         edge_hook(par, e.x, e.y);
     });
 }
@@ -881,8 +994,8 @@ int grid_for(cac_ctx *ctx, uint64_t work, int per_sm) {
     return (int)std::max<uint64_t>(1, std::min(need, cap));
 }
 
-void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s) {
-    launch_pdl(cc_compress4, grid_for(ctx, n / 4, 8), kThreads, 0, s, par, n);
+void compress_all(cac_ctx *ctx, uint32_t *par, uint32_t n, cudaStream_t s, OpenCount left) {
+    launch_pdl(cc_compress4, grid_for(ctx, n / 4, 8), kThreads, 0, s, par, n, left);
 }
 
 }  // namespace
@@ -984,16 +1097,52 @@ unsigned round_grid(cac_ctx *ctx, uint64_t warps, int threads = kRoundThreads) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((warps + per - 1) / per, (uint64_t)ctx->num_sms * 2048 / threads));
 }
 
-// Forest building without draws (every rank returns its whole slice): the rounds of kRoundDegree on
+// Forest building without draws (every rank returns its whole slice) on few edges per vertex: a round on all
+// edges, another that lists those still open, and some more on the list, each left out when the one before found
+// few open. What is left after the partial rounds below near the threshold of a giant component are open edges
+// between few large trees, and union walks of these are slow: each reads and swaps the same roots, and a line of the L2
+// serves about one access per ns (500,000 open edges of G(3 10^6, degree 2): 790 us). In a round they cost a CTA's
+// table entry each. Few: as many as are walked in the time of a round.
+//   Bound by the kernel boundaries (a round and its compression take 6 us) and, from 10^6 edges on, by the gathers of
+// parents from the L2 (3 M edges 50 us; on the list 10 to 20). Device us by one pass of union walks / by the partial rounds / so:
+// G(300,000, M) of degree 1.5 192 / 110 / 81, 1.75 116 / 218 / 81, 2 242 / 216 / 83; G(10^6, M) of degree 1.25 135 / 118 / 106,
+// 2 441 / 352 / 132; G(3 10^6, M) of degree 1.5 376 / 442 / 205, 2 400 / 808 / 267; paths of 10^6 numbered along
+// them 232 / 181 / 155, relabelled 168 / 144 / 136; random trees 118 / 123 / 122. What a pass joins at once pays for the
+// launches: stars and matchings of 300,000 vertices 34 / 46 / 48.
+int sparse_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
+    const uint64_t tiles = (L.m + 255) / 256;
+    const bool wide = tiles >= (uint64_t)ctx->num_sms * (kRoundThreads / 32);
+    const int threads = wide ? kRoundThreads : kThreads;
+    const uint32_t regions = std::min<uint32_t>(round_grid(ctx, tiles, threads), kMaxRegions);
+    const uint64_t region = (tiles + regions - 1) / regions * 256;
+    CAC_CUDA_TRY(launch_pdl(pick_edge_round(true, L.check, wide), round_grid(ctx, tiles, threads), threads, 0, s, L.par, L.u,
+                            L.v, L.m, 0u, kRoundParts, L.n, L.err));
+    compress_all(ctx, L.par, L.n, s);
+    uint32_t *open = L.total + kOpenWord;
+    auto kern = wide ? (L.check ? cc_open_edges<true, kRoundThreads> : cc_open_edges<false, kRoundThreads>)
+                     : (L.check ? cc_open_edges<true, kThreads> : cc_open_edges<false, kThreads>);
+    CAC_CUDA_TRY(launch_pdl(kern, regions, threads, 0, s, L.par, L.u, L.v, L.m, L.n, L.surv, L.region_counts, open, L.err));
+    compress_all(ctx, L.par, L.n, s);
+    const unsigned grid = (unsigned)std::min<uint64_t>((L.m + 4 * kThreads - 1) / (4 * kThreads), (uint64_t)ctx->num_sms * 8);
+    for (uint32_t k = 1; k < (L.m < kFewRoundEdges ? kFullRounds - 1 : kFullRounds); k++) {
+        const OpenCount left{open++, (uint32_t)(L.m / 128 + 4096)};
+        CAC_CUDA_TRY(launch_pdl(cc_list_round, grid, kThreads, 0, s, L.par, static_cast<const uint2 *>(L.surv),
+                                static_cast<const uint32_t *>(L.region_counts), regions, region, left, open));
+        compress_all(ctx, L.par, L.n, s, left);
+    }
+    return CAC_OK;
+}
+
+// The same on more edges: the rounds of kRoundDegree on
 // parts of the edges; where these take all edges before a giant component forms, one more round over all
 // of them, after which some hundred of 375,000 edges are left to the union walks (counted on G(300000, M),
 // average degree 2.5; 104,000 without it). Bound by the kernel boundaries (a round and its compression
 // take 6 us each). Measured against one pass of union walks: G(300000, M) of average degree 2.5 166 ->
-// 90 us a query, G(10^6, M) of degree 3 863 -> 127, of degree 1.5 153 -> 175; a path of 300,000 vertices
-// numbered along it 217 -> 151.
+// 90 us a query, G(10^6, M) of degree 3 863 -> 127.
 int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
     const double degree = 2.0 * (double)L.m / L.n;
     if (L.m < kRoundEdges || degree < 1) return CAC_OK;
+    if (degree < kSparseDegree) return sparse_rounds(ctx, L, s);
     auto round = [&](uint32_t from, uint32_t to) -> int {
         const uint64_t warps = (L.m / 256 / kRoundParts + 1) * (to - from);
         const bool wide = warps >= (uint64_t)ctx->num_sms * (kRoundThreads / 32), first = from == 0 && to < kRoundParts;
@@ -1021,7 +1170,7 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
     const uint32_t n = L.n;
     const uint64_t m = L.m;
     CAC_TRY(record(ctx, 0, capturing));
-    CAC_CUDA_TRY(cudaMemsetAsync(L.err, 0, 4, s));
+    CAC_CUDA_TRY(cudaMemsetAsync(L.err, 0, (kQueryWords - kErrWord) * 4, s));
     CAC_CUDA_TRY(launch_pdl(cc_init, grid_for(ctx, n, 8), kThreads, 0, s, L.par, n));
     if (L.draws > 0 && m > 0) {
         CAC_CUDA_TRY(cudaMemcpyAsync(L.d_ranks, L.h_ranks, sizeof(RankDesc) * L.ranks, cudaMemcpyHostToDevice, s));
