@@ -888,7 +888,7 @@ __device__ __forceinline__ void copy_entry_async(Tm *dst, const Tm *src) {
 // Q[a][b] = sum over u in group a, v in group b of A[u][v], the diagonal zeroed, with every row's
 // 32-column block prefixes and its sum (the next step's row prep). Three kernels with identical results:
 // the lower triangle of a small child (quotient_tri_kernel, see tri_fits), tiles of R rows (quotient_tile_kernel)
-// up to kTileMaxN source vertices, one row per CTA (quotient_shared_row_kernel) above.
+// up to kTileMaxN source vertices (kTileMaxN64 with u64 entries), one row per CTA (quotient_shared_row_kernel) above.
 //
 // R output rows make a tile: R rows of N entries in shared memory, so that every column index is
 // read once for R rows. The rows of a tile are interleaved in 16-byte chunks (a column's R entries
@@ -917,7 +917,12 @@ __device__ __forceinline__ void copy_entry_async(Tm *dst, const Tm *src) {
 constexpr uint32_t kTileThreads = 256;
 constexpr uint32_t kTileRows = 256;      // most output rows per CTA
 constexpr uint32_t kTileSmem = 74 * 1024;  // three CTAs per SM
-constexpr uint32_t kTileMaxN = 2900;
+// Up to these source vertices; one row per CTA above. The rows' time over the tiles' in whole queries (complete graphs,
+// 2 and 16 trials; equal weights / skewed ones, which make groups of hundreds of members), u32 entries: N = 2000 1.00,
+// 1.00 / 1.14, 1.07; 2900 1.00, 0.99 / 1.10, 1.02; 3200 1.01, 0.99 / 1.15, 1.04; 4000 0.99, 0.99 / 1.22, 1.04. u64 entries,
+// where a row's shared atomics are 64 bits wide: 2900 1.01, 1.00 / 1.42, 1.39; 4000 0.98, 0.99 / 1.47, 1.37; 5000 1.01, 1.00 / 1.53, 1.38
+// (the largest measured).
+constexpr uint32_t kTileMaxN = 2900, kTileMaxN64 = 5000;
 
 struct TilePlan {
     uint32_t rows;   // R
@@ -1236,7 +1241,7 @@ __device__ __forceinline__ void sadd(uint64_t *p, uint64_t v) {
 // vertices' columns and from those of the joined vertices before it, with shared atomics; then a warp per
 // row stores it, with its 32-column block prefixes and its sum. Half of the source is read, and a child takes
 // half the instructions of its tiles, whose setup per CTA and per tile it also spares.
-//   Taken while the triangle leaves room for three CTAs per SM (u32 entries: k <= 192; u64: 136): the
+//   Taken while the triangle leaves room for three CTAs per SM (u32 entries: k <= 192; u64: 135): the
 // children of K4000's levels of N = 255 and 182 took 320 and 350 us as tiles and take 244 and 287 us, those
 // of the Watts-Strogatz query 11.7 and 14.0 ms a group, now 7.8 and 9.1. Larger ones would leave one CTA per SM
 // or few warps, where the tiles keep three. Up to kTriSmallBytes six CTAs of 128 threads fit.
@@ -2140,8 +2145,8 @@ int KsEngine::step() {
         tasks.push_back(t);
     }
     if (tasks.empty()) return CAC_OK;
-    // sources whose row sums and block prefixes came with their matrix (warp quotient) skip the
-    // row prep; the others (roots, large-N quotients) are prepped here from their own list
+    // sources whose row sums and block prefixes came with their matrix (every quotient's) skip the
+    // row prep; the others (roots) are prepped here from their own list
     std::vector<SrcDesc> srcs(src_nodes.size()), psrcs;
     std::vector<uint64_t> row_off;
     uint64_t rows = 0, prep_elems = 0;
@@ -2288,8 +2293,8 @@ int KsEngine::step() {
         out_off[tasks.size() + i] = out_bytes;
         out_bytes += ((kq[i] + (uint64_t)kq[i] * ((kq[i] + 31) / 32)) * 8 + 15) / 16 * 16;
     }
-    // Three quotient kernels, identical outputs: triangles for small children, tiles up to kTileMaxN source
-    // vertices, one row per CTA above; the caller may force tiles (where they fit) or rows.
+    // Three quotient kernels, identical outputs: triangles for small children, tiles up to kTileMaxN or kTileMaxN64
+    // source vertices, one row per CTA above; the caller may force tiles (where they fit) or rows.
     Held out(*this);
     if (out_bytes || !leaf_list[0].empty() || !leaf_list[1].empty()) {
         if (out_bytes) CAC_TRY(out.alloc(out_bytes));
@@ -2324,7 +2329,7 @@ int KsEngine::step() {
                                   tile_groups(N, k, l.plan, kTileSmem) * tile_bytes(N, l.plan.rows, l.plan.esize);
             const bool tiles = forced == kQuotientShared                                     ? false
                                : forced == kQuotientTile || forced == kQuotientTileToo ? need <= 226 * 1024
-                                                                                       : N <= kTileMaxN;
+                                                                                       : N <= (tasks[i].src.small ? kTileMaxN : kTileMaxN64);
             if (tiles) {
                 l.plan.smem = std::max(l.plan.smem, need);
                 l.task.push_back(TileTask{tasks[i].src.mat, td[i].cols, td[i].members, td[i].memb_off, td[i].rows,

@@ -83,10 +83,11 @@ int cac_ctx_create(const cac_config *config, cac_ctx **out);
  * sparse form. */
 int cac_ctx_set_dense_limit(cac_ctx *ctx, uint32_t max_dense_vertices);
 /* The quotient kernel of the dense Karger-Stein steps: 0 (default) and 4 choose by size (triangles for
- * children of up to 192 vertices, 136 above a total weight of 2^32; tiles of output rows up to 2900
- * source vertices; eight warps per output row above); 1 and 3 force the tiles, 2 eight warps per row.
- * Children of up to 128 vertices are solved without a quotient. All give identical matrices; a kernel that does not fit a step's shared
- * memory is replaced by one that does. (No reference counterpart: a tuning control.) */
+ * children of up to 192 vertices, 135 above a total weight of 2^32; tiles of output rows up to 2900
+ * source vertices, 5000 above that weight; eight warps per output row above); 1 and 3 force the tiles, 2 eight
+ * warps per row. Children of up to 128 vertices are solved without a quotient. All give identical matrices; a
+ * kernel that does not fit a step's shared memory is replaced by one that does. (No reference counterpart: a
+ * tuning control.) */
 int cac_ctx_set_quotient_kernel(cac_ctx *ctx, int kind);
 /* Karger-Stein levels planned ahead (default 1): every child is taken to stop at its target size,
  * so the levels of a run follow one another without reading the children's sizes back; a child
