@@ -1984,8 +1984,8 @@ int KsEngine::read_err(uint32_t *err) {
 }
 
 int engine_error(uint32_t err) {
-    (void)err;  // one cause is left (kErrPlan redoes the run instead)
-    set_error("inconsistent selection prefix in the contraction kernel");
+    // (one cause: a run that planned ahead and missed is redone instead)
+    set_error("inconsistent selection prefix in the contraction kernel (error word " + std::to_string(err) + ")");
     return CAC_ERR_CUDA;
 }
 
