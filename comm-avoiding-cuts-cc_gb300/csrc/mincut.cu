@@ -1692,19 +1692,23 @@ __global__ void __launch_bounds__(kLeafThreads) sw_leaf_kernel(const LeafDesc *_
     const uint32_t N = L.N, lane = threadIdx.x & 31;
     leaf_copy(M, N, [&](uint32_t i) { return reinterpret_cast<const Tm *>(L.mat) + i * ld_of(N); },
               [&](int q) { return lane + 32 * q; });
-    // degrees: the row sums that came with the matrix, else summed here
-    uint64_t deg[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) deg[q] = L.rowsum && lane + 32 * q < N ? __ldg(L.rowsum + lane + 32 * q) : 0;
+    // degrees: the row sums that came with the matrix, else summed here, a thread per vertex (by warp 0 alone it
+    // took 10 us of a single leaf's 70)
+    __shared__ uint64_t s_deg[kLeafThreads];
+    const uint32_t v = threadIdx.x;
+    s_deg[v] = L.rowsum && v < N ? __ldg(L.rowsum + v) : 0;
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (threadIdx.x >= 32) return;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const uint32_t v = lane + 32 * q;
-        if (v < N && !L.rowsum)
-            for (uint32_t j = 0; j < N; j++) deg[q] += j == v ? 0 : (uint64_t)M[tpos(v, j)];
+    if (!L.rowsum) {
+        uint64_t sum = 0;
+        for (uint32_t j = 0; j < N && v < N; j++) sum += j == v ? 0 : (uint64_t)M[tpos(v, j)];
+        s_deg[v] = sum;
+        __syncthreads();
     }
+    if (threadIdx.x >= 32) return;
+    uint64_t deg[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) deg[q] = s_deg[lane + 32 * q];
     leaf_solve(M, N, deg, root, L.cut);
 }
 
