@@ -74,6 +74,16 @@ METRIC = "CC edges/s (parallel_cc, BA n=1,024,000 m=16)"
 KERNELS_PER_QUERY = 2 + 5 + 4 + 1 + 2 + 3
 
 
+def _profiled_traffic(name, kernels):
+    """DRAM bytes that a committed profile gives for a form of this many kernels; None for another form's."""
+    path = os.path.join(ROOT, "profiles", name)
+    if not os.path.exists(path):
+        return None
+    with open(path) as f:
+        d = json.load(f)
+    return d.get("dram_bytes_per_launch") if d.get("kernels") == kernels else None
+
+
 def _max_over_ranks(x, world):
     """The largest x over the ranks (a job takes as long as its slowest replica); the process
     group's backend decides where the reduction runs (NCCL: on the GPU, gloo: on the host)."""
@@ -576,12 +586,8 @@ def run_cac(args, rank, world):
     query_gbs = query_bytes / (r["ms_per_step"] / 1e3) / 1e9
     filt_bytes = 8 * m
     filt_gbs = filt_bytes / (r["edge_avg_ms"] / 1e3) / 1e9
-    traffic = {}
-    for key, name in (("query", "cc_query_ba1m.json"), ("filter", "cc_filter_ba1m.json")):
-        prof = os.path.join(ROOT, "profiles", name)
-        if os.path.exists(prof):
-            with open(prof) as f:
-                traffic[key] = json.load(f).get("dram_bytes_per_launch")
+    traffic = {"query": _profiled_traffic("cc_query_ba1m.json", KERNELS_PER_QUERY),
+               "filter": _profiled_traffic("cc_filter_ba1m.json", 1)}
     if rank != 0:
         g.free()
         ctx.close()
