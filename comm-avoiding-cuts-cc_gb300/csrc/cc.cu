@@ -56,10 +56,12 @@ constexpr uint32_t kRoundParts = 128;                // without draws: rounds ar
 // end a random graph has small trees only): G(10^6, M) with average degree 0.1 takes 41 us in one pass
 // and 48 in rounds, with 3 863 and 127, G(17000, M) with degree 2 87 and 66.
 constexpr uint64_t kRoundEdges = 1u << 13;
-// Up to this average degree the rounds are those of sparse_rounds, of kFullRounds - 1 below kFewRoundEdges edges.
-// Device us by them and by edge_rounds: G(10^6, M) of degree 2.25 145 and 626, 2.5 147 and 118, 3 167 and 121;
-// a 1000 x 1000 grid (4) 132 and 110.
-constexpr double kSparseDegree = 2.4;
+// Between these average degrees, and while the forest lies in the L2 (64 MB), the rounds are those of sparse_rounds, of
+// kFullRounds - 1 below kFewRoundEdges edges. Device us by them and by edge_rounds: G(10^6, M) of degree 1 86 and 81, 1.25
+// 106 and 118, 2.25 145 and 626, 2.5 147 and 118, 3 167 and 121; a 1000 x 1000 grid (4) 132 and 110. Degree 2 on 16 M
+// vertices 1165 and 1416, on 20 M 1554 and 1870, on 26 M 2379 and 2249; degree 2.3 1287 and 1625, 1720 and 1477, 2632 and 2259.
+constexpr double kSparseLow = 1.2, kSparseDegree = 2.4;
+constexpr uint32_t kSparseVertices = 1u << 24;
 constexpr uint64_t kFewRoundEdges = 1u << 18;
 constexpr uint32_t kProbes = 128;
 constexpr int kHops = 32;                            // longest walk of a compression between rounds
@@ -1108,7 +1110,7 @@ unsigned round_grid(cac_ctx *ctx, uint64_t warps, int threads = kRoundThreads) {
 // G(300,000, M) of degree 1.5 192 / 110 / 81, 1.75 116 / 218 / 81, 2 242 / 216 / 83; G(10^6, M) of degree 1.25 135 / 118 / 106,
 // 2 441 / 352 / 132; G(3 10^6, M) of degree 1.5 376 / 442 / 205, 2 400 / 808 / 267; paths of 10^6 numbered along
 // them 232 / 181 / 155, relabelled 168 / 144 / 136; random trees 118 / 123 / 122. What a pass joins at once pays for the
-// launches: stars and matchings of 300,000 vertices 34 / 46 / 48.
+// launches: stars of 300,000 vertices 34 / 46 / 48.
 int sparse_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
     const uint64_t tiles = (L.m + 255) / 256;
     const bool wide = tiles >= (uint64_t)ctx->num_sms * (kRoundThreads / 32);
@@ -1142,7 +1144,7 @@ int sparse_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
 int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
     const double degree = 2.0 * (double)L.m / L.n;
     if (L.m < kRoundEdges || degree < 1) return CAC_OK;
-    if (degree < kSparseDegree) return sparse_rounds(ctx, L, s);
+    if (degree >= kSparseLow && degree < kSparseDegree && L.n <= kSparseVertices) return sparse_rounds(ctx, L, s);
     auto round = [&](uint32_t from, uint32_t to) -> int {
         const uint64_t warps = (L.m / 256 / kRoundParts + 1) * (to - from);
         const bool wide = warps >= (uint64_t)ctx->num_sms * (kRoundThreads / 32), first = from == 0 && to < kRoundParts;

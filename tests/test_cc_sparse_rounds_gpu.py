@@ -37,6 +37,8 @@ CASES = {
     "smallest": _random(16321, 8193),
     "degree just below 1": _random(20002, 10000),
     "degree 1": _random(20000, 10000),
+    "degree below 1.2": _random(50000, 29999),
+    "degree 1.2": _random(50000, 30000),
     "below the line of degrees": _random(50000, 59999),
     "above it": _random(50000, 60001),
     "threshold of the giant": _random(200003, 110000),
@@ -95,3 +97,13 @@ def test_time_near_the_threshold_of_a_giant_component(ctx):
             t += [g.connected_components(seed=9, labels=False)[2].device_ms for _ in range(5)][2:]
         times.append(float(np.median(t)))
     assert times[0] < 2 * times[1], times
+
+
+def test_more_vertices_than_the_rounds_on_lists_take(ctx):
+    # 2^24 and one more; the labels by the device generator's graph and the oracle
+    for n in (1 << 24, (1 << 24) + 1):
+        g = ctx.generate("erdos_renyi_m", seed=5, n=n, avg_degree=1.3, wmax=1)
+        u, v, _ = g.edges()
+        want_count, want = O.cc_labels(n, u, v)
+        count, lab, _ = g.connected_components(seed=1, virtual_ranks=2)
+        assert count == want_count and np.array_equal(lab, want)
