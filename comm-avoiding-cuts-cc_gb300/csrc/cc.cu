@@ -52,9 +52,10 @@ constexpr uint32_t kSampleChunk = 32;                // consecutive edges behind
 // of twice the edges leave it in small trees).
 constexpr double kRoundDegree[] = {0.8, 0.8, 0.8, 0.8, 1.6};
 constexpr uint32_t kRoundParts = 128;                // without draws: rounds are 128ths of the 256-edge tiles
-// Without draws, smaller or sparser graphs hook every edge in one pass (below one edge per vertex at each
-// end a random graph has small trees only): G(10^6, M) with average degree 0.1 takes 41 us in one pass
-// and 48 in rounds, with 3 863 and 127, G(17000, M) with degree 2 87 and 66.
+// Without draws, smaller or sparser graphs hook every edge in one pass (up to one edge per vertex at each
+// end a random graph has small trees only, and disjoint edges have no more): G(10^6, M) with average degree 0.1 takes 41 us
+// in one pass and 48 in rounds, with 1.05 93 and 84, with 3 863 and 127, G(17000, M) with degree 2 87 and 66; a perfect
+// matching of 300,000 vertices 33 and 46, of 10^6 relabelled 49 and 69.
 constexpr uint64_t kRoundEdges = 1u << 13;
 // Between these average degrees, and while the forest lies in the L2 (64 MB), the rounds are those of sparse_rounds, of
 // kFullRounds - 1 below kFewRoundEdges edges. Device us by them and by edge_rounds: G(10^6, M) of degree 1 86 and 81, 1.25
@@ -1143,7 +1144,7 @@ int sparse_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
 // 90 us a query, G(10^6, M) of degree 3 863 -> 127.
 int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
     const double degree = 2.0 * (double)L.m / L.n;
-    if (L.m < kRoundEdges || degree < 1) return CAC_OK;
+    if (L.m < kRoundEdges || degree <= 1) return CAC_OK;
     if (degree >= kSparseLow && degree < kSparseDegree && L.n <= kSparseVertices) return sparse_rounds(ctx, L, s);
     auto round = [&](uint32_t from, uint32_t to) -> int {
         const uint64_t warps = (L.m / 256 / kRoundParts + 1) * (to - from);
