@@ -538,7 +538,7 @@ __global__ void approx_count_roots(const Forest F, uint32_t n, unsigned int *cou
 // which there was one of each, and three kernels or more, per level. Level by level over the whole
 // device (and, to 2^15 edges, a thread per edge and a block per draw) / here: R-MAT scale 9, m = 2,048 40 / 29 us;
 // G(16,000, m = 128,000), 8 levels 623 / 163 us; G(1000, m = 125,000), 10 levels 2.0 ms / 121 us; R-MAT scale 14,
-// m = 114,688, disconnected and so decided by its first level 161 / 141 us.
+// m = 114,688, disconnected and so decided by its first level 161 / 141 us (75 by rounds, which run no other level).
 //   The rule (approx_is_small): the forest fits in 64 KB of shared memory, and one CTA's pass over the edges is
 // no longer than two levels of rounds over the whole device (70 us each): with 2^20 edges it would be 0.9 ms.
 constexpr uint32_t kSmallThreads = 1024, kSmallN = 16384, kSmallM = 1u << 17;

@@ -1273,8 +1273,9 @@ void cc_graph_reset(cac_ctx *ctx) {
 }
 
 // One CTA (cc_small): the two arrays of n words fit its shared memory, host labels the ctx's pinned page,
-// and one SM still reads the edges faster than a dozen launches run (at 65,536 edges 73 us, the launches
-// 117; both grow past each other at about twice that).
+// and one SM still reads the edges faster than a dozen launches run. Device us by one CTA / by the launches, random
+// graphs: 300 vertices, 65,537 edges 37 / 67, 131,072 64 / 62, 262,144 119 / 72; 2000 vertices 43 / 71, 74 / 66, 154 / 71; 6000
+// 43 / 74, 74 / 74, 138 / 74; 16,000 68 / 88, 84 / 86, 146 / 87: the two meet at twice the line whatever the vertices.
 constexpr uint32_t kSmallVertices = (64 * 1024 - 256) / 4;
 constexpr uint64_t kSmallEdges = 1u << 16;
 bool cc_is_small(uint32_t n, uint64_t m) { return n && n <= kSmallVertices && m <= kSmallEdges; }
