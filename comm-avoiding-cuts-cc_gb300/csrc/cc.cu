@@ -500,8 +500,11 @@ __global__ void __launch_bounds__(kGiantSample) cc_compress_giant_bitmap(uint32_
 }
 
 // Closing pass without a sampling round: every edge hooks, 4 edges per thread step through
-// 16-byte streaming loads, their 8 parents requested together.
-template <bool kVec, bool kCheck>
+// 16-byte streaming loads. kFlat: after rounds, when most edges have found equal parents: the 8 parents are requested
+// together. From singletons the walks make the forest as they go, and what one has read before the others' links
+// is old by then (cac_cc_noalloc, which has this pass alone: paths of 10^6 vertices numbered along them 0.22 ms an edge at a
+// time and 0.42 with parents ahead, backwards 5.5 and 16.3; 62,500 disjoint cliques of 16 0.31 and 0.27).
+template <bool kVec, bool kCheck, bool kFlat>
 __global__ void __launch_bounds__(kThreads) cc_edge_pass(uint32_t *par, const uint32_t *__restrict__ u,
                                                          const uint32_t *__restrict__ v, uint64_t m, uint32_t n,
                                                          uint32_t *err) {
@@ -522,14 +525,19 @@ __global__ void __launch_bounds__(kThreads) cc_edge_pass(uint32_t *par, const ui
                     atomicOr(err, kErrBadId);
                     a[k] = b[k] = 0;
                 }
+            if (kFlat) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                a[k] = par[a[k]];
-                b[k] = par[b[k]];
+                for (int k = 0; k < 4; k++) {
+                    a[k] = par[a[k]];
+                    b[k] = par[b[k]];
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++)  // (equal parents: one component already, the reference drops the edge as a loop)
+                    if (a[k] != b[k]) unite(par, a[k], b[k]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) edge_hook(par, a[k], b[k]);
             }
-#pragma unroll
-            for (int k = 0; k < 4; k++)  // (equal parents: one component already, the reference drops the edge as a loop)
-                if (a[k] != b[k]) unite(par, a[k], b[k]);
         }
         done = m4 << 2;
     }
@@ -752,8 +760,9 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t x, uint32_t *sh) {
     return t;  // valid in thread 0
 }
 
-// Per-tile root counts.
-__global__ void __launch_bounds__(kThreads) cc_count_roots(const uint32_t *par, uint32_t n, uint32_t *tile_counts) {
+// Per-tile root counts. kCompress: with a full compression (roots only are written).
+template <bool kCompress>
+__global__ void __launch_bounds__(kThreads) cc_count_roots(uint32_t *par, uint32_t n, uint32_t *tile_counts) {
     pdl_wait();
     __shared__ uint32_t sh[32];
     const uint64_t base = (uint64_t)blockIdx.x * kTile;
@@ -761,7 +770,13 @@ __global__ void __launch_bounds__(kThreads) cc_count_roots(const uint32_t *par, 
 #pragma unroll
     for (int k = 0; k < kTileItems; k++) {
         const uint64_t i = base + (uint64_t)k * kThreads + threadIdx.x;
-        c += i < n && par[i] == (uint32_t)i;
+        if (kCompress) {
+            const uint32_t r = i < n ? find_root_ro(par, (uint32_t)i) : 0;
+            if (i < n) par[i] = r;
+            c += i < n && r == (uint32_t)i;
+        } else {
+            c += i < n && par[i] == (uint32_t)i;
+        }
     }
     const uint32_t t = block_sum(c, sh);
     if (threadIdx.x == 0) tile_counts[blockIdx.x] = t;
@@ -886,10 +901,12 @@ __global__ void __launch_bounds__(kThreads) cc_label_all(uint32_t *par, uint32_t
 // Count and labels of a finished forest. Up to kOwnTiles tiles each ranking CTA sums the counts before
 // its own (saves a launch; the sums together read ntiles^2 / 2 counts).
 constexpr uint32_t kOwnTiles = 4096;
+// flat: the forest's trees are a few links deep; those of union walks from singletons are compressed with the count,
+// tile after tile, before every vertex walks to its root at once.
 int label_components(int sms, uint32_t *par, uint32_t n, uint32_t ntiles, uint32_t *counts, uint32_t *offsets,
-                     uint32_t *total, uint32_t *labels, cudaStream_t s) {
+                     uint32_t *total, uint32_t *labels, bool flat, cudaStream_t s) {
     const uint32_t *cpar = par, *ccounts = counts, *coffsets = offsets;
-    CAC_CUDA_TRY(launch_pdl(cc_count_roots, ntiles, kThreads, 0, s, cpar, n, counts));
+    CAC_CUDA_TRY(launch_pdl(flat ? cc_count_roots<false> : cc_count_roots<true>, ntiles, kThreads, 0, s, par, n, counts));
     if (ntiles <= kOwnTiles) {
         CAC_CUDA_TRY(launch_pdl(cc_rank_roots<true>, ntiles, kThreads, 0, s, cpar, n, coffsets, ccounts, total, labels));
     } else {
@@ -1142,9 +1159,10 @@ int sparse_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
 // average degree 2.5; 104,000 without it). Bound by the kernel boundaries (a round and its compression
 // take 6 us each). Measured against one pass of union walks: G(300000, M) of average degree 2.5 166 ->
 // 90 us a query, G(10^6, M) of degree 3 863 -> 127.
-int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
+int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s, bool *flat) {
     const double degree = 2.0 * (double)L.m / L.n;
-    if (L.m < kRoundEdges || degree <= 1) return CAC_OK;
+    *flat = L.m >= kRoundEdges && degree > 1;
+    if (!*flat) return CAC_OK;
     if (degree >= kSparseLow && degree < kSparseDegree && L.n <= kSparseVertices) return sparse_rounds(ctx, L, s);
     auto round = [&](uint32_t from, uint32_t to) -> int {
         const uint64_t warps = (L.m / 256 / kRoundParts + 1) * (to - from);
@@ -1167,11 +1185,18 @@ int edge_rounds(cac_ctx *ctx, const CCLaunch &L, cudaStream_t s) {
     return CAC_OK;
 }
 
+template <bool kFlat>
+auto pick_edge_pass(bool vec, bool check) {
+    return vec ? (check ? cc_edge_pass<true, true, kFlat> : cc_edge_pass<true, false, kFlat>)
+               : (check ? cc_edge_pass<false, true, kFlat> : cc_edge_pass<false, false, kFlat>);
+}
+
 // Enqueues the whole query on the ctx stream (directly, or into a graph being captured).
 int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
     cudaStream_t s = ctx->stream;
     const uint32_t n = L.n;
     const uint64_t m = L.m;
+    bool flat = true;  // what the closing pass leaves: trees a few links deep, or those of union walks alone
     CAC_TRY(record(ctx, 0, capturing));
     CAC_CUDA_TRY(cudaMemsetAsync(L.err, 0, (kQueryWords - kErrWord) * 4, s));
     CAC_CUDA_TRY(launch_pdl(cc_init, grid_for(ctx, n, 8), kThreads, 0, s, L.par, n));
@@ -1222,14 +1247,13 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
                                         static_cast<const uint32_t *>(L.region_counts), regions, per * 256));
             const uint64_t done = tiles * 256;
             if (done < m)
-                (L.check ? cc_edge_pass<false, true> : cc_edge_pass<false, false>)<<<grid_for(ctx, m - done, 8), kThreads,
+                (L.check ? cc_edge_pass<false, true, true> : cc_edge_pass<false, false, true>)<<<grid_for(ctx, m - done, 8), kThreads,
                                                                                        0, s>>>(
                     L.par, L.u + done, L.v + done, m - done, n, L.err);
         } else {
-            CAC_TRY(edge_rounds(ctx, L, s));
+            CAC_TRY(edge_rounds(ctx, L, s, &flat));
             const int grid = grid_for(ctx, (m + 3) / 4, 8);
-            auto pass = L.vec ? (L.check ? cc_edge_pass<true, true> : cc_edge_pass<true, false>)
-                              : (L.check ? cc_edge_pass<false, true> : cc_edge_pass<false, false>);
+            auto pass = flat ? pick_edge_pass<true>(L.vec, L.check) : pick_edge_pass<false>(L.vec, L.check);
             pass<<<grid, kThreads, 0, s>>>(L.par, L.u, L.v, m, n, L.err);
             CAC_TRY(record(ctx, 4, capturing));
         }
@@ -1239,7 +1263,7 @@ int cc_enqueue(cac_ctx *ctx, const CCLaunch &L, bool capturing) {
     CAC_TRY(record(ctx, 2, capturing));
     // (A single-pass count and rank by decoupled look-back measured slower: BA n=1,024,000 20.4 vs
     // 18.5 us, R-MAT scale 22 48.6 vs 34.0 us for the labelling.)
-    CAC_TRY(label_components(ctx->num_sms, L.par, n, L.ntiles, L.counts, L.offsets, L.total, L.labels, s));
+    CAC_TRY(label_components(ctx->num_sms, L.par, n, L.ntiles, L.counts, L.offsets, L.total, L.labels, flat, s));
     CAC_CUDA_TRY(cudaGetLastError());
     CAC_CUDA_TRY(cudaMemcpyAsync(ctx->pinned_u32, L.total, (kErrWord + 1) * 4, cudaMemcpyDeviceToHost, s));
     CAC_TRY(record(ctx, 3, capturing));
@@ -1523,7 +1547,7 @@ int stream_enqueue(cac_ctx *ctx, const StreamLaunch &L, bool capturing) {
             // a piece of the sample (or, unfiltered, a chunk): every edge hooks, one edge per
             // thread (union walks are latency chains, so more of them run at once), then the
             // trees are flattened so the next part's walks stay one or two hops long
-            cc_edge_pass<false, true><<<grid_for(ctx, len, 8), kThreads, 0, s>>>(L.par, L.d_u + e0, L.d_v + e0, len, n,
+            cc_edge_pass<false, true, false><<<grid_for(ctx, len, 8), kThreads, 0, s>>>(L.par, L.d_u + e0, L.d_v + e0, len, n,
                                                                            L.total + kErrWord);
             if (L.filtered && c + 1 == kStreamPieces) {
                 cc_compress_giant_bitmap<<<giant_grid(ctx, n), kGiantSample, 0, s>>>(L.par, n, L.giant, L.bits, L.quads);
@@ -1547,13 +1571,13 @@ int stream_enqueue(cac_ctx *ctx, const StreamLaunch &L, bool capturing) {
             }
             const uint64_t done = tiles * 256;
             if (done < len)
-                cc_edge_pass<false, true><<<grid_for(ctx, len - done, 8), kThreads, 0, s>>>(
+                cc_edge_pass<false, true, false><<<grid_for(ctx, len - done, 8), kThreads, 0, s>>>(
                     L.par, L.d_u + e0 + done, L.d_v + e0 + done, len - done, n, L.total + kErrWord);
         }
     }
     if (!L.filtered) CAC_TRY(record(ctx, 1, capturing));
     CAC_TRY(record(ctx, 2, capturing));
-    CAC_TRY(label_components(ctx->num_sms, L.par, n, L.ntiles, L.counts, L.offsets, L.total, L.d_labels, s));
+    CAC_TRY(label_components(ctx->num_sms, L.par, n, L.ntiles, L.counts, L.offsets, L.total, L.d_labels, L.filtered, s));
     CAC_CUDA_TRY(cudaGetLastError());
     CAC_CUDA_TRY(cudaMemcpyAsync(ctx->pinned_u32, L.total, (kErrWord + 1) * 4, cudaMemcpyDeviceToHost, s));
     CAC_TRY(record(ctx, 3, capturing));
@@ -1788,11 +1812,11 @@ extern "C" int cac_cc_noalloc(uint32_t n, uint64_t m, const uint32_t *u_dev, con
     CAC_CUDA_TRY(cudaMemsetAsync(S->total + kErrWord, 0, 4, s));
     if (m > 0) {
         const bool vec = ((reinterpret_cast<uintptr_t>(u_dev) | reinterpret_cast<uintptr_t>(v_dev)) & 15) == 0;
-        if (vec) cc_edge_pass<true, true><<<grid((m + 3) / 4), kThreads, 0, s>>>(S->parent, u_dev, v_dev, m, n,
+        if (vec) cc_edge_pass<true, true, false><<<grid((m + 3) / 4), kThreads, 0, s>>>(S->parent, u_dev, v_dev, m, n,
                                                                                  S->total + kErrWord);
-        else cc_edge_pass<false, true><<<grid(m), kThreads, 0, s>>>(S->parent, u_dev, v_dev, m, n, S->total + kErrWord);
+        else cc_edge_pass<false, true, false><<<grid(m), kThreads, 0, s>>>(S->parent, u_dev, v_dev, m, n, S->total + kErrWord);
     }
-    CAC_TRY(label_components(D.sms, S->parent, n, ntiles, S->counts, S->offsets, S->total, labels_dev, s));
+    CAC_TRY(label_components(D.sms, S->parent, n, ntiles, S->counts, S->offsets, S->total, labels_dev, false, s));
     if (num_components_dev) cc_noalloc_count<<<1, 1, 0, s>>>(S->total, num_components_dev);
     CAC_CUDA_TRY(cudaGetLastError());
     return CAC_OK;
